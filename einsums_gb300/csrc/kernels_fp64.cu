@@ -10,15 +10,20 @@
 //                   (replaces GPULinearAlgebra.hpp:35-101 and GPUTensorAlgebra.hpp:146-198)
 //   k_gemv          one of the M/N groups empty: one CTA or warp per output
 //                   (replaces hipblasDgemv at GPULinearAlgebra.hpp:346-386)
-//   k_contract_f64  general case: 64x64 register-tiled DFMA contraction
+//   k_contract_f64  general case: small-tile DFMA contraction, K cut over a cluster
+//                   when the output has fewer tiles than the GPU has SMs
 //                   (replaces hipblasDgemm_64 and the atomicAdd generic kernel
 //                    GPUTensorAlgebra.hpp:28-82)
 #include <algorithm>
+#include <cmath>
 #include <utility>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace eg {
+
+int64_t mode_group_affine_stride(const ModeGroup &g, int comp);
 
 namespace {
 
@@ -292,101 +297,237 @@ __global__ void k_k_offsets(ModeGroup k, int64_t *out) {
 }
 
 // ------------------------------------------------------ tiled contraction --
-constexpr int BM = 64, BN = 64, BK = 16, kThreads = 256;
+// Bound: the FP64 pipe, which retires two FMAs per clock per SM, so a 64-bit
+// FMA of a warp takes 16 clocks of an SM while its two shared-memory reads take
+// four: register tiles buy nothing, and what counts is that every SM has its
+// share of the FMAs.  Tiles are therefore small (8, 16 or 32 square, picked by
+// contract_plan), and when there are still fewer tiles than SMs a cluster of up
+// to eight CTAs cuts K, its partial sums added over distributed shared memory
+// in rank order (deterministic, no workspace, so the launch can be captured).
+// 256 threads: KG groups along k times T*T outputs, R x R outputs per thread.
+// Chunks of BK k come through a three-slot ring of 8-byte asynchronous copies
+// (zero-filled past the edges), two chunks ahead of the FMAs.
+// Measured against 64 x 64 tiles without a K cut: 40x60x50 92 -> 26 us a call
+// (the call's host side), complex 300x170x257 (four launches) 1404 -> 156 us,
+// 144x2304x2304 2.93 -> 1.31 ms, 2304^3 21.7 -> 20.1 ms (1.22 TFLOP/s, 97 % of
+// the pipe).
+constexpr int kThreads = 256, kStages = 3;
 
-__global__ void __launch_bounds__(kThreads) k_contract_f64(ModeGroup bg, ModeGroup mg, ModeGroup ng, ModeGroup kg,
-                                                           const double *__restrict__ A, const double *__restrict__ B,
-                                                           double *C, double cp, double ab, bool zero, int a_kfast,
-                                                           int b_kfast) {
-    __shared__ double As[BK][BM + 1];
-    __shared__ double Bs[BK][BN + 1];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
-    const int64_t M = mg.total, N = ng.total, K = kg.total;
+template <int T>
+struct F64Tile {
+    static constexpr int R = T == 32 ? 2 : 1;
+    static constexpr int KG = kThreads / ((T / R) * (T / R));
+    static constexpr int BK = T == 32 ? 16 : 32;
+    static constexpr int LD = T + 1;
+    static constexpr int PER = T * BK / kThreads; // elements a thread loads per operand and chunk
+};
 
-    // Load assignment: element e = tid + 256*i of the 64x16 tile.  When the
-    // operand is contiguous along k, consecutive threads walk k; otherwise m.
-    int lm[4], lk[4], ln[4], lkb[4];
-    int64_t offA[4], offB[4];
-    bool okA[4], okB[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int e = tid + kThreads * i;
-        lm[i] = a_kfast ? e / BK : e % BM;
-        lk[i] = a_kfast ? e % BK : e / BM;
-        ln[i] = b_kfast ? e / BK : e % BN;
-        lkb[i] = b_kfast ? e % BK : e / BN;
-        int64_t oa, ob, oc;
-        okA[i] = m0 + lm[i] < M;
-        group_offsets32(mg, (uint32_t)(okA[i] ? m0 + lm[i] : 0), oa, ob, oc);
-        offA[i] = oa;
-        okB[i] = n0 + ln[i] < N;
-        group_offsets32(ng, (uint32_t)(okB[i] ? n0 + ln[i] : 0), oa, ob, oc);
-        offB[i] = ob;
-    }
+// How a k index becomes an element offset of one operand: a single stride when
+// the group's modes nest in it, else the decomposition over the modes.
+__device__ __forceinline__ int64_t k_offset(const ModeGroup &kg, int64_t stride, int comp, uint32_t k) {
+    if (stride) return (int64_t)k * stride;
+    int64_t oa, ob, oc;
+    group_offsets32(kg, k, oa, ob, oc);
+    return comp ? ob : oa;
+}
 
-    for (int64_t b = blockIdx.z; b < bg.total; b += gridDim.z) {
+__device__ __forceinline__ void copy_async8(double *dst, const double *src, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
+
+struct F64Args {
+    ModeGroup bg, mg, ng, kg;
+    const double *A, *B;
+    double *C;
+    double cp, ab;
+    int zero;
+    int a_kfast, b_kfast;  // the operand is read along k (its smaller stride), else along its rows
+    int64_t ka, kb;        // single k strides of A and B (0: none)
+    int64_t mtiles, ntiles, total; // total = batches * mtiles * ntiles
+    int cs;                // CTAs of a cluster, each taking a range of the k chunks
+};
+
+template <int T>
+__global__ void __launch_bounds__(kThreads) k_contract_f64(const __grid_constant__ F64Args p) {
+    using Q = F64Tile<T>;
+    constexpr int R = Q::R, KG = Q::KG, BK = Q::BK, LD = Q::LD, PER = Q::PER, W = T / R;
+    __shared__ double As[kStages][BK][LD];
+    __shared__ double Bs[kStages][BK][LD];
+    __shared__ double part[T * T];
+    const int tid = threadIdx.x;
+    const int kgrp = tid / (W * W), tx = tid % W, ty = (tid / W) % W;
+    const int rank = p.cs > 1 ? (int)ptx::cluster_ctarank() : 0;
+    const int64_t M = p.mg.total, N = p.ng.total, K = p.kg.total;
+    const int chunks = (int)((K + BK - 1) / BK);
+    const int cbeg = (int)((int64_t)chunks * rank / p.cs), cend = (int)((int64_t)chunks * (rank + 1) / p.cs);
+    const int64_t step = gridDim.x / p.cs;
+    for (int64_t t = blockIdx.x / p.cs; t < p.total; t += step) {
+        const int64_t q = t / p.ntiles, b = q / p.mtiles;
+        const int64_t n0 = (t - q * p.ntiles) * T, m0 = (q - b * p.mtiles) * T;
         int64_t ba, bb, bc;
-        group_offsets(bg, b, ba, bb, bc);
-        double acc[4][4];
+        group_offsets(p.bg, b, ba, bb, bc);
+        int am[PER], ak[PER], bn[PER], bk[PER];
+        const double *pa[PER], *pb[PER];
+        bool oka[PER], okb[PER];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
-
-        for (int64_t k0 = 0; k0 < K; k0 += BK) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int64_t ka = k0 + lk[i];
-                double va = 0.0;
-                if (okA[i] && ka < K) {
-                    int64_t oa, ob, oc;
-                    group_offsets32(kg, (uint32_t)ka, oa, ob, oc);
-                    va = __ldg(A + ba + offA[i] + oa);
-                }
-                As[lk[i]][lm[i]] = va;
-                const int64_t kb = k0 + lkb[i];
-                double vb = 0.0;
-                if (okB[i] && kb < K) {
-                    int64_t oa, ob, oc;
-                    group_offsets32(kg, (uint32_t)kb, oa, ob, oc);
-                    vb = __ldg(B + bb + offB[i] + ob);
-                }
-                Bs[lkb[i]][ln[i]] = vb;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int kk = 0; kk < BK; kk++) {
-                double a[4], bv[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-                for (int j = 0; j < 4; j++) bv[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) acc[i][j] = fma(a[i], bv[j], acc[i][j]);
-            }
-            __syncthreads();
+        for (int i = 0; i < PER; i++) {
+            const int e = tid + kThreads * i;
+            am[i] = p.a_kfast ? e / BK : e % T;
+            ak[i] = p.a_kfast ? e % BK : e / T;
+            bn[i] = p.b_kfast ? e / BK : e % T;
+            bk[i] = p.b_kfast ? e % BK : e / T;
+            int64_t oa, ob, oc;
+            oka[i] = m0 + am[i] < M;
+            group_offsets32(p.mg, (uint32_t)(oka[i] ? m0 + am[i] : 0), oa, ob, oc);
+            pa[i] = p.A + ba + oa;
+            okb[i] = n0 + bn[i] < N;
+            group_offsets32(p.ng, (uint32_t)(okb[i] ? n0 + bn[i] : 0), oa, ob, oc);
+            pb[i] = p.B + bb + ob;
         }
+        auto load = [&](int c) {
+            if (c < cend) {
+                const int slot = (c - cbeg) % kStages;
+#pragma unroll
+                for (int i = 0; i < PER; i++) {
+                    const int64_t ka = (int64_t)c * BK + ak[i], kb = (int64_t)c * BK + bk[i];
+                    const bool va = oka[i] && ka < K, vb = okb[i] && kb < K;
+                    copy_async8(&As[slot][ak[i]][am[i]], va ? pa[i] + k_offset(p.kg, p.ka, 0, (uint32_t)ka) : p.A, va);
+                    copy_async8(&Bs[slot][bk[i]][bn[i]], vb ? pb[i] + k_offset(p.kg, p.kb, 1, (uint32_t)kb) : p.B, vb);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        double acc[R][R] = {};
+        load(cbeg);
+        load(cbeg + 1);
+        for (int c = cbeg; c < cend; c++) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads(); // chunk c has landed for every thread, and chunk c - 1 is read
+            load(c + 2);
+            const int slot = (c - cbeg) % kStages;
+#pragma unroll 8
+            for (int kk = kgrp; kk < BK; kk += KG) {
+                double a[R], v[R];
+#pragma unroll
+                for (int i = 0; i < R; i++) a[i] = As[slot][kk][ty + W * i];
+#pragma unroll
+                for (int j = 0; j < R; j++) v[j] = Bs[slot][kk][tx + W * j];
+#pragma unroll
+                for (int i = 0; i < R; i++)
+#pragma unroll
+                    for (int j = 0; j < R; j++) acc[i][j] = fma(a[i], v[j], acc[i][j]);
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        // the k groups of the CTA, then the CTAs of the cluster, added in order
+        const bool reduce = KG > 1 || p.cs > 1;
+        if (KG > 1) {
+            static_assert(KG == 1 || (R == 1 && KG * T * T == kThreads), "one output per thread and k group");
+            double *buf = &As[0][0][0]; // KG * T * T doubles fit one slot's space
+            static_assert(KG == 1 || KG * T * T <= kStages * BK * LD, "reduction buffer");
+            __syncthreads();
+            buf[tid] = acc[0][0];
+            __syncthreads();
+            if (kgrp == 0) {
+                double v = buf[tid];
+#pragma unroll
+                for (int g = 1; g < KG; g++) v += buf[g * T * T + tid];
+                acc[0][0] = v;
+            }
+        }
+        if (p.cs > 1) {
+            if (kgrp == 0) {
+#pragma unroll
+                for (int i = 0; i < R; i++)
+#pragma unroll
+                    for (int j = 0; j < R; j++) part[(ty + W * i) * T + tx + W * j] = acc[i][j];
+            }
+            ptx::cluster_sync();
+            if (rank == 0 && kgrp == 0) {
+#pragma unroll
+                for (int i = 0; i < R; i++)
+#pragma unroll
+                    for (int j = 0; j < R; j++) {
+                        const uint32_t at = ptx::smem_u32(&part[(ty + W * i) * T + tx + W * j]);
+                        double v = acc[i][j];
+                        for (int r = 1; r < p.cs; r++) v += ptx::ld_cluster_f64(ptx::mapa(at, (uint32_t)r));
+                        acc[i][j] = v;
+                    }
+            }
+        }
+        if (rank == 0 && kgrp == 0) {
+#pragma unroll
+            for (int i = 0; i < R; i++) {
+                const int64_t m = m0 + ty + W * i;
+                if (m >= M) continue;
+                int64_t ma, mb, mc;
+                group_offsets32(p.mg, (uint32_t)m, ma, mb, mc);
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    const int64_t n = n0 + tx + W * j;
+                    if (n >= N) continue;
+                    int64_t na, nb, nc;
+                    group_offsets32(p.ng, (uint32_t)n, na, nb, nc);
+                    double *cptr = p.C + bc + mc + nc;
+                    *cptr = epilogue(acc[i][j], cptr, p.cp, p.ab, p.zero != 0);
+                }
+            }
+        }
+        if (p.cs > 1)
+            ptx::cluster_sync(); // the peers' sums are read; the next tile may overwrite them
+        else if (reduce || t + step < p.total)
+            __syncthreads();
+    }
+}
 
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int64_t m = m0 + ty + 16 * i;
-            if (m >= M) continue;
-            int64_t ma, mb, mc;
-            group_offsets32(mg, (uint32_t)m, ma, mb, mc);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int64_t n = n0 + tx + 16 * j;
-                if (n >= N) continue;
-                int64_t na, nb, nc;
-                group_offsets32(ng, (uint32_t)n, na, nb, nc);
-                double *cptr = C + bc + mc + nc;
-                *cptr = epilogue(acc[i][j], cptr, cp, ab, zero);
+// Tile edge and cluster size of a contraction: the smallest of the estimated
+// times of the busiest SM, its FMAs at two per clock plus a start-up of about
+// 2000 clocks per resident round (prologue, first loads, stores) and 1500 for a
+// cluster's exchange.  A smaller tile wins only where larger ones leave SMs
+// idle: it issues more loads and index arithmetic per FMA (the factors).
+void contract_plan(int64_t nb, int64_t M, int64_t N, int64_t K, int &T, int &cs) {
+    double best = -1.0;
+    T = 32;
+    cs = 1;
+    for (int e : {32, 16, 8}) {
+        const int bk = e == 32 ? 16 : 32;
+        const double factor = e == 32 ? 1.0 : e == 16 ? 1.05 : 1.15;
+        for (int c = 1; c <= 8; c *= 2) {
+            const int64_t chunks = (K + bk - 1) / bk;
+            if (c > 1 && chunks < 2 * c) break;
+            const double blocks = (double)nb * (double)((M + e - 1) / e) * (double)((N + e - 1) / e) * c;
+            const double rounds = std::ceil(blocks / num_sms());
+            const double fma = (double)e * e * (double)((chunks + c - 1) / c * bk) * 0.5 * factor;
+            const double cost = rounds * fma + std::ceil(rounds / 4.0) * (2000.0 + (c > 1 ? 1500.0 : 0.0));
+            if (best < 0.0 || cost < best * 0.98) {
+                best = cost;
+                T = e;
+                cs = c;
             }
         }
     }
+}
+
+template <int T>
+cudaError_t launch_f64_tiles(const F64Args &p, cudaStream_t s) {
+    const int64_t clusters = std::min<int64_t>(p.total, int64_t(1) << 24);
+    if (p.cs == 1) {
+        k_contract_f64<T><<<(unsigned)clusters, kThreads, 0, s>>>(p);
+        return cudaGetLastError();
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(clusters * p.cs));
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)p.cs;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_contract_f64<T>, p);
 }
 
 ModeGroup concat(std::initializer_list<const ModeGroup *> groups) {
@@ -531,15 +672,39 @@ eg_status launch_gemv(const Contraction &c, cudaStream_t s) {
 eg_status launch_contract_f64(const Contraction &c, cudaStream_t s) {
     if (!fits32(c.m) || !fits32(c.n) || !fits32(c.k))
         return fail(EG_ERROR_NOT_SUPPORTED, "contraction: a mode group exceeds 2^31 elements");
-    const int64_t gx = (c.n.total + BN - 1) / BN, gy = (c.m.total + BM - 1) / BM;
-    if (gy > 65535) return fail(EG_ERROR_NOT_SUPPORTED, "contraction: too many row tiles");
-    const int64_t gz = c.batch.total < 65535 ? c.batch.total : 65535;
-    const int a_kfast = c.k.n > 0 && c.k.s[0][c.k.n - 1] == 1 && !(c.m.n > 0 && c.m.s[0][c.m.n - 1] == 1);
-    const int b_kfast = c.k.n > 0 && c.k.s[1][c.k.n - 1] == 1 && !(c.n.n > 0 && c.n.s[1][c.n.n - 1] == 1);
-    dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)(gz < 1 ? 1 : gz));
-    { LaunchScope ls_("k_contract_f64", s);
-    k_contract_f64<<<grid, kThreads, 0, s>>>(c.batch, c.m, c.n, c.k, c.A, c.B, c.C, c.cp, c.ab, c.zero_when_cp_zero,
-                                             a_kfast, b_kfast);
+    if (c.m.total > int64_t(65535) * 64) return fail(EG_ERROR_NOT_SUPPORTED, "contraction: too many row tiles");
+    F64Args p;
+    p.bg = c.batch;
+    p.mg = c.m;
+    p.ng = c.n;
+    p.kg = c.k;
+    p.A = c.A;
+    p.B = c.B;
+    p.C = c.C;
+    p.cp = c.cp;
+    p.ab = c.ab;
+    p.zero = c.zero_when_cp_zero ? 1 : 0;
+    // read each operand along the smaller of its fastest k and row strides
+    auto kfast = [](const ModeGroup &k, const ModeGroup &r, int comp) {
+        if (k.n == 0) return 0;
+        return r.n == 0 || k.s[comp][k.n - 1] < r.s[comp][r.n - 1] ? 1 : 0;
+    };
+    p.a_kfast = kfast(c.k, c.m, 0);
+    p.b_kfast = kfast(c.k, c.n, 1);
+    p.ka = mode_group_affine_stride(c.k, 0);
+    p.kb = mode_group_affine_stride(c.k, 1);
+    int T = 32;
+    contract_plan(c.batch.total, c.m.total, c.n.total, c.k.total, T, p.cs);
+    p.mtiles = (c.m.total + T - 1) / T;
+    p.ntiles = (c.n.total + T - 1) / T;
+    p.total = c.batch.total * p.mtiles * p.ntiles;
+    if (p.total == 0) return EG_SUCCESS;
+    {
+        LaunchScope ls_("k_contract_f64", s);
+        const cudaError_t err = T == 32   ? launch_f64_tiles<32>(p, s)
+                                : T == 16 ? launch_f64_tiles<16>(p, s)
+                                          : launch_f64_tiles<8>(p, s);
+        if (err != cudaSuccess) return cuda_fail(err, "k_contract_f64");
     }
     EG_CHECK_LAUNCH("k_contract_f64");
     return EG_SUCCESS;

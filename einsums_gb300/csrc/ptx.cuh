@@ -116,7 +116,13 @@ __device__ __forceinline__ void st_cluster_u32(uint32_t addr_cluster, uint32_t v
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr_cluster), "r"(v) : "memory");
 }
 
-// All threads of both CTAs of the cluster.
+__device__ __forceinline__ double ld_cluster_f64(uint32_t addr_cluster) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr_cluster) : "memory");
+    return v;
+}
+
+// All threads of all CTAs of the cluster.
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
