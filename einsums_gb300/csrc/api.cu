@@ -54,18 +54,117 @@ eg_status cuda_fail(cudaError_t err, const char *what) {
     return err == cudaErrorMemoryAllocation ? EG_ERROR_OUT_OF_MEMORY : EG_ERROR_CUDA;
 }
 
-eg_status tracked_malloc(size_t bytes, void **ptr) {
+// Calls that may not run while a stream of any thread is being captured (in the
+// global capture mode) are made in the relaxed mode: they touch no captured stream.
+namespace {
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+eg_status malloc_once(size_t bytes, void **ptr) {
     std::lock_guard<std::mutex> lk(g_mem_mutex);
     if (g_budget && g_in_use + bytes > g_budget)
         return fail(EG_ERROR_OUT_OF_MEMORY, "device allocation of " + std::to_string(bytes) +
                                                 " bytes exceeds the memory budget of " + std::to_string(g_budget));
     void *p = nullptr;
     cudaError_t err = cudaMalloc(&p, bytes ? bytes : 1);
-    if (err != cudaSuccess) return cuda_fail(err, "cudaMalloc");
+    if (err != cudaSuccess) {
+        if (err == cudaErrorMemoryAllocation) cudaGetLastError(); // not sticky: leave no trace for later checks
+        return cuda_fail(err, "cudaMalloc");
+    }
     g_sizes[p] = bytes;
     g_in_use += bytes;
     *ptr = p;
     return EG_SUCCESS;
+}
+} // namespace
+
+struct SharedScratch {
+    std::mutex mu; // held from a lease's start to its end
+    void *ptr = nullptr;
+    size_t bytes = 0;
+    cudaEvent_t last = nullptr; // after the last lease's work
+};
+
+namespace {
+std::mutex &g_scratch_mutex = *new std::mutex;
+std::map<int, SharedScratch> &g_scratch = *new std::map<int, SharedScratch>;
+
+// Waits for the buffer's last user and frees it (its lock is held).
+void drop_scratch(SharedScratch &x) {
+    if (!x.ptr) return;
+    RelaxedCapture relaxed;
+    cudaEventSynchronize(x.last);
+    tracked_free(x.ptr);
+    x.ptr = nullptr;
+    x.bytes = 0;
+}
+
+// Gives back every device's shared scratch; false when there was none.
+bool trim_scratch() {
+    std::vector<SharedScratch *> all;
+    {
+        std::lock_guard<std::mutex> lk(g_scratch_mutex);
+        for (auto &kv : g_scratch) all.push_back(&kv.second);
+    }
+    bool any = false;
+    for (SharedScratch *x : all) {
+        std::lock_guard<std::mutex> lk(x->mu);
+        any |= x->ptr != nullptr;
+        drop_scratch(*x);
+    }
+    return any;
+}
+} // namespace
+
+eg_status tracked_malloc(size_t bytes, void **ptr) {
+    const eg_status st = malloc_once(bytes, ptr);
+    if (st != EG_ERROR_OUT_OF_MEMORY || !trim_scratch()) return st;
+    set_error("");
+    return malloc_once(bytes, ptr);
+}
+
+ScratchLease::ScratchLease(cudaStream_t s, size_t bytes) : s_(s) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    SharedScratch *x = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_scratch_mutex);
+        x = &g_scratch[dev];
+    }
+    x->mu.lock();
+    bool ok = x->last || cudaEventCreateWithFlags(&x->last, cudaEventDisableTiming) == cudaSuccess;
+    if (ok && x->bytes < bytes) {
+        RelaxedCapture relaxed;
+        drop_scratch(*x);
+        const size_t want = (bytes + 0x3FFFFFF) & ~size_t(0x3FFFFFF); // whole 64 MB
+        size_t free_b = 0, total_b = 0;
+        ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b >= want + total_b / 32 &&
+             malloc_once(want, &x->ptr) == EG_SUCCESS;
+        if (ok)
+            x->bytes = want;
+        else
+            set_error("");
+    } else if (ok) {
+        ok = cudaStreamWaitEvent(s, x->last, 0) == cudaSuccess;
+    }
+    if (!ok) {
+        x->mu.unlock();
+        return;
+    }
+    owner_ = x;
+    ptr_ = x->ptr;
+}
+
+ScratchLease::~ScratchLease() {
+    if (!owner_) return;
+    if (cudaEventRecord(owner_->last, s_) != cudaSuccess) { // never leave the buffer unguarded
+        cudaStreamSynchronize(s_);
+        cudaGetLastError();
+    }
+    owner_->mu.unlock();
 }
 
 eg_status tracked_free(void *ptr) {
@@ -393,6 +492,10 @@ eg_status einsum_impl(double cp, const int32_t *Cl, const eg_tensor *C, double a
     if (!has_k) return launch_elementwise(c, stream);
     if (c.batch.n == 0 && c.m.n == 0 && c.n.n == 0) return launch_dot(c, stream);
     if (c.m.n == 0 || c.n.n == 0) return launch_gemv(c, stream);
+    if (f64_tensor_pays(c)) {
+        st = launch_f64_tensor(c, stream);
+        if (st != EG_ERROR_NOT_SUPPORTED) return st;
+    }
     return launch_contract_f64(c, stream);
 }
 

@@ -124,6 +124,27 @@ struct Contraction {
 // library is loaded.  Calls that share a stream are ordered, so reuse is safe.
 eg_status workspace(cudaStream_t stream, size_t bytes, void **ptr);
 
+// A device's shared scratch for calls that need much of it for a short time: one
+// buffer per device, handed from call to call in the order of the calls (each
+// waits on the GPU for the one before, whatever its stream), locked to the
+// calling thread while its launches are issued, and given back when another
+// allocation of the library does not fit.  ptr() is null when the buffer cannot
+// be had: under the memory budget, or without leaving a thirty-second of the
+// device's memory free.
+class ScratchLease {
+  public:
+    ScratchLease(cudaStream_t s, size_t bytes);
+    ~ScratchLease();
+    ScratchLease(const ScratchLease &) = delete;
+    ScratchLease &operator=(const ScratchLease &) = delete;
+    void *ptr() const { return ptr_; }
+
+  private:
+    cudaStream_t s_;
+    struct SharedScratch *owner_ = nullptr;
+    void *ptr_ = nullptr;
+};
+
 // Device-side error word of kernels with bounded waits, one per (device,
 // stream); kernels set it with atomicCAS(ptr, 0, code) and eg_stream_status
 // reads and clears it.
@@ -162,6 +183,11 @@ eg_status launch_scale(const ModeGroup &g, double *C, double cp, cudaStream_t s)
 eg_status launch_dot(const Contraction &c, cudaStream_t s);
 eg_status launch_gemv(const Contraction &c, cudaStream_t s);
 eg_status launch_contract_f64(const Contraction &c, cudaStream_t s);
+// The blocks of 32 x 64 outputs listed at `list` ({batch, row, column}), *count of them.
+eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, const int *count, cudaStream_t s);
+double contract_f64_seconds(const Contraction &c); // its estimated time
+bool f64_tensor_pays(const Contraction &c);
+eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s);
 eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s, eg_split_report *rep);
 
 struct PermuteDesc {

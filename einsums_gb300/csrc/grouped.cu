@@ -666,6 +666,7 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
     const Contraction &c0 = cs[0];
     TcGemmParams p{};
     p.S = S;
+    p.planes = S;
     p.nbatch = 1;
     p.cp = c0.cp;
     p.ab = c0.ab;
@@ -684,7 +685,8 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
     p.timeout_ns = 2000ull * 1000 * 1000;
     p.d0 = 0; // every slice group in one launch (K fits one exact pass)
     p.d1 = S;
-    p.ksplit = 1; // no K slicing in grouped launches
+    p.t0 = INT_MAX; // no K slicing in grouped launches
+    p.ksplit = 1;
     p.kslice = 0;
     p.item_maps = (const CUtensorMap *)d_maps;
     p.rbuf = (long long *)rbuf;

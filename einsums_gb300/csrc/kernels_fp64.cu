@@ -346,6 +346,10 @@ struct F64Args {
     int64_t ka, kb;        // single k strides of A and B (0: none)
     int64_t mtiles, ntiles, total; // total = batches * mtiles * ntiles
     int cs;                // CTAs of a cluster, each taking a range of the k chunks
+    // When set, the tiles are instead the halves of the 32 x 64 blocks {batch, row,
+    // column} listed there (T = 32, one CTA each).
+    const int4 *list;
+    const int *count;
 };
 
 template <int T>
@@ -362,9 +366,20 @@ __global__ void __launch_bounds__(kThreads) k_contract_f64(const __grid_constant
     const int chunks = (int)((K + BK - 1) / BK);
     const int cbeg = (int)((int64_t)chunks * rank / p.cs), cend = (int)((int64_t)chunks * (rank + 1) / p.cs);
     const int64_t step = gridDim.x / p.cs;
-    for (int64_t t = blockIdx.x / p.cs; t < p.total; t += step) {
-        const int64_t q = t / p.ntiles, b = q / p.mtiles;
-        const int64_t n0 = (t - q * p.ntiles) * T, m0 = (q - b * p.mtiles) * T;
+    const int64_t total = p.list ? 2 * (int64_t)__ldg(p.count) : p.total;
+    for (int64_t t = blockIdx.x / p.cs; t < total; t += step) {
+        int64_t b, m0, n0;
+        if (p.list) {
+            const int4 e = p.list[t >> 1];
+            b = e.x;
+            m0 = e.y;
+            n0 = e.z + T * (t & 1);
+        } else {
+            const int64_t q = t / p.ntiles;
+            b = q / p.mtiles;
+            n0 = (t - q * p.ntiles) * T;
+            m0 = (q - b * p.mtiles) * T;
+        }
         int64_t ba, bb, bc;
         group_offsets(p.bg, b, ba, bb, bc);
         int am[PER], ak[PER], bn[PER], bk[PER];
@@ -476,7 +491,7 @@ __global__ void __launch_bounds__(kThreads) k_contract_f64(const __grid_constant
         }
         if (p.cs > 1)
             ptx::cluster_sync(); // the peers' sums are read; the next tile may overwrite them
-        else if (reduce || t + step < p.total)
+        else if (reduce || t + step < total)
             __syncthreads();
     }
 }
@@ -486,7 +501,7 @@ __global__ void __launch_bounds__(kThreads) k_contract_f64(const __grid_constant
 // 2000 clocks per resident round (prologue, first loads, stores) and 1500 for a
 // cluster's exchange.  A smaller tile wins only where larger ones leave SMs
 // idle: it issues more loads and index arithmetic per FMA (the factors).
-void contract_plan(int64_t nb, int64_t M, int64_t N, int64_t K, int &T, int &cs) {
+double contract_plan(int64_t nb, int64_t M, int64_t N, int64_t K, int &T, int &cs) { // returns the clocks
     double best = -1.0;
     T = 32;
     cs = 1;
@@ -507,6 +522,7 @@ void contract_plan(int64_t nb, int64_t M, int64_t N, int64_t K, int &T, int &cs)
             }
         }
     }
+    return best;
 }
 
 template <int T>
@@ -669,11 +685,9 @@ eg_status launch_gemv(const Contraction &c, cudaStream_t s) {
     return EG_SUCCESS;
 }
 
-eg_status launch_contract_f64(const Contraction &c, cudaStream_t s) {
-    if (!fits32(c.m) || !fits32(c.n) || !fits32(c.k))
-        return fail(EG_ERROR_NOT_SUPPORTED, "contraction: a mode group exceeds 2^31 elements");
-    if (c.m.total > int64_t(65535) * 64) return fail(EG_ERROR_NOT_SUPPORTED, "contraction: too many row tiles");
-    F64Args p;
+namespace {
+F64Args f64_args(const Contraction &c) {
+    F64Args p{};
     p.bg = c.batch;
     p.mg = c.m;
     p.ng = c.n;
@@ -693,6 +707,16 @@ eg_status launch_contract_f64(const Contraction &c, cudaStream_t s) {
     p.b_kfast = kfast(c.k, c.n, 1);
     p.ka = mode_group_affine_stride(c.k, 0);
     p.kb = mode_group_affine_stride(c.k, 1);
+    p.cs = 1;
+    return p;
+}
+} // namespace
+
+eg_status launch_contract_f64(const Contraction &c, cudaStream_t s) {
+    if (!fits32(c.m) || !fits32(c.n) || !fits32(c.k))
+        return fail(EG_ERROR_NOT_SUPPORTED, "contraction: a mode group exceeds 2^31 elements");
+    if (c.m.total > int64_t(65535) * 64) return fail(EG_ERROR_NOT_SUPPORTED, "contraction: too many row tiles");
+    F64Args p = f64_args(c);
     int T = 32;
     contract_plan(c.batch.total, c.m.total, c.n.total, c.k.total, T, p.cs);
     p.mtiles = (c.m.total + T - 1) / T;
@@ -707,6 +731,23 @@ eg_status launch_contract_f64(const Contraction &c, cudaStream_t s) {
         if (err != cudaSuccess) return cuda_fail(err, "k_contract_f64");
     }
     EG_CHECK_LAUNCH("k_contract_f64");
+    return EG_SUCCESS;
+}
+
+double contract_f64_seconds(const Contraction &c) {
+    int T = 0, cs = 0;
+    return contract_plan(c.batch.total, c.m.total, c.n.total, c.k.total, T, cs) / 2.0e9;
+}
+
+eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, const int *count, cudaStream_t s) {
+    F64Args p = f64_args(c);
+    p.list = list;
+    p.count = count;
+    {
+        LaunchScope ls_("k_contract_f64_listed", s);
+        k_contract_f64<32><<<(unsigned)(num_sms() * 4), kThreads, 0, s>>>(p);
+    }
+    EG_CHECK_LAUNCH("k_contract_f64_listed");
     return EG_SUCCESS;
 }
 

@@ -50,6 +50,8 @@ struct OperandMap {
     // are nested like a row-major block), that stride; the offset is then
     // index * stride, with no table load in the dependency chain.  0 otherwise.
     int64_t sr = 0, sk = 0;
+    // First batch index and row of the panel being split (rows, nbatch count from there).
+    int64_t b0 = 0, row0 = 0;
 };
 
 __device__ __forceinline__ int64_t comp_of(int comp, int64_t oa, int64_t ob) { return comp == 0 ? oa : ob; }
@@ -57,12 +59,12 @@ __device__ __forceinline__ int64_t comp_of(int comp, int64_t oa, int64_t ob) { r
 __device__ __forceinline__ int64_t off_b(const OperandMap &m, int64_t b) {
     if (m.bg.n == 0) return 0;
     int64_t oa, ob, oc;
-    group_offsets(m.bg, b, oa, ob, oc);
+    group_offsets(m.bg, m.b0 + b, oa, ob, oc);
     return comp_of(m.comp, oa, ob);
 }
 __device__ __forceinline__ int64_t decompose_r(const OperandMap &m, int64_t r) {
     int64_t oa, ob, oc;
-    group_offsets32(m.rg, (uint32_t)r, oa, ob, oc);
+    group_offsets32(m.rg, (uint32_t)(m.row0 + r), oa, ob, oc);
     return comp_of(m.comp, oa, ob);
 }
 __device__ __forceinline__ int64_t decompose_k(const OperandMap &m, int64_t k) {
@@ -71,7 +73,7 @@ __device__ __forceinline__ int64_t decompose_k(const OperandMap &m, int64_t k) {
     return comp_of(m.comp, oa, ob);
 }
 __device__ __forceinline__ int64_t off_r(const OperandMap &m, int64_t r) {
-    if (m.sr) return r * m.sr;
+    if (m.sr) return (m.row0 + r) * m.sr;
     return m.offr ? __ldg(m.offr + r) : decompose_r(m, r);
 }
 __device__ __forceinline__ int64_t off_k(const OperandMap &m, int64_t k) {
@@ -211,7 +213,10 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <int S>
+//
+// CHECK (FP64 form): two more planes per operand, the lower bound of every
+// magnitude and the marks of the nonzero elements (split.cuh).
+template <int S, bool CHECK>
 __global__ void __launch_bounds__(T *TR) k_split_digits(OperandMap m, const double *__restrict__ X, const int *rexp,
                                                         __nv_bfloat16 *planes, int row_fast) {
     __shared__ double tile[2][T][TK + 1];
@@ -275,17 +280,21 @@ __global__ void __launch_bounds__(T *TR) k_split_digits(OperandMap m, const doub
 #pragma unroll
             for (int j = ty; j < T; j += TR) {
                 const int64_t r = r0 + j;
-                uint32_t pk[S];
+                constexpr int P = S + (CHECK ? 2 : 0);
+                uint32_t pk[P];
                 const int e = ex[j];
+                const double x0 = tile[cur][j][2 * tx], x1 = tile[cur][j][2 * tx + 1];
                 if (e == INT_MIN) {
 #pragma unroll
-                    for (int s = 0; s < S; s++) pk[s] = 0u;
+                    for (int s = 0; s < P; s++) pk[s] = 0u;
                 } else {
-                    digits_bf16x2<S>(tile[cur][j][2 * tx], tile[cur][j][2 * tx + 1], e, pk);
+                    digits_bf16x2<S>(x0, x1, e, pk);
+                    if constexpr (CHECK) pk[S] = check_magnitude(pk[0]);
                 }
-                uint32_t *out = (uint32_t *)(planes + ((int64_t)b * S) * plane + r * m.Kp + k0) + tx;
+                if constexpr (CHECK) pk[S + 1] = check_mark(x0, x1, m.comp ? kCheckB : kCheckA);
+                uint32_t *out = (uint32_t *)(planes + ((int64_t)b * P) * plane + r * m.Kp + k0) + tx;
 #pragma unroll
-                for (int s = 0; s < S; s++) out[(int64_t)s * (plane / 2)] = pk[s];
+                for (int s = 0; s < P; s++) out[(int64_t)s * (plane / 2)] = pk[s];
             }
             __syncthreads();
         }
@@ -377,7 +386,8 @@ int64_t affine_stride(const ModeGroup &g, int comp) {
 }
 
 eg_status split_operand(OperandMap om, const double *X, unsigned long long *rowmax, int *rexp,
-                        __nv_bfloat16 *planes, int S, cudaStream_t s, int64_t *offr, int64_t *offk) {
+                        __nv_bfloat16 *planes, int S, cudaStream_t s, int64_t *offr, int64_t *offk,
+                        bool f64 = false) {
     const bool k_fast = is_fast(om.kg, om.comp);
     om.sr = affine_stride(om.rg, om.comp);
     om.sk = affine_stride(om.kg, om.comp);
@@ -394,7 +404,8 @@ eg_status split_operand(OperandMap om, const double *X, unsigned long long *rowm
         om.offk = offk;
     }
     const bool r_fast = !k_fast && is_fast(om.rg, om.comp);
-    EG_CUDA(cudaMemsetAsync(rowmax, 0, (size_t)om.nbatch * om.Rp * sizeof(unsigned long long), s));
+    if (!f64) // the FP64 form's caller clears both operands' maxima at once
+        EG_CUDA(cudaMemsetAsync(rowmax, 0, (size_t)om.nbatch * om.Rp * sizeof(unsigned long long), s));
     const int cap = num_sms() * 8;
     {
         static const int resident = resident_grid(k_split_rowmax);
@@ -415,16 +426,20 @@ eg_status split_operand(OperandMap om, const double *X, unsigned long long *rowm
     EG_CHECK_LAUNCH("k_split_exponent");
     {
         const int64_t work = (int64_t)om.nbatch * (om.Rp / T) * ((om.Kp / TK + kDigitStrip - 1) / kDigitStrip);
-        static const int resident = resident_grid(k_split_digits<5>); // the S variants share a register budget
-        const int grid = (int)(work < resident ? work : resident);
+        static const int resident = resident_grid(k_split_digits<5, false>); // the S variants share a register budget
+        static const int resident_f64 = resident_grid(k_split_digits<kF64Slices, true>);
+        const int cta = f64 ? resident_f64 : resident;
+        const int grid = (int)(work < cta ? work : cta);
         LaunchScope ls_("k_split_digits", s);
         const int rf = r_fast ? 1 : 0;
-        switch (S) {
-        case 2: k_split_digits<2><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf); break;
-        case 3: k_split_digits<3><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf); break;
-        case 4: k_split_digits<4><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf); break;
-        case 5: k_split_digits<5><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf); break;
-        default: k_split_digits<6><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf); break;
+        if (f64)
+            k_split_digits<kF64Slices, true><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf);
+        else switch (S) {
+        case 2: k_split_digits<2, false><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf); break;
+        case 3: k_split_digits<3, false><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf); break;
+        case 4: k_split_digits<4, false><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf); break;
+        case 5: k_split_digits<5, false><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf); break;
+        default: k_split_digits<6, false><<<grid, dim3(T, TR), 0, s>>>(om, X, rexp, planes, rf); break;
         }
     }
     EG_CHECK_LAUNCH("k_split_digits");
@@ -482,6 +497,52 @@ eg_status encode_planes_extent(CUtensorMap *map, void *base, int64_t K, int64_t 
     return EG_SUCCESS;
 }
 
+// Whether |ab| is a power of two: it then joins the exponent instead of costing
+// an FP64 multiplication per output.
+static void set_ab(split::TcGemmParams &p, double ab) {
+    int k = 0;
+    const double f = std::frexp(std::fabs(ab), &k); // |ab| = f 2^k
+    p.ab = ab;
+    p.ab_pow2 = (f == 0.5) ? 1 : 0;
+    p.ab_neg = (p.ab_pow2 && ab < 0) ? 1 : 0;
+    if (p.ab_pow2) p.shift_const += k - 1;
+}
+
+// Which tiles of a launch are cut along K, and how often: the whole rounds of the
+// CTAs run whole tiles; the tiles left over for the last round -- 20 of 324 on 152
+// SMs, a third of the time -- are cut into as many slices of at least two K blocks
+// as give the smallest estimated time.  The estimate counts clocks: 440 per K block
+// of a slice pair, 6000 for a tile's epilogue, 8000 more for adding a slice's sums to
+// its accumulator and 60 per accumulator plane to clear it.  Returns the clocks.
+static double choose_schedule(split::TcGemmParams &p, int64_t units, int64_t workers, int pairs, int planes) {
+    using namespace split;
+    auto entry = [&](int64_t kb) { return 440.0 * pairs * (double)kb + 6000.0; };
+    const int64_t rounds = units / workers, rem = units - rounds * workers;
+    p.t0 = (int)units;
+    p.ksplit = 1;
+    p.kslice = p.nkb;
+    const double whole = (double)rounds * entry(p.nkb);
+    double best = whole + (rem ? entry(p.nkb) : 0.0);
+    if (rem == 0) return best;
+    const int64_t unit = kKStep / kBK;
+    int64_t last = 0;
+    for (int64_t ks = 2; ks <= std::min<int64_t>(p.nkb / unit, 64); ks++) {
+        const int64_t slice = round_up((p.nkb + ks - 1) / ks, unit);
+        const int64_t n = (p.nkb + slice - 1) / slice; // slices actually used
+        if (n == last) continue;
+        last = n;
+        const int64_t r = (rem * n + workers - 1) / workers;
+        const double t = whole + (double)r * (entry(slice) + 8000.0) + 60.0 * (double)(rem * planes);
+        if (t < 0.98 * best) {
+            best = t;
+            p.t0 = (int)(rounds * workers);
+            p.ksplit = (int)n;
+            p.kslice = (int)slice;
+        }
+    }
+    return best;
+}
+
 eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s, eg_split_report *rep) {
     using namespace split;
     const int S = slices ? slices : 5;
@@ -503,16 +564,17 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     const bool tables = M + K <= (int64_t(1) << 25) && N + K <= (int64_t(1) << 25);
     const size_t offTab = offR + rbuf_bytes();
     const size_t tabBytes = tables ? (size_t)(M + N + 2 * K) * 8 : 0;
-    // K slices in parallel when the output has fewer tiles than half the SMs
     const int64_t tiles = nb * (Mp / kBM) * (Np / kBN);
-    const bool kslicing = tiles < num_sms() / 2;
     // CTA pairs (256x128 tiles) whenever the output has two or more row tiles
     const int clusters = Mp / kBM >= 2 ? tc_pair_clusters() : 0;
     const bool pair = clusters > 0;
     const size_t offRacc = round_up((int64_t)(offTab + tabBytes), 256);
-    const size_t raccBytes = kslicing ? (size_t)tiles * kBM * kBN * 8 : 0;
+    // accumulators of the tiles cut along K: fewer than the SMs (CTA pairs cut whole
+    // launches, of fewer tiles than half the SMs)
+    const size_t cut = (size_t)std::min<int64_t>(tiles, num_sms());
+    const size_t raccBytes = cut * kBM * kBN * 8;
     const size_t offRcnt = offRacc + raccBytes;
-    const size_t rcntBytes = kslicing ? (size_t)tiles * 8 * sizeof(int) : 0;
+    const size_t rcntBytes = cut * 8 * sizeof(int);
     const size_t total = offRcnt + rcntBytes;
     void *ws = nullptr;
     eg_status st = workspace(s, total, &ws);
@@ -539,6 +601,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     TcGemmParams p{};
     p.pair = pair ? 1 : 0;
     p.S = S;
+    p.planes = S;
     p.mtiles = (int)(Mp / kBM);
     p.ntiles = (int)(Np / kBN);
     p.nbatch = (int)nb;
@@ -550,22 +613,15 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     p.mg = c.m;
     p.ng = c.n;
     p.C = c.C;
-    p.ab = c.ab;
     p.eA = eA;
     p.eB = eB;
     p.shift_const = -2 * kTopBits - kBits * (S - 1);
-    {
-        int k = 0;
-        const double f = std::frexp(std::fabs(c.ab), &k); // |ab| = f 2^k
-        p.ab_pow2 = (f == 0.5) ? 1 : 0;
-        p.ab_neg = (p.ab_pow2 && c.ab < 0) ? 1 : 0;
-        if (p.ab_pow2) p.shift_const += k - 1;
-    }
+    set_ab(p, c.ab);
     p.status = status;
     p.timeout_ns = 2000ull * 1000 * 1000;
     p.rbuf = (long long *)(base + offR);
-    p.racc = kslicing ? (long long *)(base + offRacc) : nullptr;
-    p.rcnt = kslicing ? (int *)(base + offRcnt) : nullptr;
+    p.racc = (long long *)(base + offRacc);
+    p.rcnt = (int *)(base + offRcnt);
 
     // Launches: when all slice groups' exact sum fits int64 over the whole K (up to
     // 65024 for S = 5), one.  Otherwise the slice groups are cut into ranges whose
@@ -592,31 +648,21 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
         for (int64_t kb0 = 0; kb0 < nkb_total || kb0 == 0; kb0 += kb_per_pass) {
             p.kb0 = (int)kb0;
             p.nkb = (int)std::min<int64_t>(kb_per_pass, nkb_total - kb0);
-            // slices of at least 16 K blocks (one exact chunk); the count minimises the
-            // estimated makespan: rounds of work entries over the SMs times the K blocks
-            // of one entry, plus about four blocks' worth of per-entry epilogue work
-            p.ksplit = 1;
-            p.kslice = p.nkb;
-            if (kslicing && p.nkb >= 32) {
-                // schedule units: tiles over SMs, or pair tiles over CTA pairs
-                const int64_t units = pair ? nb * ((Mp / kBM + 1) / 2) * (Np / kBN) : tiles;
-                const int64_t workers = pair ? clusters : num_sms();
-                int64_t best = -1;
-                for (int ks = 1; ks <= p.nkb / 16; ks++) {
-                    const int64_t slice = round_up((p.nkb + ks - 1) / ks, kKStep / kBK);
-                    const int64_t n = (p.nkb + slice - 1) / slice; // slices actually used
-                    const int64_t rounds = (units * n + workers - 1) / workers;
-                    const int64_t cost = rounds * (slice + 4);
-                    if (best < 0 || cost < best) {
-                        best = cost;
-                        p.kslice = (int)slice;
-                        p.ksplit = (int)n;
-                    }
-                }
+            int pairs = 0;
+            for (int d = p.d0; d < p.d1; d++) pairs += d + 1;
+            // schedule units: tiles over SMs, or pair tiles over CTA pairs
+            const int64_t units = pair ? nb * ((Mp / kBM + 1) / 2) * (Np / kBN) : tiles;
+            if (pair && units >= clusters / 2) {
+                p.t0 = (int)units;
+                p.ksplit = 1;
+                p.kslice = p.nkb;
+            } else {
+                choose_schedule(p, units, pair ? clusters : num_sms(), pairs, 1);
             }
             if (p.ksplit > 1) {
-                EG_CUDA(cudaMemsetAsync(p.racc, 0, raccBytes, s));
-                EG_CUDA(cudaMemsetAsync(p.rcnt, 0, rcntBytes, s));
+                const size_t n = (size_t)(pair ? tiles : units - p.t0);
+                EG_CUDA(cudaMemsetAsync(p.racc, 0, n * kBM * kBN * 8, s));
+                EG_CUDA(cudaMemsetAsync(p.rcnt, 0, n * 8 * sizeof(int), s));
             }
             const bool first = first_launch;
             first_launch = false;
@@ -658,6 +704,177 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
         rep->error_bound = error_bound(S);
     }
     return EG_SUCCESS;
+}
+
+// The plain FP64 contraction on the tensor cores.
+//
+// This GPU's FP64 pipe retires two FMAs per clock per SM; the tensor cores run
+// the 36 BF16 slice products of an eight-slice split (63 bits below the power of
+// two above each row's largest element) an order of magnitude faster.  What the
+// split leaves out is bounded for every output before it is written:
+//
+//   |C - C_exact| <= 9.04 2^-64 N max|A_i| max|B_j|     N: the k where both are nonzero
+//
+// (7.03 from the slice pairs dropped, 2 from the digits, with max| | the power of
+// two above the row's largest element).  The check planes give, in one more slice
+// group and exactly, sum_k p_a p_b with p <= 128 |x| / max, and 20 N; where
+//   sum_k p_a p_b >= 20 N
+// the error is at most 4 2^-53 sum_k |A_ik| |B_jk| -- four roundings' worth, where
+// the bound of a chain of K FMAs is K of them.  A 32 x 64 block of outputs in
+// which it fails anywhere (rows graded against each other, infinities, NaN) is
+// not written but listed, and k_contract_f64 computes it from C as it was.  The
+// sums of all 36 products are exact in two int64 words and rounded once.
+//
+// The digit planes live in a scratch shared by the streams of the device and
+// bounded by kF64ScratchCap; larger operands are cut into panels of rows.  When
+// the scratch cannot be had (a memory budget, a full device) or the stream is
+// being captured (a graph must not hold the scratch), EG_ERROR_NOT_SUPPORTED
+// comes back with nothing launched and the FMA kernel runs instead.
+constexpr size_t kF64ScratchCap = size_t(2) << 30;
+
+eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
+    using namespace split;
+    constexpr int S = kF64Slices, P = S + 2;
+    const int64_t nb = c.batch.total, M = c.m.total, N = c.n.total, K = c.k.total;
+    const int64_t Kp = round_up(K, kKStep);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    EG_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return EG_ERROR_NOT_SUPPORTED;
+    // panels: all rows of both operands when they fit, else whole 128-row blocks of
+    // each (and, with batches, as many batch indices as fit)
+    const int64_t row_bytes = P * Kp * 2 + 32, Mp_all = round_up(M, kBM), Np_all = round_up(N, kBN);
+    const int64_t budget = (int64_t)kF64ScratchCap / row_bytes / kBM * kBM;
+    int64_t mb = Mp_all, nbk = Np_all, bb = 1;
+    if (mb + nbk > budget) {
+        const int64_t half = budget / 2 / kBM * kBM;
+        if (half < kBM) return EG_ERROR_NOT_SUPPORTED;
+        if (nbk <= half)
+            mb = budget - nbk;
+        else if (mb <= half)
+            nbk = budget - mb;
+        else
+            mb = nbk = half;
+    } else {
+        bb = std::max<int64_t>(1, std::min<int64_t>(nb, budget / (mb + nbk)));
+        bb = std::min<int64_t>(bb, (int64_t(1) << 20) / P);
+    }
+    const int64_t tiles = bb * (mb / kBM) * (nbk / kBN);
+    const int64_t cut = std::min<int64_t>(tiles, num_sms()); // tiles cut along K, at most
+    const int64_t all_tiles = nb * (Mp_all / kBM) * (Np_all / kBN);
+    const bool tables = M + K <= (int64_t(1) << 22) && N + K <= (int64_t(1) << 22);
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 1023) & ~size_t(1023);
+        return o;
+    };
+    const size_t oPA = take((size_t)bb * P * mb * Kp * 2), oPB = take((size_t)bb * P * nbk * Kp * 2);
+    const size_t oMax = take((size_t)bb * (mb + nbk) * 8); // cleared for every panel pair ...
+    const size_t oCnt = take((size_t)cut * 8 * sizeof(int)); // (with the accumulators' arrivals
+    const size_t oAcc = take((size_t)cut * 2 * kBM * kBN * 8); //  and those that the launch uses)
+    const size_t oExp = take((size_t)bb * (mb + nbk) * 4);
+    const size_t oTab = take(tables ? (size_t)(M + N + 2 * K) * 8 : 0);
+    const size_t oR = take(rbuf_bytes(2));
+    const size_t oRedoN = take(sizeof(int)), oRedo = take((size_t)all_tiles * 8 * sizeof(int4));
+    ScratchLease lease(s, at);
+    if (!lease.ptr()) return EG_ERROR_NOT_SUPPORTED;
+    int *status = nullptr;
+    eg_status st = status_word(s, &status);
+    if (st != EG_SUCCESS) return st;
+    char *base = (char *)lease.ptr();
+    __nv_bfloat16 *planesA = (__nv_bfloat16 *)(base + oPA), *planesB = (__nv_bfloat16 *)(base + oPB);
+    unsigned long long *maxA = (unsigned long long *)(base + oMax), *maxB = maxA + bb * mb;
+    int *eA = (int *)(base + oExp), *eB = eA + bb * mb;
+    int64_t *tab = tables ? (int64_t *)(base + oTab) : nullptr;
+
+    TcGemmParams p{};
+    p.S = S;
+    p.planes = P;
+    p.bg = c.batch;
+    p.mg = c.m;
+    p.ng = c.n;
+    p.C = c.C;
+    p.cp = c.cp;
+    p.zero = c.zero_when_cp_zero ? 1 : 0;
+    p.eA = eA;
+    p.eB = eB;
+    p.shift_const = -2 * kTopBits - kBits * (S - 1);
+    set_ab(p, c.ab);
+    p.status = status;
+    p.timeout_ns = 2000ull * 1000 * 1000;
+    p.rbuf = (long long *)(base + oR);
+    p.racc = (long long *)(base + oAcc);
+    p.rcnt = (int *)(base + oCnt);
+    p.d0 = 0;
+    p.d1 = S;
+    p.hid = kF64High;
+    p.redo = (int4 *)(base + oRedo);
+    p.redo_count = (int *)(base + oRedoN);
+    EG_CUDA(cudaMemsetAsync(p.redo_count, 0, sizeof(int), s));
+
+    for (int64_t b0 = 0; b0 < nb; b0 += bb) {
+        const int64_t nbc = std::min(bb, nb - b0);
+        for (int64_t m0 = 0; m0 < M; m0 += mb) {
+            const int64_t mc = std::min(mb, M - m0), Mp = round_up(mc, kBM);
+            for (int64_t n0 = 0; n0 < N; n0 += nbk) {
+                const int64_t nc = std::min(nbk, N - n0), Np = round_up(nc, kBN);
+                p.nkb = (int)(Kp / kBK);
+                choose_schedule(p, nbc * (Mp / kBM) * (Np / kBN), num_sms(), S * (S + 1) / 2 + 2, 2);
+                const size_t used = p.ksplit > 1 ? (size_t)(nbc * (Mp / kBM) * (Np / kBN) - p.t0) * 2 * kBM * kBN * 8 : 0;
+                EG_CUDA(cudaMemsetAsync(maxA, 0, oAcc - oMax + used, s));
+                OperandMap oa{c.batch, c.m, c.k, 0, mc, Mp, K, Kp, (int)nbc};
+                oa.b0 = b0;
+                oa.row0 = m0;
+                OperandMap ob{c.batch, c.n, c.k, 1, nc, Np, K, Kp, (int)nbc};
+                ob.b0 = b0;
+                ob.row0 = n0;
+                // a panel's planes stay while the other operand's panels go by
+                if (n0 == 0 && (st = split_operand(oa, c.A, maxA, eA, planesA, S, s, tab, tables ? tab + M : nullptr,
+                                                   true)) != EG_SUCCESS)
+                    return st;
+                if ((nbk < Np_all || m0 == 0) &&
+                    (st = split_operand(ob, c.B, maxB, eB, planesB, S, s, tables ? tab + M + K : nullptr,
+                                        tables ? tab + M + K + N : nullptr, true)) != EG_SUCCESS)
+                    return st;
+                CUtensorMap tmA, tmB;
+                if ((st = encode_planes(&tmA, planesA, Kp, Mp, nbc * P)) != EG_SUCCESS) return st;
+                if ((st = encode_planes(&tmB, planesB, Kp, Np, nbc * P)) != EG_SUCCESS) return st;
+                p.b0 = b0;
+                p.m0 = m0;
+                p.n0 = n0;
+                p.M = mc;
+                p.N = nc;
+                p.Mp = (int)Mp;
+                p.Np = (int)Np;
+                p.mtiles = (int)(Mp / kBM);
+                p.ntiles = (int)(Np / kBN);
+                p.nbatch = (int)nbc;
+                if ((st = launch_tc_gemm(tmA, tmB, p, s)) != EG_SUCCESS) return st;
+            }
+        }
+    }
+    return launch_contract_f64_listed(c, p.redo, p.redo_count, s);
+}
+
+// Whether an FP64 contraction is worth its detour over the tensor cores, from
+// estimates of both times: the FMA kernel's own, against 30 us of launches, the
+// splitting of both operands (36 bytes moved per element) and the tensor kernel's
+// schedule.  K below 32 is left to the FMA kernel, whose own error is then as small
+// as the check's bound; above 65536 the sums would need more bits.
+bool f64_tensor_pays(const Contraction &c) {
+    using namespace split;
+    const int64_t nb = c.batch.total, M = c.m.total, N = c.n.total, K = c.k.total;
+    if (K < 32 || K > 65536 || M < 8 || N < 8) return false;
+    if (M > int64_t(65535) * 64 || N > int64_t(65535) * 64 || nb > (int64_t(1) << 24)) return false;
+    const double fma = contract_f64_seconds(c);
+    if (fma < 40e-6) return false;
+    TcGemmParams p{};
+    p.nkb = (int)(round_up(K, kKStep) / kBK);
+    const int64_t tiles = nb * (round_up(M, kBM) / kBM) * (round_up(N, kBN) / kBN);
+    if (tiles > (int64_t(1) << 30)) return false;
+    const double clocks = choose_schedule(p, tiles, num_sms(), kF64Slices * (kF64Slices + 1) / 2 + 2, 2);
+    const double tensor = 30e-6 + (double)nb * (double)(M + N) * (double)K * 36.0 / 3e12 + clocks / 1.9e9;
+    return tensor < 0.9 * fma;
 }
 
 } // namespace eg

@@ -31,11 +31,16 @@ constexpr int kBits = 8;        // digit width
 constexpr int kTopBits = 7;     // magnitude bits of the leading digit
 constexpr int kMaxSlices = 6;   // keeps the scaled digits and the int64 accumulator in range
 constexpr int kBM = 128, kBN = 128, kBK = 64;
+// The FP64 form: eight slices (63 bits below each row's power of two) and the
+// accuracy check of launch_f64_tensor.
+constexpr int kF64Slices = 8, kF64High = 4;
+constexpr float kCheckA = 4.0f, kCheckB = -5.0f;
 constexpr int kChunkKB = 16;    // 16 x 64 = 1024 products per exact FP32 chunk
 constexpr int kKStep = 2 * kBK;  // K is padded to whole groups of two K blocks
 
 struct TcGemmParams {
     int S;
+    int planes; // planes per batch index of each operand: S, or S + 2 in the FP64 form
     int nkb;  // K blocks in this pass
     int kb0;  // first K block of this pass
     int mtiles, ntiles, nbatch;
@@ -57,12 +62,17 @@ struct TcGemmParams {
     // Per-CTA scratch of gridDim.x * 128 * 128 int64: a finished tile's sums
     // wait here until the epilogue converts them during the next tile.
     long long *rbuf;
-    // K slices run in parallel when there are few output tiles: entry t of the
-    // schedule is K slice t % ksplit (kslice K blocks, even; the last slice takes
-    // the rest) of tile t / ksplit.  The slices' exact int64 sums are added into
-    // racc ([tile][128 columns][128 rows]) and the last slice to arrive at a
-    // region of an epilogue warp (counted in rcnt, [tile][8]) finishes it.  Both
-    // are zeroed by the host before the launch; unused when ksplit == 1.
+    // The first t0 schedule entries are whole tiles.  The tiles left for the last,
+    // partly filled round of the CTAs (all of them when there are fewer tiles than
+    // CTAs) are cut along K so that the round is full: entry t >= t0 is K slice
+    // (t - t0) % ksplit (kslice K blocks, even; the last slice takes the rest) of
+    // tile t0 + (t - t0) / ksplit.  The slices' exact int64 sums are added into racc
+    // ([tile - t0][128 columns][128 rows], two planes in the FP64 form) and the last
+    // slice to arrive at a region of an epilogue warp (counted in rcnt,
+    // [tile - t0][8]) finishes it.  Both are zeroed by the host before the launch;
+    // unused when t0 is the number of tiles.  (CTA pairs number the accumulators by
+    // output tile.)
+    int t0;
     int ksplit, kslice;
     long long *racc;
     int *rcnt;
@@ -73,6 +83,16 @@ struct TcGemmParams {
     // summed by this launch: all of them (0, S) unless a long K is split into
     // group ranges whose exact sums each fit int64 (finished into C one by one).
     int d0, d1;
+    // First batch index, row and column of the panel of C this launch computes (0 when
+    // it computes all of it): mt, nt and the exponents count from there.
+    int64_t b0, m0, n0;
+    // FP64 form (redo set): the exact sums do not fit 64 bits, so the slice groups
+    // below hid form one int64 sum and the others a second; a 32 x 64 block of
+    // outputs whose accuracy check fails is left alone and listed in redo
+    // ({batch, row, column}, redo_count entries) for the FMA kernel.
+    int hid;
+    int4 *redo;
+    int *redo_count;
     // Grouped launches: two tensor maps per item (A, B) over the item's own digit
     // planes with its own row and K extents, so that TMA fills the tile's rows
     // past M (N) and K blocks past K with zeros instead of reading the padding.
@@ -99,7 +119,7 @@ __device__ __forceinline__ unsigned long long abs_bits(double x) {
     return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
 }
 
-// round(x * 2^sh) to nearest, ties to even, for |x| 2^sh < 2^52, built from the
+// round(x * 2^sh) to nearest, ties to even, for |x| 2^sh < 2^63, built from the
 // IEEE fields with integer operations (the FP64 pipe of this GPU runs about two
 // operations per clock per SM; this is the splitting kernels' inner loop).
 __device__ __forceinline__ long long scaled_round(double x, int sh) {
@@ -109,7 +129,7 @@ __device__ __forceinline__ long long scaled_round(double x, int sh) {
     const int r = 1075 - (ex != 0 ? ex : 1) - sh; // |x| 2^sh = mant 2^-r
     unsigned long long q;
     if (r <= 0) {
-        q = mant << (-r < 11 ? -r : 11); // not reached while |x| 2^sh < 2^52
+        q = mant << (-r < 63 ? -r : 63); // a whole number already
     } else if (r > 62) {
         q = 0; // below 1/2
     } else {
@@ -133,10 +153,9 @@ __device__ __forceinline__ double scale_pow2(double v, int e) {
 // the FP64 pipe -- about 1.75 operations per clock per SM on this GPU -- is
 // left for the one fused multiply-add with C.  Falls back to the FP64 path
 // when the result would not be a normal number.
-__device__ __forceinline__ double int_times_pow2_rn(long long R, int e) {
-    if (R == 0) return 0.0;
-    const unsigned long long sign = R < 0 ? 0x8000000000000000ull : 0ull;
-    const unsigned long long a = R < 0 ? (unsigned long long)(-R) : (unsigned long long)R;
+__device__ __forceinline__ double int_times_pow2_rn64(unsigned long long a, bool neg, int e) {
+    if (a == 0) return 0.0;
+    const unsigned long long sign = neg ? 0x8000000000000000ull : 0ull;
     const int lz = __clzll((long long)a);
     const unsigned long long x = a << lz;      // leading one at bit 63
     unsigned long long mant = x >> 11;         // 53 bits, leading one at bit 52
@@ -148,8 +167,27 @@ __device__ __forceinline__ double int_times_pow2_rn(long long R, int e) {
         exp++;
     }
     const int biased = exp + 1023;
-    if (biased <= 0 || biased >= 2047) return scale_pow2(__ll2double_rn(R), e);
+    if (biased <= 0 || biased >= 2047) {
+        const double v = scale_pow2(__ull2double_rn(a), e);
+        return neg ? -v : v;
+    }
     return __longlong_as_double((long long)(sign | ((unsigned long long)biased << 52) | (mant & 0xFFFFFFFFFFFFFull)));
+}
+
+__device__ __forceinline__ double int_times_pow2_rn(long long R, int e) {
+    return int_times_pow2_rn64(R < 0 ? (unsigned long long)(-R) : (unsigned long long)R, R < 0, e);
+}
+
+// The same for a 128-bit integer.
+__device__ __forceinline__ double int128_times_pow2_rn(__int128 R, int e) {
+    const bool neg = R < 0;
+    const unsigned __int128 a = neg ? (unsigned __int128)(-R) : (unsigned __int128)R;
+    unsigned long long hi = (unsigned long long)(a >> 64), lo = (unsigned long long)a;
+    if (hi == 0) return int_times_pow2_rn64(lo, neg, e);
+    const int lz = __clzll((long long)hi); // below 64
+    const unsigned long long x = lz ? (hi << lz) | (lo >> (64 - lz)) : hi; // leading one at bit 63
+    const bool sticky = (lo << lz) != 0;
+    return int_times_pow2_rn64(x | (sticky ? 1ull : 0ull), neg, e + 64 - lz); // the lowest bit only breaks ties
 }
 
 // Balanced base-256 digits of x * 2^(7 + 8(S-1) - e) rounded to an integer,
@@ -164,6 +202,18 @@ __device__ __forceinline__ void to_digits(double x, int e, int S, int *dig) {
         F = (F - d) >> 8; // exact: F - d is a multiple of 256
     }
     dig[0] = (int)F;
+}
+
+// The leading digit: G >> 8(S-1), except that with eight slices G = F + bias may
+// leave 64 bits, so there the carry out of the low bytes is added to F's own top.
+template <int S>
+__device__ __forceinline__ int top_digit(long long F, unsigned long long G, long long bias) {
+    if constexpr (S < 8) {
+        return (int)((long long)G >> (8 * (S - 1)));
+    } else {
+        constexpr unsigned long long low = (1ull << 56) - 1;
+        return (int)(F >> 56) + (int)((((unsigned long long)F & low) + (unsigned long long)bias) >> 56);
+    }
 }
 
 // The digits of two values as BF16 pairs: out[s] holds digit s of x0 in its low
@@ -182,9 +232,10 @@ __device__ __forceinline__ void digits_bf16x2(double x0, double x1, int e, uint3
         return b;
     }();
     const int sh = kTopBits + kBits * (S - 1) - e;
-    const long long G0 = scaled_round(x0, sh) + bias, G1 = scaled_round(x1, sh) + bias;
-    const uint32_t g0[2] = {(uint32_t)G0, (uint32_t)((unsigned long long)G0 >> 32)};
-    const uint32_t g1[2] = {(uint32_t)G1, (uint32_t)((unsigned long long)G1 >> 32)};
+    const long long F0 = scaled_round(x0, sh), F1 = scaled_round(x1, sh);
+    const unsigned long long G0 = (unsigned long long)F0 + bias, G1 = (unsigned long long)F1 + bias;
+    const uint32_t g0[2] = {(uint32_t)G0, (uint32_t)(G0 >> 32)};
+    const uint32_t g1[2] = {(uint32_t)G1, (uint32_t)(G1 >> 32)};
 #pragma unroll
     for (int s = 1; s < S; s++) {
         // byte S-1-s of G next to the bytes 00 00 4B: the float 2^23 + u in one permute
@@ -194,10 +245,22 @@ __device__ __forceinline__ void digits_bf16x2(double x0, double x1, int e, uint3
         const float f1 = __uint_as_float(__byte_perm(g1[w], 0x4B000000u, sel)) - 8388735.0f;
         out[s] = __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
     }
-    const int t0 = (int)(G0 >> (8 * (S - 1))), t1 = (int)(G1 >> (8 * (S - 1)));
+    const int t0 = top_digit<S>(F0, G0, bias), t1 = top_digit<S>(F1, G1, bias);
     const float f0 = __int_as_float(0x4B400000 + t0) - 12582912.0f;
     const float f1 = __int_as_float(0x4B400000 + t1) - 12582912.0f;
     out[0] = __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
+}
+
+// The two check planes of the FP64 form for the pair whose leading digits are
+// d0 (as floats in the halves of `lead`): max(|a_0| - 1, 0), at most 128 |x| 2^-e,
+// and `mark` where x is not zero (kCheckA or kCheckB by operand).
+__device__ __forceinline__ uint32_t check_magnitude(uint32_t lead) {
+    const float f0 = fmaxf(fabsf(__uint_as_float(lead << 16)) - 1.0f, 0.0f);
+    const float f1 = fmaxf(fabsf(__uint_as_float(lead & 0xFFFF0000u)) - 1.0f, 0.0f);
+    return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
+}
+__device__ __forceinline__ uint32_t check_mark(double x0, double x1, float mark) {
+    return __byte_perm(abs_bits(x0) ? __float_as_uint(mark) : 0u, abs_bits(x1) ? __float_as_uint(mark) : 0u, 0x7632);
 }
 
 // Sets the kernels' shared-memory attribute once (call outside stream capture).
@@ -211,7 +274,7 @@ eg_status launch_tc_gemm_grouped(const CUtensorMap &tmA, const CUtensorMap &tmB,
                                  const TcItem *items, const int4 *work, int ntiles_total, cudaStream_t s);
 
 // Bytes of the per-CTA sum scratch a tensor launch needs (TcGemmParams::rbuf).
-inline size_t rbuf_bytes() { return (size_t)num_sms() * kBM * kBN * sizeof(long long); }
+inline size_t rbuf_bytes(int planes = 1) { return (size_t)num_sms() * planes * kBM * kBN * sizeof(long long); }
 
 // Largest K (a multiple of kKStep) one pass may sum without the int64
 // accumulator overflowing 2^62 for S slices.

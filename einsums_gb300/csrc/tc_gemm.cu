@@ -99,12 +99,14 @@ struct TileJob {
     int zA, zB;  // digit plane of slice 0 for A / B
     int kbeg;    // first K block (of this pass) of the K slice
     int nkb;     // K blocks
-    int tid;     // linear output tile index (single-contraction form); -1: rows past the
-                 // last tile (the odd half of a CTA pair's tile), nothing to store
+    bool split;  // a K slice of a tile: its sums go to the tile's accumulator
+    int tid;     // which accumulator (single-contraction form); -1: rows past the last
+                 // tile (the odd half of a CTA pair's tile), nothing to store
     int64_t M, N;
     const ModeGroup *mg, *ng;
     const int *eA, *eB; // exponents of rows / columns of this (item, batch)
     double *C;          // output base of this (item, batch)
+    int b;              // batch index (single-contraction form)
     const CUtensorMap *mapA, *mapB; // per-item maps (grouped launches), else null
 };
 
@@ -114,16 +116,20 @@ __device__ __forceinline__ TileJob resolve(const TcGemmParams &p, const TcItem *
                                            int rank) {
     TileJob j;
     if (!GROUPED) {
-        int b, mu;
-        const int ks = t % p.ksplit;
-        t /= p.ksplit;
+        int b, mu, ks = 0;
+        j.split = t >= p.t0;
+        if (j.split) {
+            const int e = t - p.t0, q = e / p.ksplit;
+            ks = e - q * p.ksplit;
+            t = p.t0 + q;
+        }
         tile_coords<CL>(p, t, b, mu, j.nt);
         j.mt = mu * CL + rank;
-        j.zA = b * p.S;
-        j.zB = b * p.S;
+        j.zA = b * p.planes;
+        j.zB = b * p.planes;
         j.kbeg = ks * p.kslice;
-        j.nkb = min(p.kslice, p.nkb - j.kbeg);
-        j.tid = j.mt < p.mtiles ? (b * p.mtiles + j.mt) * p.ntiles + j.nt : -1;
+        j.nkb = j.split ? min(p.kslice, p.nkb - j.kbeg) : p.nkb;
+        j.tid = j.mt >= p.mtiles ? -1 : CL == 1 ? max(t - p.t0, 0) : (b * p.mtiles + j.mt) * p.ntiles + j.nt;
         j.M = p.M;
         j.N = p.N;
         j.mg = &p.mg;
@@ -131,8 +137,9 @@ __device__ __forceinline__ TileJob resolve(const TcGemmParams &p, const TcItem *
         j.eA = p.eA + (int64_t)b * p.Mp;
         j.eB = p.eB + (int64_t)b * p.Np;
         int64_t oa, ob, oc;
-        group_offsets(p.bg, b, oa, ob, oc);
+        group_offsets(p.bg, p.b0 + b, oa, ob, oc);
         j.C = p.C + oc;
+        j.b = (int)(p.b0 + b);
         j.mapA = j.mapB = nullptr;
     } else {
         const int4 w = work[t];
@@ -151,6 +158,7 @@ __device__ __forceinline__ TileJob resolve(const TcGemmParams &p, const TcItem *
         }
         j.kbeg = 0;
         j.nkb = it.nkb;
+        j.split = false;
         j.tid = 0;
         j.M = it.M;
         j.N = it.N;
@@ -161,15 +169,27 @@ __device__ __forceinline__ TileJob resolve(const TcGemmParams &p, const TcItem *
         int64_t oa, ob, oc;
         group_offsets(it.bg, b, oa, ob, oc);
         j.C = it.C + oc;
+        j.b = b;
     }
     return j;
 }
+
+// Slice groups in the order they run.  The FP64 form starts with group -1, the
+// two plane pairs of its accuracy check (planes S and S + 1 of each operand);
+// group d then holds the digit pairs (s, d - s).
+template <bool F64>
+__device__ __forceinline__ int group_pairs(int d) { return F64 && d < 0 ? 2 : d + 1; }
+template <bool F64>
+__device__ __forceinline__ int pair_a(const TcGemmParams &p, int d, int s) { return F64 && d < 0 ? p.S + s : s; }
+template <bool F64>
+__device__ __forceinline__ int pair_b(const TcGemmParams &p, int d, int s) { return F64 && d < 0 ? p.S + s : d - s; }
 
 // K blocks of schedule entry t.
 template <bool GROUPED>
 __device__ __forceinline__ int entry_nkb(const TcGemmParams &p, const TcItem *items, const int4 *work, int t) {
     if (GROUPED) return items[work[t].x].nkb;
-    const int kbeg = (t % p.ksplit) * p.kslice;
+    if (t < p.t0) return p.nkb;
+    const int kbeg = ((t - p.t0) % p.ksplit) * p.kslice;
     return min(p.kslice, p.nkb - kbeg);
 }
 
@@ -194,6 +214,21 @@ __device__ __forceinline__ int entry_nkb(const TcGemmParams &p, const TcItem *it
     " add.s64 a, %12, %14;\n add.s64 b, %13, %15;\n"                                                                   \
     " tcgen05.mma.cta_group::" CG ".kind::f16 [%1], a, b, %7, 1;\n"                                                    \
     " selp.u32 %0, 1, 0, p;\n}\n"
+
+// The FP64 value of one output's exact sums, scaled, before C is added.
+template <bool F64>
+__device__ __forceinline__ double finish_value(const TcGemmParams &p, long long lo, long long hi, int rowExp, int colExp) {
+    if (rowExp == INT_MIN || colExp == INT_MIN) return __longlong_as_double(0x7ff8000000000000ll);
+    double v;
+    if constexpr (F64) {
+        __int128 R = ((__int128)hi << (kBits * (p.S - p.hid))) + lo;
+        if (p.ab_neg) R = -R;
+        v = int128_times_pow2_rn(R, rowExp + colExp + p.shift_const);
+    } else {
+        v = int_times_pow2_rn(p.ab_neg ? -lo : lo, rowExp + colExp + p.shift_const);
+    }
+    return p.ab_pow2 ? v : v * p.ab;
+}
 
 template <int CL>
 __device__ __forceinline__ bool mma_group(uint32_t d, uint64_t a0, uint64_t b0, uint32_t idesc, uint32_t accumulate,
@@ -237,12 +272,17 @@ __device__ __forceinline__ void raise_abort(const TcGemmParams &p, volatile int 
 // each CTA's 128 rows into that CTA's tensor memory, and commits to the
 // "empty" and "accumulator full" barriers of both CTAs; both CTAs' epilogue
 // warps release an accumulator on the even CTA's barrier (16 arrivals).
-template <bool GROUPED, int CL>
+template <bool GROUPED, int CL, bool F64>
 __global__ void __launch_bounds__(THREADS, 1)
     k_tc_split_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ TcGemmParams p, const TcItem *items, const int4 *work,
                     int ntiles_total) {
     static_assert(CL == 1 || (CL == 2 && !GROUPED), "CTA pairs serve single contractions");
+    static_assert(!F64 || (CL == 1 && !GROUPED), "the FP64 form serves single contractions on single-CTA tiles");
+    // columns of a pending tile finished per chunk (the FP64 form holds two words per sum)
+    constexpr int FC = F64 ? kFinCols / 2 : kFinCols, FF = F64 ? kFinFast / 2 : kFinFast;
+    constexpr int PLANES = F64 ? 2 : 1; // int64 sums per output in the scratch and the K slices' accumulator
+    const int dbeg = F64 ? -1 : p.d0;
     using R = Ring<CL>;
     constexpr int STAGES = R::STAGES, STAGE_BYTES = R::STAGE_BYTES;
     extern __shared__ uint8_t smem_raw[];
@@ -295,7 +335,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int cta0 = blockIdx.x / CL, ctas = gridDim.x / CL;
 
     const int total_tiles =
-        GROUPED ? ntiles_total : p.nbatch * ((p.mtiles + CL - 1) / CL) * p.ntiles * p.ksplit;
+        GROUPED ? ntiles_total : p.t0 + (p.nbatch * ((p.mtiles + CL - 1) / CL) * p.ntiles - p.t0) * p.ksplit;
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
@@ -323,9 +363,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                         ptx::tma_prefetch_desc(mB);
                     }
                 }
-                for (int d = p.d0; d < p.d1 && ok; d++) {
-                    for (int s = 0; s <= d && ok; s++) {
-                        const int t = d - s;
+                for (int d = dbeg; d < p.d1 && ok; d++) {
+                    for (int s = 0; s < group_pairs<F64>(d) && ok; s++) {
+                        const int sA = pair_a<F64>(p, d, s), sB = pair_b<F64>(p, d, s);
                         for (int kb = 0; kb < job.nkb; kb += GROUP_KB) {
                             const long long t0 = p.prof ? clock64() : 0;
                             const bool got = ptx::mbar_wait(&empty[stage], phase ^ 1, p.timeout_ns, abort_flag);
@@ -342,12 +382,12 @@ __global__ void __launch_bounds__(THREADS, 1)
                                 const int kc = (p.kb0 + job.kbeg + kb + h) * kBK;
                                 uint8_t *sb = sa + GROUP_KB * A_BYTES + h * R::B_BYTES;
                                 if (CL == 1) {
-                                    ptx::tma_load_3d(sa + h * A_BYTES, mA, &full[stage], kc, arow, job.zA + s);
-                                    ptx::tma_load_3d(sb, mB, &full[stage], kc, brow, job.zB + t);
+                                    ptx::tma_load_3d(sa + h * A_BYTES, mA, &full[stage], kc, arow, job.zA + sA);
+                                    ptx::tma_load_3d(sb, mB, &full[stage], kc, brow, job.zB + sB);
                                 } else {
                                     const uint32_t fb = full_lead + (uint32_t)(stage * 8);
-                                    ptx::tma_load_3d_pair(sa + h * A_BYTES, &tmA, fb, kc, arow, job.zA + s);
-                                    ptx::tma_load_3d_pair(sb, &tmB, fb, kc, brow, job.zB + t);
+                                    ptx::tma_load_3d_pair(sa + h * A_BYTES, &tmA, fb, kc, arow, job.zA + sA);
+                                    ptx::tma_load_3d_pair(sb, &tmB, fb, kc, brow, job.zB + sB);
                                 }
                             }
                             if (issued < STAGES) issued++;
@@ -397,7 +437,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             uint32_t dt = tmem;
             // Position in the group sequence: tile, slice group d, pair s, group g
             // of the pair (gpp groups per pair), groups in the open chunk.
-            int tile = cta0, d = p.d0, s = 0, g = 0, in_chunk = 0;
+            int tile = cta0, d = dbeg, s = 0, g = 0, in_chunk = 0;
             int gpp = tile < total_tiles ? entry_nkb<GROUPED>(p, items, work, tile) / GROUP_KB : 0;
             auto close_chunk = [&]() {
                 commit(&accf[abuf]);
@@ -436,11 +476,11 @@ __global__ void __launch_bounds__(THREADS, 1)
                 if (++in_chunk == kChunkKB / GROUP_KB) close_chunk();
                 if (++g == gpp) {
                     g = 0;
-                    if (++s > d) {
+                    if (++s == group_pairs<F64>(d)) {
                         s = 0;
                         if (in_chunk > 0) close_chunk(); // the slice group ends inside a chunk
                         if (++d == p.d1) {
-                            d = p.d0;
+                            d = dbeg;
                             tile += ctas;
                             if (tile >= total_tiles) return false;
                             gpp = entry_nkb<GROUPED>(p, items, work, tile) / GROUP_KB;
@@ -497,7 +537,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         // otherwise a batch is converted with one thread per row and transposed
         // through shared memory so that the read-modify-write of C runs along a
         // row.  colOff / colExp / rowOffW / rowOkW describe the pending tile.
-        long long *const rbc = p.rbuf + (size_t)blockIdx.x * kBM * kBN;
+        constexpr size_t kPlane = (size_t)kBM * kBN; // low sums, then (FP64 form) high sums
+        long long *const rbc = p.rbuf + (size_t)blockIdx.x * PLANES * kPlane;
         bool pend = false, pend_row_ok = false;
         bool pend_rows_fast = false; // C is contiguous along the rows: one thread per row stays coalesced
         const long long *pend_src = rbc; // the pending tile's sums (scratch, or the K slices' accumulator)
@@ -507,72 +548,72 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (pend && pend_rows_fast) {
                 if (pend_row_ok) {
                     const int64_t rowOff = rowOffW[lane];
-                    for (int c0 = pend_done; c0 < upto; c0 += kFinFast) {
-                        long long Rv[kFinFast];
-                        double old[kFinFast];
+                    for (int c0 = pend_done; c0 < upto; c0 += FF) {
+                        long long Rv[FF];
+                        double old[FF];
 #pragma unroll
-                        for (int i = 0; i < kFinFast; i++) Rv[i] = __ldcg(pend_src + (size_t)(col0 + c0 + i) * kBM + row);
+                        for (int i = 0; i < FF; i++) Rv[i] = __ldcg(pend_src + (size_t)(col0 + c0 + i) * kBM + row);
+                        long long Hv[F64 ? FF : 1];
+                        if constexpr (F64) {
+#pragma unroll
+                            for (int i = 0; i < FF; i++)
+                                Hv[i] = __ldcg(pend_src + kPlane + (size_t)(col0 + c0 + i) * kBM + row);
+                        }
                         if (!plain_store) {
 #pragma unroll
-                            for (int i = 0; i < kFinFast; i++)
+                            for (int i = 0; i < FF; i++)
                                 old[i] = colExp[c0 + i] != INT_MAX ? pend_C[rowOff + colOff[c0 + i]] : 0.0;
                         }
 #pragma unroll
-                        for (int i = 0; i < kFinFast; i++) {
+                        for (int i = 0; i < FF; i++) {
                             const int ce = colExp[c0 + i];
                             if (ce == INT_MAX) continue;
-                            long long R = Rv[i];
-                            if (p.ab_neg) R = -R;
-                            double v;
-                            if (pend_rowExp == INT_MIN || ce == INT_MIN)
-                                v = __longlong_as_double(0x7ff8000000000000ll);
-                            else
-                                v = int_times_pow2_rn(R, pend_rowExp + ce + p.shift_const);
-                            if (!p.ab_pow2) v *= p.ab;
+                            const double v = finish_value<F64>(p, Rv[i], F64 ? Hv[F64 ? i : 0] : 0, pend_rowExp, ce);
                             pend_C[rowOff + colOff[c0 + i]] =
                                 plain_store ? v : (cp_one ? old[i] + v : fma(p.cp, old[i], v));
                         }
                     }
                 }
             } else if (pend) {
-                for (int c0 = pend_done; c0 < upto; c0 += kFinCols) {
-                    // Both global reads of the batch -- the old C values (lanes kFinCols*r ..
-                    // kFinCols*r + kFinCols-1 take the batch's columns of row r) and the sums
+                for (int c0 = pend_done; c0 < upto; c0 += FC) {
+                    // Both global reads of the batch -- the old C values (lanes FC*r ..
+                    // FC*r + FC-1 take the batch's columns of row r) and the sums
                     // (one thread per row) -- are issued before either is used, so their
                     // latencies overlap instead of adding up.
-                    double old[kFinCols];
+                    double old[FC];
                     if (!plain_store) {
 #pragma unroll
-                        for (int k = 0; k < kFinCols; k++) {
-                            const int e = k * 32 + lane, r = e / kFinCols, c = e % kFinCols;
+                        for (int k = 0; k < FC; k++) {
+                            const int e = k * 32 + lane, r = e / FC, c = e % FC;
                             old[k] = (rowOkW[r] && colExp[c0 + c] != INT_MAX) ? pend_C[rowOffW[r] + colOff[c0 + c]] : 0.0;
                         }
                     }
-                    long long Rv[kFinCols];
+                    long long Rv[FC];
 #pragma unroll
-                    for (int i = 0; i < kFinCols; i++)
+                    for (int i = 0; i < FC; i++)
                         Rv[i] = (pend_row_ok && colExp[c0 + i] != INT_MAX)
                                     ? __ldcg(pend_src + (size_t)(col0 + c0 + i) * kBM + row)
                                     : 0ll;
+                    long long Hv[F64 ? FC : 1];
+                    if constexpr (F64) {
 #pragma unroll
-                    for (int i = 0; i < kFinCols; i++) {
+                        for (int i = 0; i < FC; i++)
+                            Hv[i] = (pend_row_ok && colExp[c0 + i] != INT_MAX)
+                                        ? __ldcg(pend_src + kPlane + (size_t)(col0 + c0 + i) * kBM + row)
+                                        : 0ll;
+                    }
+#pragma unroll
+                    for (int i = 0; i < FC; i++) {
                         const int ce = colExp[c0 + i];
                         double v = 0.0;
-                        if (pend_row_ok && ce != INT_MAX) {
-                            long long R = Rv[i];
-                            if (p.ab_neg) R = -R;
-                            if (pend_rowExp == INT_MIN || ce == INT_MIN)
-                                v = __longlong_as_double(0x7ff8000000000000ll);
-                            else
-                                v = int_times_pow2_rn(R, pend_rowExp + ce + p.shift_const);
-                            if (!p.ab_pow2) v *= p.ab;
-                        }
+                        if (pend_row_ok && ce != INT_MAX)
+                            v = finish_value<F64>(p, Rv[i], F64 ? Hv[F64 ? i : 0] : 0, pend_rowExp, ce);
                         finT[i * FIN_T + lane] = v;
                     }
                     __syncwarp();
 #pragma unroll
-                    for (int k = 0; k < kFinCols; k++) {
-                        const int e = k * 32 + lane, r = e / kFinCols, c = e % kFinCols;
+                    for (int k = 0; k < FC; k++) {
+                        const int e = k * 32 + lane, r = e / FC, c = e % FC;
                         if (rowOkW[r] && colExp[c0 + c] != INT_MAX) {
                             const double v = finT[c * FIN_T + r];
                             pend_C[rowOffW[r] + colOff[c0 + c]] =
@@ -599,8 +640,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             for (int i = 0; i < kBN / 2; i++) L[i] = 0;
             bool hvalid = false; // H holds a part of the sum (else it reads as 0)
             int since_fold = 0;
-            for (int d = p.d0; d < p.d1 && ok; d++) {
-                const int kbs = (d + 1) * nkb;
+            bool bad = false; // FP64 form: the check of this warp's outputs failed
+            for (int d = dbeg; d < p.d1 && ok; d++) {
+                const int kbs = group_pairs<F64>(d) * nkb;
                 for (int c0 = 0; c0 < kbs; c0 += kChunkKB) {
                     const long long tw = (p.prof && ew == 0 && lane == 0) ? clock64() : 0;
                     bool w = ptx::mbar_wait(&accf[abuf], aphase, p.timeout_ns, abort_flag);
@@ -635,8 +677,28 @@ __global__ void __launch_bounds__(THREADS, 1)
                     // with the Horner step R *= 256 before the next one; after the last
                     // slice group H holds the tile's sums and L is free.
                     const bool group_end = c0 + kChunkKB >= kbs;
-                    const bool shift = group_end && d + 1 < p.d1;
-                    if (++since_fold == 64 || group_end) {
+                    const bool high_end = F64 && group_end && d + 1 == p.hid; // the high sums are complete
+                    const bool shift = group_end && d + 1 < p.d1 && !high_end;
+                    if (F64 && d < 0) {
+                        if (group_end) { // a negative margin anywhere: the FMA kernel takes this warp's outputs
+                            int worst = 0;
+#pragma unroll
+                            for (int i = 0; i < kBN / 2; i++) {
+                                worst = min(worst, L[i]);
+                                L[i] = 0;
+                            }
+                            bad = __any_sync(0xffffffffu, worst < 0);
+                        }
+                    } else if (++since_fold == 64 || group_end) {
+                        long long *dst_hi = nullptr;
+                        bool add_hi = false;
+                        if (high_end) {
+                            // the pending tile's high sums leave the scratch before this tile's enter it
+                            if (pend_done < kBN / 2) finalize_cols(kBN / 2);
+                            const TileJob jh = resolve<GROUPED, CL>(p, items, work, tile, rank);
+                            add_hi = jh.split;
+                            dst_hi = add_hi ? p.racc + ((size_t)jh.tid * PLANES + 1) * kPlane : rbc + kPlane;
+                        }
 #pragma unroll
                         for (int cc = 0; cc < kBN / 16; cc++) {
                             const uint32_t col = (uint32_t)(col0 + cc * 8);
@@ -655,16 +717,28 @@ __global__ void __launch_bounds__(THREADS, 1)
                                 hi[i] = (uint32_t)((unsigned long long)H >> 32);
                                 L[cc * 8 + i] = 0;
                             }
-                            ptx::tmem_st8(tl + 256u + col, lo);
-                            ptx::tmem_st8(tl + 384u + col, hi);
-                            ptx::tmem_wait_st();
+                            if (high_end) {
+#pragma unroll
+                                for (int i = 0; i < 8; i++) {
+                                    long long *at = dst_hi + (size_t)(col + i) * kBM + row;
+                                    const unsigned long long H = ((unsigned long long)hi[i] << 32) | lo[i];
+                                    if (add_hi)
+                                        atomicAdd((unsigned long long *)at, H);
+                                    else
+                                        *at = (long long)H;
+                                }
+                            } else {
+                                ptx::tmem_st8(tl + 256u + col, lo);
+                                ptx::tmem_st8(tl + 384u + col, hi);
+                                ptx::tmem_wait_st();
+                            }
                         }
-                        hvalid = true;
+                        hvalid = !high_end;
                         since_fold = 0;
                     }
                     if (p.prof && ew == 0 && lane == 0) prof_add(p, kProfEpiFlush, clock64() - tw1);
                     // a slice of the pending tile while the MMAs run
-                    if (pend_done < kBN / 2) finalize_cols(pend_done + (pend_rows_fast ? kFinFast : kFinCols));
+                    if (pend_done < kBN / 2) finalize_cols(pend_done + (pend_rows_fast ? FF : FC));
                 }
             }
             if (!ok) break;
@@ -686,15 +760,15 @@ __global__ void __launch_bounds__(THREADS, 1)
             int rowExp = 0;
             if (row_ok) {
                 int64_t oa, ob;
-                group_offsets32(*job.mg, (uint32_t)m, oa, ob, rowOff);
+                group_offsets32(*job.mg, (uint32_t)(GROUPED ? m : p.m0 + m), oa, ob, rowOff);
                 rowExp = job.eA[m];
             }
             // Short-K tiles (few chunks: the deferred finishing would run longer than
             // the next tile's MMAs) are finished here, straight from TMEM.
-            const bool direct = p.ksplit == 1 && nkb <= kDirectKB;
+            const bool direct = !F64 && !job.split && nkb <= kDirectKB;
             // K slices add their sums into the tile's accumulator; only the last
             // one to arrive at this warp's region finishes it
-            long long *const dst = p.ksplit > 1 ? p.racc + (size_t)job.tid * kBM * kBN : rbc;
+            long long *const dst = job.split ? p.racc + (size_t)job.tid * PLANES * kPlane : rbc;
 #pragma unroll 1
             for (int cc = 0; cc < kBN / 32 && !direct; cc++) {
                 const uint32_t col = (uint32_t)(col0 + cc * 16);
@@ -706,7 +780,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 for (int i = 0; i < 16; i++) {
                     const unsigned long long R = ((unsigned long long)hi[i] << 32) | lo[i];
                     long long *q = dst + (size_t)(col0 + cc * 16 + i) * kBM + row;
-                    if (p.ksplit > 1)
+                    if (job.split)
                         atomicAdd((unsigned long long *)q, R); // two's complement: exact for signed sums
                     else
                         *q = (long long)R;
@@ -714,20 +788,34 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
             ptx::tc_fence_before();
             bool finish = true;
-            if (p.ksplit > 1) {
+            if (job.split) {
                 __threadfence();
                 __syncwarp();
                 int last = 0;
-                if (lane == 0) last = atomicAdd(p.rcnt + job.tid * 8 + ew, 1) == p.ksplit - 1;
-                finish = __shfl_sync(0xffffffffu, last, 0) != 0;
+                if (lane == 0) {
+                    // arrivals in the low half, failed checks above them
+                    const int old = atomicAdd(p.rcnt + job.tid * 8 + ew, bad ? 0x10001 : 1);
+                    last = (old & 0xffff) == p.ksplit - 1;
+                    if (F64 && last && (old >> 16)) last = 2;
+                }
+                last = __shfl_sync(0xffffffffu, last, 0);
+                finish = last != 0;
+                if (F64 && last == 2) bad = true;
                 if (finish) __threadfence();
+            }
+            if (F64 && finish && bad) {
+                finish = false;
+                if (lane == 0) {
+                    const int at = atomicAdd(p.redo_count, 1);
+                    p.redo[at] = make_int4(job.b, (int)p.m0 + job.mt * kBM + q * 32, (int)p.n0 + job.nt * kBN + col0, 0);
+                }
             }
             for (int i = lane; i < kBN / 2; i += 32) {
                 const int64_t n = (int64_t)job.nt * kBN + col0 + i;
                 int64_t oa, ob, oc = 0;
                 int ex = INT_MAX; // marks a column beyond N
                 if (n < job.N) {
-                    group_offsets32(*job.ng, (uint32_t)n, oa, ob, oc);
+                    group_offsets32(*job.ng, (uint32_t)(GROUPED ? n : p.n0 + n), oa, ob, oc);
                     ex = job.eB[n];
                 }
                 colOff[i] = oc;
@@ -899,14 +987,17 @@ eg_status ensure_tc_attributes() {
     static std::once_flag once;
     static cudaError_t err = cudaSuccess;
     std::call_once(once, [] {
-        err = cudaFuncSetAttribute(k_tc_split_gemm<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        err = cudaFuncSetAttribute(k_tc_split_gemm<false, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    Ring<1>::SMEM_BYTES);
         if (err == cudaSuccess)
-            err = cudaFuncSetAttribute(k_tc_split_gemm<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            err = cudaFuncSetAttribute(k_tc_split_gemm<true, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        Ring<1>::SMEM_BYTES);
         if (err == cudaSuccess)
-            err = cudaFuncSetAttribute(k_tc_split_gemm<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            err = cudaFuncSetAttribute(k_tc_split_gemm<false, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        Ring<2>::SMEM_BYTES);
+        if (err == cudaSuccess)
+            err = cudaFuncSetAttribute(k_tc_split_gemm<false, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       Ring<1>::SMEM_BYTES);
     });
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(k_tc_split_gemm)");
     return EG_SUCCESS;
@@ -941,7 +1032,7 @@ int tc_pair_clusters() {
         cudaLaunchAttribute attr;
         cudaLaunchConfig_t cfg = pair_config(num_sms(), nullptr, &attr);
         int c = 0;
-        if (cudaOccupancyMaxActiveClusters(&c, (void *)k_tc_split_gemm<false, 2>, &cfg) == cudaSuccess) n = c;
+        if (cudaOccupancyMaxActiveClusters(&c, (void *)k_tc_split_gemm<false, 2, false>, &cfg) == cudaSuccess) n = c;
         cudaGetLastError();
     });
     return n;
@@ -953,7 +1044,7 @@ eg_status launch_tc_gemm(const CUtensorMap &tmA, const CUtensorMap &tmB, const T
     if (p.pair) {
         const int clusters = tc_pair_clusters();
         if (clusters < 1) return fail(EG_ERROR_CUDA, "k_tc_split_gemm: CTA pairs are not available");
-        const int total = p.nbatch * ((p.mtiles + 1) / 2) * p.ntiles * p.ksplit;
+        const int total = p.t0 + (p.nbatch * ((p.mtiles + 1) / 2) * p.ntiles - p.t0) * p.ksplit;
         if (total <= 0) return EG_SUCCESS;
         const int grid = 2 * (total < clusters ? total : clusters);
         cudaLaunchAttribute attr;
@@ -962,17 +1053,20 @@ eg_status launch_tc_gemm(const CUtensorMap &tmA, const CUtensorMap &tmB, const T
             LaunchScope ls_("k_tc_split_gemm", s);
             const TcItem *no_items = nullptr;
             const int4 *no_work = nullptr;
-            EG_CUDA(cudaLaunchKernelEx(&cfg, k_tc_split_gemm<false, 2>, tmA, tmB, p, no_items, no_work, 0));
+            EG_CUDA(cudaLaunchKernelEx(&cfg, k_tc_split_gemm<false, 2, false>, tmA, tmB, p, no_items, no_work, 0));
         }
         EG_CHECK_LAUNCH("k_tc_split_gemm");
         return EG_SUCCESS;
     }
-    const int total = p.nbatch * p.mtiles * p.ntiles * p.ksplit;
+    const int total = p.t0 + (p.nbatch * p.mtiles * p.ntiles - p.t0) * p.ksplit;
     if (total <= 0) return EG_SUCCESS;
     const int grid = total < num_sms() ? total : num_sms();
     {
-        LaunchScope ls_("k_tc_split_gemm", s);
-        k_tc_split_gemm<false, 1><<<grid, THREADS, Ring<1>::SMEM_BYTES, s>>>(tmA, tmB, p, nullptr, nullptr, 0);
+        LaunchScope ls_(p.redo ? "k_tc_split_gemm_f64" : "k_tc_split_gemm", s);
+        if (p.redo)
+            k_tc_split_gemm<false, 1, true><<<grid, THREADS, Ring<1>::SMEM_BYTES, s>>>(tmA, tmB, p, nullptr, nullptr, 0);
+        else
+            k_tc_split_gemm<false, 1, false><<<grid, THREADS, Ring<1>::SMEM_BYTES, s>>>(tmA, tmB, p, nullptr, nullptr, 0);
     }
     EG_CHECK_LAUNCH("k_tc_split_gemm");
     return EG_SUCCESS;
@@ -986,7 +1080,7 @@ eg_status launch_tc_gemm_grouped(const CUtensorMap &tmA, const CUtensorMap &tmB,
     const int grid = ntiles_total < num_sms() ? ntiles_total : num_sms();
     {
         LaunchScope ls_("k_tc_split_gemm_grouped", s);
-        k_tc_split_gemm<true, 1><<<grid, THREADS, Ring<1>::SMEM_BYTES, s>>>(tmA, tmB, p, items, work, ntiles_total);
+        k_tc_split_gemm<true, 1, false><<<grid, THREADS, Ring<1>::SMEM_BYTES, s>>>(tmA, tmB, p, items, work, ntiles_total);
     }
     EG_CHECK_LAUNCH("k_tc_split_gemm_grouped");
     return EG_SUCCESS;
