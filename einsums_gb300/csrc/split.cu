@@ -508,39 +508,53 @@ static void set_ab(split::TcGemmParams &p, double ab) {
     if (p.ab_pow2) p.shift_const += k - 1;
 }
 
-// Which tiles of a launch are cut along K, and how often: the whole rounds of the
-// CTAs run whole tiles; the tiles left over for the last round -- 20 of 324 on 152
-// SMs, a third of the time -- are cut into as many slices of at least two K blocks
-// as give the smallest estimated time.  The estimate counts clocks: 440 per K block
-// of a slice pair, 6000 for a tile's epilogue, 8000 more for adding a slice's sums to
-// its accumulator and 60 per accumulator plane to clear it.  Returns the clocks.
-static double choose_schedule(split::TcGemmParams &p, int64_t units, int64_t workers, int pairs, int planes) {
+// Single CTAs or CTA pairs, which tiles of a launch are cut along K, and how often:
+// the whole rounds of the CTAs run whole tiles; the tiles left over for the last
+// round -- 20 of 324 on 152 SMs, a third of the time -- are cut into as many slices
+// of at least two K blocks as give the smallest estimated time.  The estimate counts
+// clocks: 360 per K block of a slice pair (320 on CTA pairs, which need two row
+// tiles), 6000 for a tile's epilogue, 8000 more for adding a slice's sums to its
+// accumulator and 60 per accumulator plane to clear it.  Returns the clocks.
+static double choose_schedule(split::TcGemmParams &p, int64_t nb, int64_t mtiles, int64_t ntiles, int pairs,
+                              int planes) {
     using namespace split;
-    auto entry = [&](int64_t kb) { return 440.0 * pairs * (double)kb + 6000.0; };
-    const int64_t rounds = units / workers, rem = units - rounds * workers;
-    p.t0 = (int)units;
-    p.ksplit = 1;
-    p.kslice = p.nkb;
-    const double whole = (double)rounds * entry(p.nkb);
-    double best = whole + (rem ? entry(p.nkb) : 0.0);
-    if (rem == 0) return best;
-    const int64_t unit = kKStep / kBK;
-    int64_t last = 0;
-    for (int64_t ks = 2; ks <= std::min<int64_t>(p.nkb / unit, 64); ks++) {
-        const int64_t slice = round_up((p.nkb + ks - 1) / ks, unit);
-        const int64_t n = (p.nkb + slice - 1) / slice; // slices actually used
-        if (n == last) continue;
-        last = n;
-        const int64_t r = (rem * n + workers - 1) / workers;
-        const double t = whole + (double)r * (entry(slice) + 8000.0) + 60.0 * (double)(rem * planes);
-        if (t < 0.98 * best) {
+    double best = -1.0;
+    const int clusters = mtiles >= 2 ? tc_pair_clusters() : 0;
+    for (int cl = clusters > 0 && tc_pairs_forced() ? 2 : 1; cl <= (clusters > 0 ? 2 : 1); cl++) {
+        const int64_t units = nb * ((mtiles + cl - 1) / cl) * ntiles, workers = cl == 2 ? clusters : num_sms();
+        auto entry = [&](int64_t kb) { return (cl == 2 ? 320.0 : 360.0) * pairs * (double)kb + 6000.0; };
+        const int64_t rounds = units / workers, rem = units - rounds * workers;
+        const double whole = (double)rounds * entry(p.nkb);
+        auto offer = [&](double t, int64_t t0, int64_t ks, int64_t slice, double margin) {
+            if (best >= 0.0 && t >= margin * best) return;
             best = t;
-            p.t0 = (int)(rounds * workers);
-            p.ksplit = (int)n;
+            p.pair = cl - 1;
+            p.t0 = (int)t0;
+            p.ksplit = (int)ks;
             p.kslice = (int)slice;
+        };
+        offer(whole + (rem ? entry(p.nkb) : 0.0), units, 1, p.nkb, 1.0);
+        if (rem == 0) continue;
+        const int64_t unit = kKStep / kBK;
+        int64_t last = 0;
+        for (int64_t ks = 2; ks <= std::min<int64_t>(p.nkb / unit, 64); ks++) {
+            const int64_t slice = round_up((p.nkb + ks - 1) / ks, unit);
+            const int64_t n = (p.nkb + slice - 1) / slice; // slices actually used
+            if (n == last) continue;
+            last = n;
+            const int64_t r = (rem * n + workers - 1) / workers;
+            offer(whole + (double)r * (entry(slice) + 8000.0) + 60.0 * (double)(rem * cl * planes), rounds * workers, n,
+                  slice, 0.98);
         }
     }
     return best;
+}
+
+// The accumulators of the tiles cut along K in a launch of choose_schedule (at most
+// one per SM).
+static int64_t cut_tiles(const split::TcGemmParams &p, int64_t nb, int64_t mtiles, int64_t ntiles) {
+    const int cl = p.pair ? 2 : 1;
+    return p.ksplit > 1 ? (nb * ((mtiles + cl - 1) / cl) * ntiles - p.t0) * cl : 0;
 }
 
 eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s, eg_split_report *rep) {
@@ -565,16 +579,12 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     const size_t offTab = offR + rbuf_bytes();
     const size_t tabBytes = tables ? (size_t)(M + N + 2 * K) * 8 : 0;
     const int64_t tiles = nb * (Mp / kBM) * (Np / kBN);
-    // CTA pairs (256x128 tiles) whenever the output has two or more row tiles
-    const int clusters = Mp / kBM >= 2 ? tc_pair_clusters() : 0;
-    const bool pair = clusters > 0;
     const size_t offRacc = round_up((int64_t)(offTab + tabBytes), 256);
-    // accumulators of the tiles cut along K: fewer than the SMs (CTA pairs cut whole
-    // launches, of fewer tiles than half the SMs)
-    const size_t cut = (size_t)std::min<int64_t>(tiles, num_sms());
+    // accumulators of the tiles cut along K: at most one per SM
+    const size_t cut = (size_t)std::min<int64_t>(2 * tiles, num_sms());
     const size_t raccBytes = cut * kBM * kBN * 8;
     const size_t offRcnt = offRacc + raccBytes;
-    const size_t rcntBytes = cut * 8 * sizeof(int);
+    const size_t rcntBytes = cut * kTileRegions * sizeof(int);
     const size_t total = offRcnt + rcntBytes;
     void *ws = nullptr;
     eg_status st = workspace(s, total, &ws);
@@ -594,12 +604,12 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
                             tables ? tab + M + K + N : nullptr)) != EG_SUCCESS)
         return st;
 
-    CUtensorMap tmA, tmB;
+    CUtensorMap tmA, tmB, tmBh;
     if ((st = encode_planes(&tmA, planesA, Kp, Mp, nb * S)) != EG_SUCCESS) return st;
-    if ((st = encode_planes(&tmB, planesB, Kp, Np, nb * S, pair ? kBN / 2 : kBN)) != EG_SUCCESS) return st;
+    if ((st = encode_planes(&tmB, planesB, Kp, Np, nb * S)) != EG_SUCCESS) return st;
+    if ((st = encode_planes(&tmBh, planesB, Kp, Np, nb * S, kBN / 2)) != EG_SUCCESS) return st;
 
     TcGemmParams p{};
-    p.pair = pair ? 1 : 0;
     p.S = S;
     p.planes = S;
     p.mtiles = (int)(Mp / kBM);
@@ -650,19 +660,10 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
             p.nkb = (int)std::min<int64_t>(kb_per_pass, nkb_total - kb0);
             int pairs = 0;
             for (int d = p.d0; d < p.d1; d++) pairs += d + 1;
-            // schedule units: tiles over SMs, or pair tiles over CTA pairs
-            const int64_t units = pair ? nb * ((Mp / kBM + 1) / 2) * (Np / kBN) : tiles;
-            if (pair && units >= clusters / 2) {
-                p.t0 = (int)units;
-                p.ksplit = 1;
-                p.kslice = p.nkb;
-            } else {
-                choose_schedule(p, units, pair ? clusters : num_sms(), pairs, 1);
-            }
-            if (p.ksplit > 1) {
-                const size_t n = (size_t)(pair ? tiles : units - p.t0);
+            choose_schedule(p, nb, p.mtiles, p.ntiles, pairs, 1);
+            if (const size_t n = (size_t)cut_tiles(p, nb, p.mtiles, p.ntiles)) {
                 EG_CUDA(cudaMemsetAsync(p.racc, 0, n * kBM * kBN * 8, s));
-                EG_CUDA(cudaMemsetAsync(p.rcnt, 0, n * 8 * sizeof(int), s));
+                EG_CUDA(cudaMemsetAsync(p.rcnt, 0, n * kTileRegions * sizeof(int), s));
             }
             const bool first = first_launch;
             first_launch = false;
@@ -676,7 +677,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
                 EG_CUDA(cudaMemsetAsync(prof, 0, (size_t)num_sms() * 8 * sizeof(unsigned long long), s));
             }
             p.prof = prof;
-            if ((st = launch_tc_gemm(tmA, tmB, p, s)) != EG_SUCCESS) return st;
+            if ((st = launch_tc_gemm(tmA, tmB, tmBh, p, s)) != EG_SUCCESS) return st;
             if (prof) {
                 // Per-role wait/busy cycles summed over CTAs (a tracing aid, off by default).
                 std::vector<unsigned long long> h((size_t)num_sms() * 8);
@@ -759,7 +760,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
         bb = std::min<int64_t>(bb, (int64_t(1) << 20) / P);
     }
     const int64_t tiles = bb * (mb / kBM) * (nbk / kBN);
-    const int64_t cut = std::min<int64_t>(tiles, num_sms()); // tiles cut along K, at most
+    const int64_t cut = std::min<int64_t>(2 * tiles, num_sms()); // tiles cut along K, at most
     const int64_t all_tiles = nb * (Mp_all / kBM) * (Np_all / kBN);
     const bool tables = M + K <= (int64_t(1) << 22) && N + K <= (int64_t(1) << 22);
     size_t at = 0;
@@ -770,12 +771,12 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
     };
     const size_t oPA = take((size_t)bb * P * mb * Kp * 2), oPB = take((size_t)bb * P * nbk * Kp * 2);
     const size_t oMax = take((size_t)bb * (mb + nbk) * 8); // cleared for every panel pair ...
-    const size_t oCnt = take((size_t)cut * 8 * sizeof(int)); // (with the accumulators' arrivals
+    const size_t oCnt = take((size_t)cut * kTileRegions * sizeof(int)); // (with the accumulators' arrivals
     const size_t oAcc = take((size_t)cut * 2 * kBM * kBN * 8); //  and those that the launch uses)
     const size_t oExp = take((size_t)bb * (mb + nbk) * 4);
     const size_t oTab = take(tables ? (size_t)(M + N + 2 * K) * 8 : 0);
-    const size_t oR = take(rbuf_bytes(2));
-    const size_t oRedoN = take(sizeof(int)), oRedo = take((size_t)all_tiles * 8 * sizeof(int4));
+    const size_t oR = take(rbuf_bytes(3));
+    const size_t oRedoN = take(sizeof(int)), oRedo = take((size_t)all_tiles * kTileRegions * sizeof(int4));
     ScratchLease lease(s, at);
     if (!lease.ptr()) return EG_ERROR_NOT_SUPPORTED;
     int *status = nullptr;
@@ -819,8 +820,8 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
             for (int64_t n0 = 0; n0 < N; n0 += nbk) {
                 const int64_t nc = std::min(nbk, N - n0), Np = round_up(nc, kBN);
                 p.nkb = (int)(Kp / kBK);
-                choose_schedule(p, nbc * (Mp / kBM) * (Np / kBN), num_sms(), S * (S + 1) / 2 + 2, 2);
-                const size_t used = p.ksplit > 1 ? (size_t)(nbc * (Mp / kBM) * (Np / kBN) - p.t0) * 2 * kBM * kBN * 8 : 0;
+                choose_schedule(p, nbc, Mp / kBM, Np / kBN, S * (S + 1) / 2 + 2, 2);
+                const size_t used = (size_t)cut_tiles(p, nbc, Mp / kBM, Np / kBN) * 2 * kBM * kBN * 8;
                 EG_CUDA(cudaMemsetAsync(maxA, 0, oAcc - oMax + used, s));
                 OperandMap oa{c.batch, c.m, c.k, 0, mc, Mp, K, Kp, (int)nbc};
                 oa.b0 = b0;
@@ -836,9 +837,10 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
                     (st = split_operand(ob, c.B, maxB, eB, planesB, S, s, tables ? tab + M + K : nullptr,
                                         tables ? tab + M + K + N : nullptr, true)) != EG_SUCCESS)
                     return st;
-                CUtensorMap tmA, tmB;
+                CUtensorMap tmA, tmB, tmBh;
                 if ((st = encode_planes(&tmA, planesA, Kp, Mp, nbc * P)) != EG_SUCCESS) return st;
                 if ((st = encode_planes(&tmB, planesB, Kp, Np, nbc * P)) != EG_SUCCESS) return st;
+                if ((st = encode_planes(&tmBh, planesB, Kp, Np, nbc * P, kBN / 2)) != EG_SUCCESS) return st;
                 p.b0 = b0;
                 p.m0 = m0;
                 p.n0 = n0;
@@ -849,7 +851,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
                 p.mtiles = (int)(Mp / kBM);
                 p.ntiles = (int)(Np / kBN);
                 p.nbatch = (int)nbc;
-                if ((st = launch_tc_gemm(tmA, tmB, p, s)) != EG_SUCCESS) return st;
+                if ((st = launch_tc_gemm(tmA, tmB, tmBh, p, s)) != EG_SUCCESS) return st;
             }
         }
     }
@@ -870,9 +872,9 @@ bool f64_tensor_pays(const Contraction &c) {
     if (fma < 40e-6) return false;
     TcGemmParams p{};
     p.nkb = (int)(round_up(K, kKStep) / kBK);
-    const int64_t tiles = nb * (round_up(M, kBM) / kBM) * (round_up(N, kBN) / kBN);
-    if (tiles > (int64_t(1) << 30)) return false;
-    const double clocks = choose_schedule(p, tiles, num_sms(), kF64Slices * (kF64Slices + 1) / 2 + 2, 2);
+    const int64_t mtiles = round_up(M, kBM) / kBM, ntiles = round_up(N, kBN) / kBN;
+    if (nb * mtiles * ntiles > (int64_t(1) << 30)) return false;
+    const double clocks = choose_schedule(p, nb, mtiles, ntiles, kF64Slices * (kF64Slices + 1) / 2 + 2, 2);
     const double tensor = 30e-6 + (double)nb * (double)(M + N) * (double)K * 36.0 / 3e12 + clocks / 1.9e9;
     return tensor < 0.9 * fma;
 }

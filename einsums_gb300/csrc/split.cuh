@@ -35,6 +35,7 @@ constexpr int kBM = 128, kBN = 128, kBK = 64;
 // accuracy check of launch_f64_tensor.
 constexpr int kF64Slices = 8, kF64High = 4;
 constexpr float kCheckA = 4.0f, kCheckB = -5.0f;
+constexpr int kTileRegions = 8; // 32 x 64 blocks of a tile, one per epilogue warp
 constexpr int kChunkKB = 16;    // 16 x 64 = 1024 products per exact FP32 chunk
 constexpr int kKStep = 2 * kBK;  // K is padded to whole groups of two K blocks
 
@@ -59,8 +60,8 @@ struct TcGemmParams {
     unsigned long long timeout_ns;
     // Optional per-CTA cycle counters (null in normal runs): see kProf* in tc_gemm.cu.
     unsigned long long *prof;
-    // Per-CTA scratch of gridDim.x * 128 * 128 int64: a finished tile's sums
-    // wait here until the epilogue converts them during the next tile.
+    // Per-CTA scratch of gridDim.x * 128 * 128 int64, where a finished tile's sums wait
+    // (in the FP64 form three such planes: the low sums, and the high sums of two tiles).
     long long *rbuf;
     // The first t0 schedule entries are whole tiles.  The tiles left for the last,
     // partly filled round of the CTAs (all of them when there are fewer tiles than
@@ -70,14 +71,13 @@ struct TcGemmParams {
     // ([tile - t0][128 columns][128 rows], two planes in the FP64 form) and the last
     // slice to arrive at a region of an epilogue warp (counted in rcnt,
     // [tile - t0][8]) finishes it.  Both are zeroed by the host before the launch;
-    // unused when t0 is the number of tiles.  (CTA pairs number the accumulators by
-    // output tile.)
+    // unused when t0 is the number of tiles.  (With CTA pairs an entry is two tiles,
+    // and so has two accumulators.)
     int t0;
     int ksplit, kslice;
     long long *racc;
     int *rcnt;
-    // Launch as CTA pairs (cta_group::2, 256x128 tiles; B's tensor map has
-    // 64-row boxes): single contractions only.
+    // Launch as CTA pairs (cta_group::2, 256x128 tiles): single contractions only.
     int pair;
     // Slice groups d0 <= d < d1 (anti-diagonals s + t = d of the digit pairs)
     // summed by this launch: all of them (0, S) unless a long K is split into
@@ -140,68 +140,68 @@ __device__ __forceinline__ long long scaled_round(double x, int sh) {
     return (bits >> 63) ? -(long long)q : (long long)q;
 }
 
-__device__ __forceinline__ double scale_pow2(double v, int e) {
-    if (v == 0.0) return v;
-    const long long bits = __double_as_longlong(v);
-    const int ex = (int)((bits >> 52) & 0x7ff);
-    const int ne = ex + e;
-    if (ex != 0 && ne > 0 && ne < 2047) return __longlong_as_double(bits + ((long long)e << 52));
-    return scalbn(v, e);
-}
-
-// R * 2^e rounded to nearest (ties to even), built with integer operations so
-// the FP64 pipe -- about 1.75 operations per clock per SM on this GPU -- is
-// left for the one fused multiply-add with C.  Falls back to the FP64 path
-// when the result would not be a normal number.
-__device__ __forceinline__ double int_times_pow2_rn64(unsigned long long a, bool neg, int e) {
-    if (a == 0) return 0.0;
+// |sum| * 2^e rounded to nearest (ties to even), built with integer operations so the
+// FP64 pipe -- about 1.75 operations per clock per SM on this GPU -- is left for
+// the one fused multiply-add with C.  x holds the leading one at bit 63 (or is 0),
+// its value x 2^(e - lz); the bits below its lowest are known to be zero or only
+// break ties (they are or-ed into bit 0).
+//   FAST: e lies in [kFastMin, kFastMax], so the result is a normal number;
+//   otherwise one rounding also where the result is subnormal, and infinity beyond
+//   the largest number -- with no floating-point fallback, which the compiler would
+//   run for every element beside the integer path.
+constexpr int kFastMin = -1000, kFastMax = 900; // sums have up to 96 bits
+template <bool FAST>
+__device__ __forceinline__ double pack_rn(unsigned long long x, int lz, bool neg, int e) {
+    const int biased = 1086 - lz + e; // exponent field of the leading one
     const unsigned long long sign = neg ? 0x8000000000000000ull : 0ull;
-    const int lz = __clzll((long long)a);
-    const unsigned long long x = a << lz;      // leading one at bit 63
-    unsigned long long mant = x >> 11;         // 53 bits, leading one at bit 52
-    const unsigned long long rem = x & 0x7FFull;
-    if (rem > 0x400ull || (rem == 0x400ull && (mant & 1ull))) mant++;
-    int exp = 63 - lz + e;
-    if (mant >> 53) {
-        mant >>= 1;
-        exp++;
+    unsigned long long bits;
+    if constexpr (FAST) {
+        const uint32_t low = (uint32_t)x;
+        const uint32_t up = (low & 0x7FFu) + ((low >> 11) & 1u) > 0x400u ? 1u : 0u;
+        // the leading one of the 53-bit mantissa carries into the exponent field
+        bits = ((unsigned long long)(uint32_t)(biased - 1) << 52) + (x >> 11) + up;
+    } else {
+        const int drop = 11 + (biased > 0 ? 0 : min(1 - biased, 54)); // fewer bits below the smallest normal number
+        const int r = min(drop, 63);
+        unsigned long long mant = x >> r;
+        const unsigned long long rem = x << (64 - r); // the dropped bits, the half at bit 63
+        const unsigned long long half = 0x8000000000000000ull;
+        mant += (rem > half || (rem == half && (mant & 1ull))) ? 1ull : 0ull;
+        if (drop > 63) mant = drop == 64 && x > half ? 1ull : 0ull; // at most half of the smallest subnormal
+        bits = ((unsigned long long)(biased > 0 ? biased - 1 : 0) << 52) + mant;
+        if (biased > 2047) bits = 0x7FF0000000000000ull;
+        bits = min(bits, 0x7FF0000000000000ull);
     }
-    const int biased = exp + 1023;
-    if (biased <= 0 || biased >= 2047) {
-        const double v = scale_pow2(__ull2double_rn(a), e);
-        return neg ? -v : v;
-    }
-    return __longlong_as_double((long long)(sign | ((unsigned long long)biased << 52) | (mant & 0xFFFFFFFFFFFFFull)));
+    return x ? __longlong_as_double((long long)(bits | sign)) : 0.0;
 }
 
+template <bool FAST = false>
 __device__ __forceinline__ double int_times_pow2_rn(long long R, int e) {
-    return int_times_pow2_rn64(R < 0 ? (unsigned long long)(-R) : (unsigned long long)R, R < 0, e);
+    const unsigned long long a = R < 0 ? (unsigned long long)(-R) : (unsigned long long)R;
+    const int lz = __clzll((long long)a);
+    return pack_rn<FAST>(a << (lz & 63), lz, R < 0, e);
 }
 
-// The same for a 128-bit integer.
-__device__ __forceinline__ double int128_times_pow2_rn(__int128 R, int e) {
-    const bool neg = R < 0;
-    const unsigned __int128 a = neg ? (unsigned __int128)(-R) : (unsigned __int128)R;
-    unsigned long long hi = (unsigned long long)(a >> 64), lo = (unsigned long long)a;
-    if (hi == 0) return int_times_pow2_rn64(lo, neg, e);
-    const int lz = __clzll((long long)hi); // below 64
-    const unsigned long long x = lz ? (hi << lz) | (lo >> (64 - lz)) : hi; // leading one at bit 63
-    const bool sticky = (lo << lz) != 0;
-    return int_times_pow2_rn64(x | (sticky ? 1ull : 0ull), neg, e + 64 - lz); // the lowest bit only breaks ties
-}
-
-// Balanced base-256 digits of x * 2^(7 + 8(S-1) - e) rounded to an integer,
-// most significant first: dig[0] in [-128, 128], the others in [-127, 128].
-__device__ __forceinline__ void to_digits(double x, int e, int S, int *dig) {
-    long long F = scaled_round(x, kTopBits + kBits * (S - 1) - e);
-#pragma unroll
-    for (int s = S - 1; s >= 1; s--) {
-        int d = (int)(F & 255);
-        if (d > 128) d -= 256;
-        dig[s] = d;
-        F = (F - d) >> 8; // exact: F - d is a multiple of 256
+// The same for the exact sum (hi 2^32 + lo), negated if neg; |hi| < 2^62.
+template <bool FAST>
+__device__ __forceinline__ double words_times_pow2_rn(long long hi, long long lo, bool neg, int e) {
+    hi += lo >> 32;
+    uint32_t w = (uint32_t)lo; // the sum is hi 2^32 + w
+    const bool minus = hi < 0;
+    if (minus) {
+        hi = ~hi + (w == 0 ? 1 : 0);
+        w = 0u - w;
     }
-    dig[0] = (int)F;
+    if (hi == 0) {
+        hi = w;
+        w = 0;
+        e -= 32;
+    }
+    const int lz = __clzll(hi);
+    const unsigned long long below = (unsigned long long)w << 32;
+    const unsigned long long x = ((unsigned long long)hi << (lz & 63)) | (lz > 0 && lz < 64 ? below >> (64 - lz) : 0ull) |
+                                 ((below << (lz & 63)) != 0 ? 1ull : 0ull);
+    return pack_rn<FAST>(x, lz, minus != neg, e + 32);
 }
 
 // The leading digit: G >> 8(S-1), except that with eight slices G = F + bias may
@@ -265,10 +265,14 @@ __device__ __forceinline__ uint32_t check_mark(double x0, double x1, float mark)
 
 // Sets the kernels' shared-memory attribute once (call outside stream capture).
 eg_status ensure_tc_attributes();
-// Clusters of two k_tc_split_gemm CTAs that fit on the GPU at once, when CTA
-// pairs are requested with EINSUMS_GB300_TC_PAIRS=1 (else 0: single-CTA tiles).
+// Clusters of two k_tc_split_gemm CTAs that fit on the GPU at once (0 when CTA pairs
+// are switched off with EINSUMS_GB300_TC_PAIRS=0), and whether they are asked for
+// wherever they can run (EINSUMS_GB300_TC_PAIRS=1).
 int tc_pair_clusters();
-eg_status launch_tc_gemm(const CUtensorMap &tmA, const CUtensorMap &tmB, const TcGemmParams &p, cudaStream_t s);
+bool tc_pairs_forced();
+// tmBh: B's planes in boxes of 64 rows (half a tile), read by CTA pairs.
+eg_status launch_tc_gemm(const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmBh, const TcGemmParams &p,
+                         cudaStream_t s);
 // Grouped form: `ntiles_total` work entries, per-tile parameters from `items`.
 eg_status launch_tc_gemm_grouped(const CUtensorMap &tmA, const CUtensorMap &tmB, const TcGemmParams &p,
                                  const TcItem *items, const int4 *work, int ntiles_total, cudaStream_t s);

@@ -289,10 +289,12 @@ eg_status eg_stream_synchronize(void *stream);
 eg_status eg_measure_fp64_peak(double *dfma_tflops, double *dmma_tflops);
 eg_status eg_measure_fp64_peak_clock(double *dfma_tflops, double *dmma_tflops, double *probe_mhz);
 
-/* *clusters receives the number of two-CTA clusters the split-BF16 tensor kernel
- * runs single contractions on (256x128 output tiles, cta_group::2 MMAs), or 0
- * when it runs one CTA per 128x128 tile.  Pairs are used when the process
- * starts with EINSUMS_GB300_TC_PAIRS=1.  No reference counterpart. */
+/* *clusters receives the number of two-CTA clusters (256x128 output tiles,
+ * cta_group::2 MMAs) that the tensor kernel fits on the GPU when the process asked
+ * for them wherever the output has two row tiles (EINSUMS_GB300_TC_PAIRS=1), else 0:
+ * each call then takes pairs or single CTAs by its estimated time, or always single
+ * CTAs with EINSUMS_GB300_TC_PAIRS=0.  Results are the same bit for bit.  No
+ * reference counterpart. */
 eg_status eg_tc_pair_clusters(int32_t *clusters);
 
 /* Kernel accounting.  eg_kernel_launches: kernels this library has launched in the
