@@ -88,6 +88,10 @@ __device__ __forceinline__ void tma_load_3d_at(uint32_t dst, const void *tmap, u
 __device__ __forceinline__ void cp_async8(double *dst, const double *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async16(double *dst, const double *src, bool valid) { // zeros when not valid
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ---------------------------------------------------------------- clusters --
@@ -123,6 +127,12 @@ __device__ __forceinline__ void st_cluster_u32(uint32_t addr_cluster, uint32_t v
 __device__ __forceinline__ double ld_cluster_f64(uint32_t addr_cluster) {
     double v;
     asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr_cluster) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ unsigned long long ld_cluster_u64(uint32_t addr_cluster) {
+    unsigned long long v;
+    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(addr_cluster) : "memory");
     return v;
 }
 

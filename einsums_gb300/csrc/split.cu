@@ -21,10 +21,12 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
 
+#include "ptx.cuh"
 #include "split.cuh"
 
 namespace eg {
@@ -180,16 +182,18 @@ __global__ void __launch_bounds__(T *TR, 5) k_split_rowmax(OperandMap m, const d
     }
 }
 
+// The exponent of a row whose largest |x| has the given bits: |x| < 2^e (INT_MIN for
+// a row holding an infinity or NaN, 0 for a row of zeros).
+__device__ __forceinline__ int row_exponent(unsigned long long bits) {
+    const int field = (int)(bits >> 52);
+    if (field == 0x7ff) return INT_MIN;
+    if (field) return field - 1022;
+    return bits ? -1010 - __clzll((long long)bits) : 0; // subnormal: 2^-1074 times the bits
+}
+
 __global__ void k_split_exponent(const unsigned long long *rowmax, int *e, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double mx = __longlong_as_double((long long)rowmax[i]);
-        int ex = 0;
-        if (!isfinite(mx))
-            ex = INT_MIN;
-        else if (mx > 0.0)
-            frexp(mx, &ex); // mx = f 2^ex with f in [0.5, 1): |x| <= mx < 2^ex
-        e[i] = ex;
-    }
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        e[i] = row_exponent(rowmax[i]);
 }
 
 // Tiles of 32 rows x 64 k staged through shared memory so that the operand is
@@ -301,6 +305,135 @@ __global__ void __launch_bounds__(T *TR) k_split_digits(OperandMap m, const doub
     }
 }
 
+// Row maxima, exponents and digit planes of both operands in one launch that reads
+// every element once: a cluster of C CTAs takes R rows, each CTA a range of kc of
+// the K elements, which it holds in shared memory (asynchronous 8-byte copies, all
+// in flight at once); the CTAs' row maxima meet over distributed shared memory, and
+// each writes its range of the digit planes.  Bound: memory, 8 bytes read and 2 per
+// plane written per element.  Against the passes above (memset, maxima, exponents,
+// digits for each operand, with every element read twice): see split_both.
+struct SplitJob {
+    OperandMap m;
+    const double *X;
+    int *rexp;
+    __nv_bfloat16 *planes;
+    int row_fast;  // consecutive lanes walk rows (the smaller stride), else k
+    int pairs;     // (k, k + 1) with even k are neighbours on a 16-byte boundary in every row
+    int64_t tiles; // batches x R-row tiles
+};
+
+constexpr int kFusedThreads = 256;
+
+template <int S, bool CHECK, int R>
+__global__ void __launch_bounds__(kFusedThreads) k_split_rows(const __grid_constant__ SplitJob ja,
+                                                              const __grid_constant__ SplitJob jb, int kc, int ld,
+                                                              int C) {
+    extern __shared__ __align__(16) double tile[]; // [R][ld], then the tables
+    int64_t *koff = (int64_t *)(tile + (size_t)R * ld);
+    int64_t *roff = koff + kc;
+    unsigned long long *pmax = (unsigned long long *)(roff + R);
+    int *ex = (int *)(pmax + R);
+    constexpr int W = kFusedThreads / 32, P = S + (CHECK ? 2 : 0);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t id = blockIdx.x / C;
+    const int rank = C > 1 ? (int)ptx::cluster_ctarank() : 0;
+    const bool second = id >= ja.tiles;
+    const SplitJob &jj = second ? jb : ja;
+    const OperandMap &m = jj.m;
+    const int64_t t = second ? id - ja.tiles : id, rt = m.Rp / R;
+    const int64_t b = t / rt, r0 = (t - b * rt) * R;
+    const int64_t k0 = (int64_t)rank * kc;
+    const int nk = (int)max((int64_t)0, min((int64_t)kc, m.K - k0)); // real elements of this CTA's range
+    const int64_t ob = off_b(m, b);
+    for (int k = tid; k < nk; k += kFusedThreads) koff[k] = off_k(m, k0 + k);
+    if (tid < R) roff[tid] = r0 + tid < m.rows ? ob + off_r(m, r0 + tid) : -1;
+    __syncthreads();
+    const double *X = jj.X;
+    if (jj.row_fast) {
+        constexpr int KP = 32 / (R < 32 ? R : 32); // k a warp takes at a time
+        const int r = lane % R, kk = lane / R;
+        const int64_t ro = roff[r];
+        for (int k = warp * KP + kk; k < kc; k += W * KP) {
+            const bool ok = ro >= 0 && k < nk;
+            cp_async8(&tile[r * ld + k], ok ? X + ro + koff[k] : X, ok);
+        }
+    } else if (jj.pairs) {
+        for (int r = warp; r < R; r += W) {
+            const int64_t ro = roff[r];
+            for (int k = 2 * lane; k < kc; k += 64) { // the real elements are even in number too
+                const bool ok = ro >= 0 && k < nk;
+                ptx::cp_async16(&tile[r * ld + k], ok ? X + ro + koff[k] : X, ok);
+            }
+        }
+    } else {
+        for (int r = warp; r < R; r += W) {
+            const int64_t ro = roff[r];
+            for (int k = lane; k < kc; k += 32) {
+                const bool ok = ro >= 0 && k < nk;
+                cp_async8(&tile[r * ld + k], ok ? X + ro + koff[k] : X, ok);
+            }
+        }
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    for (int r = warp; r < R; r += W) {
+        unsigned long long mx = 0;
+        for (int k = 2 * lane; k < kc; k += 64) {
+            const double2 v = *(const double2 *)&tile[r * ld + k];
+            mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
+        }
+        for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (lane == 0) pmax[r] = mx;
+    }
+    if (C > 1)
+        ptx::cluster_sync();
+    else
+        __syncthreads();
+    if (tid < R) {
+        unsigned long long mx = pmax[tid];
+        for (int c = 1; c < C; c++) {
+            const int peer = rank + c < C ? rank + c : rank + c - C;
+            mx = max(mx, ptx::ld_cluster_u64(ptx::mapa(ptx::smem_u32(&pmax[tid]), (uint32_t)peer)));
+        }
+        const int e = row_exponent(mx);
+        ex[tid] = e;
+        if (rank == 0) jj.rexp[b * m.Rp + r0 + tid] = e;
+    }
+    if (C > 1)
+        ptx::cluster_sync(); // the peers have read this CTA's maxima
+    else
+        __syncthreads();
+    const int64_t plane = m.Rp * m.Kp;
+    const int kw = (int)max((int64_t)0, min((int64_t)kc, m.Kp - k0)); // range written, a multiple of 4
+    for (int r = warp; r < R; r += W) {
+        const int e = ex[r];
+        __nv_bfloat16 *row = jj.planes + (int64_t)b * P * plane + (r0 + r) * m.Kp + k0;
+        for (int k = 4 * lane; k < kw; k += 128) {
+            const double2 v0 = *(const double2 *)&tile[r * ld + k], v1 = *(const double2 *)&tile[r * ld + k + 2];
+            uint32_t p0[P], p1[P];
+            if (e == INT_MIN) {
+#pragma unroll
+                for (int s = 0; s < P; s++) p0[s] = p1[s] = 0u;
+            } else {
+                digits_bf16x2<S>(v0.x, v0.y, e, p0);
+                digits_bf16x2<S>(v1.x, v1.y, e, p1);
+                if constexpr (CHECK) {
+                    p0[S] = check_magnitude(p0[0]);
+                    p1[S] = check_magnitude(p1[0]);
+                }
+            }
+            if constexpr (CHECK) {
+                const float mark = m.comp ? kCheckB : kCheckA;
+                p0[S + 1] = check_mark(v0.x, v0.y, mark);
+                p1[S + 1] = check_mark(v1.x, v1.y, mark);
+            }
+#pragma unroll
+            for (int s = 0; s < P; s++) *(uint2 *)(row + s * plane + k) = make_uint2(p0[s], p1[s]);
+        }
+    }
+}
+
 // CTAs of `kernel` (256 threads, static shared memory) that fit on the GPU at
 // once: the splitting kernels launch exactly one wave of them and loop over
 // their work units, so no partial second wave trails the launch.
@@ -404,8 +537,7 @@ eg_status split_operand(OperandMap om, const double *X, unsigned long long *rowm
         om.offk = offk;
     }
     const bool r_fast = !k_fast && is_fast(om.rg, om.comp);
-    if (!f64) // the FP64 form's caller clears both operands' maxima at once
-        EG_CUDA(cudaMemsetAsync(rowmax, 0, (size_t)om.nbatch * om.Rp * sizeof(unsigned long long), s));
+    EG_CUDA(cudaMemsetAsync(rowmax, 0, (size_t)om.nbatch * om.Rp * sizeof(unsigned long long), s));
     const int cap = num_sms() * 8;
     {
         static const int resident = resident_grid(k_split_rowmax);
@@ -443,6 +575,112 @@ eg_status split_operand(OperandMap om, const double *X, unsigned long long *rowm
         }
     }
     EG_CHECK_LAUNCH("k_split_digits");
+    return EG_SUCCESS;
+}
+
+template <int S, bool CHECK, int R>
+cudaError_t launch_split_rows(const SplitJob &a, const SplitJob &b, int kc, int ld, int C, size_t smem, cudaStream_t s) {
+    static const cudaError_t attr = cudaFuncSetAttribute(k_split_rows<S, CHECK, R>,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (attr != cudaSuccess) return attr;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((a.tiles + b.tiles) * C));
+    cfg.blockDim = dim3(kFusedThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute la;
+    la.id = cudaLaunchAttributeClusterDimension;
+    la.val.clusterDim.x = (unsigned)C;
+    la.val.clusterDim.y = 1;
+    la.val.clusterDim.z = 1;
+    cfg.attrs = &la;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_split_rows<S, CHECK, R>, a, b, kc, ld, C);
+}
+
+// Splits the operands of a contraction (an operand without rows is left out).  The
+// fused launch when a range of K fits shared memory (K to about 25000); beyond, the
+// passes over each operand, with tables of offsets at tab (rows and K of each operand;
+// may be null).  Fused against passes, device time: both operands of 2304^3 in FP64
+// 165 -> 68 us, the six splits of a ring contraction with adjoints at o = 24, v = 96
+// 515 -> 211 us, the four of n = 75 quarter transformations 1.90 -> 1.05 ms (1.3 GB
+// each: 5.0 TB/s).
+eg_status split_both(OperandMap oa, const double *A, int *eA, __nv_bfloat16 *pA, OperandMap ob, const double *B, int *eB,
+                     __nv_bfloat16 *pB, unsigned long long *maxima, int64_t *tab, int S, bool f64, cudaStream_t s) {
+    for (OperandMap *o : {&oa, &ob}) {
+        o->sr = affine_stride(o->rg, o->comp);
+        o->sk = affine_stride(o->kg, o->comp);
+    }
+    const int64_t Kp = oa.Kp;
+    int R = 32, C = 1;
+    int64_t kc = 0;
+    size_t smem = 0;
+    auto fits = [&](int r, int c, size_t limit) {
+        const int64_t k = round_up((Kp + c - 1) / c, 4), ld = round_up(k, 16) + 2;
+        const size_t bytes = (size_t)r * ld * 8 + (size_t)k * 8 + (size_t)r * 20;
+        if (bytes > limit) return false;
+        R = r;
+        C = c;
+        kc = k;
+        smem = bytes;
+        return true;
+    };
+    bool ok = false;
+    // 32 rows, then 8, and up to eight CTAs along K, such that three CTAs fit an SM and,
+    // where K allows, there are a few for every SM; the longest K takes an SM per CTA
+    for (int r : {32, 8})
+        for (int c = 1; c <= 8 && !ok; c *= 2)
+            if (fits(r, c, 75 * 1024)) {
+                const int64_t tiles = (oa.nbatch * oa.Rp + ob.nbatch * ob.Rp) / r;
+                ok = tiles * c >= (r == 32 ? 2 : 4) * num_sms() || c == 8 || Kp / (2 * c) < 128;
+            }
+    if (!ok) ok = fits(8, 8, 227 * 1024);
+    const int64_t tiles = (oa.rows ? oa.nbatch * oa.Rp / R : 0) + (ob.rows ? ob.nbatch * ob.Rp / R : 0);
+    if (ok && tiles * C < (int64_t(1) << 31)) {
+        auto job = [&](const OperandMap &o, const double *X, int *e, __nv_bfloat16 *pl) {
+            const int64_t kstride = o.kg.n ? o.kg.s[o.comp][o.kg.n - 1] : 0, rstride = o.rg.n ? o.rg.s[o.comp][o.rg.n - 1] : 0;
+            SplitJob j{o, X, e, pl, rstride > 0 && (kstride == 0 || rstride < kstride) ? 1 : 0,
+                       0, o.rows ? o.nbatch * o.Rp / R : 0};
+            bool even = !j.row_fast && kstride == 1 && o.kg.ext[o.kg.n - 1] % 2 == 0 && ((uintptr_t)X & 15) == 0;
+            for (const ModeGroup *g : {&o.bg, &o.rg, &o.kg})
+                for (int d = 0; d < g->n - (g == &o.kg ? 1 : 0); d++) even = even && g->s[o.comp][d] % 2 == 0;
+            j.pairs = even ? 1 : 0;
+            return j;
+        };
+        const SplitJob ja = job(oa, A, eA, pA), jb = job(ob, B, eB, pB);
+        const int ld = (int)round_up(kc, 16) + 2;
+        cudaError_t err;
+        {
+            LaunchScope ls_("k_split_rows", s);
+            auto go = [&](auto slices, auto check) {
+                constexpr int SL = decltype(slices)::value;
+                constexpr bool CH = decltype(check)::value;
+                return R == 32 ? launch_split_rows<SL, CH, 32>(ja, jb, (int)kc, ld, C, smem, s)
+                               : launch_split_rows<SL, CH, 8>(ja, jb, (int)kc, ld, C, smem, s);
+            };
+            using std::integral_constant;
+            if (f64)
+                err = go(integral_constant<int, kF64Slices>{}, std::true_type{});
+            else
+                switch (S) {
+                case 2: err = go(integral_constant<int, 2>{}, std::false_type{}); break;
+                case 3: err = go(integral_constant<int, 3>{}, std::false_type{}); break;
+                case 4: err = go(integral_constant<int, 4>{}, std::false_type{}); break;
+                case 5: err = go(integral_constant<int, 5>{}, std::false_type{}); break;
+                default: err = go(integral_constant<int, 6>{}, std::false_type{}); break;
+                }
+        }
+        if (err != cudaSuccess) return cuda_fail(err, "k_split_rows");
+        EG_CHECK_LAUNCH("k_split_rows");
+        return EG_SUCCESS;
+    }
+    unsigned long long *maxA = maxima, *maxB = maxima + (int64_t)oa.nbatch * oa.Rp;
+    eg_status st;
+    if (oa.rows && (st = split_operand(oa, A, maxA, eA, pA, S, s, tab, tab ? tab + oa.rows : nullptr, f64)) != EG_SUCCESS)
+        return st;
+    int64_t *tabB = tab ? tab + oa.rows + oa.K : nullptr;
+    if (ob.rows && (st = split_operand(ob, B, maxB, eB, pB, S, s, tabB, tab ? tabB + ob.rows : nullptr, f64)) != EG_SUCCESS)
+        return st;
     return EG_SUCCESS;
 }
 
@@ -570,8 +808,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     const size_t bytesA = (size_t)nb * S * Mp * Kp * 2, bytesB = (size_t)nb * S * Np * Kp * 2;
     const size_t offB = round_up((int64_t)bytesA, 1024);
     const size_t offMaxA = offB + round_up((int64_t)bytesB, 1024);
-    const size_t offMaxB = offMaxA + round_up(nb * Mp * 8, 256);
-    const size_t offEA = offMaxB + round_up(nb * Np * 8, 256);
+    const size_t offEA = offMaxA + round_up(nb * (Mp + Np) * 8, 256);
     const size_t offEB = offEA + round_up(nb * Mp * 4, 256);
     const size_t offR = offEB + round_up(nb * Np * 4, 256);
     // offset tables (rows and k of each operand) unless they would be large
@@ -591,7 +828,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     if (st != EG_SUCCESS) return st;
     char *base = (char *)ws;
     __nv_bfloat16 *planesA = (__nv_bfloat16 *)base, *planesB = (__nv_bfloat16 *)(base + offB);
-    unsigned long long *maxA = (unsigned long long *)(base + offMaxA), *maxB = (unsigned long long *)(base + offMaxB);
+    unsigned long long *maxA = (unsigned long long *)(base + offMaxA);
     int *eA = (int *)(base + offEA), *eB = (int *)(base + offEB);
     int *status = nullptr;
     if ((st = status_word(s, &status)) != EG_SUCCESS) return st;
@@ -599,10 +836,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     OperandMap oa{c.batch, c.m, c.k, 0, M, Mp, K, Kp, (int)nb};
     OperandMap ob{c.batch, c.n, c.k, 1, N, Np, K, Kp, (int)nb};
     int64_t *tab = tables ? (int64_t *)(base + offTab) : nullptr;
-    if ((st = split_operand(oa, c.A, maxA, eA, planesA, S, s, tab, tables ? tab + M : nullptr)) != EG_SUCCESS) return st;
-    if ((st = split_operand(ob, c.B, maxB, eB, planesB, S, s, tables ? tab + M + K : nullptr,
-                            tables ? tab + M + K + N : nullptr)) != EG_SUCCESS)
-        return st;
+    if ((st = split_both(oa, c.A, eA, planesA, ob, c.B, eB, planesB, maxA, tab, S, false, s)) != EG_SUCCESS) return st;
 
     CUtensorMap tmA, tmB, tmBh;
     if ((st = encode_planes(&tmA, planesA, Kp, Mp, nb * S)) != EG_SUCCESS) return st;
@@ -770,9 +1004,9 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
         return o;
     };
     const size_t oPA = take((size_t)bb * P * mb * Kp * 2), oPB = take((size_t)bb * P * nbk * Kp * 2);
-    const size_t oMax = take((size_t)bb * (mb + nbk) * 8); // cleared for every panel pair ...
-    const size_t oCnt = take((size_t)cut * kTileRegions * sizeof(int)); // (with the accumulators' arrivals
-    const size_t oAcc = take((size_t)cut * 2 * kBM * kBN * 8); //  and those that the launch uses)
+    const size_t oMax = take((size_t)bb * (mb + nbk) * 8);
+    const size_t oCnt = take((size_t)cut * kTileRegions * sizeof(int)); // cleared for every panel pair, with
+    const size_t oAcc = take((size_t)cut * 2 * kBM * kBN * 8);          // those accumulators that the launch uses
     const size_t oExp = take((size_t)bb * (mb + nbk) * 4);
     const size_t oTab = take(tables ? (size_t)(M + N + 2 * K) * 8 : 0);
     const size_t oR = take(rbuf_bytes(3));
@@ -784,7 +1018,6 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
     if (st != EG_SUCCESS) return st;
     char *base = (char *)lease.ptr();
     __nv_bfloat16 *planesA = (__nv_bfloat16 *)(base + oPA), *planesB = (__nv_bfloat16 *)(base + oPB);
-    unsigned long long *maxA = (unsigned long long *)(base + oMax), *maxB = maxA + bb * mb;
     int *eA = (int *)(base + oExp), *eB = eA + bb * mb;
     int64_t *tab = tables ? (int64_t *)(base + oTab) : nullptr;
 
@@ -822,7 +1055,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
                 p.nkb = (int)(Kp / kBK);
                 choose_schedule(p, nbc, Mp / kBM, Np / kBN, S * (S + 1) / 2 + 2, 2);
                 const size_t used = (size_t)cut_tiles(p, nbc, Mp / kBM, Np / kBN) * 2 * kBM * kBN * 8;
-                EG_CUDA(cudaMemsetAsync(maxA, 0, oAcc - oMax + used, s));
+                if (used) EG_CUDA(cudaMemsetAsync(base + oCnt, 0, oAcc - oCnt + used, s));
                 OperandMap oa{c.batch, c.m, c.k, 0, mc, Mp, K, Kp, (int)nbc};
                 oa.b0 = b0;
                 oa.row0 = m0;
@@ -830,12 +1063,10 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
                 ob.b0 = b0;
                 ob.row0 = n0;
                 // a panel's planes stay while the other operand's panels go by
-                if (n0 == 0 && (st = split_operand(oa, c.A, maxA, eA, planesA, S, s, tab, tables ? tab + M : nullptr,
-                                                   true)) != EG_SUCCESS)
-                    return st;
-                if ((nbk < Np_all || m0 == 0) &&
-                    (st = split_operand(ob, c.B, maxB, eB, planesB, S, s, tables ? tab + M + K : nullptr,
-                                        tables ? tab + M + K + N : nullptr, true)) != EG_SUCCESS)
+                if (n0 > 0) oa.rows = 0;
+                if (nbk >= Np_all && m0 > 0) ob.rows = 0;
+                if ((st = split_both(oa, c.A, eA, planesA, ob, c.B, eB, planesB, (unsigned long long *)(base + oMax), tab,
+                                     S, true, s)) != EG_SUCCESS)
                     return st;
                 CUtensorMap tmA, tmB, tmBh;
                 if ((st = encode_planes(&tmA, planesA, Kp, Mp, nbc * P)) != EG_SUCCESS) return st;

@@ -112,23 +112,33 @@ struct TcItem {
     ModeGroup bg, mg, ng;
 };
 
-// IEEE bit pattern of |x|: for non-negative doubles (and NaN above Inf) the
-// unsigned order of the patterns is the numeric order.  Integer ops only: an
-// FP64 abs would run on this GPU's slow FP64 pipe, once per element.
-__device__ __forceinline__ unsigned long long abs_bits(double x) {
-    return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+// The bits of x, by way of an instruction the compiler does not look into: it turns
+// tests on the fields of a double's bits into FP64 comparisons, which run on this
+// GPU's slow FP64 pipe (a third of the splitting kernels' time).
+__device__ __forceinline__ unsigned long long bits_of(double x) {
+    unsigned long long b;
+    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+    return b;
 }
+
+// IEEE bit pattern of |x|: for non-negative doubles (and NaN above Inf) the
+// unsigned order of the patterns is the numeric order.
+__device__ __forceinline__ unsigned long long abs_bits(double x) { return bits_of(x) & 0x7FFFFFFFFFFFFFFFull; }
 
 // round(x * 2^sh) to nearest, ties to even, for |x| 2^sh < 2^63, built from the
 // IEEE fields with integer operations (the FP64 pipe of this GPU runs about two
 // operations per clock per SM; this is the splitting kernels' inner loop).
+// SHRINKS: |x| 2^sh < 2^48, so that there is always a bit to drop.
+template <bool SHRINKS = false>
 __device__ __forceinline__ long long scaled_round(double x, int sh) {
-    const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
-    const int ex = (int)((bits >> 52) & 0x7ff);
-    const unsigned long long mant = (bits & 0xFFFFFFFFFFFFFull) | ((unsigned long long)(ex != 0) << 52);
-    const int r = 1075 - (ex != 0 ? ex : 1) - sh; // |x| 2^sh = mant 2^-r
+    const unsigned long long bits = bits_of(x);
+    const uint32_t hi = (uint32_t)(bits >> 32);
+    const int ex = (int)((hi >> 20) & 0x7ff);
+    const uint32_t top = (hi & 0xFFFFFu) | (ex != 0 ? 0x100000u : 0u);
+    const unsigned long long mant = ((unsigned long long)top << 32) | (uint32_t)bits;
+    const int r = 1075 - max(ex, 1) - sh; // |x| 2^sh = mant 2^-r
     unsigned long long q;
-    if (r <= 0) {
+    if (!SHRINKS && r <= 0) {
         q = mant << (-r < 63 ? -r : 63); // a whole number already
     } else if (r > 62) {
         q = 0; // below 1/2
@@ -137,7 +147,7 @@ __device__ __forceinline__ long long scaled_round(double x, int sh) {
         // exactly when they exceed half, or equal half with an odd quotient
         q = (mant + ((1ull << (r - 1)) - 1ull) + ((mant >> r) & 1ull)) >> r;
     }
-    return (bits >> 63) ? -(long long)q : (long long)q;
+    return (int)hi < 0 ? -(long long)q : (long long)q;
 }
 
 // |sum| * 2^e rounded to nearest (ties to even), built with integer operations so the
@@ -232,7 +242,8 @@ __device__ __forceinline__ void digits_bf16x2(double x0, double x1, int e, uint3
         return b;
     }();
     const int sh = kTopBits + kBits * (S - 1) - e;
-    const long long F0 = scaled_round(x0, sh), F1 = scaled_round(x1, sh);
+    constexpr bool SHRINKS = S <= 6; // below 2^(7 + 8 (S - 1)), at most 2^47
+    const long long F0 = scaled_round<SHRINKS>(x0, sh), F1 = scaled_round<SHRINKS>(x1, sh);
     const unsigned long long G0 = (unsigned long long)F0 + bias, G1 = (unsigned long long)F1 + bias;
     const uint32_t g0[2] = {(uint32_t)G0, (uint32_t)(G0 >> 32)};
     const uint32_t g1[2] = {(uint32_t)G1, (uint32_t)(G1 >> 32)};

@@ -111,3 +111,40 @@ def test_subnormal_and_huge_results(eg):
         # one rounding of the exact sum against two: at most one unit of the last place apart
         ok = np.abs(C.cpu().numpy() - want) <= np.maximum(np.abs(np.spacing(want)), 5e-324)
         assert np.all(ok | (C.cpu().numpy() == want))
+
+
+@pytest.mark.parametrize("K", [65, 130, 1111, 5000, 20000, 26000])
+@pytest.mark.parametrize("layout", ["k", "k odd base", "k odd stride", "rows", "both strided", "two k modes"])
+def test_operand_splitting(eg, K, layout):
+    """The splitting launch: K of one CTA and of clusters, 32 and 8 rows, and beyond (the passes);
+    operands read along k (in pairs when aligned), along rows, or strided both ways."""
+    from test_split_math import split_product_fast
+    M, N, S = 45, 6, 3
+    rng = np.random.default_rng(K + len(layout))
+    A = rng.standard_normal((M, K)) * np.exp2(rng.integers(-9, 9, size=(M, 1)))
+    B = rng.standard_normal((N, K))
+    A[7] = 0.0
+    labels = "ik"
+    if layout == "k":
+        tA = cu(A)
+    elif layout == "k odd base":
+        tA = cu(np.concatenate([np.zeros(1), A.ravel()]))[1:].view(M, K)
+    elif layout == "k odd stride":
+        tA = cu(np.concatenate([A, np.zeros((M, 1 + K % 2))], 1))[:, :K]
+    elif layout == "rows":
+        tA = cu(A.T).T
+    elif layout == "both strided":
+        big = torch.zeros((M, 2 * K), dtype=torch.float64, device="cuda")
+        big[:, ::2] = cu(A)
+        tA = big[:, ::2]
+    else:
+        q = next(d for d in (13, 11, 5, 2) if K % d == 0)
+        tA, labels = cu(A.reshape(M, q, K // q).transpose(1, 0, 2)), "kil"
+    tB = cu(B)
+    C = torch.full((M, N), float("nan"), dtype=torch.float64, device="cuda")
+    if labels == "ik":
+        eg.einsum(0.0, "ij", C, 1.0, "ik", tA, "jk", tB, precision="split_bf16", slices=S)
+    else:
+        eg.einsum(0.0, "ij", C, 1.0, "kil", tA, "jkl", tB.view(N, q, K // q), precision="split_bf16", slices=S)
+    want = split_product_fast(A, B, S)
+    assert np.array_equal(C.cpu().numpy().view(np.uint64), np.ascontiguousarray(want).view(np.uint64))
