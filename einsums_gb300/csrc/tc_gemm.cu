@@ -41,14 +41,14 @@ constexpr int kFin = 8;      // columns finished at a time
 constexpr int FIN_T = 33;    // padded row count of a warp's transposition buffer
 constexpr int kCols = kBN / (kEpiWarps / 4); // columns of an epilogue warp
 static_assert(kTileRegions == kEpiWarps, "a region per epilogue warp");
-// per epilogue warp: its column offsets and exponents, the transposition buffer of
-// one batch, and its 32 rows' output offsets and validity
-constexpr int EPI_WARP_BYTES = kCols * (8 + 4) + kFin * FIN_T * 8 + 32 * (8 + 4);
+// per epilogue warp: its column offsets and (of two tiles) exponents, the
+// transposition buffer of one batch, and its 32 rows' addresses
+constexpr int EPI_WARP_BYTES = kCols * (8 + 2 * 4) + kFin * FIN_T * 8 + 32 * 8;
 constexpr int SMEM_BYTES = 1024 + 2 * kSlots * TILE_BYTES + AUX_BYTES + kEpiWarps * EPI_WARP_BYTES + 64;
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 // setmaxnreg: the epilogue warps' sums take 128 registers; what they hold beyond the
 // launch's 168 a thread, the four other warps give up.
-constexpr int kRegsIssue = 40, kRegsEpilogue = 232;
+constexpr int kRegsIssue = 56, kRegsEpilogue = 224;
 static_assert(128 * kRegsIssue + 32 * kEpiWarps * kRegsEpilogue <= THREADS * 168, "registers of the launch");
 constexpr int GROUP_M = 16; // tile rasterisation: groups of 16 row tiles share B tiles in L2
 constexpr unsigned long long DRAIN_NS = 200ull * 1000 * 1000;
@@ -254,10 +254,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     // per-epilogue-warp copies of the tile's column offsets and exponents, so
     // the epilogue warps never wait on one another
     int64_t *colOffAll = (int64_t *)(smem + 2 * kSlots * TILE_BYTES + AUX_BYTES);
-    int *colExpAll = (int *)(colOffAll + kEpiWarps * kCols);
-    double *finTAll = (double *)(colExpAll + kEpiWarps * kCols);            // a warp: kFin x FIN_T
-    int64_t *rowOffAll = (int64_t *)(finTAll + kEpiWarps * kFin * FIN_T); // a warp: 32 rows
-    int *rowOkAll = (int *)(rowOffAll + kEpiWarps * 32);
+    int *colExpAll = (int *)(colOffAll + kEpiWarps * kCols);                // a warp: the running and the pending tile's
+    double *finTAll = (double *)(colExpAll + 2 * kEpiWarps * kCols);            // a warp: kFin x FIN_T
+    double **rowAtAll = (double **)(finTAll + kEpiWarps * kFin * FIN_T); // a warp: 32 rows (null: past the output)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = CL == 2 ? (int)ptx::cluster_ctarank() : 0;
@@ -482,10 +481,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         const int row = quad * 32 + lane;     // tile row owned by this thread
         const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)col0;
         int64_t *colOff = colOffAll + ew * kCols;
-        int *colExp = colExpAll + ew * kCols;
+        int *colExp = colExpAll + 2 * ew * kCols; // the pending tile's; the running tile's are at colExp + run_exp
+        int run_exp = kCols;
         double *finT = finTAll + ew * (kFin * FIN_T);
-        int64_t *rowOffW = rowOffAll + ew * 32;
-        int *rowOkW = rowOkAll + ew * 32;
+        double **rowAt = rowAtAll + ew * 32;
         int abuf = 0;
         uint32_t aphase = 0;
         bool ok = true;
@@ -503,17 +502,17 @@ __global__ void __launch_bounds__(THREADS, 1)
         // K = 1024: 16.1 ms against 13).  When C runs along
         // the rows a thread keeps its row; otherwise a batch is transposed through
         // shared memory so that the read-modify-write of C runs along a row (lanes
-        // FIN*r .. FIN*r + FIN-1 take the batch's columns of row r).  colOff, colExp,
-        // rowOffW and rowOkW describe the pending tile.  One copy of this code, in a
+        // FIN*r .. FIN*r + FIN-1 take the batch's columns of row r).  colOff, colExp and rowAt
+        // describe the pending tile.  One copy of this code, in a
         // loop: finishing a tile's columns straight from the registers is as many times
         // the code, which ran at the rate of instruction fetch (80k clocks a tile).
         long long *const rbc = p.rbuf + (size_t)blockIdx.x * (F64 ? 3 : 1) * kPlane + (size_t)col0 * kBM + row;
         int parity = 0; // FP64 form: which of two scratch planes takes this tile's high sums
         int pend_cols = 0, pend_done = 0; // columns of the pending tile, and how many are done
-        bool pend_row_ok = false, pend_rows_fast = false, pend_fast = false;
+        bool pend_rows_fast = false, pend_fast = false;
         int pend_rowExp = 0;
-        const long long *pend_lo = rbc, *pend_hi = rbc;
-        double *pend_C = nullptr, *pend_row = nullptr; // the output, and this thread's row of it
+        const long long *pend_lo = rbc; // its sums, and how far on its high sums are
+        int pend_hi = 0;
         long long Rv[FIN], Hv[F64 ? FIN : 1];
         auto load_batch = [&]() {
             const int c0 = pend_done;
@@ -522,14 +521,14 @@ __global__ void __launch_bounds__(THREADS, 1)
                 for (int i = 0; i < FIN; i++) {
                     const int e = i * 32 + lane;
                     const int r = pend_rows_fast ? lane : e / FIN, c = pend_rows_fast ? i : e % FIN;
-                    if (rowOkW[r] && c0 + c < pend_cols)
-                        ptx::cp_async8(&finT[c * FIN_T + r], pend_C + rowOffW[r] + colOff[c0 + c]);
+                    if (rowAt[r] && c0 + c < pend_cols)
+                        ptx::cp_async8(&finT[c * FIN_T + r], rowAt[r] + colOff[c0 + c]);
                 }
             }
 #pragma unroll
             for (int i = 0; i < FIN; i++) {
                 Rv[i] = __ldcg(pend_lo + (c0 + i) * kBM);
-                if constexpr (F64) Hv[i] = __ldcg(pend_hi + (c0 + i) * kBM);
+                if constexpr (F64) Hv[i] = __ldcg(pend_lo + pend_hi + (c0 + i) * kBM);
             }
         };
         for (int tile = cta0;; tile += ctas) {
@@ -538,16 +537,19 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (drain && pend_done >= pend_cols) break;
             // only the K block count and the exponents (loaded early, like the batches) are
             // held through the chunks
-            int nkb = 0, my_rowExp = 0, my_colExp[kCols / 32] = {};
+            int nkb = 0, my_rowExp = 0;
+            int live = 0; // this warp's columns inside the output (none when its rows are not): the others are skipped
             if (!drain) {
                 const TileJob job = resolve<GROUPED, CL>(p, items, work, tile, rank);
                 nkb = job.nkb;
+                const int64_t left = job.N - (int64_t)job.nt * kBN - col0;
+                if ((int64_t)job.mt * kBM + quad * 32 < job.M && left > 0) live = left < kCols ? (int)left : kCols;
                 const int64_t m = (int64_t)job.mt * kBM + row;
                 if (m < job.M) my_rowExp = job.eA[m];
 #pragma unroll
                 for (int i = 0; i < kCols / 32; i++) {
                     const int64_t n = (int64_t)job.nt * kBN + col0 + lane + 32 * i;
-                    if (n < job.N) my_colExp[i] = job.eB[n];
+                    colExp[run_exp + lane + 32 * i] = n < job.N ? job.eB[n] : 0;
                 }
             }
             // This thread's 64 exact sums, a Horner sum over the steps:
@@ -573,18 +575,26 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                     ptx::tc_fence_after();
                     const uint32_t at = tl + (uint32_t)(abuf * 2 * kBN);
+                    if (st.two) {
 #pragma unroll
-                    for (int cc = 0; cc < kCols; cc += 16) {
-                        uint32_t lo[16], hi[16];
-                        ptx::tmem_ld16(at + cc, lo);
-                        if (st.two) ptx::tmem_ld16(at + kBN + cc, hi);
-                        ptx::tmem_wait_ld();
-                        if (st.two) {
+                        for (int cc = 0; cc < kCols; cc += 16) {
+                            if (cc >= live) break;
+                            uint32_t lo[16], hi[16];
+                            ptx::tmem_ld16(at + cc, lo);
+                            ptx::tmem_ld16(at + kBN + cc, hi);
+                            ptx::tmem_wait_ld();
 #pragma unroll
                             for (int i = 0; i < 16; i++)
                                 H[cc + i] += (long long)__float2int_rn(__uint_as_float(hi[i])) * (1 << kBits) +
                                              __float2int_rn(__uint_as_float(lo[i]));
-                        } else {
+                        }
+                    } else {
+#pragma unroll
+                        for (int cc = 0; cc < kCols; cc += 16) {
+                            if (cc >= live) break;
+                            uint32_t lo[16];
+                            ptx::tmem_ld16(at + cc, lo);
+                            ptx::tmem_wait_ld();
 #pragma unroll
                             for (int i = 0; i < 16; i++) H[cc + i] += __float2int_rn(__uint_as_float(lo[i]));
                         }
@@ -664,8 +674,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if (pend_rows_fast) {
 #pragma unroll
                         for (int i = 0; i < FIN; i++)
-                            if (pend_row_ok && c0 + i < pend_cols)
-                                pend_row[colOff[c0 + i]] = plain_store ? val[i] : fma(p.cp, finT[i * FIN_T + lane], val[i]);
+                            if (rowAt[lane] && c0 + i < pend_cols)
+                                rowAt[lane][colOff[c0 + i]] = plain_store ? val[i] : fma(p.cp, finT[i * FIN_T + lane], val[i]);
                     } else {
 #pragma unroll
                         for (int i = 0; i < FIN; i++) {
@@ -676,7 +686,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
                         for (int i = 0; i < FIN; i++) {
                             const int e = i * 32 + lane, r = e / FIN, c = e % FIN;
-                            if (rowOkW[r] && c0 + c < pend_cols) pend_C[rowOffW[r] + colOff[c0 + c]] = finT[c * FIN_T + r];
+                            if (rowAt[r] && c0 + c < pend_cols) rowAt[r][colOff[c0 + c]] = finT[c * FIN_T + r];
                         }
                         __syncwarp();
                     }
@@ -730,40 +740,37 @@ __global__ void __launch_bounds__(THREADS, 1)
                     p.redo[at] = make_int4(job.b, (int)p.m0 + job.mt * kBM + quad * 32, (int)p.n0 + job.nt * kBN + col0, 0);
                 }
             }
-            const int64_t nleft = job.N - (int64_t)job.nt * kBN - col0;
-            if (!finish || nleft <= 0) continue;
-            pend_cols = nleft < kCols ? (int)nleft : kCols;
+            if (!finish || live == 0) continue;
+            pend_cols = live;
             pend_lo = sums;
-            pend_hi = job.split ? sums + kPlane : own_hi;
-            pend_C = job.C;
+            pend_hi = (int)(job.split ? kPlane : (size_t)(own_hi - sums));
             pend_rows_fast = job.mg->n > 0 && job.mg->s[2][job.mg->n - 1] == 1;
             const int64_t m = (int64_t)job.mt * kBM + row;
-            pend_row_ok = m < job.M;
+            const bool row_ok = m < job.M;
             int64_t rowOff = 0;
             pend_rowExp = my_rowExp;
-            if (pend_row_ok) {
+            if (row_ok) {
                 int64_t oa, ob;
                 group_offsets32(*job.mg, (uint32_t)(GROUPED ? m : p.m0 + m), oa, ob, rowOff);
             }
-            pend_row = pend_C + rowOff;
             // the largest and smallest exponents (a non-finite row or column counts as far below)
             int emax = INT_MIN, emin = INT_MAX;
 #pragma unroll
             for (int k = 0; k < kCols / 32; k++) {
-                const int i = lane + 32 * k, ex = my_colExp[k];
+                const int i = lane + 32 * k, ex = colExp[run_exp + i];
                 const int64_t n = (int64_t)job.nt * kBN + col0 + i;
                 int64_t oa, ob, oc = 0;
-                if (i < pend_cols) group_offsets32(*job.ng, (uint32_t)(GROUPED ? n : p.n0 + n), oa, ob, oc);
+                if (i < live) group_offsets32(*job.ng, (uint32_t)(GROUPED ? n : p.n0 + n), oa, ob, oc);
                 colOff[i] = oc;
-                colExp[i] = ex;
                 emax = max(emax, ex);
                 emin = min(emin, max(ex, -(1 << 20)));
             }
+            colExp += run_exp;
+            run_exp = -run_exp;
             emax = __reduce_max_sync(0xffffffffu, emax) + __reduce_max_sync(0xffffffffu, pend_rowExp);
             emin = __reduce_min_sync(0xffffffffu, emin) + __reduce_min_sync(0xffffffffu, max(pend_rowExp, -(1 << 20)));
             pend_fast = emin + p.shift_const >= kFastMin && emax + p.shift_const <= kFastMax;
-            rowOffW[lane] = rowOff;
-            rowOkW[lane] = pend_row_ok ? 1 : 0;
+            rowAt[lane] = row_ok ? job.C + rowOff : nullptr;
             __syncwarp();
         }
     }
