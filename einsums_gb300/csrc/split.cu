@@ -749,7 +749,7 @@ static void set_ab(split::TcGemmParams &p, double ab) {
 // Single CTAs or CTA pairs, which tiles of a launch are cut along K, and how often:
 // the whole rounds of the CTAs run whole tiles; the tiles left over for the last
 // round -- 20 of 324 on 152 SMs, a third of the time -- are cut into as many slices
-// of at least two K blocks as give the smallest estimated time.  The estimate counts
+// of K blocks as give the smallest estimated time.  The estimate counts
 // clocks: 360 per K block of a slice pair (320 on CTA pairs, which need two row
 // tiles), 6000 for a tile's epilogue, 8000 more for adding a slice's sums to its
 // accumulator and 60 per accumulator plane to clear it.  Returns the clocks.
@@ -773,10 +773,9 @@ static double choose_schedule(split::TcGemmParams &p, int64_t nb, int64_t mtiles
         };
         offer(whole + (rem ? entry(p.nkb) : 0.0), units, 1, p.nkb, 1.0);
         if (rem == 0) continue;
-        const int64_t unit = kKStep / kBK;
         int64_t last = 0;
-        for (int64_t ks = 2; ks <= std::min<int64_t>(p.nkb / unit, 64); ks++) {
-            const int64_t slice = round_up((p.nkb + ks - 1) / ks, unit);
+        for (int64_t ks = 2; ks <= std::min<int64_t>(p.nkb, 64); ks++) {
+            const int64_t slice = (p.nkb + ks - 1) / ks;
             const int64_t n = (p.nkb + slice - 1) / slice; // slices actually used
             if (n == last) continue;
             last = n;
@@ -802,7 +801,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     const int64_t nb = c.batch.total, M = c.m.total, N = c.n.total, K = c.k.total;
     if (M >= (int64_t(1) << 31) || N >= (int64_t(1) << 31) || K >= (int64_t(1) << 31) || nb * S >= (int64_t(1) << 31))
         return fail(EG_ERROR_NOT_SUPPORTED, "split form: a mode group exceeds 2^31 elements");
-    const int64_t Kp = round_up(K, kKStep), Mp = round_up(M, kBM), Np = round_up(N, kBN);
+    const int64_t Kp = round_up(K, kBK), Mp = round_up(M, kBM), Np = round_up(N, kBN);
 
     // workspace: digit planes of A and B, row maxima, exponents, status word
     const size_t bytesA = (size_t)nb * S * Mp * Kp * 2, bytesB = (size_t)nb * S * Np * Kp * 2;
@@ -971,7 +970,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
     using namespace split;
     constexpr int S = kF64Slices, P = S + 2;
     const int64_t nb = c.batch.total, M = c.m.total, N = c.n.total, K = c.k.total;
-    const int64_t Kp = round_up(K, kKStep);
+    const int64_t Kp = round_up(K, kBK);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     EG_CUDA(cudaStreamIsCapturing(s, &cap));
     if (cap != cudaStreamCaptureStatusNone) return EG_ERROR_NOT_SUPPORTED;
@@ -1102,7 +1101,7 @@ bool f64_tensor_pays(const Contraction &c) {
     const double fma = contract_f64_seconds(c);
     if (fma < 40e-6) return false;
     TcGemmParams p{};
-    p.nkb = (int)(round_up(K, kKStep) / kBK);
+    p.nkb = (int)(round_up(K, kBK) / kBK);
     const int64_t mtiles = round_up(M, kBM) / kBM, ntiles = round_up(N, kBN) / kBN;
     if (nb * mtiles * ntiles > (int64_t(1) << 30)) return false;
     const double clocks = choose_schedule(p, nb, mtiles, ntiles, kF64Slices * (kF64Slices + 1) / 2 + 2, 2);

@@ -37,7 +37,7 @@ constexpr int kF64Slices = 8, kF64High = 4;
 constexpr float kCheckA = 4.0f, kCheckB = -5.0f;
 constexpr int kTileRegions = 8; // 32 x 64 blocks of a tile, one per epilogue warp
 constexpr int kChunkKB = 16;    // 16 x 64 = 1024 products per exact FP32 chunk
-constexpr int kKStep = 2 * kBK;  // K is padded to whole groups of two K blocks
+constexpr int kKStep = 2 * kBK;  // granularity of the longest exact pass (K itself is padded to kBK)
 
 struct TcGemmParams {
     int S;
@@ -66,7 +66,7 @@ struct TcGemmParams {
     // The first t0 schedule entries are whole tiles.  The tiles left for the last,
     // partly filled round of the CTAs (all of them when there are fewer tiles than
     // CTAs) are cut along K so that the round is full: entry t >= t0 is K slice
-    // (t - t0) % ksplit (kslice K blocks, even; the last slice takes the rest) of
+    // (t - t0) % ksplit (kslice K blocks; the last slice takes the rest) of
     // tile t0 + (t - t0) / ksplit.  The slices' exact int64 sums are added into racc
     // ([tile - t0][128 columns][128 rows], two planes in the FP64 form) and the last
     // slice to arrive at a region of an epilogue warp (counted in rcnt,

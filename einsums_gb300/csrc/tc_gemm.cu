@@ -47,7 +47,10 @@ constexpr int EPI_WARP_BYTES = kCols * (8 + 2 * 4) + kFin * FIN_T * 8 + 32 * 8;
 constexpr int SMEM_BYTES = 1024 + 2 * kSlots * TILE_BYTES + AUX_BYTES + kEpiWarps * EPI_WARP_BYTES + 64;
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 // setmaxnreg: the epilogue warps' sums take 128 registers; what they hold beyond the
-// launch's 168 a thread, the four other warps give up.
+// launch's 168 a thread, the four other warps give up.  No role may spill: a local load
+// that misses the few KB of L1 left beside the ring waits some 4000 clocks behind the
+// tiles in flight (25600 x 25600, K = 1024: 16.0 ms with 60 bytes of spills a thread,
+// 12.9 without).
 constexpr int kRegsIssue = 56, kRegsEpilogue = 224;
 static_assert(128 * kRegsIssue + 32 * kEpiWarps * kRegsEpilogue <= THREADS * 168, "registers of the launch");
 constexpr int GROUP_M = 16; // tile rasterisation: groups of 16 row tiles share B tiles in L2
