@@ -21,6 +21,7 @@ eg_status lower_for_group(double cp, const int32_t *Cl, const eg_tensor *C, doub
                           const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options &opt,
                           Contraction &out, int32_t *alg_out, bool &gemm_shaped);
 void set_split_report(const eg_split_report &r);
+void set_error(const std::string &msg);
 void count_launches(uint64_t n);
 } // namespace eg
 
@@ -84,12 +85,16 @@ eg_status create_plan(double cp, const int32_t *Cl, const eg_tensor *Cs, double 
         cs.push_back(c);
     }
     if (!groupable) return EG_SUCCESS;
-    auto plan = std::make_unique<Plan>();
-    cudaGetDevice(&plan->device);
-    plan->precision = opt.precision;
-    plan->slices = opt.slices;
-    plan->count = count;
-    plan->algorithm = alg0;
+    auto new_plan = [&] {
+        auto p = std::make_unique<Plan>();
+        cudaGetDevice(&p->device);
+        p->precision = opt.precision;
+        p->slices = opt.slices;
+        p->count = count;
+        p->algorithm = alg0;
+        return p;
+    };
+    auto plan = new_plan();
     StreamForCapture cap(stream);
     if (!cap.s) return eg::fail(EG_ERROR_CUDA, "could not create a capture stream");
     eg_status st;
@@ -100,7 +105,16 @@ eg_status create_plan(double cp, const int32_t *Cl, const eg_tensor *Cs, double 
             return EG_SUCCESS;
         }
     } else {
-        st = eg::grouped::build_f64_plan(*plan, cs, cap.s);
+        st = EG_ERROR_NOT_SUPPORTED;
+        if (eg::grouped::f64_tensor_plan_pays(cs)) {
+            st = eg::grouped::build_split_plan(*plan, cs, 0, cap.s, true);
+            if (st == EG_ERROR_OUT_OF_MEMORY) st = EG_ERROR_NOT_SUPPORTED; // the FMA plan needs next to none
+            if (st == EG_ERROR_NOT_SUPPORTED) {
+                eg::set_error("");
+                plan = new_plan();
+            }
+        }
+        if (st == EG_ERROR_NOT_SUPPORTED) st = eg::grouped::build_f64_plan(*plan, cs, cap.s);
     }
     if (st != EG_SUCCESS) return st;
     out = std::move(plan);
@@ -108,8 +122,17 @@ eg_status create_plan(double cp, const int32_t *Cl, const eg_tensor *Cs, double 
 }
 
 eg_status run_plan(Plan &plan, cudaStream_t stream) {
+    std::unique_lock<std::mutex> lk;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    const bool ordered = plan.last && cudaStreamIsCapturing(stream, &capturing) == cudaSuccess &&
+                         capturing == cudaStreamCaptureStatusNone;
+    if (ordered) {
+        lk = std::unique_lock<std::mutex>(plan.mu);
+        EG_CUDA(cudaStreamWaitEvent(stream, plan.last, 0));
+    }
     cudaError_t err = cudaGraphLaunch(plan.exec, stream);
     if (err != cudaSuccess) return eg::cuda_fail(err, "cudaGraphLaunch");
+    if (ordered) EG_CUDA(cudaEventRecord(plan.last, stream));
     eg::count_launches(plan.kernels);
     if (plan.precision == EG_PRECISION_SPLIT_BF16) eg::set_split_report(plan.report);
     return EG_SUCCESS;
@@ -136,6 +159,7 @@ Plan::~Plan() {
                              100 * tot[2] / tot[6], 100 * tot[3] / tot[6], 100 * tot[4] / tot[6], 100 * tot[5] / tot[6]);
         }
     }
+    if (last) cudaEventDestroy(last);
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     for (void *p : owned) tracked_free(p);

@@ -5,13 +5,15 @@
 // A plan lowers every item to the canonical contraction, builds a device-side
 // work list of output tiles (largest first), and captures the whole batch as
 // a CUDA graph that later calls replay:
-//   * FP64: one persistent launch of k_grouped_f64 over the work list; each
+//   * FP64, when it pays (f64_tensor_plan_pays): as split-BF16 with eight slices and
+//     the accuracy check of split.cu's launch_f64_tensor, then one launch of the FMA
+//     kernel over the blocks that failed it;
+//   * FP64 otherwise: one persistent launch of k_grouped_f64 over the work list; each
 //     entry computes a 32x32 or 64x64 tile with the DFMA core, the tile size
 //     chosen per shape bucket by the autotuner (autotune.cpp);
-//   * split-BF16: three digit-splitting launches per operand covering every
-//     item (grouped variants of split.cu's kernels, unit -> item by binary
-//     search over a prefix table), then one persistent launch of the
-//     tcgen05 GEMM over the work list (k_tc_split_gemm<true>).
+//   * split-BF16: one digit-splitting launch over every operand of every item, then
+//     one persistent launch of the tcgen05 GEMM over the work list
+//     (k_tc_split_gemm<true>).
 #include <algorithm>
 #include <climits>
 #include <cstdio>
@@ -23,18 +25,19 @@
 #include <mutex>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_bf16.h>
 
 #include "grouped.cuh"
+#include "ptx.cuh"
 #include "split.cuh"
 
 namespace eg {
 eg_status lower_for_group(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al,
                           const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options &opt,
                           Contraction &out, int32_t *alg_out, bool &gemm_shaped);
-eg_status encode_planes_public(CUtensorMap *map, void *base, int64_t Kp, int64_t rows, int64_t planes);
 int64_t mode_group_affine_stride(const ModeGroup &g, int comp);
 eg_status encode_planes_extent(CUtensorMap *map, void *base, int64_t K, int64_t rows, int64_t planes, int64_t Kp,
                                int64_t Rp);
@@ -157,6 +160,19 @@ __global__ void __launch_bounds__(THREADS) k_grouped_f64(const F64Item *items, c
     }
 }
 
+// The 32 x 64 blocks of outputs that the FP64 form on the tensor cores left out:
+// {item, batch index, row, column}, *count of them.
+__global__ void __launch_bounds__(THREADS) k_grouped_f64_listed(const F64Item *items, const int4 *list, const int *count,
+                                                                 double cp, double ab, int zero) {
+    __shared__ double As[BK][LD];
+    __shared__ double Bs[BK][LD];
+    const int n = 2 * __ldg(count);
+    for (int w = blockIdx.x; w < n; w += gridDim.x) {
+        const int4 e = list[w >> 1];
+        f64_tile<32>(items[e.x], e.y, e.z / 32, e.w / 32 + (w & 1), cp, ab, zero != 0, As, Bs);
+    }
+}
+
 // --------------------------------------------------- grouped digit split --
 struct GOp {
     const double *X;
@@ -166,7 +182,8 @@ struct GOp {
     int nbatch;
     int64_t rows, Rp, K, Kp;
     int64_t rowbase;      // first entry in the row-max / exponent arrays
-    int64_t zbase;        // first digit plane
+    int64_t plane0;       // element offset of the first digit plane
+    int64_t pitch, pstride; // elements between rows and between planes (16-byte multiples)
     int64_t rtab, ktab;   // first entries of this operand's row and K offsets in the plan's offset table
     int64_t sr, sk;       // the single element stride of the rows / of K when the modes nest (else 0: tables)
 };
@@ -186,7 +203,7 @@ template <int S>
 __global__ void __launch_bounds__(kGThreads, 4) k_grouped_split(const GOp *ops, const int4 *units, int nunits,
                                                              const long long *__restrict__ offs, int *rexpA,
                                                              int *rexpB, __nv_bfloat16 *planesA,
-                                                             __nv_bfloat16 *planesB, int64_t Rmax, int64_t Kmaxp) {
+                                                             __nv_bfloat16 *planesB) {
     __shared__ double tile[kGU][kGK + 1];
     __shared__ unsigned long long red[kGWarps][kGU];
     __shared__ int ex[kGU];
@@ -256,7 +273,6 @@ __global__ void __launch_bounds__(kGThreads, 4) k_grouped_split(const GOp *ops, 
         __syncthreads();
         // phase 2: digit planes, 64 K at a time
         __nv_bfloat16 *planes = g.comp ? planesB : planesA;
-        const int64_t z0 = g.zbase + b * S;
         for (int64_t k0 = 0; k0 < K; k0 += kGK) {
             if (row_fast) {
 #pragma unroll
@@ -291,7 +307,7 @@ __global__ void __launch_bounds__(kGThreads, 4) k_grouped_split(const GOp *ops, 
                     }
 #pragma unroll
                     for (int q = 0; q < S; q++)
-                        *reinterpret_cast<uint32_t *>(planes + ((z0 + q) * Rmax + r0 + rr) * Kmaxp + k) = pk[q];
+                        *reinterpret_cast<uint32_t *>(planes + g.plane0 + (b * S + q) * g.pstride + (r0 + rr) * g.pitch + k) = pk[q];
                 }
             }
             __syncthreads();
@@ -299,22 +315,153 @@ __global__ void __launch_bounds__(kGThreads, 4) k_grouped_split(const GOp *ops, 
     }
 }
 
-template <int S>
-void launch_grouped_split_s(const GOp *ops, const int4 *units, int nunits, const long long *offs, int *eA, int *eB,
-                            __nv_bfloat16 *pA, __nv_bfloat16 *pB, int64_t Rmax, int64_t Kmaxp, cudaStream_t s) {
-    const int grid = (int)std::min<int64_t>(std::max(nunits, 1), (int64_t)num_sms() * 8);
-    k_grouped_split<S><<<grid, kGThreads, 0, s>>>(ops, units, nunits, offs, eA, eB, pA, pB, Rmax, Kmaxp);
+// The same when every item's K is short (kRowsMaxK): a unit is 32 rows or fewer (int4
+// .w, a power of two), as many as keep it within 32 KB of shared memory, so that every
+// element is read once, all of a unit's loads in flight at once while the unit before is
+// converted, and the maxima and digits are taken from shared memory.  Bound: integer
+// instructions and memory about equally; the unit above read each element twice, a few
+// loads per thread at a time.
+constexpr int64_t kRowsElems = 4096, kRowsMaxK = 1152;
+
+__host__ __device__ inline int rows_ld(int64_t K) { return (int)((K + 15) / 16 * 16 + 2); }
+
+template <int S, bool CHECK>
+__global__ void __launch_bounds__(kGThreads, 3) k_grouped_rows(const GOp *ops, const int4 *units, int nunits,
+                                                               const long long *__restrict__ offs, int *rexpA, int *rexpB,
+                                                               __nv_bfloat16 *planesA, __nv_bfloat16 *planesB,
+                                                               int tile_elems) {
+    extern __shared__ __align__(16) double tiles[]; // two of [rows of the unit][rows_ld(K)]
+    constexpr int P = S + (CHECK ? 2 : 0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto load = [&](int u, double *tile) {
+        if (u < nunits) {
+            const int4 un = units[u];
+            const GOp &g = ops[un.x];
+            const int64_t b = un.y, r0 = un.z;
+            const int R = un.w, K = (int)g.K, ld = rows_ld(K), kw = (K + 3) & ~3;
+            const int nr = (int)(g.rows - r0 < R ? g.rows - r0 : R);
+            const int64_t sr = g.sr, sk = g.sk;
+            int64_t oa, ob, oc;
+            group_offsets(g.bg, b, oa, ob, oc);
+            const double *X = g.X + pick(g.comp, oa, ob);
+            auto row_at = [&](int r) { return sr ? (r0 + r) * sr : (int64_t)__ldg(offs + g.rtab + r0 + r); };
+            auto k_at = [&](int k) { return (int64_t)__ldg(offs + g.ktab + k); };
+            // (a single k stride is added up: the loop is two copies for it)
+            auto row_copy = [&](int r, int k, int step) { // k, k + step, ... of row r
+                const double *x = X + row_at(r);
+                double *t = tile + r * ld;
+                if (sk) {
+                    const int64_t inc = (int64_t)step * sk;
+                    x += (int64_t)k * sk;
+#pragma unroll 4
+                    for (; k < K; k += step, x += inc) ptx::cp_async8(t + k, x);
+                } else {
+#pragma unroll 4
+                    for (; k < K; k += step) ptx::cp_async8(t + k, x + k_at(k));
+                }
+                for (; k < kw; k += step) t[k] = 0.0;
+            };
+            if (g.row_fast) {
+                const int r = lane & (R - 1), per = 32 / R;
+                if (r < nr) row_copy(r, warp * per + lane / R, kGWarps * per);
+            } else {
+                for (int r = warp; r < nr; r += kGWarps) row_copy(r, lane, 32);
+            }
+        }
+        ptx::cp_async_commit();
+    };
+    int buf = 0;
+    load(blockIdx.x, tiles);
+    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
+        load(u + gridDim.x, tiles + (buf ^ 1) * tile_elems);
+        ptx::cp_async_wait<1>();
+        __syncthreads();
+        const double *tile = tiles + buf * tile_elems;
+        const int4 un = units[u];
+        const GOp &g = ops[un.x];
+        const int64_t b = un.y, r0 = un.z;
+        const int K = (int)g.K, ld = rows_ld(K), kw = (K + 3) & ~3;
+        const int nr = (int)(g.rows - r0 < un.w ? g.rows - r0 : un.w);
+        const int64_t pstride = g.pstride, pitch = g.pitch;
+        // a warp takes whole rows: the maximum, then the digits of four k a lane at a time
+        __nv_bfloat16 *planes = (g.comp ? planesB : planesA) + g.plane0 + b * P * pstride + r0 * pitch;
+        int *rexp = (g.comp ? rexpB : rexpA) + g.rowbase + b * g.Rp + r0;
+        const float mark = g.comp ? split::kCheckB : split::kCheckA;
+        for (int r = warp; r < nr; r += kGWarps) {
+            const int e = split::row_exponent(split::row_max_bits(tile + r * ld, kw, lane));
+            if (lane == 0) rexp[r] = e;
+            __nv_bfloat16 *row = planes + r * pitch;
+            for (int k = 4 * lane; k < kw; k += 128) {
+                const double2 v0 = *(const double2 *)&tile[r * ld + k], v1 = *(const double2 *)&tile[r * ld + k + 2];
+                uint32_t p0[P], p1[P];
+                if (e == INT_MIN) {
+#pragma unroll
+                    for (int s = 0; s < P; s++) p0[s] = p1[s] = 0u;
+                } else {
+                    split::digits_bf16x2<S>(v0.x, v0.y, e, p0);
+                    split::digits_bf16x2<S>(v1.x, v1.y, e, p1);
+                    if constexpr (CHECK) {
+                        p0[S] = split::check_magnitude(p0[0]);
+                        p1[S] = split::check_magnitude(p1[0]);
+                    }
+                }
+                if constexpr (CHECK) {
+                    p0[S + 1] = split::check_mark(v0.x, v0.y, mark);
+                    p1[S + 1] = split::check_mark(v1.x, v1.y, mark);
+                }
+#pragma unroll
+                for (int s = 0; s < P; s++) *(uint2 *)(row + s * pstride + k) = make_uint2(p0[s], p1[s]);
+            }
+        }
+        __syncthreads(); // the tile is read before the loads of the unit after next replace it
+        buf ^= 1;
+    }
 }
 
-void launch_grouped_split(int S, const GOp *ops, const int4 *units, int nunits, const long long *offs, int *eA,
-                          int *eB, __nv_bfloat16 *pA, __nv_bfloat16 *pB, int64_t Rmax, int64_t Kmaxp, cudaStream_t s) {
+// f(std::integral_constant<int, S>, std::bool_constant<FP64 form>) for a run-time form.
+template <typename F>
+auto with_slices(int S, bool f64, F f) {
+    using std::integral_constant;
+    if (f64) return f(integral_constant<int, split::kF64Slices>{}, std::true_type{});
     switch (S) {
-    case 2: launch_grouped_split_s<2>(ops, units, nunits, offs, eA, eB, pA, pB, Rmax, Kmaxp, s); break;
-    case 3: launch_grouped_split_s<3>(ops, units, nunits, offs, eA, eB, pA, pB, Rmax, Kmaxp, s); break;
-    case 4: launch_grouped_split_s<4>(ops, units, nunits, offs, eA, eB, pA, pB, Rmax, Kmaxp, s); break;
-    case 5: launch_grouped_split_s<5>(ops, units, nunits, offs, eA, eB, pA, pB, Rmax, Kmaxp, s); break;
-    default: launch_grouped_split_s<6>(ops, units, nunits, offs, eA, eB, pA, pB, Rmax, Kmaxp, s); break;
+    case 2: return f(integral_constant<int, 2>{}, std::false_type{});
+    case 3: return f(integral_constant<int, 3>{}, std::false_type{});
+    case 4: return f(integral_constant<int, 4>{}, std::false_type{});
+    case 5: return f(integral_constant<int, 5>{}, std::false_type{});
+    default: return f(integral_constant<int, 6>{}, std::false_type{});
     }
+}
+
+// Outside any capture, before launch_grouped_rows is captured.
+cudaError_t allow_grouped_rows(int S, bool f64) {
+    return with_slices(S, f64, [](auto slices, auto check) {
+        return cudaFuncSetAttribute(k_grouped_rows<decltype(slices)::value, decltype(check)::value>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 76 * 1024);
+    });
+}
+
+eg_status launch_grouped_rows(int S, bool f64, const GOp *ops, const int4 *units, int nunits, const long long *offs, int *eA,
+                              int *eB, __nv_bfloat16 *pA, __nv_bfloat16 *pB, size_t smem, cudaStream_t s) {
+    const int per_sm = std::max(1, std::min<int>(8, (int)(220 * 1024 / (smem + 1024))));
+    const int grid = std::min(std::max(nunits, 1), num_sms() * per_sm);
+    with_slices(S, f64, [&](auto slices, auto check) {
+        k_grouped_rows<decltype(slices)::value, decltype(check)::value>
+            <<<grid, kGThreads, smem, s>>>(ops, units, nunits, offs, eA, eB, pA, pB, (int)(smem / 16));
+        return 0;
+    });
+    EG_CHECK_LAUNCH("k_grouped_rows");
+    return EG_SUCCESS;
+}
+
+eg_status launch_grouped_split(int S, const GOp *ops, const int4 *units, int nunits, const long long *offs, int *eA,
+                               int *eB, __nv_bfloat16 *pA, __nv_bfloat16 *pB, cudaStream_t s) {
+    const int grid = (int)std::min<int64_t>(std::max(nunits, 1), (int64_t)num_sms() * 8);
+    with_slices(S, false, [&](auto slices, auto) {
+        k_grouped_split<decltype(slices)::value><<<grid, kGThreads, 0, s>>>(ops, units, nunits, offs, eA, eB, pA, pB);
+        return 0;
+    });
+    EG_CHECK_LAUNCH("grouped digit splitting");
+    return EG_SUCCESS;
 }
 
 int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
@@ -516,21 +663,42 @@ eg_status build_f64_plan(Plan &plan, const std::vector<Contraction> &cs, cudaStr
     return EG_SUCCESS;
 }
 
-// Builds and captures the split-BF16 plan; returns EG_ERROR_NOT_SUPPORTED when
-// an item's K needs more than one exact pass (the caller then runs items one by one).
-eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int slices, cudaStream_t s) {
+// Whether an FP64 list is worth the tensor cores (the FP64 form of split.cu's
+// launch_f64_tensor, every item a tile or a few): from estimates of both times, the
+// FMAs of 32 x 32 tiles at the FP64 pipe's rate against 30 us of launches, the splitting
+// (28 bytes per element) and the tiles, each at least its chain of loads.  The digit
+// planes stay below 1 GB; items with K below 8 or beyond the row-wise splitting keep the
+// list on the FMA kernel.
+bool f64_tensor_plan_pays(const std::vector<Contraction> &cs) {
+    double fma = 0.0, bytes = 0.0, clocks = 0.0, planes = 0.0;
+    for (const Contraction &c : cs) {
+        const double nb = (double)c.batch.total, M = (double)c.m.total, N = (double)c.n.total, K = (double)c.k.total;
+        if (c.k.total < 8 || c.k.total > kRowsMaxK || c.m.total >= (1ll << 31) || c.n.total >= (1ll << 31)) return false;
+        fma += nb * std::ceil(M / 32) * std::ceil(N / 32) * 1024.0 * K;
+        bytes += nb * (M + N) * K * 28.0;
+        planes += nb * (M + N) * (K + 16) * 2.0 * (split::kF64Slices + 2);
+        clocks += nb * std::ceil(M / 128) * std::ceil(N / 128) * (std::ceil(K / 64) * 38 * 420 + 16000);
+    }
+    const double sms = num_sms();
+    const double t_fma = 1.1 * fma / (2.0 * sms * 1.9e9);
+    const double t_tensor = 30e-6 + bytes / 2.2e12 + std::max(clocks / sms, 60000.0) / 1.9e9;
+    return planes < 1e9 && t_tensor < 0.8 * t_fma;
+}
+
+// Builds and captures the split-BF16 plan, or (f64) the FP64 one on the tensor cores;
+// returns EG_ERROR_NOT_SUPPORTED when an item's K needs more than one exact pass (the
+// caller then runs items one by one).
+eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int slices, cudaStream_t s, bool f64) {
     using namespace split;
-    const int S = slices ? slices : 5;
-    if (S < 2 || S > kMaxSlices) return fail(EG_ERROR_INVALID_ARGUMENT, "split form: slices must be in 2..6");
-    const int64_t kmax = max_k_per_pass(S);
-    int64_t Rmax = kBM, Kmaxp = kBK, zA = 0, zB = 0, rowsA = 0, rowsB = 0;
+    const int S = f64 ? kF64Slices : slices ? slices : 5, P = f64 ? S + 2 : S;
+    if (!f64 && (S < 2 || S > kMaxSlices)) return fail(EG_ERROR_INVALID_ARGUMENT, "split form: slices must be in 2..6");
+    const int64_t kmax = f64 ? kRowsMaxK : max_k_per_pass(S);
+    int64_t elemsA = 0, elemsB = 0, rowsA = 0, rowsB = 0;
     for (auto &c : cs) {
         if (c.k.total > kmax) return fail(EG_ERROR_NOT_SUPPORTED, "grouped split: K above one exact pass");
         if (c.k.total <= 0) return fail(EG_ERROR_NOT_SUPPORTED, "grouped split: an item sums over no index");
         if (c.m.total >= (1ll << 31) || c.n.total >= (1ll << 31) || c.k.total >= (1ll << 31))
             return fail(EG_ERROR_NOT_SUPPORTED, "grouped split: extent above 2^31");
-        Rmax = std::max({Rmax, round_up(c.m.total, kBM), round_up(c.n.total, kBN)});
-        Kmaxp = std::max(Kmaxp, round_up(c.k.total, kBK));
     }
     std::vector<GOp> opsA, opsB;
     std::vector<TcItem> items;
@@ -553,7 +721,10 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
         a.K = K;
         a.Kp = Kp;
         a.rowbase = rowsA;
-        a.zbase = zA;
+        // an item's planes are packed: its own rows, at a pitch of 32-byte multiples
+        a.pitch = round_up(K, 16);
+        a.pstride = M * a.pitch;
+        a.plane0 = elemsA;
         a.sr = mode_group_affine_stride(c.m, 0);
         a.sk = mode_group_affine_stride(c.k, 0);
         GOp b = a;
@@ -564,7 +735,8 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
         b.rows = N;
         b.Rp = Np;
         b.rowbase = rowsB;
-        b.zbase = zB;
+        b.pstride = N * b.pitch;
+        b.plane0 = elemsB;
         b.sr = mode_group_affine_stride(c.n, 1);
         b.sk = mode_group_affine_stride(c.k, 1);
         opsA.push_back(a);
@@ -574,8 +746,6 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
         it.M = M;
         it.N = N;
         it.nkb = (int)(Kp / kBK);
-        it.zA = (int)zA;
-        it.zB = (int)zB;
         it.eAoff = (int)rowsA;
         it.eBoff = (int)rowsB;
         it.Mp = (int)Mp;
@@ -590,10 +760,10 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
                     work.push_back({Kp, make_int4((int)i, (int)bb, (int)x, (int)y)});
         rowsA += nb * Mp;
         rowsB += nb * Np;
-        zA += nb * S;
-        zB += nb * S;
+        elemsA += round_up(nb * P * a.pstride, 64);
+        elemsB += round_up(nb * P * b.pstride, 64);
     }
-    if (zA >= (1ll << 31) || rowsA >= (1ll << 31) || rowsB >= (1ll << 31))
+    if (rowsA >= (1ll << 31) || rowsB >= (1ll << 31))
         return fail(EG_ERROR_NOT_SUPPORTED, "grouped split: batch too large");
     std::stable_sort(work.begin(), work.end(), [](auto &x, auto &y) { return x.first > y.first; });
     std::vector<int4> wl;
@@ -606,32 +776,40 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
     for (auto &op : ops) {
         int64_t oa, ob, oc;
         op.rtab = (int64_t)offs.size();
-        for (int64_t r = 0; r < op.rows; r++) {
+        for (int64_t r = 0; r < op.rows && !op.sr; r++) { // (none where one stride serves)
             group_offsets(op.rg, r, oa, ob, oc);
             offs.push_back(op.comp ? ob : oa);
         }
         op.ktab = (int64_t)offs.size();
-        for (int64_t k = 0; k < op.K; k++) {
+        for (int64_t k = 0; k < op.K && !op.sk; k++) {
             group_offsets(op.kg, k, oa, ob, oc);
             offs.push_back(op.comp ? ob : oa);
         }
     }
-    for (size_t i = 0; i < ops.size(); i++)
+    int64_t Kmax = 0;
+    for (const auto &op : ops) Kmax = std::max(Kmax, op.K);
+    const bool by_rows = Kmax <= kRowsMaxK;
+    size_t rows_smem = 0;
+    for (size_t i = 0; i < ops.size(); i++) {
+        int R = 32;
+        if (by_rows) {
+            while (R > 4 && (int64_t)R * ops[i].K > kRowsElems) R /= 2;
+            rows_smem = std::max(rows_smem, (size_t)R * rows_ld(ops[i].K) * 16); // two tiles
+        }
         for (int64_t bb = 0; bb < ops[i].nbatch; bb++)
-            for (int64_t r0 = 0; r0 < ops[i].rows; r0 += 32) units.push_back(make_int4((int)i, (int)bb, (int)r0, 0));
+            for (int64_t r0 = 0; r0 < ops[i].rows; r0 += R) units.push_back(make_int4((int)i, (int)bb, (int)r0, R));
+    }
     if (units.size() >= (size_t)INT_MAX) return fail(EG_ERROR_NOT_SUPPORTED, "grouped split: batch too large");
 
     void *planesA, *planesB, *eA, *eB, *d_ops, *d_units, *d_offs, *d_items, *d_work, *rbuf;
     eg_status st;
-    if ((st = dev_alloc(plan, rbuf_bytes(), &rbuf)) != EG_SUCCESS) return st;
-    const size_t pbytesA = (size_t)zA * Rmax * Kmaxp * 2, pbytesB = (size_t)zB * Rmax * Kmaxp * 2;
+    if ((st = dev_alloc(plan, rbuf_bytes(f64 ? 3 : 1), &rbuf)) != EG_SUCCESS) return st;
+    const size_t pbytesA = (size_t)elemsA * 2, pbytesB = (size_t)elemsB * 2;
     if ((st = dev_alloc(plan, pbytesA, &planesA)) != EG_SUCCESS) return st;
     if ((st = dev_alloc(plan, pbytesB, &planesB)) != EG_SUCCESS) return st;
     if ((st = dev_alloc(plan, (size_t)rowsA * 4, &eA)) != EG_SUCCESS) return st;
     if ((st = dev_alloc(plan, (size_t)rowsB * 4, &eB)) != EG_SUCCESS) return st;
-    // padded rows and K are never written by the splitting kernel: zero them once
-    EG_CUDA(cudaMemsetAsync(planesA, 0, pbytesA, s));
-    EG_CUDA(cudaMemsetAsync(planesB, 0, pbytesB, s));
+    // the exponents of padded rows are never written: zero them once
     EG_CUDA(cudaMemsetAsync(eA, 0, (size_t)rowsA * 4, s));
     EG_CUDA(cudaMemsetAsync(eB, 0, (size_t)rowsB * 4, s));
     if ((st = dev_copy(plan, ops.data(), ops.size() * sizeof(GOp), &d_ops)) != EG_SUCCESS) return st;
@@ -640,22 +818,18 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
     if ((st = dev_copy(plan, items.data(), items.size() * sizeof(TcItem), &d_items)) != EG_SUCCESS) return st;
     if ((st = dev_copy(plan, wl.data(), wl.size() * sizeof(int4), &d_work)) != EG_SUCCESS) return st;
 
-    CUtensorMap tmA, tmB;
-    if ((st = encode_planes_public(&tmA, planesA, Kmaxp, Rmax, zA)) != EG_SUCCESS) return st;
-    if ((st = encode_planes_public(&tmB, planesB, Kmaxp, Rmax, zB)) != EG_SUCCESS) return st;
     // per-item maps: each item's planes with its own M (N) and K as the extents
     std::vector<CUtensorMap> maps(2 * items.size());
     for (size_t i = 0; i < items.size(); i++) {
         const TcItem &it = items[i];
         const Contraction &c = cs[i];
         if (it.M == 0 || it.N == 0 || c.batch.total == 0) continue; // no tiles: the maps are never used
-        const int64_t planes = c.batch.total * S, K = c.k.total;
-        const size_t plane = (size_t)Rmax * Kmaxp;
-        if ((st = encode_planes_extent(&maps[2 * i], (__nv_bfloat16 *)planesA + (size_t)it.zA * plane, K, it.M, planes,
-                                       Kmaxp, Rmax)) != EG_SUCCESS)
+        const int64_t planes = c.batch.total * P, K = c.k.total;
+        if ((st = encode_planes_extent(&maps[2 * i], (__nv_bfloat16 *)planesA + opsA[i].plane0, K, it.M, planes,
+                                       opsA[i].pitch, it.M)) != EG_SUCCESS)
             return st;
-        if ((st = encode_planes_extent(&maps[2 * i + 1], (__nv_bfloat16 *)planesB + (size_t)it.zB * plane, K, it.N,
-                                       planes, Kmaxp, Rmax)) != EG_SUCCESS)
+        if ((st = encode_planes_extent(&maps[2 * i + 1], (__nv_bfloat16 *)planesB + opsB[i].plane0, K, it.N, planes,
+                                       opsB[i].pitch, it.N)) != EG_SUCCESS)
             return st;
     }
     void *d_maps = nullptr;
@@ -666,7 +840,7 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
     const Contraction &c0 = cs[0];
     TcGemmParams p{};
     p.S = S;
-    p.planes = S;
+    p.planes = P;
     p.nbatch = 1;
     p.cp = c0.cp;
     p.ab = c0.ab;
@@ -702,15 +876,38 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
     }
 
     if ((st = ensure_tc_attributes()) != EG_SUCCESS) return st;
+    if (by_rows) EG_CUDA(allow_grouped_rows(S, f64));
+    void *d_fma = nullptr, *redo = nullptr, *redo_count = nullptr;
+    if (f64) {
+        std::vector<F64Item> fma;
+        for (auto &c : cs) fma.push_back(f64_item(c));
+        if ((st = dev_copy(plan, fma.data(), fma.size() * sizeof(F64Item), &d_fma)) != EG_SUCCESS) return st;
+        if ((st = dev_alloc(plan, wl.size() * kTileRegions * sizeof(int4), &redo)) != EG_SUCCESS) return st;
+        if ((st = dev_alloc(plan, sizeof(int), &redo_count)) != EG_SUCCESS) return st;
+        p.hid = kF64High;
+        p.redo = (int4 *)redo;
+        p.redo_count = (int *)redo_count;
+    }
+    EG_CUDA(cudaEventCreateWithFlags(&plan.last, cudaEventDisableTiming));
     EG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     {
         CaptureGuard g;
         auto issue = [&]() -> eg_status {
-            launch_grouped_split(S, (const GOp *)d_ops, (const int4 *)d_units, (int)units.size(),
-                                 (const long long *)d_offs, (int *)eA, (int *)eB,
-                                 (__nv_bfloat16 *)planesA, (__nv_bfloat16 *)planesB, Rmax, Kmaxp, s);
-            EG_CHECK_LAUNCH("grouped digit splitting");
-            return launch_tc_gemm_grouped(tmA, tmB, p, (TcItem *)d_items, (int4 *)d_work, (int)wl.size(), s);
+            if (f64) EG_CUDA(cudaMemsetAsync(redo_count, 0, sizeof(int), s));
+            eg_status is =
+                by_rows ? launch_grouped_rows(S, f64, (const GOp *)d_ops, (const int4 *)d_units, (int)units.size(),
+                                              (const long long *)d_offs, (int *)eA, (int *)eB, (__nv_bfloat16 *)planesA,
+                                              (__nv_bfloat16 *)planesB, rows_smem, s)
+                        : launch_grouped_split(S, (const GOp *)d_ops, (const int4 *)d_units, (int)units.size(),
+                                               (const long long *)d_offs, (int *)eA, (int *)eB, (__nv_bfloat16 *)planesA,
+                                               (__nv_bfloat16 *)planesB, s);
+            if (is != EG_SUCCESS) return is;
+            is = launch_tc_gemm_grouped(maps[0], maps[1], p, (TcItem *)d_items, (int4 *)d_work, (int)wl.size(), s);
+            if (is != EG_SUCCESS || !f64) return is;
+            k_grouped_f64_listed<<<num_sms() * 4, THREADS, 0, s>>>((const F64Item *)d_fma, (const int4 *)redo,
+                                                                   (const int *)redo_count, c0.cp, c0.ab, p.zero);
+            EG_CHECK_LAUNCH("k_grouped_f64_listed");
+            return EG_SUCCESS;
         };
         st = issue();
     }
@@ -723,8 +920,8 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
     if (err != cudaSuccess) return cuda_fail(err, "cudaStreamEndCapture");
     plan.graph = graph;
     EG_CUDA(cudaGraphInstantiate(&plan.exec, graph, 0));
-    plan.kernels = 2;
-    plan.report = eg_split_report{S, S * (S + 1) / 2, kBits, error_bound(S)};
+    plan.kernels = f64 ? 3 : 2;
+    if (!f64) plan.report = eg_split_report{S, S * (S + 1) / 2, kBits, error_bound(S)};
     return EG_SUCCESS;
 }
 

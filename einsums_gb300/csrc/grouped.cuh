@@ -1,6 +1,7 @@
 // Grouped (batched) execution plans and the tile autotuner.
 #pragma once
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -34,9 +35,13 @@ struct Plan {
     eg_split_report report{};
     // per-role cycle counters of the tensor kernel, summed over replays (EINSUMS_GB300_TC_PROFILE)
     unsigned long long *prof = nullptr;
+    // plans with scratch of their own: a replay waits for the one before, on whatever stream
+    std::mutex mu;
+    cudaEvent_t last = nullptr;
     ~Plan();
 };
 eg_status build_f64_plan(Plan &plan, const std::vector<Contraction> &cs, cudaStream_t s);
-eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int slices, cudaStream_t s);
+bool f64_tensor_plan_pays(const std::vector<Contraction> &cs);
+eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int slices, cudaStream_t s, bool f64 = false);
 eg_status choose_f64_tiles(const std::vector<Contraction> &cs, cudaStream_t s, std::vector<int> &tiles);
 } // namespace eg::grouped

@@ -84,13 +84,23 @@ __device__ __forceinline__ void tma_load_3d_at(uint32_t dst, const void *tmap, u
                      : "memory");
 }
 
-// Asynchronous 8-byte copies into shared memory, and the wait for all of this thread's.
+// Asynchronous 8- and 16-byte copies into shared memory (the first form: zeros when not
+// valid), and the waits for this thread's: for all, or for all but the last N committed
+// groups.
+__device__ __forceinline__ void cp_async8(double *dst, const double *src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 8 : 0)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async8(double *dst, const double *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async16(double *dst, const double *src, bool valid) { // zeros when not valid
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0)
-                 : "memory");
+__device__ __forceinline__ void cp_async16(double *dst, const double *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 

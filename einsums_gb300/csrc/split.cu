@@ -182,15 +182,6 @@ __global__ void __launch_bounds__(T *TR, 5) k_split_rowmax(OperandMap m, const d
     }
 }
 
-// The exponent of a row whose largest |x| has the given bits: |x| < 2^e (INT_MIN for
-// a row holding an infinity or NaN, 0 for a row of zeros).
-__device__ __forceinline__ int row_exponent(unsigned long long bits) {
-    const int field = (int)(bits >> 52);
-    if (field == 0x7ff) return INT_MIN;
-    if (field) return field - 1022;
-    return bits ? -1010 - __clzll((long long)bits) : 0; // subnormal: 2^-1074 times the bits
-}
-
 __global__ void k_split_exponent(const unsigned long long *rowmax, int *e, int64_t n) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         e[i] = row_exponent(rowmax[i]);
@@ -209,17 +200,6 @@ __global__ void k_split_exponent(const unsigned long long *rowmax, int *e, int64
 // operand) bring tile t+1 into shared memory while tile t is converted.
 constexpr int TK = 2 * T;
 constexpr int64_t kDigitStrip = 8; // k tiles per work unit
-__device__ __forceinline__ void cp_async8(double *dst, const double *src, bool valid) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-//
-// CHECK (FP64 form): two more planes per operand, the lower bound of every
-// magnitude and the marks of the nonzero elements (split.cuh).
 template <int S, bool CHECK>
 __global__ void __launch_bounds__(T *TR) k_split_digits(OperandMap m, const double *__restrict__ X, const int *rexp,
                                                         __nv_bfloat16 *planes, int row_fast) {
@@ -251,7 +231,7 @@ __global__ void __launch_bounds__(T *TR) k_split_digits(OperandMap m, const doub
                 for (int j = ty; j < TK; j += TR) {
                     const int64_t k = k0 + j;
                     const bool ok = xr[0] && k < m.K;
-                    cp_async8(&tile[buf][tx][j], ok ? xr[0] + off_k(m, k) : X, ok);
+                    ptx::cp_async8(&tile[buf][tx][j], ok ? xr[0] + off_k(m, k) : X, ok);
                 }
             } else {
 #pragma unroll
@@ -262,11 +242,11 @@ __global__ void __launch_bounds__(T *TR) k_split_digits(OperandMap m, const doub
 #pragma unroll
                     for (int j = 0; j < RPT; j++) {
                         const bool ok = xr[j] && kin;
-                        cp_async8(&tile[buf][ty + TR * j][h * T + tx], ok ? xr[j] + okk : X, ok);
+                        ptx::cp_async8(&tile[buf][ty + TR * j][h * T + tx], ok ? xr[j] + okk : X, ok);
                     }
                 }
             }
-            cp_async_commit();
+            ptx::cp_async_commit();
         };
         const int64_t kt_beg = sg * kDigitStrip, kt_end = min(kt, (sg + 1) * kDigitStrip);
         load_tile(0, kt_beg * TK);
@@ -275,9 +255,9 @@ __global__ void __launch_bounds__(T *TR) k_split_digits(OperandMap m, const doub
             const int64_t k0 = ktile * TK;
             if (ktile + 1 < kt_end) {
                 load_tile(cur ^ 1, k0 + TK);
-                cp_async_wait<1>();
+                ptx::cp_async_wait<1>();
             } else {
-                cp_async_wait<0>();
+                ptx::cp_async_wait<0>();
             }
             __syncthreads();
             // write: thread tx converts k0 + 2tx and k0 + 2tx + 1 of each of its rows
@@ -345,45 +325,52 @@ __global__ void __launch_bounds__(kFusedThreads) k_split_rows(const __grid_const
     const int64_t k0 = (int64_t)rank * kc;
     const int nk = (int)max((int64_t)0, min((int64_t)kc, m.K - k0)); // real elements of this CTA's range
     const int64_t ob = off_b(m, b);
-    for (int k = tid; k < nk; k += kFusedThreads) koff[k] = off_k(m, k0 + k);
+    if (!m.sk)
+        for (int k = tid; k < nk; k += kFusedThreads) koff[k] = off_k(m, k0 + k);
     if (tid < R) roff[tid] = r0 + tid < m.rows ? ob + off_r(m, r0 + tid) : -1;
     __syncthreads();
-    const double *X = jj.X;
-    if (jj.row_fast) {
-        constexpr int KP = 32 / (R < 32 ? R : 32); // k a warp takes at a time
-        const int r = lane % R, kk = lane / R;
+    // k, k + step, ... of row r: copies of the real elements, then zeros (a single k
+    // stride is added up: the loop is two copies for it)
+    auto row_copy = [&](int r, int k, int step) {
         const int64_t ro = roff[r];
-        for (int k = warp * KP + kk; k < kc; k += W * KP) {
-            const bool ok = ro >= 0 && k < nk;
-            cp_async8(&tile[r * ld + k], ok ? X + ro + koff[k] : X, ok);
+        double *t = tile + r * ld;
+        if (ro >= 0) {
+            const double *x = jj.X + ro;
+            if (m.sk) {
+                const int64_t inc = (int64_t)step * m.sk;
+                x += (k0 + k) * m.sk;
+#pragma unroll 4
+                for (; k < nk; k += step, x += inc) ptx::cp_async8(t + k, x);
+            } else {
+#pragma unroll 4
+                for (; k < nk; k += step) ptx::cp_async8(t + k, x + koff[k]);
+            }
         }
+        for (; k < kc; k += step) t[k] = 0.0;
+    };
+    if (jj.row_fast) {
+        constexpr int KP = 32 / R; // k a warp takes at a time
+        row_copy(lane % R, warp * KP + lane / R, W * KP);
     } else if (jj.pairs) {
         for (int r = warp; r < R; r += W) {
             const int64_t ro = roff[r];
-            for (int k = 2 * lane; k < kc; k += 64) { // the real elements are even in number too
-                const bool ok = ro >= 0 && k < nk;
-                ptx::cp_async16(&tile[r * ld + k], ok ? X + ro + koff[k] : X, ok);
+            double *t = tile + r * ld;
+            int k = 2 * lane; // the real elements are even in number
+            if (ro >= 0) {
+                const double *x = jj.X + ro;
+#pragma unroll 4
+                for (; k < nk; k += 64) ptx::cp_async16(t + k, x + (m.sk ? k0 + k : koff[k]));
             }
+            for (; k < kc; k += 64) t[k] = t[k + 1] = 0.0;
         }
     } else {
-        for (int r = warp; r < R; r += W) {
-            const int64_t ro = roff[r];
-            for (int k = lane; k < kc; k += 32) {
-                const bool ok = ro >= 0 && k < nk;
-                cp_async8(&tile[r * ld + k], ok ? X + ro + koff[k] : X, ok);
-            }
-        }
+        for (int r = warp; r < R; r += W) row_copy(r, lane, 32);
     }
-    cp_async_commit();
-    cp_async_wait<0>();
+    ptx::cp_async_commit();
+    ptx::cp_async_wait<0>();
     __syncthreads();
     for (int r = warp; r < R; r += W) {
-        unsigned long long mx = 0;
-        for (int k = 2 * lane; k < kc; k += 64) {
-            const double2 v = *(const double2 *)&tile[r * ld + k];
-            mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
-        }
-        for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const unsigned long long mx = row_max_bits(tile + r * ld, kc, lane);
         if (lane == 0) pmax[r] = mx;
     }
     if (C > 1)
@@ -689,10 +676,6 @@ eg_status split_both(OperandMap oa, const double *A, int *eA, __nv_bfloat16 *pA,
 } // namespace eg::split
 
 namespace eg {
-
-eg_status encode_planes_public(CUtensorMap *map, void *base, int64_t Kp, int64_t rows, int64_t planes) {
-    return split::encode_planes(map, base, Kp, rows, planes);
-}
 
 int64_t mode_group_affine_stride(const ModeGroup &g, int comp) { return split::affine_stride(g, comp); }
 

@@ -88,8 +88,9 @@ struct TcGemmParams {
     int64_t b0, m0, n0;
     // FP64 form (redo set): the exact sums do not fit 64 bits, so the slice groups
     // below hid form one int64 sum and the others a second; a 32 x 64 block of
-    // outputs whose accuracy check fails is left alone and listed in redo
-    // ({batch, row, column}, redo_count entries) for the FMA kernel.
+    // outputs whose accuracy check fails is left alone and listed in redo ({batch, row,
+    // column}, in grouped launches {item, batch, row, column}; redo_count entries) for
+    // the FMA kernel.
     int hid;
     int4 *redo;
     int *redo_count;
@@ -99,14 +100,13 @@ struct TcGemmParams {
     const CUtensorMap *item_maps;
 };
 
-// One item of a grouped launch: an independent contraction whose digit planes
-// start at plane zA / zB of the shared plane arrays and whose exponents start
-// at eAoff / eBoff.  Work entries (int4) are {item, batch index, mt, nt}.
+// One item of a grouped launch: an independent contraction whose digit planes have
+// tensor maps of their own (TcGemmParams::item_maps) and whose exponents start at
+// eAoff / eBoff.  Work entries (int4) are {item, batch index, mt, nt}.
 struct TcItem {
     double *C;
     int64_t M, N;
     int nkb;
-    int zA, zB;
     int eAoff, eBoff;
     int Mp, Np;
     ModeGroup bg, mg, ng;
@@ -124,6 +124,33 @@ __device__ __forceinline__ unsigned long long bits_of(double x) {
 // IEEE bit pattern of |x|: for non-negative doubles (and NaN above Inf) the
 // unsigned order of the patterns is the numeric order.
 __device__ __forceinline__ unsigned long long abs_bits(double x) { return bits_of(x) & 0x7FFFFFFFFFFFFFFFull; }
+
+// The exponent of a row whose largest |x| has the given bits: |x| < 2^e (INT_MIN for
+// a row holding an infinity or NaN, 0 for a row of zeros).
+__device__ __forceinline__ int row_exponent(unsigned long long bits) {
+    const int field = (int)(bits >> 52);
+    if (field == 0x7ff) return INT_MIN;
+    if (field) return field - 1022;
+    return bits ? -1010 - __clzll((long long)bits) : 0; // subnormal: 2^-1074 times the bits
+}
+
+// For row_exponent: the largest |x|'s bits among n values of a row in shared memory
+// (16-byte aligned, readable and zero up to an even count), found by a warp.  The
+// exponent field decides, so the upper words do, at two instructions a value and with a
+// lower word of zero, unless all are subnormal.
+__device__ __forceinline__ unsigned long long row_max_bits(const double *row, int n, int lane) {
+    uint32_t mx = 0;
+    for (int k = 2 * lane; k < n; k += 64) {
+        const uint4 v = *(const uint4 *)&row[k];
+        mx = max(mx, max(v.y & 0x7FFFFFFFu, v.w & 0x7FFFFFFFu));
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (mx >= 0x00100000u) return (unsigned long long)mx << 32;
+    unsigned long long m = 0;
+    for (int k = lane; k < n; k += 32) m = max(m, abs_bits(row[k]));
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    return m;
+}
 
 // round(x * 2^sh) to nearest, ties to even, for |x| 2^sh < 2^63, built from the
 // IEEE fields with integer operations (the FP64 pipe of this GPU runs about two

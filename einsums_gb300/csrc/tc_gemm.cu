@@ -95,7 +95,8 @@ struct TileJob {
     const ModeGroup *mg, *ng;
     const int *eA, *eB; // exponents of rows / columns of this (item, batch)
     double *C;          // output base of this (item, batch)
-    int b;              // batch index (single-contraction form)
+    int b;              // batch index
+    int item;           // item of a grouped launch
     const CUtensorMap *mapA, *mapB; // per-item maps (grouped launches), else null
 };
 
@@ -136,15 +137,10 @@ __device__ __forceinline__ TileJob resolve(const TcGemmParams &p, const TcItem *
         const int b = w.y;
         j.mt = w.z;
         j.nt = w.w;
-        if (p.item_maps) { // planes numbered within the item
-            j.mapA = p.item_maps + 2 * w.x;
-            j.mapB = j.mapA + 1;
-            j.zA = j.zB = b * p.S;
-        } else {
-            j.mapA = j.mapB = nullptr;
-            j.zA = it.zA + b * p.S;
-            j.zB = it.zB + b * p.S;
-        }
+        j.mapA = p.item_maps + 2 * w.x;
+        j.mapB = j.mapA + 1;
+        j.zA = j.zB = b * p.planes; // planes are numbered within the item
+        j.item = w.x;
         j.kbeg = 0;
         j.nkb = it.nkb;
         j.split = false;
@@ -240,7 +236,6 @@ __global__ void __launch_bounds__(THREADS, 1)
                     const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ TcGemmParams p,
                     const TcItem *items, const int4 *work, int ntiles_total) {
     static_assert(CL == 1 || (CL == 2 && !GROUPED), "CTA pairs serve single contractions");
-    static_assert(!F64 || !GROUPED, "the FP64 form serves single contractions");
     constexpr int PLANES = F64 ? 2 : 1; // int64 sums per output in the K slices' accumulator
     constexpr size_t kPlane = (size_t)kBM * kBN;
     const int qbeg = F64 ? -1 : 0, qend = step_count(p);
@@ -319,7 +314,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const int row0 = (isB ? job.nt : job.mt) * kBM, z0 = isB ? job.zB : job.zA;
                 const int kc0 = (p.kb0 + job.kbeg) * kBK, nkb = job.nkb;
                 const void *map = isB ? &tmB : &tmA;
-                if (GROUPED && job.mapA) {
+                if (GROUPED) {
                     map = isB ? job.mapB : job.mapA;
                     if (leader) {
                         if (tile + ctas < total_tiles) // the next tile's map, while this one runs
@@ -740,7 +735,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                 finish = false;
                 if (lane == 0) {
                     const int at = atomicAdd(p.redo_count, 1);
-                    p.redo[at] = make_int4(job.b, (int)p.m0 + job.mt * kBM + quad * 32, (int)p.n0 + job.nt * kBN + col0, 0);
+                    const int m0 = job.mt * kBM + quad * 32, n0 = job.nt * kBN + col0;
+                    p.redo[at] = GROUPED ? make_int4(job.item, job.b, m0, n0)
+                                         : make_int4(job.b, (int)p.m0 + m0, (int)p.n0 + n0, 0);
                 }
             }
             if (!finish || live == 0) continue;
@@ -797,7 +794,7 @@ eg_status ensure_tc_attributes() {
     std::call_once(once, [] {
         for (const void *f : {(const void *)k_tc_split_gemm<false, 1, false>, (const void *)k_tc_split_gemm<true, 1, false>,
                               (const void *)k_tc_split_gemm<false, 2, false>, (const void *)k_tc_split_gemm<false, 1, true>,
-                              (const void *)k_tc_split_gemm<false, 2, true>})
+                              (const void *)k_tc_split_gemm<false, 2, true>, (const void *)k_tc_split_gemm<true, 1, true>})
             if (err == cudaSuccess) err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     });
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(k_tc_split_gemm)");
@@ -886,8 +883,11 @@ eg_status launch_tc_gemm_grouped(const CUtensorMap &tmA, const CUtensorMap &tmB,
     if (ntiles_total <= 0) return EG_SUCCESS;
     const int grid = ntiles_total < num_sms() ? ntiles_total : num_sms();
     {
-        LaunchScope ls_("k_tc_split_gemm_grouped", s);
-        k_tc_split_gemm<true, 1, false><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmB, p, items, work, ntiles_total);
+        LaunchScope ls_(p.redo ? "k_tc_split_gemm_grouped_f64" : "k_tc_split_gemm_grouped", s);
+        if (p.redo)
+            k_tc_split_gemm<true, 1, true><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmB, p, items, work, ntiles_total);
+        else
+            k_tc_split_gemm<true, 1, false><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmB, p, items, work, ntiles_total);
     }
     EG_CHECK_LAUNCH("k_tc_split_gemm_grouped");
     return EG_SUCCESS;

@@ -209,3 +209,81 @@ def test_streams_and_threads_share_the_scratch(eg):
     for A, B, Cs, want in sets:
         for C in Cs:
             assert np.allclose(C.cpu().numpy(), want, rtol=0, atol=1e-11)
+
+
+def launches():
+    from einsums_gb300 import _lib
+    n = ctypes.c_uint64()
+    _lib.check(_lib.load().eg_kernel_launches(ctypes.byref(n)))
+    return n.value
+
+
+@pytest.mark.parametrize("pattern", [("ab", "ija", "ijb"), ("zab", "zai", "zbi")])
+def test_lists(eg, pattern):
+    """A list long enough for the tensor cores (three kernels a replay): items of one and of several
+    tiles, hard items among them, replays on changed inputs and on two streams; the FMA plan under a
+    memory budget."""
+    from einsums_gb300 import _lib
+    Cl, Al, Bl = pattern
+    rng = np.random.default_rng(len(Cl))
+    As, Bs = [], []
+    for q in range(300):
+        d = dict(i=int(rng.integers(9, 33)), j=int(rng.integers(9, 33)), a=int(rng.integers(40, 130)),
+                 b=int(rng.integers(40, 130)), z=1 + q % 2)
+        if q == 0:
+            d = dict(i=32, j=34, a=300, b=7, z=3)
+        As.append(rng.standard_normal([d[c] for c in Al]))
+        Bs.append(rng.standard_normal([d[c] for c in Bl]))
+    if Cl == "ab":  # graded against each other over the summed indices, an infinity, a row of zeros
+        g = 10.0 ** np.linspace(-9, 9, As[5].shape[0])[:, None, None]
+        As[5], Bs[5] = As[5] * g, Bs[5] / g
+        As[6][0, 0, 3] = np.inf
+        Bs[7][:, :, 2] = 0.0
+    tA, tB = [cu(x) for x in As], [cu(x) for x in Bs]
+    want = lambda k: np.einsum(f"{Al},{Bl}->{Cl}", As[k], Bs[k])
+    scale = lambda k: np.einsum(f"{Al},{Bl}->{Cl}", np.abs(As[k]), np.abs(Bs[k]))
+
+    def check(tC, factor=1.0):
+        for k in range(len(As)):
+            K = As[k].size // tC[k].shape[-2] // (As[k].shape[0] if Cl == "zab" else 1)
+            with np.errstate(invalid="ignore"):
+                w, s, got = want(k) * factor, scale(k), tC[k].cpu().numpy()
+                off = np.abs(got - w)
+            fin = np.isfinite(s)
+            assert np.all(off[fin] <= 2 * (K + 4) * U * s[fin] * abs(factor)), k
+            assert np.array_equal(np.isfinite(got), np.isfinite(w)), k
+
+    empty = lambda: [torch.full(want(k).shape, float("nan"), dtype=torch.float64, device="cuda") for k in range(len(As))]
+    tC = empty()
+    plan = eg.GroupedPlan(0.0, Cl, tC, 1.0, Al, tA, Bl, tB)
+    n = launches()
+    plan.execute()
+    assert launches() - n == 3
+    torch.cuda.synchronize()
+    check(tC)
+    for t in tA:
+        t.mul_(-2.0)
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(3):  # each replay writes all of C; they share the plan's scratch
+        plan.execute(stream=s1)
+        plan.execute(stream=s2)
+    torch.cuda.synchronize()
+    check(tC, -2.0)
+    plan.close()
+    for t in tA:
+        t.mul_(-0.5)
+    used = ctypes.c_size_t()
+    _lib.check(_lib.load().eg_memory_in_use(ctypes.byref(used)))
+    try:
+        _lib.check(_lib.load().eg_set_memory_budget(used.value + (64 << 20)))
+        tC = empty()
+        plan = eg.GroupedPlan(0.0, Cl, tC, 1.0, Al, tA, Bl, tB)
+        n = launches()
+        plan.execute()
+        assert launches() - n == 1
+        torch.cuda.synchronize()
+        check(tC)
+        plan.close()
+    finally:
+        _lib.check(_lib.load().eg_set_memory_budget(0))
