@@ -15,7 +15,9 @@
 // Arithmetic follows HPTT, the reference's host transposer: cp == 0 stores
 // ap*A without reading C (a plain copy when ap == 1, so the copy is bit-exact),
 // otherwise ap*A + cp*C without fused multiply-adds.
+#include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -46,44 +48,90 @@ __device__ __forceinline__ void rest_offsets(const PermuteMap &r, int64_t i, int
     }
 }
 
-template <int MODE> // 0: copy, 1: ap*a (cp == 0), 2: ap*a + cp*c
+// 0: copy, 1: ap*a (cp == 0), 2: ap*a + cp*c, 3: c + a or c - a (cp == 1, ap == +-1).
+// The last saves two of three FP64 operations, the same bits: three an element take the
+// pipe 75 us for 15e6 elements, as long as memory takes.
+template <int MODE>
 __device__ __forceinline__ double combine(double a, const double *c, double ap, double cp) {
     if (MODE == 0) return a;
     if (MODE == 1) return __dmul_rn(ap, a);
+    if (MODE == 3) {
+        const long long sign = __double_as_longlong(ap) & (long long)(1ull << 63);
+        return __dadd_rn(__longlong_as_double(__double_as_longlong(a) ^ sign), *c);
+    }
     return __dadd_rn(__dmul_rn(ap, a), __dmul_rn(cp, *c));
 }
 
-// Fastest modes shared: rows of length L with strides sa/sc along the row.  A
-// warp takes a chunk of up to kRowChunk elements of one row (the decomposition
-// of the row index is paid once per chunk) and keeps four loads in flight.
-constexpr int64_t kRowChunk = 2048;
+// Fastest modes shared: rows of length L with strides sa/sc along the row, in elements
+// of T -- double, or double2 when rows are contiguous and every address is on a 16-byte
+// boundary.  A warp takes kRowChunk elements: a chunk of one row, or as many whole rows
+// as make it up, NR at a time.  The decomposition of the row index is paid once per run
+// along the fastest rest mode; eight loads of a thread are in flight (NR rows of 8 / NR
+// each), so rows shorter than 256 elements keep as many as long ones.  Bound: memory.
+// Rows of 126: 15e6 elements in 49 us (5.0 TB/s), scaled in place of a copy 47 us; a warp
+// per row took 54 us.
+constexpr int kRowChunk = 2048;
+
+__host__ __device__ inline int rows_per_unit(int64_t L) { return L >= kRowChunk ? 1 : kRowChunk / (int)(L < 1 ? 1 : L); }
+
 template <int MODE>
+__device__ __forceinline__ double2 combine(double2 a, const double2 *c, double ap, double cp) {
+    return make_double2(combine<MODE>(a.x, &c->x, ap, cp), combine<MODE>(a.y, &c->y, ap, cp));
+}
+
+template <int MODE, typename T, int NR>
 __global__ void __launch_bounds__(256) k_permute_rows(PermuteMap rest, int64_t L, int64_t sa, int64_t sc,
-                                                      const double *__restrict__ A, double *C, double ap, double cp) {
+                                                      const T *__restrict__ A, T *C, double ap, double cp) {
+    constexpr int Q = 8 / NR; // loads of a row at a time
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = rows_per_unit(L);
     const int64_t chunks = (L + kRowChunk - 1) / kRowChunk;
-    const int64_t units = rest.total * chunks;
+    const int64_t groups = (rest.total + per - 1) / per, units = groups * chunks;
+    const int last = rest.n - 1;
+    const int64_t run = rest.n ? rest.ext[last] : 1, runA = rest.n ? rest.sA[last] : 0, runC = rest.n ? rest.sC[last] : 0;
     for (int64_t u = (int64_t)blockIdx.x * 8 + warp; u < units; u += (int64_t)gridDim.x * 8) {
-        const int64_t row = u / chunks, ch = u - row * chunks;
-        int64_t oa, oc;
-        rest_offsets(rest, row, oa, oc);
-        const double *a = A + oa;
-        double *c = C + oc;
-        const int64_t x0 = ch * kRowChunk, x1 = min(L, x0 + kRowChunk);
-        int64_t x = x0 + lane;
-        for (; x + 96 < x1; x += 128) {
-            double v[4];
+        const int64_t grp = u / chunks, x0 = (u - grp * chunks) * kRowChunk;
+        const int len = (int)min((int64_t)kRowChunk, L - x0); // this chunk's part of a row
+        const int64_t row0 = grp * per;
+        const int rows = (int)min((int64_t)per, rest.total - row0);
+        int64_t oa, oc, left = run - row0 % run; // rows to the end of the run along the fastest rest mode
+        rest_offsets(rest, row0, oa, oc);
+        for (int r = 0; r < rows; r += NR) {
+            const T *a[NR];
+            T *c[NR];
 #pragma unroll
-            for (int q = 0; q < 4; q++) v[q] = __ldg(a + (x + 32 * q) * sa);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                double *cptr = c + (x + 32 * q) * sc;
-                *cptr = combine<MODE>(v[q], cptr, ap, cp);
+            for (int k = 0; k < NR; k++) {
+                a[k] = A + oa + (x0 + lane) * sa;
+                c[k] = C + oc + (x0 + lane) * sc;
+                if (--left > 0 || r + k + 1 >= rows) {
+                    oa += runA;
+                    oc += runC;
+                } else {
+                    left = run;
+                    rest_offsets(rest, row0 + r + k + 1, oa, oc);
+                }
             }
-        }
-        for (; x < x1; x += 32) {
-            double *cptr = c + x * sc;
-            *cptr = combine<MODE>(__ldg(a + x * sa), cptr, ap, cp);
+            for (int xb = lane; xb < len; xb += 32 * Q) {
+                T v[NR][Q], old[NR][Q];
+#pragma unroll
+                for (int k = 0; k < NR; k++)
+#pragma unroll
+                    for (int q = 0; q < Q; q++) {
+                        const bool in = r + k < rows && xb + 32 * q < len;
+                        v[k][q] = in ? __ldg(a[k] + 32 * q * sa) : T{};
+                        if (MODE >= 2) old[k][q] = in ? c[k][32 * q * sc] : T{};
+                    }
+#pragma unroll
+                for (int k = 0; k < NR; k++)
+#pragma unroll
+                    for (int q = 0; q < Q; q++)
+                        if (r + k < rows && xb + 32 * q < len) c[k][32 * q * sc] = combine<MODE>(v[k][q], &old[k][q], ap, cp);
+#pragma unroll
+                for (int k = 0; k < NR; k++) {
+                    a[k] += 32 * Q * sa;
+                    c[k] += 32 * Q * sc;
+                }
+            }
         }
     }
 }
@@ -91,14 +139,19 @@ __global__ void __launch_bounds__(256) k_permute_rows(PermuteMap rest, int64_t L
 constexpr int TILE = 32, ROWS = 8;
 constexpr int64_t kStrip = 8; // tiles along C's fastest mode per work unit
 
+constexpr int kTileStages = 4; // tiles of a strip in shared memory: three in flight while one is written
+
 // ia runs along A's fastest mode (extent EA, strides saA in A / scA in C);
 // ic runs along C's fastest mode (extent EC, strides saC in A / scC in C).
+// Bound: memory; the tiles of a strip arrive by asynchronous copies, three ahead, and
+// with C_prefactor the old values of C are loaded a tile ahead.  15e6 elements: 43 us
+// (5.7 TB/s), accumulating 66 us (5.6 TB/s); one tile at a time 54 and 110 us.
 template <int MODE>
 __global__ void __launch_bounds__(TILE *ROWS) k_permute_tiles(PermuteMap rest, int64_t EA, int64_t EC, int64_t saA,
                                                               int64_t scA, int64_t saC, int64_t scC,
                                                               const double *__restrict__ A, double *C, double ap,
                                                               double cp) {
-    __shared__ double tile[TILE][TILE + 1];
+    __shared__ double tile[kTileStages][TILE][TILE + 1];
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int64_t tilesA = (EA + TILE - 1) / TILE, tilesC = (EC + TILE - 1) / TILE;
     // a work unit is a strip: one index of the rest modes, one tile row along A's
@@ -114,29 +167,48 @@ __global__ void __launch_bounds__(TILE *ROWS) k_permute_tiles(PermuteMap rest, i
         const double *Ar = A + oa + (a0 + tx) * saA;       // this thread's reads: ia = a0 + tx
         const bool a_in = a0 + tx < EA;
         const int64_t cbeg = sg * kStrip * TILE, cend = min(EC, cbeg + kStrip * TILE);
-        for (int64_t c0 = cbeg; c0 < cend; c0 += TILE) {
-            // read: consecutive threads walk A's fastest mode
-#pragma unroll
-            for (int j = 0; j < TILE; j += ROWS) {
-                const int64_t ic = c0 + ty + j;
-                if (a_in && ic < cend) tile[ty + j][tx] = __ldg(Ar + ic * saC);
-            }
-            __syncthreads();
-            // write: consecutive threads walk C's fastest mode
-            const int64_t ic = c0 + tx;
-            if (ic < cend) {
-                double *Cc = C + oc + ic * scC;
+        const int n = (int)((cend - cbeg + TILE - 1) / TILE);
+        auto load = [&](int t) { // consecutive threads walk A's fastest mode
+            if (t < n && a_in) {
 #pragma unroll
                 for (int j = 0; j < TILE; j += ROWS) {
-                    const int64_t ia = a0 + ty + j;
-                    if (ia < EA) {
-                        double *cptr = Cc + ia * scA;
-                        *cptr = combine<MODE>(tile[tx][ty + j], cptr, ap, cp);
-                    }
+                    const int64_t ic = cbeg + t * TILE + ty + j;
+                    if (ic < cend) ptx::cp_async8(&tile[t % kTileStages][ty + j][tx], Ar + ic * saC);
                 }
             }
-            __syncthreads();
+            ptx::cp_async_commit();
+        };
+        double old[TILE / ROWS], next[TILE / ROWS]; // C's old values at this thread's writes of this and the next tile
+        auto load_old = [&](int t, double (&o)[TILE / ROWS]) {
+            const int64_t ic = cbeg + t * TILE + tx; // consecutive threads walk C's fastest mode
+#pragma unroll
+            for (int j = 0; j < TILE / ROWS; j++) {
+                const int64_t ia = a0 + ty + j * ROWS;
+                o[j] = ic < cend && ia < EA ? C[oc + ic * scC + ia * scA] : 0.0;
+            }
+        };
+        for (int t = 0; t < kTileStages - 1; t++) load(t);
+        if (MODE >= 2) load_old(0, next);
+        for (int t = 0; t < n; t++) {
+            if (MODE >= 2) {
+#pragma unroll
+                for (int j = 0; j < TILE / ROWS; j++) old[j] = next[j];
+                if (t + 1 < n) load_old(t + 1, next);
+            }
+            const int64_t ic = cbeg + t * TILE + tx;
+            double *Cc = C + oc + ic * scC;
+            ptx::cp_async_wait<kTileStages - 2>();
+            __syncthreads(); // tile t has landed for every thread, and tile t - 1 is read
+            load(t + kTileStages - 1);
+            if (ic < cend) {
+#pragma unroll
+                for (int j = 0; j < TILE / ROWS; j++) {
+                    const int64_t ia = a0 + ty + j * ROWS;
+                    if (ia < EA) Cc[ia * scA] = combine<MODE>(tile[t % kTileStages][tx][ty + j * ROWS], &old[j], ap, cp);
+                }
+            }
         }
+        __syncthreads(); // the strip's last tiles are read before the next one's replace them
     }
 }
 
@@ -313,7 +385,7 @@ eg_status encode_tiled_f64(CUtensorMap *map, const void *base, int rank, const u
 struct PermuteLaunch {
     bool empty = false;
     bool rows = false; // fastest modes shared: row copies, else tiles
-    int mode = 0;      // 0: copy, 1: ap*a, 2: ap*a + cp*c
+    int mode = 0;      // of combine()
     int grid = 0;
     PermuteMap rest;
     int64_t L = 0, sa = 0, sc = 0;                                 // rows
@@ -363,7 +435,7 @@ PermuteLaunch prepare_permute(const PermuteDesc &p) {
         return best;
     };
     const int fa = argmin(sA), fc = argmin(sC);
-    pl.mode = (p.cp == 0.0) ? (p.ap == 1.0 ? 0 : 1) : 2;
+    pl.mode = p.cp == 0.0 ? (p.ap == 1.0 ? 0 : 1) : (p.cp == 1.0 && (p.ap == 1.0 || p.ap == -1.0) ? 3 : 2);
     const int cap = num_sms() * 16;
     for (int d = 0; d < n; d++) {
         if (d == fa || d == fc) continue;
@@ -378,8 +450,6 @@ PermuteLaunch prepare_permute(const PermuteDesc &p) {
         pl.L = ext[fc];
         pl.sa = sA[fc];
         pl.sc = sC[fc];
-        const int64_t work = (pl.rest.total * ((pl.L + kRowChunk - 1) / kRowChunk) + 7) / 8;
-        pl.grid = (int)(work < cap ? work : cap);
         return pl;
     }
     pl.EA = ext[fa];
@@ -509,14 +579,46 @@ eg_status run_permute(const PermuteLaunch &pl, const double *A, double *C, cudaS
         set_error(""); // the tile kernel below takes the case the TMA form declined
     }
     if (pl.rows) {
+        bool pairs = pl.sa == 1 && pl.sc == 1 && pl.L % 2 == 0 && (((uintptr_t)A | (uintptr_t)C) & 15) == 0;
+        for (int d = 0; d < pl.rest.n; d++) pairs = pairs && pl.rest.sA[d] % 2 == 0 && pl.rest.sC[d] % 2 == 0;
+        PermuteMap rest = pl.rest;
+        int64_t L = pl.L;
+        if (pairs) {
+            L /= 2;
+            for (int d = 0; d < rest.n; d++) {
+                rest.sA[d] /= 2;
+                rest.sC[d] /= 2;
+            }
+        }
+        const int64_t per = rows_per_unit(L);
+        const int64_t work = ((rest.total + per - 1) / per * ((L + kRowChunk - 1) / kRowChunk) + 7) / 8;
+        const int grid = (int)std::min<int64_t>(work, (int64_t)num_sms() * 16);
+        auto go = [&](auto mode, auto nr) {
+            constexpr int MODE = decltype(mode)::value, NR = decltype(nr)::value;
+            if (pairs)
+                k_permute_rows<MODE, double2, NR><<<grid, 256, 0, s>>>(rest, L, 1, 1, (const double2 *)A, (double2 *)C,
+                                                                       pl.ap, pl.cp);
+            else
+                k_permute_rows<MODE, double, NR><<<grid, 256, 0, s>>>(rest, L, pl.sa, pl.sc, A, C, pl.ap, pl.cp);
+        };
+        auto rows_at_once = [&](auto mode) {
+            if (L <= 64)
+                go(mode, std::integral_constant<int, 4>{});
+            else if (L <= 128)
+                go(mode, std::integral_constant<int, 2>{});
+            else
+                go(mode, std::integral_constant<int, 1>{});
+        };
         {
             LaunchScope ls_("k_permute_rows", s);
             if (pl.mode == 0)
-                k_permute_rows<0><<<pl.grid, 256, 0, s>>>(pl.rest, pl.L, pl.sa, pl.sc, A, C, pl.ap, pl.cp);
+                rows_at_once(std::integral_constant<int, 0>{});
             else if (pl.mode == 1)
-                k_permute_rows<1><<<pl.grid, 256, 0, s>>>(pl.rest, pl.L, pl.sa, pl.sc, A, C, pl.ap, pl.cp);
+                rows_at_once(std::integral_constant<int, 1>{});
+            else if (pl.mode == 2)
+                rows_at_once(std::integral_constant<int, 2>{});
             else
-                k_permute_rows<2><<<pl.grid, 256, 0, s>>>(pl.rest, pl.L, pl.sa, pl.sc, A, C, pl.ap, pl.cp);
+                rows_at_once(std::integral_constant<int, 3>{});
         }
         EG_CHECK_LAUNCH("k_permute_rows");
         return EG_SUCCESS;
@@ -530,8 +632,11 @@ eg_status run_permute(const PermuteLaunch &pl, const double *A, double *C, cudaS
         else if (pl.mode == 1)
             k_permute_tiles<1><<<pl.grid, block, 0, s>>>(pl.rest, pl.EA, pl.EC, pl.saA, pl.scA, pl.saC, pl.scC, A, C,
                                                         pl.ap, pl.cp);
-        else
+        else if (pl.mode == 2)
             k_permute_tiles<2><<<pl.grid, block, 0, s>>>(pl.rest, pl.EA, pl.EC, pl.saA, pl.scA, pl.saC, pl.scC, A, C,
+                                                        pl.ap, pl.cp);
+        else
+            k_permute_tiles<3><<<pl.grid, block, 0, s>>>(pl.rest, pl.EA, pl.EC, pl.saA, pl.scA, pl.saC, pl.scC, A, C,
                                                         pl.ap, pl.cp);
     }
     EG_CHECK_LAUNCH("k_permute_tiles");
