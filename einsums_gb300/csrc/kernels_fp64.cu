@@ -293,13 +293,37 @@ __global__ void __launch_bounds__(256) k_gemv(ModeGroup rows, ModeGroup k, const
     }
 }
 
+// Adds RB values of each lane over the warp: lane q < RB (spread over the lanes: the
+// bits of a lane above the lowest log2(32 / RB)) ends up with the sum of value q.  Each
+// step halves the values a lane holds, so four sums take 6 additions a lane, not 20 (the
+// FP64 pipe bounds the kernel below).
+template <int RB>
+__device__ __forceinline__ double warp_sums(double (&v)[RB], int lane, int &which) {
+    which = 0;
+    int o = 16;
+#pragma unroll
+    for (int n = RB; n > 1; n /= 2, o /= 2) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int q = 0; q < n / 2; q++) {
+            const double keep = up ? v[q + n / 2] : v[q], give = up ? v[q] : v[q + n / 2];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+        which = 2 * which + (up ? 1 : 0);
+    }
+    for (; o > 0; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
 // Long k: one CTA takes RB outputs at a time, each k of B (the vector, shared
-// by every output) and each pair of table offsets is loaded once and used for
-// RB rows of A, so the vector's L1 traffic and the reductions are divided by
-// RB.  Contig: k is one mode of stride 1 in A and B (with 16-byte pairs when
-// aligned); otherwise offk[0..K) / offk[K..2K) hold the offsets of every k in A
-// and B.
-template <int RB, bool Contig>
+// by every output) is loaded once and used for RB rows of A, so the vector's L1 traffic
+// is divided by RB.  Bound: the FP64 pipe at two FMAs per clock per SM, 8 bytes of A
+// each (5 TB/s), ahead of memory.  10^4 rows of 10^4: one run 188 us, nested runs 203 us
+// (208 us with a tree per row, 227 us with offset tables).  FORM 0: k is one mode of stride 1 in A and B, with
+// 16-byte pairs when aligned; 1: two modes, the inner of stride 1 in both, walked by a
+// running index (r, s) per thread; 2: offk[0..K) / offk[K..2K) hold the offsets of every
+// k in A and B.
+template <int RB, int FORM>
 __global__ void __launch_bounds__(256) k_gemv_rows(ModeGroup rows, ModeGroup k, const double *__restrict__ A,
                                                    const double *__restrict__ B, double *C, double cp, double ab,
                                                    bool zero, const int64_t *__restrict__ offk) {
@@ -323,55 +347,70 @@ __global__ void __launch_bounds__(256) k_gemv_rows(ModeGroup rows, ModeGroup k, 
         double acc[RB];
 #pragma unroll
         for (int q = 0; q < RB; q++) acc[q] = 0.0;
-        if (Contig && aligned) {
+        auto pair = [&](int64_t oa, int64_t ob) {
+            const double2 y = __ldg((const double2 *)(b + ob));
+            double2 x[RB];
+#pragma unroll
+            for (int q = 0; q < RB; q++) x[q] = __ldg((const double2 *)(a[q] + oa));
+#pragma unroll
+            for (int q = 0; q < RB; q++) acc[q] = fma(x[q].y, y.y, fma(x[q].x, y.x, acc[q]));
+        };
+        auto single = [&](int64_t oa, int64_t ob) {
+            const double y = __ldg(b + ob);
+#pragma unroll
+            for (int q = 0; q < RB; q++) acc[q] = fma(__ldg(a[q] + oa), y, acc[q]);
+        };
+        if (FORM == 0 && aligned) {
             const int64_t K2 = K / 2;
             // CTAs start at different points of k so that concurrently read rows
             // (a fixed stride apart) do not hit the same memory channels in step
             const int64_t start = K2 > 4096 ? ((r0 / RB) * 1031 % (K2 / 256)) * 256 : 0;
-            auto body = [&](int64_t j) {
-                const double2 y = __ldg((const double2 *)b + j);
-#pragma unroll
-                for (int q = 0; q < RB; q++) {
-                    const double2 x = __ldg((const double2 *)a[q] + j);
-                    acc[q] = fma(x.x, y.x, acc[q]);
-                    acc[q] = fma(x.y, y.y, acc[q]);
+#pragma unroll 2
+            for (int64_t j = start + tid; j < K2; j += 256) pair(2 * j, 2 * j);
+#pragma unroll 2
+            for (int64_t j = tid; j < start; j += 256) pair(2 * j, 2 * j);
+            if ((K & 1) && tid == 0) single(K - 1, K - 1);
+        } else if (FORM == 0) {
+#pragma unroll 2
+            for (int64_t i = tid; i < K; i += 256) single(i, i);
+        } else if (FORM == 1) {
+            // the inner mode's pairs are aligned when its extent and all other strides are even
+            const int64_t sa = k.s[0][0], sb = k.s[1][0];
+            const bool pairs = aligned && k.ext[1] % 2 == 0 && sa % 2 == 0 && sb % 2 == 0;
+            const int w = pairs ? 2 : 1;
+            const uint32_t inner = (uint32_t)(k.ext[1] / w), n = (uint32_t)(K / w);
+            const uint32_t dr = 256u / inner, ds = 256u - dr * inner;
+            uint32_t r = (uint32_t)tid / inner, s = (uint32_t)tid - r * inner;
+            int64_t oa = (int64_t)r * sa, ob = (int64_t)r * sb;
+            auto walk = [&](auto &&use) {
+#pragma unroll 2
+                for (uint32_t i = tid; i < n; i += 256) {
+                    use(oa + w * (int64_t)s, ob + w * (int64_t)s);
+                    s += ds;
+                    const uint32_t step = dr + (s >= inner ? 1u : 0u);
+                    s -= s >= inner ? inner : 0u;
+                    oa += (int64_t)step * sa;
+                    ob += (int64_t)step * sb;
                 }
             };
-            for (int64_t j = start + tid; j < K2; j += 256) body(j);
-            for (int64_t j = tid; j < start; j += 256) body(j);
-            if ((K & 1) && tid == 0) {
-                const double y = __ldg(b + K - 1);
-#pragma unroll
-                for (int q = 0; q < RB; q++) acc[q] = fma(__ldg(a[q] + K - 1), y, acc[q]);
-            }
-        } else if (Contig) {
-            for (int64_t i = tid; i < K; i += 256) {
-                const double y = __ldg(b + i);
-#pragma unroll
-                for (int q = 0; q < RB; q++) acc[q] = fma(__ldg(a[q] + i), y, acc[q]);
-            }
+            if (pairs)
+                walk(pair);
+            else
+                walk(single);
         } else {
-            for (int64_t i = tid; i < K; i += 256) {
-                const int64_t oa = __ldg(offk + i);
-                const double y = __ldg(b + __ldg(offk + K + i));
-#pragma unroll
-                for (int q = 0; q < RB; q++) acc[q] = fma(__ldg(a[q] + oa), y, acc[q]);
-            }
+            for (int64_t i = tid; i < K; i += 256) single(__ldg(offk + i), __ldg(offk + K + i));
         }
         // fixed-order reduction: warp trees, then the warps in order
-#pragma unroll
-        for (int q = 0; q < RB; q++) {
-            double v = acc[q];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) red[warp][q] = v;
-        }
+        int which;
+        const double v = warp_sums<RB>(acc, lane, which);
+        if ((lane & (32 / RB - 1)) == 0) red[warp][which] = v;
         __syncthreads();
         if (tid < RB && r0 + tid < rows.total) {
-            double v = 0.0;
-            for (int w = 0; w < 8; w++) v += red[w][tid];
+            double t = 0.0;
+            for (int w = 0; w < 8; w++) t += red[w][tid];
             int64_t ra, rb, oc;
             group_offsets(rows, r0 + tid, ra, rb, oc);
-            C[oc] = epilogue(v, C + oc, cp, ab, zero);
+            C[oc] = epilogue(t, C + oc, cp, ab, zero);
         }
         __syncthreads();
     }
@@ -770,9 +809,10 @@ eg_status launch_gemv(const Contraction &c, cudaStream_t s) {
         for (int d = 0; d < k.n; d++) std::swap(k.s[0][d], k.s[1][d]);
         std::swap(X, Y);
     }
+    const bool nested = k.n == 2 && k.s[0][1] == 1 && k.s[1][1] == 1;
     // offset tables for a strided k, built once and shared by every output
     int64_t *offk = nullptr;
-    if (!contig && k.total <= (int64_t(1) << 24) && rows.total > 1) {
+    if (!contig && !(rows_kernel && nested) && k.total <= (int64_t(1) << 24) && rows.total > 1) {
         void *ws = nullptr;
         eg_status st = workspace(s, (size_t)k.total * 2 * sizeof(int64_t), &ws);
         if (st != EG_SUCCESS) return st;
@@ -783,14 +823,18 @@ eg_status launch_gemv(const Contraction &c, cudaStream_t s) {
         }
         EG_CHECK_LAUNCH("k_k_offsets");
     }
-    if (rows_kernel && (contig || offk)) {
+    if (rows_kernel && (contig || nested || offk)) {
         constexpr int RB = 4;
+        // one unit of RB rows per CTA, handed out by the hardware: persistent CTAs (4 to 8
+        // per SM) took 193 to 246 us where these take 188 (n = 100, 10^4 rows of 10^4)
         const int grid = grid_for(rows.total, RB);
         LaunchScope ls_("k_gemv", s);
         if (contig)
-            k_gemv_rows<RB, true><<<grid, 256, 0, s>>>(rows, k, X, Y, c.C, c.cp, c.ab, c.zero_when_cp_zero, nullptr);
+            k_gemv_rows<RB, 0><<<grid, 256, 0, s>>>(rows, k, X, Y, c.C, c.cp, c.ab, c.zero_when_cp_zero, nullptr);
+        else if (nested)
+            k_gemv_rows<RB, 1><<<grid, 256, 0, s>>>(rows, k, X, Y, c.C, c.cp, c.ab, c.zero_when_cp_zero, nullptr);
         else
-            k_gemv_rows<RB, false><<<grid, 256, 0, s>>>(rows, k, X, Y, c.C, c.cp, c.ab, c.zero_when_cp_zero, offk);
+            k_gemv_rows<RB, 2><<<grid, 256, 0, s>>>(rows, k, X, Y, c.C, c.cp, c.ab, c.zero_when_cp_zero, offk);
     } else if (k.total >= 2048) {
         const int grid = grid_for(rows.total, 1);
         LaunchScope ls_("k_gemv", s);
