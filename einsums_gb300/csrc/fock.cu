@@ -35,11 +35,12 @@
 // shared-memory tiles, no atomics.  Every partial has one home and the last
 // passes add them in a fixed order, so the result is deterministic.
 //   k_fock_digits_d   (split form) the digits of every row of D.
-//   k_fock_rows<S>    unit r, a lane per pair (p, q): T1 and T4, sums over s
+//   k_fock_lines<S>   the three line passes in one launch:
+//     fock_rows<S>      unit r, a lane per pair (p, q): T1 and T4, sums over s
 //                     of g[r,s,p,q] (= g[p,q,r,s]), consecutive lanes along q.
-//   k_fock_cols<S>    unit p, a lane per pair (r, s): T2, T5 and T3, sums over
+//     fock_cols<S>      unit p, a lane per pair (r, s): T2, T5 and T3, sums over
 //                     q of g[p,q,r,s], consecutive lanes along s.
-//   k_fock_exchange   warp (q, p, 32 s): T6, sums over r of g[q,p,r,s]
+//     fock_exchange     warp (q, p, 32 s): T6, sums over r of g[q,p,r,s]
 //                     (= g[p,q,r,s]) D[p,r], lanes along s.
 //   k_fock_reduce     CTA (i, 32 j): YJ and XK from the partials.
 //   k_fock_combine    J = 2 (YJ + YJ^T), K = XK + XK^T and the prefactors.
@@ -58,7 +59,7 @@ using split::int_times_pow2_rn;
 using split::scaled_round;
 
 constexpr int kWarps = 4;      // warps per CTA of the line passes (consecutive r)
-constexpr int kRedWarps = 8;   // warps of a reduction CTA
+constexpr int kRedWarps = 16;  // warps of a reduction CTA
 constexpr int kFockMaxN = 384; // g is 174 GB at n = 384
 constexpr int kFlush = 64;     // elements per exact FP32 digit-group sum (a multiple of kBatch)
 constexpr int kBatch = 8;      // independent loads in flight per lane in the line passes
@@ -224,10 +225,10 @@ __device__ __forceinline__ int cols_pairs(int p) { return (p + 1) * (p + 2) / 2;
 // consecutive q.  The loop runs over the warp's common range in batches of
 // kBatch independent loads (a lane outside its own range adds nothing).
 template <int S>
-__global__ void __launch_bounds__(kWarps * 32) k_fock_rows(const double *__restrict__ g,
-                                                           const double *__restrict__ D, int n, FockScratch sc) {
+__device__ __forceinline__ void fock_rows(int cta, const double *__restrict__ g, const double *__restrict__ D, int n,
+                                          const FockScratch &sc) {
     int r, first;
-    unit_of_cta(blockIdx.x, n, [&](int u) { return rows_pairs(n, u); }, r, first);
+    unit_of_cta(cta, n, [&](int u) { return rows_pairs(n, u); }, r, first);
     if (r < 0) return;
     const int f = first + threadIdx.x;
     const bool on = f < rows_pairs(n, r);
@@ -318,10 +319,10 @@ __global__ void __launch_bounds__(kWarps * 32) k_fock_rows(const double *__restr
 // batches of kBatch loads as in the rows pass.  Each lane's T3 sum over q is
 // added over s by the reduction.
 template <int S>
-__global__ void __launch_bounds__(kWarps * 32) k_fock_cols(const double *__restrict__ g,
-                                                           const double *__restrict__ D, int n, FockScratch sc) {
+__device__ __forceinline__ void fock_cols(int cta, const double *__restrict__ g, const double *__restrict__ D, int n,
+                                          const FockScratch &sc) {
     int p, first;
-    unit_of_cta(blockIdx.x, n, [&](int u) { return cols_pairs(u); }, p, first);
+    unit_of_cta(cta, n, [&](int u) { return cols_pairs(u); }, p, first);
     if (p < 0) return;
     const int f = first + threadIdx.x;
     const bool on = f < cols_pairs(p);
@@ -414,11 +415,11 @@ __global__ void __launch_bounds__(kWarps * 32) k_fock_cols(const double *__restr
 // when q < s -- of f g[q,p,r,s] D[p,r].  Warp (q, 32 s, p), lane = s: the sum
 // over r for one p, so that every warp has at most n terms (the sums over p
 // would leave a few long warps running alone); the reduction adds over p.
-__global__ void __launch_bounds__(kWarps * 32) k_fock_exchange(const double *__restrict__ g,
-                                                               const double *__restrict__ D, int n, int nsc,
-                                                               double *__restrict__ X6) {
-    const int q = blockIdx.x / nsc, s0 = (blockIdx.x - q * nsc) * 32;
-    const int p = blockIdx.y * kWarps + (threadIdx.x >> 5);
+__device__ __forceinline__ void fock_exchange(int cta, const double *__restrict__ g, const double *__restrict__ D, int n,
+                                              int nsc, double *__restrict__ X6) {
+    const int py = cta / (n * nsc), qx = cta - py * (n * nsc);
+    const int q = qx / nsc, s0 = (qx - q * nsc) * 32;
+    const int p = py * kWarps + (threadIdx.x >> 5);
     const int s = s0 + (threadIdx.x & 31);
     if (p >= n || p < q || p < s0) return; // whole warps leave together
     const int sl = s < n ? s : n - 1;
@@ -446,9 +447,22 @@ __global__ void __launch_bounds__(kWarps * 32) k_fock_exchange(const double *__r
     if (s < n) X6[((size_t)q * n + p) * n + s] = acc;
 }
 
+// The three passes in one launch, the longest units first: each pass alone ends in a
+// tail of few CTAs, which the next one's now fill (n = 100: 167 us, against 196 us one
+// after the other).
+template <int S>
+__global__ void __launch_bounds__(kWarps * 32) k_fock_lines(const double *__restrict__ g, const double *__restrict__ D,
+                                                            int n, FockScratch sc, int cols_ctas, int rows_ctas) {
+    int cta = blockIdx.x;
+    if (cta < cols_ctas) return fock_cols<S>(cta, g, D, n, sc);
+    cta -= cols_ctas;
+    if (cta < rows_ctas) return fock_rows<S>(cta, g, D, n, sc);
+    fock_exchange(cta - rows_ctas, g, D, n, sc.nsc, sc.X6);
+}
+
 // Row i, columns j of one chunk of 32, of YJ (j <= i) and XK from the partials.
 // Lanes run over j (every read is contiguous); warp w takes the terms t = w,
-// w + 8, ... of each sum over p or r, and the eight warps' sums are added in
+// w + kRedWarps, ... of each sum over p or r, and the warps' sums are added in
 // warp order.
 __global__ void __launch_bounds__(kRedWarps * 32) k_fock_reduce(int n, FockScratch sc) {
     __shared__ double sr[2][kRedWarps][32];
@@ -457,9 +471,6 @@ __global__ void __launch_bounds__(kRedWarps * 32) k_fock_reduce(int n, FockScrat
     const int j = blockIdx.y * 32 + lane;
     if (j < n) {
         double xk = 0.0, yj = 0.0;
-        if (warp == 0) {
-
-        }
         for (int t = warp; t < n; t += kRedWarps) {
             if (t >= max(i, j)) xk += sc.S4[((size_t)i * n + t) * n + j]; // T4 of (p = t, r = j), q = i
             if (t >= max(i, j & ~31)) xk += sc.X6[((size_t)i * n + t) * n + j]; // T6 of (q = i, p = t), s = j
@@ -514,15 +525,12 @@ eg_status launch_lines(const double *g, const double *D, int n, const FockScratc
         EG_CHECK_LAUNCH("k_fock_digits_d");
     }
     {
-        LaunchScope ls_("k_fock_rows", s);
-        k_fock_rows<S><<<rows_ctas, kWarps * 32, 0, s>>>(g, D, n, sc);
+        const unsigned exchange_ctas = (unsigned)(n * sc.nsc) * (unsigned)((n + kWarps - 1) / kWarps);
+        LaunchScope ls_("k_fock_lines", s);
+        k_fock_lines<S><<<cols_ctas + rows_ctas + exchange_ctas, kWarps * 32, 0, s>>>(g, D, n, sc, (int)cols_ctas,
+                                                                                     (int)rows_ctas);
     }
-    EG_CHECK_LAUNCH("k_fock_rows");
-    {
-        LaunchScope ls_("k_fock_cols", s);
-        k_fock_cols<S><<<cols_ctas, kWarps * 32, 0, s>>>(g, D, n, sc);
-    }
-    EG_CHECK_LAUNCH("k_fock_cols");
+    EG_CHECK_LAUNCH("k_fock_lines");
     return EG_SUCCESS;
 }
 
@@ -578,12 +586,6 @@ extern "C" eg_status eg_fock_jk_symmetric(double F_prefactor, double *F, double 
     default: st = launch_lines<6>(g, D, nn, sc, s); break;
     }
     if (st != EG_SUCCESS) return st;
-    {
-        LaunchScope ls_("k_fock_exchange", s);
-        k_fock_exchange<<<dim3((unsigned)(nn * nsc), (unsigned)((nn + kWarps - 1) / kWarps)), kWarps * 32, 0, s>>>(
-            g, D, nn, nsc, sc.X6);
-    }
-    EG_CHECK_LAUNCH("k_fock_exchange");
     {
         LaunchScope ls_("k_fock_reduce", s);
         k_fock_reduce<<<dim3((unsigned)nn, (unsigned)nsc), kRedWarps * 32, 0, s>>>(nn, sc);
