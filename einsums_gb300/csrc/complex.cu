@@ -15,12 +15,26 @@
 // and both precisions (FP64 and split-BF16) serve complex operands.  A real
 // C_prefactor rides on the first contraction into each part, keeping the real
 // path's zeroing rules; a complex one is applied first by k_complex_scale.
+//
+// An FP64 contraction with a real AB_prefactor that the FMA kernel would take four times
+// runs once: the real and imaginary parts become a mode p of C and a mode q of the sums,
+// the larger operand serves both as it is stored, and the smaller is written out as the
+// 2 x 2 real block of each of its elements.  One launch of four times the work fills the
+// chip where four did not, and the summed modes of an interleaved operand are contiguous.
+#include <algorithm>
+#include <climits>
+
 #include "common.cuh"
 
 namespace eg {
 eg_status einsum_impl(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al,
                       const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options *opt_in,
                       cudaStream_t stream, int32_t *alg_out);
+eg_status lower_for_group(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al,
+                          const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options &opt,
+                          Contraction &out, int32_t *alg_out, bool &gemm_shaped);
+bool f64_tensor_pays(const Contraction &c);
+void set_split_report(const eg_split_report &r);
 eg_status classify_call(const int32_t *Cl, const eg_tensor *C, const int32_t *Al, const eg_tensor *A,
                         const int32_t *Bl, const eg_tensor *B, const eg_options *opt_in, int32_t *alg_out);
 
@@ -44,6 +58,105 @@ eg_tensor part_view(const eg_tensor &t, int part) {
     v.data = t.data ? t.data + part : nullptr;
     for (int d = 0; d < t.rank && d < EG_MAX_RANK; d++) v.stride[d] = 2 * t.stride[d];
     return v;
+}
+
+// Element i of the smaller operand (g: its modes, strides 0 in the source and 1 in E) as
+// the block E[q, p]: {re, -own other im} for the real part, {own im, other re} for the
+// imaginary one, own and other -1 for a conjugated operand.
+__global__ void __launch_bounds__(256) k_complex_blocks(ModeGroup g, const double *__restrict__ src, double *E,
+                                                        int64_t sq, int64_t sp, double own, double other) {
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (uint32_t)g.total; i += stride) {
+        int64_t os, oe, unused;
+        group_offsets32(g, i, os, oe, unused);
+        const double re = __ldg(src + os), im = __ldg(src + os + 1);
+        double *e = E + oe;
+        e[0] = re;
+        e[sq] = -(own * other) * im;
+        e[sp] = own * im;
+        e[sq + sp] = other * re;
+    }
+}
+
+// g with a mode of extent 2 and the given strides as its fastest, its modes merged where
+// all three operands allow; false when there is no room.
+bool append_part(ModeGroup &g, int64_t s0, int64_t s1, int64_t s2) {
+    if (g.n == kMaxModes) return false;
+    const int64_t s[3] = {s0, s1, s2};
+    ModeGroup out;
+    for (int d = 0; d <= g.n; d++) {
+        const bool part = d == g.n;
+        const int64_t ext = part ? 2 : g.ext[d];
+        bool merge = out.n > 0;
+        for (int t = 0; t < 3 && merge; t++) merge = out.s[t][out.n - 1] == (part ? s[t] : g.s[t][d]) * ext;
+        if (!merge) out.ext[out.n++] = 1;
+        out.ext[out.n - 1] *= ext;
+        for (int t = 0; t < 3; t++) out.s[t][out.n - 1] = part ? s[t] : g.s[t][d];
+    }
+    out.total = 2 * g.total;
+    g = out;
+    return true;
+}
+
+// The contraction c of the real parts as one real contraction of the whole complex
+// operands (file comment).  NOT_SUPPORTED: the caller's four contractions, when the shape,
+// the tensor cores (better from about 40 us each), a capture or the scratch say so.
+// Bound: the FP64 pipe (83 us for 300 x 170 x 257, which take 125 us; in four launches
+// 156 us, each with a last wave of its own and operands at stride 2).
+constexpr int64_t kBlocksMax = int64_t(1) << 23; // elements of the smaller operand: 256 MB of blocks
+eg_status launch_complex_blocks(Contraction c, double sa, double sb, cudaStream_t s) {
+    if (c.k.n == 0 || c.m.n == 0 || c.n.n == 0 || f64_tensor_pays(c)) return EG_ERROR_NOT_SUPPORTED;
+    if (c.batch.n + c.m.n + c.n.n >= kMaxModes) return EG_ERROR_NOT_SUPPORTED;
+    const int t = c.m.total < c.n.total ? 0 : 1; // the operand written out as blocks
+    ModeGroup &f = t == 0 ? c.m : c.n, &k = c.k, &b = c.batch;
+    if (b.n + f.n + k.n > kMaxModes || k.n == kMaxModes || f.n == kMaxModes) return EG_ERROR_NOT_SUPPORTED;
+    const double rows = (double)f.total * (double)b.total;
+    if (rows * (double)k.total > (double)kBlocksMax) return EG_ERROR_NOT_SUPPORTED;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    EG_CUDA(cudaStreamIsCapturing(s, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return EG_ERROR_NOT_SUPPORTED;
+
+    // E's strides: batch, then the free modes and p, then the summed modes and q, or the
+    // last two the other way round, as the operand itself is faster along the one or other
+    auto fastest = [&](const ModeGroup &g) { return *std::min_element(g.s[t], g.s[t] + g.n); };
+    const bool k_inner = fastest(k) <= fastest(f);
+    ModeGroup src; // source strides 0, E's strides 1, slowest mode first
+    int64_t step = 1, part[2] = {0, 0}; // strides of q and p
+    ModeGroup *order[3] = {k_inner ? &k : &f, k_inner ? &f : &k, &b};
+    int at = b.n + f.n + k.n;
+    src.n = at;
+    for (ModeGroup *g : order) {
+        if (g != &b) {
+            part[g == &k ? 0 : 1] = step;
+            step *= 2;
+        }
+        for (int d = g->n - 1; d >= 0; d--) {
+            at--;
+            src.ext[at] = g->ext[d];
+            src.s[0][at] = g->s[t][d];
+            src.s[1][at] = step;
+            src.total *= g->ext[d];
+            g->s[t][d] = step;
+            step *= g->ext[d];
+        }
+    }
+    ScratchLease lease(s, (size_t)step * sizeof(double));
+    if (!lease.ptr()) return EG_ERROR_NOT_SUPPORTED;
+    double *E = (double *)lease.ptr();
+    const double *from = t == 0 ? c.A : c.B;
+    const bool room = t == 0 ? append_part(k, part[0], 1, 0) && append_part(f, part[1], 0, 1)
+                             : append_part(k, 1, part[0], 0) && append_part(f, 0, part[1], 1);
+    if (!room) return EG_ERROR_NOT_SUPPORTED;
+    (t == 0 ? c.A : c.B) = E;
+    {
+        LaunchScope ls_("k_complex_blocks", s);
+        const int64_t blocks = std::min<int64_t>((src.total + 255) / 256, (int64_t)num_sms() * 8);
+        k_complex_blocks<<<(unsigned)blocks, 256, 0, s>>>(src, from, E, part[0], part[1], t == 0 ? sa : sb,
+                                                          t == 0 ? sb : sa);
+    }
+    EG_CHECK_LAUNCH("k_complex_blocks");
+    set_split_report(eg_split_report{0, 0, 0, 0.0});
+    return launch_contract_f64(c, s);
 }
 
 } // namespace
@@ -94,6 +207,18 @@ extern "C" eg_status eg_einsum_complex(const double *C_prefactor, const int32_t 
     const eg_tensor Cr = part_view(*C, 0), Ci = part_view(*C, 1);
     const eg_tensor Ar = part_view(*A, 0), Ai = part_view(*A, 1);
     const eg_tensor Br = part_view(*B, 0), Bi = part_view(*B, 1);
+    eg_options o;
+    eg_options_default(&o);
+    if (opt) o = *opt;
+    if (abi == 0.0 && abr != 0.0 && o.precision == EG_PRECISION_FP64 &&
+        (o.semantics == EG_SEMANTICS_CPP || o.semantics == EG_SEMANTICS_PYTHON)) {
+        Contraction c;
+        int32_t alg = 0;
+        bool gemm_shaped = false;
+        eg_status st = lower_for_group(cp0, C_labels, &Cr, abr, A_labels, &Ar, B_labels, &Br, o, c, &alg, gemm_shaped);
+        if (st != EG_SUCCESS) return st;
+        if (gemm_shaped && (st = launch_complex_blocks(c, sa, sb, s)) != EG_ERROR_NOT_SUPPORTED) return st;
+    }
     // (destination, A part, B part, coefficient): Re gets abr Pr - abi Pi, Im gets abr Pi + abi Pr
     struct Term {
         const eg_tensor *c, *a, *b;
