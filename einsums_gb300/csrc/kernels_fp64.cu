@@ -38,7 +38,7 @@ __device__ __forceinline__ double epilogue(double acc, double *cptr, double cp, 
 // 16 bytes, two pairs of a thread in flight.  Bound: memory, 24 bytes per element (32
 // with C_prefactor), if the FP64 pipe is spared -- three operations an element took as
 // long: a multiplication by ab = 1 and the sum with C are left out where they do nothing.
-// 20e6 elements: 69 us (7.0 TB/s); mode by mode 105 us.  One element off alignment, or
+// 15e6 elements: 69 us (5.3 TB/s); mode by mode 81 us.  One element off alignment, or
 // with a mode between, the kernel below takes it.
 template <bool PLAIN, bool AB_ONE>
 __global__ void __launch_bounds__(256) k_elementwise_contiguous(int64_t n, const double *__restrict__ A,
@@ -118,7 +118,9 @@ __device__ __forceinline__ double block_sum(double v, double *smem) {
 }
 
 // -------------------------------------------------------------------- dot --
-constexpr int kDotThreads = 256;
+// Four blocks per SM: the compensated sum over blocks, serial FP64 work on one SM, took
+// 6 us of 54 with twice as many partials and threads.
+constexpr int kDotThreads = 256, kDotBlocksPerSm = 4, kDotFinalThreads = 128;
 
 template <bool Contig>
 __global__ void __launch_bounds__(kDotThreads) k_dot_partial(ModeGroup k, const double *__restrict__ A,
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(kDotThreads) k_dot_partial(ModeGroup k, const 
     double acc0 = 0.0, acc1 = 0.0;
     if (Contig) {
         // 16-byte pairs where both operands allow (chunks are even), four pairs of each in
-        // flight: 15e6 elements with the final sum 54 us, element by element 69 us
+        // flight: 15e6 elements with the final sum 50 us, element by element 69 us
         int64_t i = begin + threadIdx.x;
         if ((((uintptr_t)A | (uintptr_t)B) & 15) == 0) {
             const double2 *A2 = (const double2 *)(A + begin), *B2 = (const double2 *)(B + begin);
@@ -174,7 +176,7 @@ __global__ void __launch_bounds__(kDotThreads) k_dot_partial(ModeGroup k, const 
 // A short sum in one CTA and one launch: up to kDotSmall elements, eight of a thread in
 // flight, each in a sum of its own: at most 4 + 3 + 9 additions lie on a path, against
 // 8 + 1 + 8 before the compensated sum over blocks of the two launches of longer sums.
-// Bound: latency.  10^4 elements: 6.2 us (8.4 us in two launches); above kDotSmall the
+// Bound: latency.  10^4 elements: 6.2 us (10.0 us in two launches); above kDotSmall the
 // CTA's one SM takes longer than a second launch.
 constexpr int64_t kDotSmall = 16384;
 constexpr int kDotSmallThreads = 512;
@@ -207,17 +209,17 @@ __global__ void __launch_bounds__(kDotSmallThreads) k_dot_small(ModeGroup k, con
 
 // Sums the per-block partials in a fixed order: Neumaier compensation within a
 // thread, then a compensated tree across the block.
-__global__ void __launch_bounds__(kDotThreads) k_dot_final(const double *partial, int nparts, double *C, double cp,
+__global__ void __launch_bounds__(kDotFinalThreads) k_dot_final(const double *partial, int nparts, double *C, double cp,
                                                            double ab, bool zero) {
-    __shared__ double sh_s[kDotThreads / 32], sh_c[kDotThreads / 32];
+    __shared__ double sh_s[kDotFinalThreads / 32], sh_c[kDotFinalThreads / 32];
     double s = 0.0, c = 0.0;
-    for (int i = threadIdx.x; i < nparts; i += kDotThreads) {
+    for (int i = threadIdx.x; i < nparts; i += kDotFinalThreads) {
         const double x = partial[i];
         const double t = s + x;
         c += (fabs(s) >= fabs(x)) ? (s - t) + x : (x - t) + s;
         s = t;
     }
-    const double sum = block_sum_compensated<kDotThreads>(s, c, sh_s, sh_c);
+    const double sum = block_sum_compensated<kDotFinalThreads>(s, c, sh_s, sh_c);
     if (threadIdx.x == 0) *C = epilogue(sum, C, cp, ab, zero);
 }
 
@@ -767,7 +769,7 @@ eg_status launch_dot(const Contraction &c, cudaStream_t s) {
     }
     const int64_t per_block_min = 4096;
     int64_t nblocks = (k.total + per_block_min - 1) / per_block_min;
-    const int64_t cap = (int64_t)num_sms() * 8;
+    const int64_t cap = (int64_t)num_sms() * kDotBlocksPerSm;
     if (nblocks > cap) nblocks = cap;
     if (nblocks < 1) nblocks = 1;
     const int64_t chunk = ((k.total + nblocks - 1) / nblocks + 1) & ~int64_t(1); // even: pairs stay aligned
@@ -787,7 +789,7 @@ eg_status launch_dot(const Contraction &c, cudaStream_t s) {
         }
     EG_CHECK_LAUNCH("k_dot_partial");
     { LaunchScope ls_("k_dot_final", s);
-    k_dot_final<<<1, kDotThreads, 0, s>>>(partial, (int)nblocks, c.C, c.cp, c.ab, c.zero_when_cp_zero);
+    k_dot_final<<<1, kDotFinalThreads, 0, s>>>(partial, (int)nblocks, c.C, c.cp, c.ab, c.zero_when_cp_zero);
     }
     EG_CHECK_LAUNCH("k_dot_final");
     return EG_SUCCESS;
