@@ -183,7 +183,8 @@ eg_status launch_scale(const ModeGroup &g, double *C, double cp, cudaStream_t s)
 eg_status launch_dot(const Contraction &c, cudaStream_t s);
 eg_status launch_gemv(const Contraction &c, cudaStream_t s);
 eg_status launch_contract_f64(const Contraction &c, cudaStream_t s);
-// The blocks of 32 x 64 outputs listed at `list` ({batch, row, column}), *count of them.
+// The blocks of outputs listed at `list` ({batch, row, column}), *count of them: 32 rows by
+// the 16 columns from `column` and from 32, 64 and 96 further on.
 eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, const int *count, cudaStream_t s);
 double contract_f64_seconds(const Contraction &c); // its estimated time
 bool f64_tensor_pays(const Contraction &c);

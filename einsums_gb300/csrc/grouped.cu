@@ -60,11 +60,10 @@ struct F64Item {
 constexpr int BK = 16, THREADS = 256, LD = 65;
 
 template <int T>
-__device__ __forceinline__ void f64_tile(const F64Item &it, int64_t bidx, int mt, int nt, double cp, double ab,
-                                         bool zero, double (*As)[LD], double (*Bs)[LD]) {
+__device__ __forceinline__ void f64_tile(const F64Item &it, int64_t bidx, int64_t m0, int64_t n0, int gap, double cp,
+                                         double ab, bool zero, double (*As)[LD], double (*Bs)[LD]) {
     constexpr int R = T / 16; // outputs per thread per dimension, and loads per thread per operand
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int64_t m0 = (int64_t)mt * T, n0 = (int64_t)nt * T;
     const int64_t M = it.m.total, N = it.n.total, K = it.k.total;
     int64_t ba, bb, bc;
     group_offsets(it.b, bidx, ba, bb, bc);
@@ -82,8 +81,9 @@ __device__ __forceinline__ void f64_tile(const F64Item &it, int64_t bidx, int mt
         okA[i] = m0 + lm[i] < M;
         group_offsets32(it.m, (uint32_t)(okA[i] ? m0 + lm[i] : 0), oa, ob, oc);
         offA[i] = ba + oa;
-        okB[i] = n0 + ln[i] < N;
-        group_offsets32(it.n, (uint32_t)(okB[i] ? n0 + ln[i] : 0), oa, ob, oc);
+        const int64_t n = n0 + ln[i] + (ln[i] & gap);
+        okB[i] = n < N;
+        group_offsets32(it.n, (uint32_t)(okB[i] ? n : 0), oa, ob, oc);
         offB[i] = bb + ob;
     }
     double acc[R][R];
@@ -134,7 +134,7 @@ __device__ __forceinline__ void f64_tile(const F64Item &it, int64_t bidx, int mt
         group_offsets32(it.m, (uint32_t)m, ma, mb, mc);
 #pragma unroll
         for (int j = 0; j < R; j++) {
-            const int64_t n = n0 + tx + 16 * j;
+            const int64_t n = n0 + tx + 16 * j + ((tx + 16 * j) & gap);
             if (n >= N) continue;
             int64_t na, nb, nc;
             group_offsets32(it.n, (uint32_t)n, na, nb, nc);
@@ -154,14 +154,15 @@ __global__ void __launch_bounds__(THREADS) k_grouped_f64(const F64Item *items, c
         const int4 e = work[w];
         const F64Item &it = items[e.x];
         if (tiles[e.x] == 64)
-            f64_tile<64>(it, e.y, e.z, e.w, cp, ab, zero != 0, As, Bs);
+            f64_tile<64>(it, e.y, int64_t(64) * e.z, int64_t(64) * e.w, 0, cp, ab, zero != 0, As, Bs);
         else
-            f64_tile<32>(it, e.y, e.z, e.w, cp, ab, zero != 0, As, Bs);
+            f64_tile<32>(it, e.y, int64_t(32) * e.z, int64_t(32) * e.w, 0, cp, ab, zero != 0, As, Bs);
     }
 }
 
-// The 32 x 64 blocks of outputs that the FP64 form on the tensor cores left out:
-// {item, batch index, row, column}, *count of them.
+// The blocks of outputs that the FP64 form on the tensor cores left out, *count of them:
+// {item, batch index, row, column}, 32 rows by the 16 columns from `column` and from 32,
+// 64 and 96 further on.  Tile column j is column j + (j & gap) from the tile's first.
 __global__ void __launch_bounds__(THREADS) k_grouped_f64_listed(const F64Item *items, const int4 *list, const int *count,
                                                                  double cp, double ab, int zero) {
     __shared__ double As[BK][LD];
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(THREADS) k_grouped_f64_listed(const F64Item *i
     const int n = 2 * __ldg(count);
     for (int w = blockIdx.x; w < n; w += gridDim.x) {
         const int4 e = list[w >> 1];
-        f64_tile<32>(items[e.x], e.y, e.z / 32, e.w / 32 + (w & 1), cp, ab, zero != 0, As, Bs);
+        f64_tile<32>(items[e.x], e.y, e.z, e.w + 64 * (w & 1), 16, cp, ab, zero != 0, As, Bs);
     }
 }
 

@@ -479,8 +479,9 @@ struct F64Args {
     int64_t ka, kb;        // single k strides of A and B (0: none)
     int64_t mtiles, ntiles, total; // total = batches * mtiles * ntiles
     int cs;                // CTAs of a cluster, each taking a range of the k chunks
-    // When set, the tiles are instead the halves of the 32 x 64 blocks {batch, row,
-    // column} listed there (T = 32, one CTA each).
+    // When set, the tiles are instead the halves of the blocks {batch, row, column}
+    // listed there (T = 32, one CTA each): 32 rows by the 16 columns from `column` and
+    // from 32, 64 and 96 further on.
     const int4 *list;
     const int *count;
 };
@@ -500,13 +501,14 @@ __global__ void __launch_bounds__(kThreads) k_contract_f64(const __grid_constant
     const int cbeg = (int)((int64_t)chunks * rank / p.cs), cend = (int)((int64_t)chunks * (rank + 1) / p.cs);
     const int64_t step = gridDim.x / p.cs;
     const int64_t total = p.list ? 2 * (int64_t)__ldg(p.count) : p.total;
+    const int gap = p.list ? 16 : 0; // tile column j is column j + (j & gap) from the tile's first
     for (int64_t t = blockIdx.x / p.cs; t < total; t += step) {
         int64_t b, m0, n0;
         if (p.list) {
             const int4 e = p.list[t >> 1];
             b = e.x;
             m0 = e.y;
-            n0 = e.z + T * (t & 1);
+            n0 = e.z + 2 * T * (t & 1);
         } else {
             const int64_t q = t / p.ntiles;
             b = q / p.mtiles;
@@ -529,8 +531,9 @@ __global__ void __launch_bounds__(kThreads) k_contract_f64(const __grid_constant
             oka[i] = m0 + am[i] < M;
             group_offsets32(p.mg, (uint32_t)(oka[i] ? m0 + am[i] : 0), oa, ob, oc);
             pa[i] = p.A + ba + oa;
-            okb[i] = n0 + bn[i] < N;
-            group_offsets32(p.ng, (uint32_t)(okb[i] ? n0 + bn[i] : 0), oa, ob, oc);
+            const int64_t n = n0 + bn[i] + (bn[i] & gap);
+            okb[i] = n < N;
+            group_offsets32(p.ng, (uint32_t)(okb[i] ? n : 0), oa, ob, oc);
             pb[i] = p.B + bb + ob;
         }
         auto load = [&](int c) {
@@ -613,7 +616,7 @@ __global__ void __launch_bounds__(kThreads) k_contract_f64(const __grid_constant
                 group_offsets32(p.mg, (uint32_t)m, ma, mb, mc);
 #pragma unroll
                 for (int j = 0; j < R; j++) {
-                    const int64_t n = n0 + tx + W * j;
+                    const int64_t n = n0 + tx + W * j + ((tx + W * j) & gap);
                     if (n >= N) continue;
                     int64_t na, nb, nc;
                     group_offsets32(p.ng, (uint32_t)n, na, nb, nc);

@@ -937,7 +937,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
 // group and exactly, sum_k p_a p_b with p <= 128 |x| / max, and 20 N; where
 //   sum_k p_a p_b >= 20 N
 // the error is at most 4 2^-53 sum_k |A_ik| |B_jk| -- four roundings' worth, where
-// the bound of a chain of K FMAs is K of them.  A 32 x 64 block of outputs in
+// the bound of a chain of K FMAs is K of them.  A region of a tile in
 // which it fails anywhere (rows graded against each other, infinities, NaN) is
 // not written but listed, and k_contract_f64 computes it from C as it was.  The
 // sums of all 36 products are exact in two int64 words and rounded once.

@@ -35,7 +35,7 @@ constexpr int kBM = 128, kBN = 128, kBK = 64;
 // accuracy check of launch_f64_tensor.
 constexpr int kF64Slices = 8, kF64High = 4;
 constexpr float kCheckA = 4.0f, kCheckB = -5.0f;
-constexpr int kTileRegions = 8; // 32 x 64 blocks of a tile, one per epilogue warp
+constexpr int kTileRegions = 8; // parts of a tile, one per epilogue warp: 32 rows by 64 columns in turns of 16
 constexpr int kChunkKB = 16;    // 16 x 64 = 1024 products per exact FP32 chunk
 constexpr int kKStep = 2 * kBK;  // granularity of the longest exact pass (K itself is padded to kBK)
 
@@ -87,8 +87,8 @@ struct TcGemmParams {
     // it computes all of it): mt, nt and the exponents count from there.
     int64_t b0, m0, n0;
     // FP64 form (redo set): the exact sums do not fit 64 bits, so the slice groups
-    // below hid form one int64 sum and the others a second; a 32 x 64 block of
-    // outputs whose accuracy check fails is left alone and listed in redo ({batch, row,
+    // below hid form one int64 sum and the others a second; a region of
+    // a tile whose accuracy check fails is left alone and listed in redo ({batch, row,
     // column}, in grouped launches {item, batch, row, column}; redo_count entries) for
     // the FMA kernel.
     int hid;

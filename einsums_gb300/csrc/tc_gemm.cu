@@ -9,7 +9,7 @@
 //               kind::f16 (N = 256: two slice groups at once, step_of below) into
 //               one of two FP32 accumulators of 256 columns, committing each slot
 //               and each chunk of at most 1024 products per accumulated sum;
-//   warps 4-11  epilogue (two warps per TMEM lane quadrant, 64 columns each): after
+//   warps 4-11  epilogue (two warps per TMEM lane quadrant, 64 columns each in turns of 16): after
 //               every chunk convert the exact FP32 sums to integers and add them to
 //               int64 sums in registers (128 of them; setmaxnreg moves registers
 //               from the other warps); a finished tile's sums wait in a scratch and
@@ -80,6 +80,12 @@ __device__ __forceinline__ void tile_coords(const TcGemmParams &p, int t, int &b
     mt = first_m + r % gsize;
     nt = r / gsize;
 }
+
+// Column of a tile that is an epilogue warp's column i: the two warps of a lane quadrant
+// take turns of 16 columns, so that a narrow tile (N = 57: 32 and 25 columns, not 57 and
+// none) keeps both busy.  421875 x 75, K = 75 in FP64: 673 us, with the columns in two
+// runs of 64 793 us.
+__device__ __forceinline__ int tile_col(int half, int i) { return (i >> 4) * 32 + half * 16 + (i & 15); }
 
 // Everything one role needs about a tile, for both the single-contraction and
 // the grouped form.
@@ -475,9 +481,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         constexpr int FIN = F64 ? kFin / 2 : kFin; // the FP64 form holds two words per sum
         const int ew = warp - 4;              // 0..7
         const int quad = warp & 3;            // TMEM lane quadrant this warp may access
-        const int col0 = (ew >> 2) * kCols;
+        const int half = ew >> 2; // of the columns, in turns of 16: columns 32 g + 16 half .. + 15
         const int row = quad * 32 + lane;     // tile row owned by this thread
-        const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)col0;
+        const uint32_t tl = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * 16);
         int64_t *colOff = colOffAll + ew * kCols;
         int *colExp = colExpAll + 2 * ew * kCols; // the pending tile's; the running tile's are at colExp + run_exp
         int run_exp = kCols;
@@ -504,7 +510,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         // describe the pending tile.  One copy of this code, in a
         // loop: finishing a tile's columns straight from the registers is as many times
         // the code, which ran at the rate of instruction fetch (80k clocks a tile).
-        long long *const rbc = p.rbuf + (size_t)blockIdx.x * (F64 ? 3 : 1) * kPlane + (size_t)col0 * kBM + row;
+        long long *const rbc = p.rbuf + (size_t)blockIdx.x * (F64 ? 3 : 1) * kPlane + (size_t)(half * kCols) * kBM + row;
         int parity = 0; // FP64 form: which of two scratch planes takes this tile's high sums
         int pend_cols = 0, pend_done = 0; // columns of the pending tile, and how many are done
         bool pend_rows_fast = false, pend_fast = false;
@@ -540,13 +546,14 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (!drain) {
                 const TileJob job = resolve<GROUPED, CL>(p, items, work, tile, rank);
                 nkb = job.nkb;
-                const int64_t left = job.N - (int64_t)job.nt * kBN - col0;
-                if ((int64_t)job.mt * kBM + quad * 32 < job.M && left > 0) live = left < kCols ? (int)left : kCols;
+                const int cols = (int)min((int64_t)kBN, job.N - (int64_t)job.nt * kBN);
+                if ((int64_t)job.mt * kBM + quad * 32 < job.M)
+                    live = cols / 32 * 16 + min(max(cols % 32 - half * 16, 0), 16);
                 const int64_t m = (int64_t)job.mt * kBM + row;
                 if (m < job.M) my_rowExp = job.eA[m];
 #pragma unroll
                 for (int i = 0; i < kCols / 32; i++) {
-                    const int64_t n = (int64_t)job.nt * kBN + col0 + lane + 32 * i;
+                    const int64_t n = (int64_t)job.nt * kBN + tile_col(half, lane + 32 * i);
                     colExp[run_exp + lane + 32 * i] = n < job.N ? job.eB[n] : 0;
                 }
             }
@@ -578,8 +585,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                         for (int cc = 0; cc < kCols; cc += 16) {
                             if (cc >= live) break;
                             uint32_t lo[16], hi[16];
-                            ptx::tmem_ld16(at + cc, lo);
-                            ptx::tmem_ld16(at + kBN + cc, hi);
+                            ptx::tmem_ld16(at + 2 * cc, lo);
+                            ptx::tmem_ld16(at + kBN + 2 * cc, hi);
                             ptx::tmem_wait_ld();
 #pragma unroll
                             for (int i = 0; i < 16; i++)
@@ -591,7 +598,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                         for (int cc = 0; cc < kCols; cc += 16) {
                             if (cc >= live) break;
                             uint32_t lo[16];
-                            ptx::tmem_ld16(at + cc, lo);
+                            ptx::tmem_ld16(at + 2 * cc, lo);
                             ptx::tmem_wait_ld();
 #pragma unroll
                             for (int i = 0; i < 16; i++) H[cc + i] += __float2int_rn(__uint_as_float(lo[i]));
@@ -701,7 +708,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             const TileJob job = resolve<GROUPED, CL>(p, items, work, tile, rank);
             if (!GROUPED && job.tid < 0) continue; // the odd half of a pair's last row of tiles
             bool finish = true;
-            long long *const sums = job.split ? p.racc + (size_t)job.tid * PLANES * kPlane + (size_t)col0 * kBM + row : rbc;
+            long long *const sums = job.split ? p.racc + (size_t)job.tid * PLANES * kPlane + (size_t)(half * kCols) * kBM + row : rbc;
             long long *const own_hi = rbc + (F64 ? 1 + parity : 0) * kPlane;
             parity ^= 1;
             if (job.split) {
@@ -735,7 +742,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 finish = false;
                 if (lane == 0) {
                     const int at = atomicAdd(p.redo_count, 1);
-                    const int m0 = job.mt * kBM + quad * 32, n0 = job.nt * kBN + col0;
+                    const int m0 = job.mt * kBM + quad * 32, n0 = job.nt * kBN + half * 16;
                     p.redo[at] = GROUPED ? make_int4(job.item, job.b, m0, n0)
                                          : make_int4(job.b, (int)p.m0 + m0, (int)p.n0 + n0, 0);
                 }
@@ -758,7 +765,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
             for (int k = 0; k < kCols / 32; k++) {
                 const int i = lane + 32 * k, ex = colExp[run_exp + i];
-                const int64_t n = (int64_t)job.nt * kBN + col0 + i;
+                const int64_t n = (int64_t)job.nt * kBN + tile_col(half, i);
                 int64_t oa, ob, oc = 0;
                 if (i < live) group_offsets32(*job.ng, (uint32_t)(GROUPED ? n : p.n0 + n), oa, ob, oc);
                 colOff[i] = oc;
