@@ -734,10 +734,11 @@ static void set_ab(split::TcGemmParams &p, double ab) {
 // round -- 20 of 324 on 152 SMs, a third of the time -- are cut into as many slices
 // of K blocks as give the smallest estimated time.  The estimate counts
 // clocks: 360 per K block of a slice pair (320 on CTA pairs, which need two row
-// tiles), 6000 for a tile's epilogue, 8000 more for adding a slice's sums to its
-// accumulator and 60 per accumulator plane to clear it.  Returns the clocks.
-static double choose_schedule(split::TcGemmParams &p, int64_t nb, int64_t mtiles, int64_t ntiles, int pairs,
-                              int planes) {
+// tiles), 6000 for a tile's epilogue, and where tiles are cut 8000 for the launch that
+// adds the slices up and 100 per plane of a slice's sums to write and read it.  At most
+// max_slices tiles' sums are kept.  Returns the clocks.
+static double choose_schedule(split::TcGemmParams &p, int64_t nb, int64_t mtiles, int64_t ntiles, int pairs, int planes,
+                              int64_t max_slices) {
     using namespace split;
     double best = -1.0;
     const int clusters = mtiles >= 2 ? tc_pair_clusters() : 0;
@@ -762,19 +763,19 @@ static double choose_schedule(split::TcGemmParams &p, int64_t nb, int64_t mtiles
             const int64_t n = (p.nkb + slice - 1) / slice; // slices actually used
             if (n == last) continue;
             last = n;
+            if (rem * n * cl > max_slices) break;
             const int64_t r = (rem * n + workers - 1) / workers;
-            offer(whole + (double)r * (entry(slice) + 8000.0) + 60.0 * (double)(rem * cl * planes), rounds * workers, n,
+            offer(whole + (double)r * entry(slice) + 8000.0 + 100.0 * (double)(rem * n * cl * planes), rounds * workers, n,
                   slice, 0.98);
         }
     }
     return best;
 }
 
-// The accumulators of the tiles cut along K in a launch of choose_schedule (at most
-// one per SM).
-static int64_t cut_tiles(const split::TcGemmParams &p, int64_t nb, int64_t mtiles, int64_t ntiles) {
-    const int cl = p.pair ? 2 : 1;
-    return p.ksplit > 1 ? (nb * ((mtiles + cl - 1) / cl) * ntiles - p.t0) * cl : 0;
+// Scratch for the slices of tiles cut along K, in tiles of sums: as many as a schedule of
+// `tiles` tiles of nkb K blocks may use, at most two per SM.
+static int64_t slice_room(int64_t tiles, int64_t nkb) {
+    return std::min<int64_t>(2 * tiles * std::min<int64_t>(nkb, 64), 2 * num_sms());
 }
 
 eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s, eg_split_report *rep) {
@@ -799,14 +800,16 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     const size_t tabBytes = tables ? (size_t)(M + N + 2 * K) * 8 : 0;
     const int64_t tiles = nb * (Mp / kBM) * (Np / kBN);
     const size_t offRacc = round_up((int64_t)(offTab + tabBytes), 256);
-    // accumulators of the tiles cut along K: at most one per SM
-    const size_t cut = (size_t)std::min<int64_t>(2 * tiles, num_sms());
-    const size_t raccBytes = cut * kBM * kBN * 8;
-    const size_t offRcnt = offRacc + raccBytes;
-    const size_t rcntBytes = cut * kTileRegions * sizeof(int);
-    const size_t total = offRcnt + rcntBytes;
+    int64_t slices_max = slice_room(tiles, Kp / kBK); // tiles cut along K
+    const size_t raccBytes = (size_t)slices_max * kBM * kBN * 8;
+    size_t total = offRacc + raccBytes;
     void *ws = nullptr;
     eg_status st = workspace(s, total, &ws);
+    if (st == EG_ERROR_OUT_OF_MEMORY) { // without tiles cut along K
+        set_error("");
+        slices_max = 0;
+        st = workspace(s, total = offRacc, &ws);
+    }
     if (st != EG_SUCCESS) return st;
     char *base = (char *)ws;
     __nv_bfloat16 *planesA = (__nv_bfloat16 *)base, *planesB = (__nv_bfloat16 *)(base + offB);
@@ -846,8 +849,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     p.status = status;
     p.timeout_ns = 2000ull * 1000 * 1000;
     p.rbuf = (long long *)(base + offR);
-    p.racc = (long long *)(base + offRacc);
-    p.rcnt = (int *)(base + offRcnt);
+    p.parts = (long long *)(base + offRacc);
 
     // Launches: when all slice groups' exact sum fits int64 over the whole K (up to
     // 65024 for S = 5), one.  Otherwise the slice groups are cut into ranges whose
@@ -876,11 +878,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
             p.nkb = (int)std::min<int64_t>(kb_per_pass, nkb_total - kb0);
             int pairs = 0;
             for (int d = p.d0; d < p.d1; d++) pairs += d + 1;
-            choose_schedule(p, nb, p.mtiles, p.ntiles, pairs, 1);
-            if (const size_t n = (size_t)cut_tiles(p, nb, p.mtiles, p.ntiles)) {
-                EG_CUDA(cudaMemsetAsync(p.racc, 0, n * kBM * kBN * 8, s));
-                EG_CUDA(cudaMemsetAsync(p.rcnt, 0, n * kTileRegions * sizeof(int), s));
-            }
+            choose_schedule(p, nb, p.mtiles, p.ntiles, pairs, 1, slices_max);
             const bool first = first_launch;
             first_launch = false;
             p.cp = first ? c.cp : 1.0;
@@ -976,7 +974,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
         bb = std::min<int64_t>(bb, (int64_t(1) << 20) / P);
     }
     const int64_t tiles = bb * (mb / kBM) * (nbk / kBN);
-    const int64_t cut = std::min<int64_t>(2 * tiles, num_sms()); // tiles cut along K, at most
+    const int64_t slices_max = slice_room(tiles, Kp / kBK); // tiles cut along K
     const int64_t all_tiles = nb * (Mp_all / kBM) * (Np_all / kBN);
     const bool tables = M + K <= (int64_t(1) << 22) && N + K <= (int64_t(1) << 22);
     size_t at = 0;
@@ -987,8 +985,8 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
     };
     const size_t oPA = take((size_t)bb * P * mb * Kp * 2), oPB = take((size_t)bb * P * nbk * Kp * 2);
     const size_t oMax = take((size_t)bb * (mb + nbk) * 8);
-    const size_t oCnt = take((size_t)cut * kTileRegions * sizeof(int)); // cleared for every panel pair, with
-    const size_t oAcc = take((size_t)cut * 2 * kBM * kBN * 8);          // those accumulators that the launch uses
+    const size_t oBad = take((size_t)slices_max * kTileRegions * sizeof(int));
+    const size_t oParts = take((size_t)slices_max * 2 * kBM * kBN * 8);
     const size_t oExp = take((size_t)bb * (mb + nbk) * 4);
     const size_t oTab = take(tables ? (size_t)(M + N + 2 * K) * 8 : 0);
     const size_t oR = take(rbuf_bytes(3));
@@ -1019,8 +1017,8 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
     p.status = status;
     p.timeout_ns = 2000ull * 1000 * 1000;
     p.rbuf = (long long *)(base + oR);
-    p.racc = (long long *)(base + oAcc);
-    p.rcnt = (int *)(base + oCnt);
+    p.parts = (long long *)(base + oParts);
+    p.parts_bad = (int *)(base + oBad);
     p.d0 = 0;
     p.d1 = S;
     p.hid = kF64High;
@@ -1035,9 +1033,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
             for (int64_t n0 = 0; n0 < N; n0 += nbk) {
                 const int64_t nc = std::min(nbk, N - n0), Np = round_up(nc, kBN);
                 p.nkb = (int)(Kp / kBK);
-                choose_schedule(p, nbc, Mp / kBM, Np / kBN, S * (S + 1) / 2 + 2, 2);
-                const size_t used = (size_t)cut_tiles(p, nbc, Mp / kBM, Np / kBN) * 2 * kBM * kBN * 8;
-                if (used) EG_CUDA(cudaMemsetAsync(base + oCnt, 0, oAcc - oCnt + used, s));
+                choose_schedule(p, nbc, Mp / kBM, Np / kBN, S * (S + 1) / 2 + 2, 2, slices_max);
                 OperandMap oa{c.batch, c.m, c.k, 0, mc, Mp, K, Kp, (int)nbc};
                 oa.b0 = b0;
                 oa.row0 = m0;
@@ -1087,7 +1083,8 @@ bool f64_tensor_pays(const Contraction &c) {
     p.nkb = (int)(round_up(K, kBK) / kBK);
     const int64_t mtiles = round_up(M, kBM) / kBM, ntiles = round_up(N, kBN) / kBN;
     if (nb * mtiles * ntiles > (int64_t(1) << 30)) return false;
-    const double clocks = choose_schedule(p, nb, mtiles, ntiles, kF64Slices * (kF64Slices + 1) / 2 + 2, 2);
+    const double clocks = choose_schedule(p, nb, mtiles, ntiles, kF64Slices * (kF64Slices + 1) / 2 + 2, 2,
+                                           slice_room(nb * mtiles * ntiles, p.nkb));
     const double tensor = 30e-6 + (double)nb * (double)(M + N) * (double)K * 36.0 / 3e12 + clocks / 1.9e9;
     return tensor < 0.9 * fma;
 }

@@ -67,16 +67,14 @@ struct TcGemmParams {
     // partly filled round of the CTAs (all of them when there are fewer tiles than
     // CTAs) are cut along K so that the round is full: entry t >= t0 is K slice
     // (t - t0) % ksplit (kslice K blocks; the last slice takes the rest) of
-    // tile t0 + (t - t0) / ksplit.  The slices' exact int64 sums are added into racc
-    // ([tile - t0][128 columns][128 rows], two planes in the FP64 form) and the last
-    // slice to arrive at a region of an epilogue warp (counted in rcnt,
-    // [tile - t0][8]) finishes it.  Both are zeroed by the host before the launch;
-    // unused when t0 is the number of tiles.  (With CTA pairs an entry is two tiles,
-    // and so has two accumulators.)
+    // tile t0 + (t - t0) / ksplit.  A slice's exact int64 sums go to parts ([t - t0]
+    // [128 columns][128 rows], two planes in the FP64 form; with CTA pairs an entry is
+    // two tiles, one after the other) and whether its check failed to parts_bad
+    // ([t - t0][8]); k_tc_finish_slices adds them up.  Unused when t0 is the number of tiles.
     int t0;
     int ksplit, kslice;
-    long long *racc;
-    int *rcnt;
+    long long *parts;
+    int *parts_bad;
     // Launch as CTA pairs (cta_group::2, 256x128 tiles): single contractions only.
     int pair;
     // Slice groups d0 <= d < d1 (anti-diagonals s + t = d of the digit pairs)

@@ -94,9 +94,8 @@ struct TileJob {
     int zA, zB;  // digit plane of slice 0 for A / B
     int kbeg;    // first K block (of this pass) of the K slice
     int nkb;     // K blocks
-    bool split;  // a K slice of a tile: its sums go to the tile's accumulator
-    int tid;     // which accumulator (single-contraction form); -1: rows past the last
-                 // tile (the odd half of a CTA pair's tile), nothing to store
+    int part;    // a K slice of a tile: where its sums go (-1: a whole tile); -2: rows past
+                 // the last tile (the odd half of a CTA pair's tile), nothing to store
     int64_t M, N;
     const ModeGroup *mg, *ng;
     const int *eA, *eB; // exponents of rows / columns of this (item, batch)
@@ -113,8 +112,9 @@ __device__ __forceinline__ TileJob resolve(const TcGemmParams &p, const TcItem *
     TileJob j;
     if (!GROUPED) {
         int b, mu, ks = 0;
-        j.split = t >= p.t0;
-        if (j.split) {
+        const bool split = t >= p.t0;
+        j.part = split ? (t - p.t0) * CL + rank : -1;
+        if (split) {
             const int e = t - p.t0, q = e / p.ksplit;
             ks = e - q * p.ksplit;
             t = p.t0 + q;
@@ -124,8 +124,8 @@ __device__ __forceinline__ TileJob resolve(const TcGemmParams &p, const TcItem *
         j.zA = b * p.planes;
         j.zB = b * p.planes;
         j.kbeg = ks * p.kslice;
-        j.nkb = j.split ? min(p.kslice, p.nkb - j.kbeg) : p.nkb;
-        j.tid = j.mt >= p.mtiles ? -1 : max(t - p.t0, 0) * CL + rank;
+        j.nkb = split ? min(p.kslice, p.nkb - j.kbeg) : p.nkb;
+        if (j.mt >= p.mtiles) j.part = -2;
         j.M = p.M;
         j.N = p.N;
         j.mg = &p.mg;
@@ -149,8 +149,7 @@ __device__ __forceinline__ TileJob resolve(const TcGemmParams &p, const TcItem *
         j.item = w.x;
         j.kbeg = 0;
         j.nkb = it.nkb;
-        j.split = false;
-        j.tid = 0;
+        j.part = -1;
         j.M = it.M;
         j.N = it.N;
         j.mg = &it.mg;
@@ -511,6 +510,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         // loop: finishing a tile's columns straight from the registers is as many times
         // the code, which ran at the rate of instruction fetch (80k clocks a tile).
         long long *const rbc = p.rbuf + (size_t)blockIdx.x * (F64 ? 3 : 1) * kPlane + (size_t)(half * kCols) * kBM + row;
+        // a K slice's sums: [128 columns][128 rows], two planes in the FP64 form
+        auto part_of = [&](int tile) {
+            return p.parts + (size_t)((tile - p.t0) * CL + rank) * PLANES * kPlane + (size_t)(half * kCols) * kBM + row;
+        };
         int parity = 0; // FP64 form: which of two scratch planes takes this tile's high sums
         int pend_cols = 0, pend_done = 0; // columns of the pending tile, and how many are done
         bool pend_rows_fast = false, pend_fast = false;
@@ -627,7 +630,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                             }
                             bad = __any_sync(0xffffffffu, worst < 0);
                         } else if (F64 && st.hi + 1 == p.hid) { // the high sums are complete
-                            long long *const at_hi = rbc + (1 + parity) * kPlane;
+                            long long *const at_hi = !GROUPED && tile >= p.t0 ? part_of(tile) + kPlane : rbc + (1 + parity) * kPlane;
 #pragma unroll
                             for (int i = 0; i < kCols; i++) {
                                 at_hi[i * kBM] = H[i];
@@ -706,51 +709,30 @@ __global__ void __launch_bounds__(THREADS, 1)
             // ---- end of tile: park its sums and make it the pending one
             pend_done = pend_cols = 0;
             const TileJob job = resolve<GROUPED, CL>(p, items, work, tile, rank);
-            if (!GROUPED && job.tid < 0) continue; // the odd half of a pair's last row of tiles
-            bool finish = true;
-            long long *const sums = job.split ? p.racc + (size_t)job.tid * PLANES * kPlane + (size_t)(half * kCols) * kBM + row : rbc;
+            if (!GROUPED && job.part == -2) continue; // the odd half of a pair's last row of tiles
+            const bool slice = !GROUPED && job.part >= 0; // k_tc_finish_slices adds it up
+            long long *const sums = slice ? part_of(tile) : rbc;
+#pragma unroll
+            for (int i = 0; i < kCols; i++) sums[i * kBM] = H[i];
+            if (slice) {
+                if (F64 && lane == 0) p.parts_bad[job.part * kTileRegions + ew] = bad ? 1 : 0;
+                continue;
+            }
             long long *const own_hi = rbc + (F64 ? 1 + parity : 0) * kPlane;
             parity ^= 1;
-            if (job.split) {
-                // K slices add their sums into the tile's accumulator; only the last
-                // one to arrive at this warp's region finishes it
-#pragma unroll
-                for (int i = 0; i < kCols; i++) atomicAdd((unsigned long long *)sums + i * kBM, (unsigned long long)H[i]);
-                if constexpr (F64) {
-#pragma unroll 8
-                    for (int i = 0; i < kCols; i++)
-                        atomicAdd((unsigned long long *)sums + kPlane + i * kBM, (unsigned long long)own_hi[i * kBM]);
-                }
-                __threadfence();
-                __syncwarp();
-                int arrived = 0;
-                if (lane == 0) {
-                    // arrivals in the low half, failed checks above them
-                    const int before = atomicAdd(p.rcnt + job.tid * kEpiWarps + ew, bad ? 0x10001 : 1);
-                    arrived = (before & 0xffff) == p.ksplit - 1;
-                    if (F64 && arrived && (before >> 16)) arrived = 2;
-                }
-                arrived = __shfl_sync(0xffffffffu, arrived, 0);
-                finish = arrived != 0;
-                if (F64 && arrived == 2) bad = true;
-                if (finish) __threadfence();
-            } else {
-#pragma unroll
-                for (int i = 0; i < kCols; i++) sums[i * kBM] = H[i];
-            }
-            if (F64 && finish && bad) {
-                finish = false;
+            if (F64 && bad) {
                 if (lane == 0) {
                     const int at = atomicAdd(p.redo_count, 1);
                     const int m0 = job.mt * kBM + quad * 32, n0 = job.nt * kBN + half * 16;
                     p.redo[at] = GROUPED ? make_int4(job.item, job.b, m0, n0)
                                          : make_int4(job.b, (int)p.m0 + m0, (int)p.n0 + n0, 0);
                 }
+                continue;
             }
-            if (!finish || live == 0) continue;
+            if (live == 0) continue;
             pend_cols = live;
             pend_lo = sums;
-            pend_hi = (int)(job.split ? kPlane : (size_t)(own_hi - sums));
+            pend_hi = (int)(own_hi - sums);
             pend_rows_fast = job.mg->n > 0 && job.mg->s[2][job.mg->n - 1] == 1;
             const int64_t m = (int64_t)job.mt * kBM + row;
             const bool row_ok = m < job.M;
@@ -791,6 +773,91 @@ __global__ void __launch_bounds__(THREADS, 1)
         ptx::tc_fence_after();
         ptx::tmem_dealloc<CL>(tmem, TMEM_COLS);
     }
+}
+
+// The tiles cut along K: a CTA adds up the slices of half the columns of a region of a
+// tile (a region is one epilogue warp's), checks and scales the sums and applies them to C.  Bound: memory (8 or
+// 16 bytes of sums per output and slice, mostly from L2).  Slices that add themselves to
+// one accumulator with atomics, the last to arrive finishing it, took 36 us for the
+// atomics (they retire some 70 a clock) and 29 us for the finishing of 144 x 2304, K =
+// 2304 in FP64, while the other CTAs were done; stores and this kernel take about 15 us
+// (the whole contraction 190 -> 132 us, 2304 x 2304 715 -> 672 us).
+constexpr int kFinishRows = 8, kFinishCols = 32, kFinishParts = kCols / kFinishCols; // warps and columns of its CTAs
+template <int CL, bool F64>
+__global__ void __launch_bounds__(32 * kFinishRows) k_tc_finish_slices(const __grid_constant__ TcGemmParams p) {
+    __shared__ double tile[kFinishCols][33];
+    constexpr int PLANES = F64 ? 2 : 1, PER = kFinishCols / kFinishRows;
+    constexpr size_t kPlane = (size_t)kBM * kBN;
+    const int c0 = blockIdx.x % kFinishParts * kFinishCols; // of the region's columns
+    const int ew = blockIdx.x / kFinishParts % kTileRegions, u = blockIdx.x / (kFinishParts * kTileRegions);
+    const int rank = u % CL, q = u / CL;
+    int b, mu, nt;
+    tile_coords<CL>(p, p.t0 + q, b, mu, nt);
+    const int mt = mu * CL + rank;
+    if (mt >= p.mtiles) return;
+    const int quad = ew & 3, half = ew >> 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t m0 = (int64_t)mt * kBM + quad * 32, n0 = (int64_t)nt * kBN;
+    const int rows = (int)min((int64_t)32, p.M - m0), cols = (int)min((int64_t)kBN, p.N - n0);
+    const int live = min(cols / 32 * 16 + min(max(cols % 32 - half * 16, 0), 16) - c0, kFinishCols);
+    if (rows <= 0 || live <= 0) return;
+    const int e0 = q * p.ksplit * CL + rank; // the tile's first slice; the next ones are CL further on
+    if (F64) {
+        int bad = 0;
+        for (int k = 0; k < p.ksplit; k++) bad |= p.parts_bad[(e0 + k * CL) * kTileRegions + ew];
+        if (bad) {
+            if (threadIdx.x == 0 && c0 == 0)
+                p.redo[atomicAdd(p.redo_count, 1)] =
+                    make_int4((int)p.b0 + b, (int)(p.m0 + m0), (int)(p.n0 + n0) + half * 16, 0);
+            return;
+        }
+    }
+    // where this thread will write, along C's rows or columns, and C's old values there
+    const bool plain_store = p.zero && p.cp == 0.0;
+    const bool rows_fast = p.mg.n > 0 && p.mg.s[2][p.mg.n - 1] == 1;
+    int64_t oa, ob, oc;
+    group_offsets(p.bg, p.b0 + b, oa, ob, oc);
+    double *out[PER], old[PER];
+    const double *from[PER];
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        const int x = (threadIdx.x >> 5) + i * kFinishRows;
+        const int r = rows_fast ? lane : x, c = rows_fast ? x : lane;
+        from[i] = &tile[c][r];
+        out[i] = nullptr;
+        old[i] = 0.0;
+        if (r < rows && c < live) {
+            int64_t om, on;
+            group_offsets32(p.mg, (uint32_t)(p.m0 + m0 + r), oa, ob, om);
+            group_offsets32(p.ng, (uint32_t)(p.n0 + n0 + tile_col(half, c0 + c)), oa, ob, on);
+            out[i] = p.C + oc + om + on;
+            if (!plain_store) old[i] = *out[i];
+        }
+    }
+    // a warp takes every kFinishRows-th column, lanes along the rows
+    long long lo[PER] = {}, hi[PER] = {};
+    const long long *at =
+        p.parts + (size_t)e0 * PLANES * kPlane + (size_t)(half * kCols + c0 + warp) * kBM + quad * 32 + lane;
+#pragma unroll 2
+    for (int k = 0; k < p.ksplit; k++, at += CL * PLANES * kPlane) {
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            lo[i] += __ldcg(at + i * kFinishRows * kBM);
+            if (F64) hi[i] += __ldcg(at + kPlane + i * kFinishRows * kBM);
+        }
+    }
+    const int rowExp = lane < rows ? p.eA[(int64_t)b * p.Mp + m0 + lane] : 0;
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        const int c = warp + i * kFinishRows;
+        if (c >= live) break;
+        const int colExp = p.eB[(int64_t)b * p.Np + n0 + tile_col(half, c0 + c)];
+        const double v = finish_value<F64, false>(p, lo[i], hi[i], rowExp, colExp);
+        tile[c][lane] = p.ab_pow2 ? v : p.ab * v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; i++)
+        if (out[i]) *out[i] = plain_store ? *from[i] : fma(p.cp, old[i], *from[i]);
 }
 
 } // namespace
@@ -880,6 +947,16 @@ eg_status launch_tc_gemm(const CUtensorMap &tmA, const CUtensorMap &tmB, const C
         }
     }
     EG_CHECK_LAUNCH("k_tc_split_gemm");
+    const int slices = total - p.t0;
+    if (p.ksplit > 1 && slices > 0) {
+        {
+            LaunchScope ls_("k_tc_finish_slices", s);
+            auto finish = p.pair ? (f64 ? k_tc_finish_slices<2, true> : k_tc_finish_slices<2, false>)
+                                 : (f64 ? k_tc_finish_slices<1, true> : k_tc_finish_slices<1, false>);
+            finish<<<(unsigned)(slices / p.ksplit * CL * kTileRegions * kFinishParts), 32 * kFinishRows, 0, s>>>(p);
+        }
+        EG_CHECK_LAUNCH("k_tc_finish_slices");
+    }
     return EG_SUCCESS;
 }
 
