@@ -393,30 +393,42 @@ __global__ void __launch_bounds__(kFusedThreads) k_split_rows(const __grid_const
         __syncthreads();
     const int64_t plane = m.Rp * m.Kp;
     const int kw = (int)max((int64_t)0, min((int64_t)kc, m.Kp - k0)); // range written, a multiple of 4
-    for (int r = warp; r < R; r += W) {
+    // four elements a thread, rows one after the other: a warp runs across the ends of rows,
+    // so that rows of few elements keep all lanes busy (a row to a warp at a time left 12 of
+    // 32 idle at K = 75)
+    const int quads = kw / 4;
+    __nv_bfloat16 *const first = jj.planes + (int64_t)b * P * plane + r0 * m.Kp + k0;
+    int r = tid / max(quads, 1), k = tid - r * quads;
+    const int dr = kFusedThreads / max(quads, 1), dk = kFusedThreads - dr * quads;
+    for (int i = tid; i < R * quads; i += kFusedThreads) {
+        const double *x = tile + r * ld + 4 * k;
+        const double2 v0 = *(const double2 *)x, v1 = *(const double2 *)(x + 2);
+        uint32_t p0[P], p1[P];
         const int e = ex[r];
-        __nv_bfloat16 *row = jj.planes + (int64_t)b * P * plane + (r0 + r) * m.Kp + k0;
-        for (int k = 4 * lane; k < kw; k += 128) {
-            const double2 v0 = *(const double2 *)&tile[r * ld + k], v1 = *(const double2 *)&tile[r * ld + k + 2];
-            uint32_t p0[P], p1[P];
-            if (e == INT_MIN) {
+        if (e == INT_MIN) {
 #pragma unroll
-                for (int s = 0; s < P; s++) p0[s] = p1[s] = 0u;
-            } else {
-                digits_bf16x2<S>(v0.x, v0.y, e, p0);
-                digits_bf16x2<S>(v1.x, v1.y, e, p1);
-                if constexpr (CHECK) {
-                    p0[S] = check_magnitude(p0[0]);
-                    p1[S] = check_magnitude(p1[0]);
-                }
-            }
+            for (int s = 0; s < P; s++) p0[s] = p1[s] = 0u;
+        } else {
+            digits_bf16x2<S>(v0.x, v0.y, e, p0);
+            digits_bf16x2<S>(v1.x, v1.y, e, p1);
             if constexpr (CHECK) {
-                const float mark = m.comp ? kCheckB : kCheckA;
-                p0[S + 1] = check_mark(v0.x, v0.y, mark);
-                p1[S + 1] = check_mark(v1.x, v1.y, mark);
+                p0[S] = check_magnitude(p0[0]);
+                p1[S] = check_magnitude(p1[0]);
             }
+        }
+        if constexpr (CHECK) {
+            const float mark = m.comp ? kCheckB : kCheckA;
+            p0[S + 1] = check_mark(v0.x, v0.y, mark);
+            p1[S + 1] = check_mark(v1.x, v1.y, mark);
+        }
+        __nv_bfloat16 *row = first + r * m.Kp + 4 * k;
 #pragma unroll
-            for (int s = 0; s < P; s++) *(uint2 *)(row + s * plane + k) = make_uint2(p0[s], p1[s]);
+        for (int s = 0; s < P; s++) *(uint2 *)(row + s * plane) = make_uint2(p0[s], p1[s]);
+        r += dr;
+        k += dk;
+        if (k >= quads) {
+            k -= quads;
+            r++;
         }
     }
 }
@@ -467,7 +479,7 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
-// 3-D map over [planes][rows][Kp] BF16, box 64 (k) x box_rows rows x 1, 128-byte swizzle.
+// 3-D map over [planes][rows][Kp] BF16 (zeros beyond Kp), box 64 (k) x box_rows rows x 1, 128-byte swizzle.
 eg_status encode_planes(CUtensorMap *map, void *base, int64_t Kp, int64_t rows, int64_t planes, int box_rows = kBM) {
     auto fn = encode_fn();
     if (!fn) return fail(EG_ERROR_CUDA, "cuTensorMapEncodeTiled is unavailable");
@@ -585,13 +597,23 @@ cudaError_t launch_split_rows(const SplitJob &a, const SplitJob &b, int kc, int 
     return cudaLaunchKernelEx(&cfg, k_split_rows<S, CHECK, R>, a, b, kc, ld, C);
 }
 
+// Elements from row to row of the digit planes: K in whole blocks of 64, or for a short K
+// of which those would be an eighth padding or more, in 32-byte sectors (the tensor maps
+// fill the rest of the last block with zeros; only the fused launch writes such rows).
+// 421875 x 75: 68 MB a plane instead of 108; with ten of them the splitting takes 222 us
+// instead of 228, and 180 with the rows' elements spread over all lanes (k_split_rows).
+int64_t plane_pitch(int64_t K) {
+    const int64_t sectors = round_up(K, 16), blocks = round_up(K, kBK);
+    return K <= 512 && 8 * sectors <= 7 * blocks ? sectors : blocks;
+}
+
 // Splits the operands of a contraction (an operand without rows is left out).  The
 // fused launch when a range of K fits shared memory (K to about 25000); beyond, the
 // passes over each operand, with tables of offsets at tab (rows and K of each operand;
 // may be null).  Fused against passes, device time: both operands of 2304^3 in FP64
 // 165 -> 68 us, the six splits of a ring contraction with adjoints at o = 24, v = 96
-// 515 -> 211 us, the four of n = 75 quarter transformations 1.90 -> 1.05 ms (1.3 GB
-// each: 5.0 TB/s).
+// 515 -> 211 us, the four of n = 75 quarter transformations 1.90 -> 0.72 ms (0.9 GB
+// each: 5.2 TB/s).
 eg_status split_both(OperandMap oa, const double *A, int *eA, __nv_bfloat16 *pA, OperandMap ob, const double *B, int *eB,
                      __nv_bfloat16 *pB, unsigned long long *maxima, int64_t *tab, int S, bool f64, cudaStream_t s) {
     for (OperandMap *o : {&oa, &ob}) {
@@ -785,7 +807,8 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     const int64_t nb = c.batch.total, M = c.m.total, N = c.n.total, K = c.k.total;
     if (M >= (int64_t(1) << 31) || N >= (int64_t(1) << 31) || K >= (int64_t(1) << 31) || nb * S >= (int64_t(1) << 31))
         return fail(EG_ERROR_NOT_SUPPORTED, "split form: a mode group exceeds 2^31 elements");
-    const int64_t Kp = round_up(K, kBK), Mp = round_up(M, kBM), Np = round_up(N, kBN);
+    const int64_t Kp = plane_pitch(K), Mp = round_up(M, kBM), Np = round_up(N, kBN);
+    const int64_t nkb_total = (K + kBK - 1) / kBK;
 
     // workspace: digit planes of A and B, row maxima, exponents, status word
     const size_t bytesA = (size_t)nb * S * Mp * Kp * 2, bytesB = (size_t)nb * S * Np * Kp * 2;
@@ -800,7 +823,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     const size_t tabBytes = tables ? (size_t)(M + N + 2 * K) * 8 : 0;
     const int64_t tiles = nb * (Mp / kBM) * (Np / kBN);
     const size_t offRacc = round_up((int64_t)(offTab + tabBytes), 256);
-    int64_t slices_max = slice_room(tiles, Kp / kBK); // tiles cut along K
+    int64_t slices_max = slice_room(tiles, nkb_total); // tiles cut along K
     const size_t raccBytes = (size_t)slices_max * kBM * kBN * 8;
     size_t total = offRacc + raccBytes;
     void *ws = nullptr;
@@ -857,7 +880,6 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     // into C in FP64 by its own launch -- one extra rounding per range instead of a
     // launch (and a read and write of C) per 128 of K; a range that still cannot
     // take the whole K runs K passes.
-    const int64_t nkb_total = Kp / kBK;
     std::vector<std::pair<int, int>> ranges;
     for (int d0 = 0; d0 < S;) {
         int d1 = d0 + 1;
@@ -951,7 +973,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
     using namespace split;
     constexpr int S = kF64Slices, P = S + 2;
     const int64_t nb = c.batch.total, M = c.m.total, N = c.n.total, K = c.k.total;
-    const int64_t Kp = round_up(K, kBK);
+    const int64_t Kp = plane_pitch(K), nkb = (K + kBK - 1) / kBK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     EG_CUDA(cudaStreamIsCapturing(s, &cap));
     if (cap != cudaStreamCaptureStatusNone) return EG_ERROR_NOT_SUPPORTED;
@@ -974,7 +996,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
         bb = std::min<int64_t>(bb, (int64_t(1) << 20) / P);
     }
     const int64_t tiles = bb * (mb / kBM) * (nbk / kBN);
-    const int64_t slices_max = slice_room(tiles, Kp / kBK); // tiles cut along K
+    const int64_t slices_max = slice_room(tiles, nkb); // tiles cut along K
     const int64_t all_tiles = nb * (Mp_all / kBM) * (Np_all / kBN);
     const bool tables = M + K <= (int64_t(1) << 22) && N + K <= (int64_t(1) << 22);
     size_t at = 0;
@@ -1032,7 +1054,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
             const int64_t mc = std::min(mb, M - m0), Mp = round_up(mc, kBM);
             for (int64_t n0 = 0; n0 < N; n0 += nbk) {
                 const int64_t nc = std::min(nbk, N - n0), Np = round_up(nc, kBN);
-                p.nkb = (int)(Kp / kBK);
+                p.nkb = (int)nkb;
                 choose_schedule(p, nbc, Mp / kBM, Np / kBN, S * (S + 1) / 2 + 2, 2, slices_max);
                 OperandMap oa{c.batch, c.m, c.k, 0, mc, Mp, K, Kp, (int)nbc};
                 oa.b0 = b0;
