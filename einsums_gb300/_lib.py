@@ -7,6 +7,7 @@ every entry point raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 
@@ -126,6 +127,8 @@ _LOCK = threading.Lock()
 def load(path: str | None = None):
     """Load the library (once) and attach prototypes.  Raises when absent."""
     global _LIB
+    if _LIB is not None:
+        return _LIB
     with _LOCK:
         if _LIB is None:
             p = path or LIB_PATH
@@ -158,9 +161,11 @@ def label_id(name) -> int:
     return h & 0x7FFFFFFF
 
 
+@functools.lru_cache(maxsize=1024)
+def _label_array(names: tuple) -> ctypes.Array:
+    return (ctypes.c_int32 * max(1, len(names)))(*map(label_id, names))
+
+
 def labels(names) -> ctypes.Array:
-    ids = [label_id(n) for n in names]
-    arr = (ctypes.c_int32 * max(1, len(ids)))()
-    for i, v in enumerate(ids):
-        arr[i] = v
-    return arr
+    """The labels of index names, as the library's calls read them (never written to)."""
+    return _label_array(tuple(map(str, names)))
