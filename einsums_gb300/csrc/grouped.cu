@@ -189,7 +189,7 @@ struct GOp {
     int64_t sr, sk;       // the single element stride of the rows / of K when the modes nest (else 0: tables)
 };
 
-__device__ __forceinline__ int64_t pick(int comp, int64_t oa, int64_t ob) { return comp == 0 ? oa : ob; }
+__host__ __device__ __forceinline__ int64_t pick(int comp, int64_t oa, int64_t ob) { return comp == 0 ? oa : ob; }
 
 // One work unit = 32 rows of one operand of one item (and batch index): the
 // rows' maxima (the operand is read once along its contiguous direction), their
@@ -316,40 +316,52 @@ __global__ void __launch_bounds__(kGThreads, 4) k_grouped_split(const GOp *ops, 
     }
 }
 
-// The same when every item's K is short (kRowsMaxK): a unit is 32 rows or fewer (int4
-// .w, a power of two), as many as keep it within 32 KB of shared memory, so that every
-// element is read once, all of a unit's loads in flight at once while the unit before is
-// converted, and the maxima and digits are taken from shared memory.  Bound: integer
-// instructions and memory about equally; the unit above read each element twice, a few
-// loads per thread at a time.
+// The same when every item's K is short (kRowsMaxK): a unit is 32 rows or fewer (a power
+// of two), as many as keep it within 32 KB of shared memory, so that every element is read
+// once, all of a unit's loads in flight at once while the unit before is converted, and
+// the maxima and digits are taken from shared memory.  Bound: latency and integer
+// instructions; the unit above read each element twice, a few loads per thread at a time.
+// What a unit needs to be known stands in one record, itself fetched three units ahead:
+// looked up through the operand's, its loads waited for three chains of loads first
+// (2048 items of 4-32 x 4-32 summed, 20-120 x 20-120, S = 5: 286 us, now 241).
 constexpr int64_t kRowsElems = 4096, kRowsMaxK = 1152;
+
+struct alignas(16) RowsUnit {
+    const double *X;       // the operand at this batch index (and at the first row, when sr)
+    __nv_bfloat16 *planes; // the first row's leading digits
+    int *rexp;             // the rows' exponents
+    int64_t sr, sk;        // strides of the rows and of k, 0: the tables at rtab (first row), ktab
+    int64_t rtab, ktab;
+    int64_t pitch, pstride;
+    int K, R, rows; // rows: of the R, those that exist
+    int flags;      // 1: contiguous along the rows, 2: the operand is B
+};
+constexpr int kUnitSlots = 4;
+static_assert(sizeof(RowsUnit) % 16 == 0 && sizeof(RowsUnit) / 16 <= 32, "fetched by one warp, 16 bytes a lane");
 
 __host__ __device__ inline int rows_ld(int64_t K) { return (int)((K + 15) / 16 * 16 + 2); }
 
 template <int S, bool CHECK>
-__global__ void __launch_bounds__(kGThreads, 3) k_grouped_rows(const GOp *ops, const int4 *units, int nunits,
-                                                               const long long *__restrict__ offs, int *rexpA, int *rexpB,
-                                                               __nv_bfloat16 *planesA, __nv_bfloat16 *planesB,
-                                                               int tile_elems) {
+__global__ void __launch_bounds__(kGThreads, 3) k_grouped_rows(const RowsUnit *units, int nunits,
+                                                               const long long *__restrict__ offs, int tile_elems) {
     extern __shared__ __align__(16) double tiles[]; // two of [rows of the unit][rows_ld(K)]
+    __shared__ RowsUnit slots[kUnitSlots];
+    __shared__ int ex[32];
     constexpr int P = S + (CHECK ? 2 : 0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    auto load = [&](int u, double *tile) {
+    auto fetch = [&](int64_t u, int n) { // the record of this CTA's n-th unit
+        if (u < nunits && threadIdx.x < sizeof(RowsUnit) / 16)
+            ptx::cp_async16((double *)&slots[n % kUnitSlots] + 2 * threadIdx.x, (const double *)(units + u) + 2 * threadIdx.x);
+    };
+    auto load = [&](int64_t u, int n, double *tile) {
         if (u < nunits) {
-            const int4 un = units[u];
-            const GOp &g = ops[un.x];
-            const int64_t b = un.y, r0 = un.z;
-            const int R = un.w, K = (int)g.K, ld = rows_ld(K), kw = (K + 3) & ~3;
-            const int nr = (int)(g.rows - r0 < R ? g.rows - r0 : R);
-            const int64_t sr = g.sr, sk = g.sk;
-            int64_t oa, ob, oc;
-            group_offsets(g.bg, b, oa, ob, oc);
-            const double *X = g.X + pick(g.comp, oa, ob);
-            auto row_at = [&](int r) { return sr ? (r0 + r) * sr : (int64_t)__ldg(offs + g.rtab + r0 + r); };
-            auto k_at = [&](int k) { return (int64_t)__ldg(offs + g.ktab + k); };
+            const RowsUnit &g = slots[n % kUnitSlots];
+            const int R = g.R, K = g.K, ld = rows_ld(K), kw = (K + 3) & ~3, nr = g.rows;
+            const int64_t sr = g.sr, sk = g.sk, rtab = g.rtab, ktab = g.ktab;
+            const double *X = g.X;
             // (a single k stride is added up: the loop is two copies for it)
             auto row_copy = [&](int r, int k, int step) { // k, k + step, ... of row r
-                const double *x = X + row_at(r);
+                const double *x = X + (sr ? r * sr : (int64_t)__ldg(offs + rtab + r));
                 double *t = tile + r * ld;
                 if (sk) {
                     const int64_t inc = (int64_t)step * sk;
@@ -358,60 +370,76 @@ __global__ void __launch_bounds__(kGThreads, 3) k_grouped_rows(const GOp *ops, c
                     for (; k < K; k += step, x += inc) ptx::cp_async8(t + k, x);
                 } else {
 #pragma unroll 4
-                    for (; k < K; k += step) ptx::cp_async8(t + k, x + k_at(k));
+                    for (; k < K; k += step) ptx::cp_async8(t + k, x + __ldg(offs + ktab + k));
                 }
                 for (; k < kw; k += step) t[k] = 0.0;
             };
-            if (g.row_fast) {
+            if (g.flags & 1) {
                 const int r = lane & (R - 1), per = 32 / R;
                 if (r < nr) row_copy(r, warp * per + lane / R, kGWarps * per);
             } else {
                 for (int r = warp; r < nr; r += kGWarps) row_copy(r, lane, 32);
             }
         }
-        ptx::cp_async_commit();
     };
-    int buf = 0;
-    load(blockIdx.x, tiles);
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-        load(u + gridDim.x, tiles + (buf ^ 1) * tile_elems);
+    const int64_t u0 = blockIdx.x, step = gridDim.x;
+    for (int n = 0; n < 3; n++) fetch(u0 + n * step, n);
+    ptx::cp_async_commit();
+    ptx::cp_async_wait<0>();
+    __syncthreads();
+    load(u0, 0, tiles);
+    ptx::cp_async_commit();
+    int n = 0, buf = 0;
+    for (int64_t u = u0; u < nunits; u += step, n++) {
+        load(u + step, n + 1, tiles + (buf ^ 1) * tile_elems);
+        fetch(u + 3 * step, n + 3); // has landed two units on: its slot was read up to the unit before
+        ptx::cp_async_commit();
         ptx::cp_async_wait<1>();
         __syncthreads();
         const double *tile = tiles + buf * tile_elems;
-        const int4 un = units[u];
-        const GOp &g = ops[un.x];
-        const int64_t b = un.y, r0 = un.z;
-        const int K = (int)g.K, ld = rows_ld(K), kw = (K + 3) & ~3;
-        const int nr = (int)(g.rows - r0 < un.w ? g.rows - r0 : un.w);
+        const RowsUnit &g = slots[n % kUnitSlots];
+        const int K = g.K, ld = rows_ld(K), kw = (K + 3) & ~3, nr = g.rows;
         const int64_t pstride = g.pstride, pitch = g.pitch;
-        // a warp takes whole rows: the maximum, then the digits of four k a lane at a time
-        __nv_bfloat16 *planes = (g.comp ? planesB : planesA) + g.plane0 + b * P * pstride + r0 * pitch;
-        int *rexp = (g.comp ? rexpB : rexpA) + g.rowbase + b * g.Rp + r0;
-        const float mark = g.comp ? split::kCheckB : split::kCheckA;
+        // the rows' exponents, a warp to a row, then the digits, four k a thread and the rows
+        // one after the other, so that rows of few k keep all lanes busy
+        __nv_bfloat16 *const planes = g.planes;
+        int *const rexp = g.rexp;
+        const float mark = g.flags & 2 ? split::kCheckB : split::kCheckA;
         for (int r = warp; r < nr; r += kGWarps) {
             const int e = split::row_exponent(split::row_max_bits(tile + r * ld, kw, lane));
-            if (lane == 0) rexp[r] = e;
-            __nv_bfloat16 *row = planes + r * pitch;
-            for (int k = 4 * lane; k < kw; k += 128) {
-                const double2 v0 = *(const double2 *)&tile[r * ld + k], v1 = *(const double2 *)&tile[r * ld + k + 2];
-                uint32_t p0[P], p1[P];
-                if (e == INT_MIN) {
+            if (lane == 0) ex[r] = rexp[r] = e;
+        }
+        __syncthreads();
+        const int quads = kw / 4, dr = kGThreads / quads, dk = kGThreads - dr * quads;
+        int r = threadIdx.x / quads, k = threadIdx.x - r * quads;
+        for (int i = threadIdx.x; i < nr * quads; i += kGThreads) {
+            const double *x = tile + r * ld + 4 * k;
+            const double2 v0 = *(const double2 *)x, v1 = *(const double2 *)(x + 2);
+            uint32_t p0[P], p1[P];
+            const int e = ex[r];
+            if (e == INT_MIN) {
 #pragma unroll
-                    for (int s = 0; s < P; s++) p0[s] = p1[s] = 0u;
-                } else {
-                    split::digits_bf16x2<S>(v0.x, v0.y, e, p0);
-                    split::digits_bf16x2<S>(v1.x, v1.y, e, p1);
-                    if constexpr (CHECK) {
-                        p0[S] = split::check_magnitude(p0[0]);
-                        p1[S] = split::check_magnitude(p1[0]);
-                    }
-                }
+                for (int s = 0; s < P; s++) p0[s] = p1[s] = 0u;
+            } else {
+                split::digits_bf16x2<S>(v0.x, v0.y, e, p0);
+                split::digits_bf16x2<S>(v1.x, v1.y, e, p1);
                 if constexpr (CHECK) {
-                    p0[S + 1] = split::check_mark(v0.x, v0.y, mark);
-                    p1[S + 1] = split::check_mark(v1.x, v1.y, mark);
+                    p0[S] = split::check_magnitude(p0[0]);
+                    p1[S] = split::check_magnitude(p1[0]);
                 }
+            }
+            if constexpr (CHECK) {
+                p0[S + 1] = split::check_mark(v0.x, v0.y, mark);
+                p1[S + 1] = split::check_mark(v1.x, v1.y, mark);
+            }
+            __nv_bfloat16 *row = planes + r * pitch + 4 * k;
 #pragma unroll
-                for (int s = 0; s < P; s++) *(uint2 *)(row + s * pstride + k) = make_uint2(p0[s], p1[s]);
+            for (int s = 0; s < P; s++) *(uint2 *)(row + s * pstride) = make_uint2(p0[s], p1[s]);
+            r += dr;
+            k += dk;
+            if (k >= quads) {
+                k -= quads;
+                r++;
             }
         }
         __syncthreads(); // the tile is read before the loads of the unit after next replace it
@@ -441,13 +469,13 @@ cudaError_t allow_grouped_rows(int S, bool f64) {
     });
 }
 
-eg_status launch_grouped_rows(int S, bool f64, const GOp *ops, const int4 *units, int nunits, const long long *offs, int *eA,
-                              int *eB, __nv_bfloat16 *pA, __nv_bfloat16 *pB, size_t smem, cudaStream_t s) {
+eg_status launch_grouped_rows(int S, bool f64, const RowsUnit *units, int nunits, const long long *offs, size_t smem,
+                              cudaStream_t s) {
     const int per_sm = std::max(1, std::min<int>(8, (int)(220 * 1024 / (smem + 1024))));
     const int grid = std::min(std::max(nunits, 1), num_sms() * per_sm);
     with_slices(S, f64, [&](auto slices, auto check) {
         k_grouped_rows<decltype(slices)::value, decltype(check)::value>
-            <<<grid, kGThreads, smem, s>>>(ops, units, nunits, offs, eA, eB, pA, pB, (int)(smem / 16));
+            <<<grid, kGThreads, smem, s>>>(units, nunits, offs, (int)(smem / 16));
         return 0;
     });
     EG_CHECK_LAUNCH("k_grouped_rows");
@@ -814,7 +842,35 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
     EG_CUDA(cudaMemsetAsync(eA, 0, (size_t)rowsA * 4, s));
     EG_CUDA(cudaMemsetAsync(eB, 0, (size_t)rowsB * 4, s));
     if ((st = dev_copy(plan, ops.data(), ops.size() * sizeof(GOp), &d_ops)) != EG_SUCCESS) return st;
-    if ((st = dev_copy(plan, units.data(), units.size() * sizeof(int4), &d_units)) != EG_SUCCESS) return st;
+    if (by_rows) {
+        std::vector<RowsUnit> rows;
+        rows.reserve(units.size());
+        for (const int4 &u : units) {
+            const GOp &g = ops[u.x];
+            int64_t oa, ob, oc;
+            group_offsets(g.bg, u.y, oa, ob, oc);
+            const int64_t r0 = u.z;
+            RowsUnit x{};
+            x.X = g.X + pick(g.comp, oa, ob) + (g.sr ? r0 * g.sr : 0);
+            x.planes = (__nv_bfloat16 *)(g.comp ? planesB : planesA) + g.plane0 + u.y * P * g.pstride + r0 * g.pitch;
+            x.rexp = (int *)(g.comp ? eB : eA) + g.rowbase + u.y * g.Rp + r0;
+            x.sr = g.sr;
+            x.sk = g.sk;
+            x.rtab = g.rtab + r0;
+            x.ktab = g.ktab;
+            x.pitch = g.pitch;
+            x.pstride = g.pstride;
+            x.K = (int)g.K;
+            x.R = u.w;
+            x.rows = (int)std::min<int64_t>(g.rows - r0, u.w);
+            x.flags = (g.row_fast ? 1 : 0) | (g.comp ? 2 : 0);
+            rows.push_back(x);
+        }
+        st = dev_copy(plan, rows.data(), rows.size() * sizeof(RowsUnit), &d_units);
+    } else {
+        st = dev_copy(plan, units.data(), units.size() * sizeof(int4), &d_units);
+    }
+    if (st != EG_SUCCESS) return st;
     if ((st = dev_copy(plan, offs.data(), offs.size() * sizeof(long long), &d_offs)) != EG_SUCCESS) return st;
     if ((st = dev_copy(plan, items.data(), items.size() * sizeof(TcItem), &d_items)) != EG_SUCCESS) return st;
     if ((st = dev_copy(plan, wl.data(), wl.size() * sizeof(int4), &d_work)) != EG_SUCCESS) return st;
@@ -896,9 +952,8 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int s
         auto issue = [&]() -> eg_status {
             if (f64) EG_CUDA(cudaMemsetAsync(redo_count, 0, sizeof(int), s));
             eg_status is =
-                by_rows ? launch_grouped_rows(S, f64, (const GOp *)d_ops, (const int4 *)d_units, (int)units.size(),
-                                              (const long long *)d_offs, (int *)eA, (int *)eB, (__nv_bfloat16 *)planesA,
-                                              (__nv_bfloat16 *)planesB, rows_smem, s)
+                by_rows ? launch_grouped_rows(S, f64, (const RowsUnit *)d_units, (int)units.size(),
+                                              (const long long *)d_offs, rows_smem, s)
                         : launch_grouped_split(S, (const GOp *)d_ops, (const int4 *)d_units, (int)units.size(),
                                                (const long long *)d_offs, (int *)eA, (int *)eB, (__nv_bfloat16 *)planesA,
                                                (__nv_bfloat16 *)planesB, s);
