@@ -717,8 +717,28 @@ bool f64_tensor_plan_pays(const std::vector<Contraction> &cs) {
 // Builds and captures the split-BF16 plan, or (f64) the FP64 one on the tensor cores;
 // returns EG_ERROR_NOT_SUPPORTED when an item's K needs more than one exact pass (the
 // caller then runs items one by one).
-eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &cs, int slices, cudaStream_t s, bool f64) {
+// C = B A instead of A B, for an item whose tiles then end sooner: a tile's time is its
+// epilogue's, that of the columns of one warp of each lane quadrant, whether or not its
+// rows fill the four quadrants (30 x 100: 64 columns a warp, 100 x 30: 16).  The sums are
+// exact either way, so the results are the same bits.  2048 uneven items in five
+// slices: 557 -> 523 us, 512 in FP64: 328 -> 319.
+Contraction better_side_first(const Contraction &c) {
     using namespace split;
+    auto warp_columns = [](int64_t n) { return n / 32 * 16 + std::min<int64_t>(n % 32, 16); };
+    auto cost = [&](int64_t m, int64_t n) { return (m + kBM - 1) / kBM * warp_columns(n); };
+    if (cost(c.n.total, c.m.total) >= cost(c.m.total, c.n.total)) return c;
+    Contraction t = c;
+    std::swap(t.A, t.B);
+    std::swap(t.m, t.n);
+    for (ModeGroup *g : {&t.batch, &t.m, &t.n, &t.k})
+        for (int d = 0; d < g->n; d++) std::swap(g->s[0][d], g->s[1][d]);
+    return t;
+}
+
+eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, int slices, cudaStream_t s, bool f64) {
+    using namespace split;
+    std::vector<Contraction> cs;
+    for (auto &c : given) cs.push_back(better_side_first(c));
     const int S = f64 ? kF64Slices : slices ? slices : 5, P = f64 ? S + 2 : S;
     if (!f64 && (S < 2 || S > kMaxSlices)) return fail(EG_ERROR_INVALID_ARGUMENT, "split form: slices must be in 2..6");
     const int64_t kmax = f64 ? kRowsMaxK : max_k_per_pass(S);
