@@ -20,10 +20,12 @@
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <numeric>
+#include <queue>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -714,17 +716,14 @@ bool f64_tensor_plan_pays(const std::vector<Contraction> &cs) {
     return planes < 1e9 && t_tensor < 0.8 * t_fma;
 }
 
-// Builds and captures the split-BF16 plan, or (f64) the FP64 one on the tensor cores;
-// returns EG_ERROR_NOT_SUPPORTED when an item's K needs more than one exact pass (the
-// caller then runs items one by one).
 // C = B A instead of A B, for an item whose tiles then end sooner: a tile's time is its
 // epilogue's, that of the columns of one warp of each lane quadrant, whether or not its
 // rows fill the four quadrants (30 x 100: 64 columns a warp, 100 x 30: 16).  The sums are
 // exact either way, so the results are the same bits.  2048 uneven items in five
 // slices: 557 -> 523 us, 512 in FP64: 328 -> 319.
+int64_t warp_columns(int64_t n) { return n / 32 * 16 + std::min<int64_t>(n % 32, 16); }
 Contraction better_side_first(const Contraction &c) {
     using namespace split;
-    auto warp_columns = [](int64_t n) { return n / 32 * 16 + std::min<int64_t>(n % 32, 16); };
     auto cost = [&](int64_t m, int64_t n) { return (m + kBM - 1) / kBM * warp_columns(n); };
     if (cost(c.n.total, c.m.total) >= cost(c.m.total, c.n.total)) return c;
     Contraction t = c;
@@ -735,6 +734,9 @@ Contraction better_side_first(const Contraction &c) {
     return t;
 }
 
+// Builds and captures the split-BF16 plan, or (f64) the FP64 one on the tensor cores;
+// returns EG_ERROR_NOT_SUPPORTED when an item's K needs more than one exact pass (the
+// caller then runs items one by one).
 eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, int slices, cudaStream_t s, bool f64) {
     using namespace split;
     std::vector<Contraction> cs;
@@ -806,7 +808,9 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
         for (int64_t bb = 0; bb < nb; bb++)
             for (int64_t x = 0; x < Mp / kBM; x++)
                 for (int64_t y = 0; y < Np / kBN; y++)
-                    work.push_back({Kp, make_int4((int)i, (int)bb, (int)x, (int)y)});
+                    work.push_back({Kp / kBK * 256 * (S * (S + 1) / 2) + 6000 +
+                                        (f64 ? 700 : 350) * warp_columns(std::min<int64_t>(N - y * kBN, kBN)),
+                                    make_int4((int)i, (int)bb, (int)x, (int)y)});
         rowsA += nb * Mp;
         rowsB += nb * Np;
         elemsA += round_up(nb * P * a.pstride, 64);
@@ -815,8 +819,26 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
     if (rowsA >= (1ll << 31) || rowsB >= (1ll << 31))
         return fail(EG_ERROR_NOT_SUPPORTED, "grouped split: batch too large");
     std::stable_sort(work.begin(), work.end(), [](auto &x, auto &y) { return x.first > y.first; });
+    // the tiles, the longest first, each to the CTA with the least to do (first: estimated
+    // clocks of the MMAs and of the epilogue).  512 uneven items in FP64, dealt round in
+    // that order: 222 us, of which the CTA with the longest first item took twice the mean;
+    // 160 us so.
+    const int grid = (int)std::min<size_t>(work.size(), (size_t)num_sms());
+    std::vector<std::vector<int4>> of_cta(grid);
+    std::priority_queue<std::pair<int64_t, int>, std::vector<std::pair<int64_t, int>>, std::greater<>> least;
+    for (int c = 0; c < grid; c++) least.push({0, c});
+    for (auto &w : work) {
+        const auto [load, c] = least.top();
+        least.pop();
+        of_cta[c].push_back(w.second);
+        least.push({load + w.first, c});
+    }
     std::vector<int4> wl;
-    for (auto &w : work) wl.push_back(w.second);
+    std::vector<int> ranges(1, 0);
+    for (auto &l : of_cta) {
+        wl.insert(wl.end(), l.begin(), l.end());
+        ranges.push_back((int)wl.size());
+    }
     // one splitting unit per 32 real rows of every operand (and batch index)
     std::vector<GOp> ops(opsA);
     ops.insert(ops.end(), opsB.begin(), opsB.end());
@@ -894,6 +916,8 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
     if ((st = dev_copy(plan, offs.data(), offs.size() * sizeof(long long), &d_offs)) != EG_SUCCESS) return st;
     if ((st = dev_copy(plan, items.data(), items.size() * sizeof(TcItem), &d_items)) != EG_SUCCESS) return st;
     if ((st = dev_copy(plan, wl.data(), wl.size() * sizeof(int4), &d_work)) != EG_SUCCESS) return st;
+    void *d_ranges = nullptr;
+    if ((st = dev_copy(plan, ranges.data(), ranges.size() * sizeof(int), &d_ranges)) != EG_SUCCESS) return st;
 
     // per-item maps: each item's planes with its own M (N) and K as the extents
     std::vector<CUtensorMap> maps(2 * items.size());
@@ -940,6 +964,7 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
     p.ksplit = 1;
     p.kslice = 0;
     p.item_maps = (const CUtensorMap *)d_maps;
+    p.ranges = (const int *)d_ranges;
     p.rbuf = (long long *)rbuf;
     static const bool prof_on = std::getenv("EINSUMS_GB300_TC_PROFILE") != nullptr;
     if (prof_on) {
@@ -978,7 +1003,7 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
                                                (const long long *)d_offs, (int *)eA, (int *)eB, (__nv_bfloat16 *)planesA,
                                                (__nv_bfloat16 *)planesB, s);
             if (is != EG_SUCCESS) return is;
-            is = launch_tc_gemm_grouped(maps[0], maps[1], p, (TcItem *)d_items, (int4 *)d_work, (int)wl.size(), s);
+            is = launch_tc_gemm_grouped(maps[0], maps[1], p, (TcItem *)d_items, (int4 *)d_work, grid, s);
             if (is != EG_SUCCESS || !f64) return is;
             k_grouped_f64_listed<<<num_sms() * 4, THREADS, 0, s>>>((const F64Item *)d_fma, (const int4 *)redo,
                                                                    (const int *)redo_count, c0.cp, c0.ab, p.zero);

@@ -96,6 +96,7 @@ struct TcGemmParams {
     // planes with its own row and K extents, so that TMA fills the tile's rows
     // past M (N) and K blocks past K with zeros instead of reading the padding.
     const CUtensorMap *item_maps;
+    const int *ranges; // each CTA's work entries
 };
 
 // One item of a grouped launch: an independent contraction whose digit planes have
@@ -309,9 +310,10 @@ bool tc_pairs_forced();
 // tmBh: B's planes in boxes of 64 rows (half a tile), read by CTA pairs.
 eg_status launch_tc_gemm(const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmBh, const TcGemmParams &p,
                          cudaStream_t s);
-// Grouped form: `ntiles_total` work entries, per-tile parameters from `items`.
+// Grouped form: CTA c of `grid` runs the work entries of TcGemmParams::ranges[c] ..
+// ranges[c + 1], per-tile parameters from `items`.
 eg_status launch_tc_gemm_grouped(const CUtensorMap &tmA, const CUtensorMap &tmB, const TcGemmParams &p,
-                                 const TcItem *items, const int4 *work, int ntiles_total, cudaStream_t s);
+                                 const TcItem *items, const int4 *work, int grid, cudaStream_t s);
 
 // Bytes of the per-CTA sum scratch a tensor launch needs (TcGemmParams::rbuf).
 inline size_t rbuf_bytes(int planes = 1) { return (size_t)num_sms() * planes * kBM * kBN * sizeof(long long); }

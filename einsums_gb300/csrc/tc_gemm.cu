@@ -239,7 +239,7 @@ template <bool GROUPED, int CL, bool F64>
 __global__ void __launch_bounds__(THREADS, 1)
     k_tc_split_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ TcGemmParams p,
-                    const TcItem *items, const int4 *work, int ntiles_total) {
+                    const TcItem *items, const int4 *work) {
     static_assert(CL == 1 || (CL == 2 && !GROUPED), "CTA pairs serve single contractions");
     constexpr int PLANES = F64 ? 2 : 1; // int64 sums per output in the K slices' accumulator
     constexpr size_t kPlane = (size_t)kBM * kBN;
@@ -290,11 +290,11 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (CL == 2) ptx::cluster_sync(); // the peer's barriers are initialised before any remote arrival
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    // schedule index and stride of this CTA (of its pair when CL = 2)
-    const int cta0 = blockIdx.x / CL, ctas = gridDim.x / CL;
+    // first schedule entry and stride of this CTA (of its pair when CL = 2)
+    const int cta0 = GROUPED ? p.ranges[blockIdx.x] : blockIdx.x / CL, ctas = GROUPED ? 1 : gridDim.x / CL;
 
     const int total_tiles =
-        GROUPED ? ntiles_total : p.t0 + (p.nbatch * ((p.mtiles + CL - 1) / CL) * p.ntiles - p.t0) * p.ksplit;
+        GROUPED ? p.ranges[blockIdx.x + 1] : p.t0 + (p.nbatch * ((p.mtiles + CL - 1) / CL) * p.ntiles - p.t0) * p.ksplit;
 
     if (warp < 4) {
         ptx::regs_dec<kRegsIssue>();
@@ -944,13 +944,13 @@ eg_status launch_tc_gemm(const CUtensorMap &tmA, const CUtensorMap &tmB, const C
             cudaLaunchAttribute attr;
             cudaLaunchConfig_t cfg = pair_config(grid, s, &attr);
             if (f64)
-                EG_CUDA(cudaLaunchKernelEx(&cfg, k_tc_split_gemm<false, 2, true>, tmA, tmB, tmBh, p, no_items, no_work, 0));
+                EG_CUDA(cudaLaunchKernelEx(&cfg, k_tc_split_gemm<false, 2, true>, tmA, tmB, tmBh, p, no_items, no_work));
             else
-                EG_CUDA(cudaLaunchKernelEx(&cfg, k_tc_split_gemm<false, 2, false>, tmA, tmB, tmBh, p, no_items, no_work, 0));
+                EG_CUDA(cudaLaunchKernelEx(&cfg, k_tc_split_gemm<false, 2, false>, tmA, tmB, tmBh, p, no_items, no_work));
         } else if (f64) {
-            k_tc_split_gemm<false, 1, true><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmBh, p, no_items, no_work, 0);
+            k_tc_split_gemm<false, 1, true><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmBh, p, no_items, no_work);
         } else {
-            k_tc_split_gemm<false, 1, false><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmBh, p, no_items, no_work, 0);
+            k_tc_split_gemm<false, 1, false><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmBh, p, no_items, no_work);
         }
     }
     EG_CHECK_LAUNCH("k_tc_split_gemm");
@@ -968,17 +968,16 @@ eg_status launch_tc_gemm(const CUtensorMap &tmA, const CUtensorMap &tmB, const C
 }
 
 eg_status launch_tc_gemm_grouped(const CUtensorMap &tmA, const CUtensorMap &tmB, const TcGemmParams &p,
-                                 const TcItem *items, const int4 *work, int ntiles_total, cudaStream_t s) {
+                                 const TcItem *items, const int4 *work, int grid, cudaStream_t s) {
     eg_status st = ensure_tc_attributes();
     if (st != EG_SUCCESS) return st;
-    if (ntiles_total <= 0) return EG_SUCCESS;
-    const int grid = ntiles_total < num_sms() ? ntiles_total : num_sms();
+    if (grid <= 0) return EG_SUCCESS;
     {
         LaunchScope ls_(p.redo ? "k_tc_split_gemm_grouped_f64" : "k_tc_split_gemm_grouped", s);
         if (p.redo)
-            k_tc_split_gemm<true, 1, true><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmB, p, items, work, ntiles_total);
+            k_tc_split_gemm<true, 1, true><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmB, p, items, work);
         else
-            k_tc_split_gemm<true, 1, false><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmB, p, items, work, ntiles_total);
+            k_tc_split_gemm<true, 1, false><<<grid, THREADS, SMEM_BYTES, s>>>(tmA, tmB, tmB, p, items, work);
     }
     EG_CHECK_LAUNCH("k_tc_split_gemm_grouped");
     return EG_SUCCESS;
