@@ -1007,7 +1007,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
     };
     const size_t oPA = take((size_t)bb * P * mb * Kp * 2), oPB = take((size_t)bb * P * nbk * Kp * 2);
     const size_t oMax = take((size_t)bb * (mb + nbk) * 8);
-    const size_t oBad = take((size_t)slices_max * kTileRegions * sizeof(int));
+    const size_t oMargin = take((size_t)slices_max * kTileRegions * sizeof(int));
     const size_t oParts = take((size_t)slices_max * 2 * kBM * kBN * 8);
     const size_t oExp = take((size_t)bb * (mb + nbk) * 4);
     const size_t oTab = take(tables ? (size_t)(M + N + 2 * K) * 8 : 0);
@@ -1040,7 +1040,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
     p.timeout_ns = 2000ull * 1000 * 1000;
     p.rbuf = (long long *)(base + oR);
     p.parts = (long long *)(base + oParts);
-    p.parts_bad = (int *)(base + oBad);
+    p.parts_margin = (int *)(base + oMargin);
     p.d0 = 0;
     p.d1 = S;
     p.hid = kF64High;

@@ -69,12 +69,12 @@ struct TcGemmParams {
     // (t - t0) % ksplit (kslice K blocks; the last slice takes the rest) of
     // tile t0 + (t - t0) / ksplit.  A slice's exact int64 sums go to parts ([t - t0]
     // [128 columns][128 rows], two planes in the FP64 form; with CTA pairs an entry is
-    // two tiles, one after the other) and whether its check failed to parts_bad
+    // two tiles, one after the other) and the least sum of its check to parts_margin
     // ([t - t0][8]); k_tc_finish_slices adds them up.  Unused when t0 is the number of tiles.
     int t0;
     int ksplit, kslice;
     long long *parts;
-    int *parts_bad;
+    int *parts_margin;
     // Launch as CTA pairs (cta_group::2, 256x128 tiles): single contractions only.
     int pair;
     // Slice groups d0 <= d < d1 (anti-diagonals s + t = d of the digit pairs)

@@ -43,7 +43,7 @@ constexpr int kCols = kBN / (kEpiWarps / 4); // columns of an epilogue warp
 static_assert(kTileRegions == kEpiWarps, "a region per epilogue warp");
 // per epilogue warp: its column offsets and (of two tiles) exponents, the
 // transposition buffer of one batch, and its 32 rows' addresses
-constexpr int EPI_WARP_BYTES = kCols * (8 + 2 * 4) + kFin * FIN_T * 8 + 32 * 8;
+constexpr int EPI_WARP_BYTES = kCols * (8 + 2 * 4) + kFin * FIN_T * 8 + 33 * 8;
 constexpr int SMEM_BYTES = 1024 + 2 * kSlots * TILE_BYTES + AUX_BYTES + kEpiWarps * EPI_WARP_BYTES + 64;
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 // setmaxnreg: the epilogue warps' sums take 128 registers; what they hold beyond the
@@ -51,8 +51,10 @@ static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 // that misses the few KB of L1 left beside the ring waits some 4000 clocks behind the
 // tiles in flight (25600 x 25600, K = 1024: 16.0 ms with 60 bytes of spills a thread,
 // 12.9 without).
-constexpr int kRegsIssue = 56, kRegsEpilogue = 224;
-static_assert(128 * kRegsIssue + 32 * kEpiWarps * kRegsEpilogue <= THREADS * 168, "registers of the launch");
+constexpr int regs_issue(int cl) { return cl == 2 ? 40 : 56; } // (single CTAs' issuer watches two slots)
+constexpr int regs_epilogue(int cl) { return cl == 2 ? 232 : 224; }
+static_assert(128 * regs_issue(1) + 32 * kEpiWarps * regs_epilogue(1) <= THREADS * 168, "registers of the launch");
+static_assert(128 * regs_issue(2) + 32 * kEpiWarps * regs_epilogue(2) <= THREADS * 168, "registers of the launch");
 constexpr int GROUP_M = 16; // tile rasterisation: groups of 16 row tiles share B tiles in L2
 constexpr unsigned long long DRAIN_NS = 200ull * 1000 * 1000;
 
@@ -297,7 +299,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         GROUPED ? p.ranges[blockIdx.x + 1] : p.t0 + (p.nbatch * ((p.mtiles + CL - 1) / CL) * p.ntiles - p.t0) * p.ksplit;
 
     if (warp < 4) {
-        ptx::regs_dec<kRegsIssue>();
+        ptx::regs_dec<regs_issue(CL)>();
         if (warp == 0 || warp == 2) {
             // -------------------------------------------- TMA producers: A tiles, B tiles
             // Two warps, each with uniform control flow and one elected lane issuing:
@@ -476,7 +478,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     } else {
         // ------------------------------------------------ epilogue (warps 4..11)
         // Two warps per TMEM lane quadrant; each owns 64 of the tile's 128 columns.
-        ptx::regs_inc<kRegsEpilogue>();
+        ptx::regs_inc<regs_epilogue(CL)>();
         constexpr int FIN = F64 ? kFin / 2 : kFin; // the FP64 form holds two words per sum
         const int ew = warp - 4;              // 0..7
         const int quad = warp & 3;            // TMEM lane quadrant this warp may access
@@ -487,7 +489,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         int *colExp = colExpAll + 2 * ew * kCols; // the pending tile's; the running tile's are at colExp + run_exp
         int run_exp = kCols;
         double *finT = finTAll + ew * (kFin * FIN_T);
-        double **rowAt = rowAtAll + ew * 32;
+        double **rowAt = rowAtAll + ew * 33;
+        // FP64 form: the least sum of the check in the running tile, negative where it fails
+        volatile int *const margin = (volatile int *)(rowAt + 32);
         int abuf = 0;
         uint32_t aphase = 0;
         bool ok = true;
@@ -558,7 +562,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 if ((int64_t)job.mt * kBM + quad * 32 < job.M)
                     live = cols / 32 * 16 + min(max(cols % 32 - half * 16, 0), 16);
                 const int64_t m = (int64_t)job.mt * kBM + row;
-                if (m < job.M) my_rowExp = job.eA[m];
+                my_rowExp = m < job.M ? job.eA[m] : INT_MAX; // INT_MAX: past the output
 #pragma unroll
                 for (int i = 0; i < kCols / 32; i++) {
                     const int64_t n = (int64_t)job.nt * kBN + tile_col(half, lane + 32 * i);
@@ -570,7 +574,6 @@ __global__ void __launch_bounds__(THREADS, 1)
             long long H[kCols];
 #pragma unroll
             for (int i = 0; i < kCols; i++) H[i] = 0;
-            bool bad = false; // FP64 form: the check of this warp's outputs failed
             int q = drain ? qend : qbeg, kb = 0;
             Step st = step_of(p, q);
             while (true) {
@@ -627,13 +630,13 @@ __global__ void __launch_bounds__(THREADS, 1)
                         kb = 0;
                         q++;
                         if (F64 && q == 0) { // a negative margin anywhere: the FMA kernel takes this warp's outputs
-                            long long worst = 0;
+                            int worst = INT_MAX; // (the sums stay below 2^30)
 #pragma unroll
                             for (int i = 0; i < kCols; i++) {
-                                worst = min(worst, H[i]);
+                                if (i < live) worst = min(worst, (int)H[i]);
                                 H[i] = 0;
                             }
-                            bad = __any_sync(0xffffffffu, worst < 0);
+                            *margin = __reduce_min_sync(0xffffffffu, my_rowExp != INT_MAX ? worst : INT_MAX);
                         } else if (F64 && st.hi + 1 == p.hid) { // the high sums are complete
                             long long *const at_hi = !GROUPED && tile >= p.t0 ? part_of(tile) + kPlane : rbc + (1 + parity) * kPlane;
 #pragma unroll
@@ -721,12 +724,12 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
             for (int i = 0; i < kCols; i++) sums[i * kBM] = H[i];
             if (slice) {
-                if (F64 && lane == 0) p.parts_bad[job.part * kTileRegions + ew] = bad ? 1 : 0;
+                if (F64 && lane == 0) p.parts_margin[job.part * kTileRegions + ew] = *margin;
                 continue;
             }
             long long *const own_hi = rbc + (F64 ? 1 + parity : 0) * kPlane;
             parity ^= 1;
-            if (F64 && bad) {
+            if (F64 && *margin < 0) {
                 if (lane == 0) {
                     const int at = atomicAdd(p.redo_count, 1);
                     const int m0 = job.mt * kBM + quad * 32, n0 = job.nt * kBN + half * 16;
@@ -743,7 +746,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             const int64_t m = (int64_t)job.mt * kBM + row;
             const bool row_ok = m < job.M;
             int64_t rowOff = 0;
-            pend_rowExp = my_rowExp;
+            pend_rowExp = row_ok ? my_rowExp : 0;
             if (row_ok) {
                 int64_t oa, ob;
                 group_offsets32(*job.mg, (uint32_t)(GROUPED ? m : p.m0 + m), oa, ob, rowOff);
@@ -809,9 +812,10 @@ __global__ void __launch_bounds__(32 * kFinishRows) k_tc_finish_slices(const __g
     if (rows <= 0 || live <= 0) return;
     const int e0 = q * p.ksplit * CL + rank; // the tile's first slice; the next ones are CL further on
     if (F64) {
-        int bad = 0;
-        for (int k = 0; k < p.ksplit; k++) bad |= p.parts_bad[(e0 + k * CL) * kTileRegions + ew];
-        if (bad) {
+        // the slices' least check sums add up to no more than the least of their sum
+        long long margin = 0;
+        for (int k = 0; k < p.ksplit; k++) margin += p.parts_margin[(e0 + k * CL) * kTileRegions + ew];
+        if (margin < 0) {
             if (threadIdx.x == 0 && c0 == 0)
                 p.redo[atomicAdd(p.redo_count, 1)] =
                     make_int4((int)p.b0 + b, (int)(p.m0 + m0), (int)(p.n0 + n0) + half * 16, 0);
