@@ -7,6 +7,7 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <functional>
 #include <string>
 
 #include "../../include/einsums_gb300.h"
@@ -188,7 +189,10 @@ eg_status launch_contract_f64(const Contraction &c, cudaStream_t s);
 eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, const int *count, cudaStream_t s);
 double contract_f64_seconds(const Contraction &c); // its estimated time
 bool f64_tensor_pays(const Contraction &c);
-eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s);
+// `front` bytes of the scratch are the caller's: fill(c, them) issues what writes them and
+// points c at them, once the scratch is there and before c is read.
+eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front = 0,
+                            const std::function<eg_status(Contraction &, void *)> &fill = nullptr);
 eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s, eg_split_report *rep);
 
 struct PermuteDesc {

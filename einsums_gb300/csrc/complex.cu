@@ -16,11 +16,12 @@
 // C_prefactor rides on the first contraction into each part, keeping the real
 // path's zeroing rules; a complex one is applied first by k_complex_scale.
 //
-// An FP64 contraction with a real AB_prefactor that the FMA kernel would take four times
-// runs once: the real and imaginary parts become a mode p of C and a mode q of the sums,
-// the larger operand serves both as it is stored, and the smaller is written out as the
-// 2 x 2 real block of each of its elements.  One launch of four times the work fills the
-// chip where four did not, and the summed modes of an interleaved operand are contiguous.
+// An FP64 contraction with a real AB_prefactor runs once instead of four times: the real
+// and imaginary parts become a mode p of C and a mode q of the sums, the larger operand
+// serves both as it is stored, and the smaller is written out as the 2 x 2 real block of
+// each of its elements.  One launch of four times the work fills the chip where four did
+// not, the summed modes of an interleaved operand are contiguous, and the tensor cores pay
+// for sizes where they would not for each of the four.
 #include <algorithm>
 #include <climits>
 
@@ -33,7 +34,6 @@ eg_status einsum_impl(double cp, const int32_t *Cl, const eg_tensor *C, double a
 eg_status lower_for_group(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al,
                           const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options &opt,
                           Contraction &out, int32_t *alg_out, bool &gemm_shaped);
-bool f64_tensor_pays(const Contraction &c);
 void set_split_report(const eg_split_report &r);
 eg_status classify_call(const int32_t *Cl, const eg_tensor *C, const int32_t *Al, const eg_tensor *A,
                         const int32_t *Bl, const eg_tensor *B, const eg_options *opt_in, int32_t *alg_out);
@@ -100,12 +100,13 @@ bool append_part(ModeGroup &g, int64_t s0, int64_t s1, int64_t s2) {
 
 // The contraction c of the real parts as one real contraction of the whole complex
 // operands (file comment).  NOT_SUPPORTED: the caller's four contractions, when the shape,
-// the tensor cores (better from about 40 us each), a capture or the scratch say so.
-// Bound: the FP64 pipe (83 us for 300 x 170 x 257, which take 125 us; in four launches
-// 156 us, each with a last wave of its own and operands at stride 2).
+// a capture or the scratch say so.  300 x 170 x 257: 55 us on the tensor cores; FMAs take
+// 125 us in one launch (83 us of the FP64 pipe) and in four 156 us, each with a last wave
+// of its own and operands at stride 2.
 constexpr int64_t kBlocksMax = int64_t(1) << 23; // elements of the smaller operand: 256 MB of blocks
 eg_status launch_complex_blocks(Contraction c, double sa, double sb, cudaStream_t s) {
-    if (c.k.n == 0 || c.m.n == 0 || c.n.n == 0 || f64_tensor_pays(c)) return EG_ERROR_NOT_SUPPORTED;
+    if (c.k.n == 0 || c.m.n == 0 || c.n.n == 0) return EG_ERROR_NOT_SUPPORTED;
+    const bool four_tensor = f64_tensor_pays(c); // each of the four contractions
     if (c.batch.n + c.m.n + c.n.n >= kMaxModes) return EG_ERROR_NOT_SUPPORTED;
     const int t = c.m.total < c.n.total ? 0 : 1; // the operand written out as blocks
     ModeGroup &f = t == 0 ? c.m : c.n, &k = c.k, &b = c.batch;
@@ -140,23 +141,32 @@ eg_status launch_complex_blocks(Contraction c, double sa, double sb, cudaStream_
             step *= g->ext[d];
         }
     }
-    ScratchLease lease(s, (size_t)step * sizeof(double));
-    if (!lease.ptr()) return EG_ERROR_NOT_SUPPORTED;
-    double *E = (double *)lease.ptr();
     const double *from = t == 0 ? c.A : c.B;
     const bool room = t == 0 ? append_part(k, part[0], 1, 0) && append_part(f, part[1], 0, 1)
                              : append_part(k, 1, part[0], 0) && append_part(f, 0, part[1], 1);
     if (!room) return EG_ERROR_NOT_SUPPORTED;
-    (t == 0 ? c.A : c.B) = E;
-    {
-        LaunchScope ls_("k_complex_blocks", s);
-        const int64_t blocks = std::min<int64_t>((src.total + 255) / 256, (int64_t)num_sms() * 8);
-        k_complex_blocks<<<(unsigned)blocks, 256, 0, s>>>(src, from, E, part[0], part[1], t == 0 ? sa : sb,
-                                                          t == 0 ? sb : sa);
+    const size_t bytes = (size_t)step * sizeof(double);
+    auto fill = [&](Contraction &x, void *E) -> eg_status {
+        (t == 0 ? x.A : x.B) = (double *)E;
+        {
+            LaunchScope ls_("k_complex_blocks", s);
+            const int64_t blocks = std::min<int64_t>((src.total + 255) / 256, (int64_t)num_sms() * 8);
+            k_complex_blocks<<<(unsigned)blocks, 256, 0, s>>>(src, from, (double *)E, part[0], part[1], t == 0 ? sa : sb,
+                                                              t == 0 ? sb : sa);
+        }
+        EG_CHECK_LAUNCH("k_complex_blocks");
+        set_split_report(eg_split_report{0, 0, 0, 0.0});
+        return EG_SUCCESS;
+    };
+    if (f64_tensor_pays(c)) {
+        const eg_status st = launch_f64_tensor(c, s, bytes, fill);
+        if (st != EG_ERROR_NOT_SUPPORTED) return st;
     }
-    EG_CHECK_LAUNCH("k_complex_blocks");
-    set_split_report(eg_split_report{0, 0, 0, 0.0});
-    return launch_contract_f64(c, s);
+    if (four_tensor) return EG_ERROR_NOT_SUPPORTED; // better than FMAs in one launch
+    ScratchLease lease(s, bytes);
+    if (!lease.ptr()) return EG_ERROR_NOT_SUPPORTED;
+    const eg_status st = fill(c, lease.ptr());
+    return st == EG_SUCCESS ? launch_contract_f64(c, s) : st;
 }
 
 } // namespace

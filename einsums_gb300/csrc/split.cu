@@ -969,7 +969,8 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
 // comes back with nothing launched and the FMA kernel runs instead.
 constexpr size_t kF64ScratchCap = size_t(2) << 30;
 
-eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
+eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
+                            const std::function<eg_status(Contraction &, void *)> &fill) {
     using namespace split;
     constexpr int S = kF64Slices, P = S + 2;
     const int64_t nb = c.batch.total, M = c.m.total, N = c.n.total, K = c.k.total;
@@ -1005,6 +1006,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
         at += (bytes + 1023) & ~size_t(1023);
         return o;
     };
+    const size_t oFront = take(front);
     const size_t oPA = take((size_t)bb * P * mb * Kp * 2), oPB = take((size_t)bb * P * nbk * Kp * 2);
     const size_t oMax = take((size_t)bb * (mb + nbk) * 8);
     const size_t oMargin = take((size_t)slices_max * kTileRegions * sizeof(int));
@@ -1019,6 +1021,7 @@ eg_status launch_f64_tensor(const Contraction &c, cudaStream_t s) {
     eg_status st = status_word(s, &status);
     if (st != EG_SUCCESS) return st;
     char *base = (char *)lease.ptr();
+    if (fill && (st = fill(c, base + oFront)) != EG_SUCCESS) return st;
     __nv_bfloat16 *planesA = (__nv_bfloat16 *)(base + oPA), *planesB = (__nv_bfloat16 *)(base + oPB);
     int *eA = (int *)(base + oExp), *eB = eA + bb * mb;
     int64_t *tab = tables ? (int64_t *)(base + oTab) : nullptr;

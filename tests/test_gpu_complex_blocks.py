@@ -85,3 +85,22 @@ def test_one_contraction(eg, Cl, Al, Bl, dims, conj):
             graph.replay()
             four = C.cpu().numpy()
             assert np.all(np.abs(four - got) <= 2 * bound)
+
+
+@pytest.mark.parametrize("Cl,Al,Bl", [("ij", "ik", "kj"), ("ji", "ki", "jk"), ("bij", "bik", "bkj")])
+@pytest.mark.parametrize("i,j,k", [(300, 170, 257), (129, 400, 300), (640, 640, 130)])
+def test_on_the_tensor_cores(eg, Cl, Al, Bl, i, j, k):
+    """Above the FMA kernel's sizes: no more than four roundings' worth of the magnitudes a part."""
+    rng = np.random.default_rng(i + j)
+    dims = dict(i=i, j=j, k=k, b=2)
+    A, B, C = (rand(rng, dims, l, False) for l in (Al, Bl, Cl))
+    a, b, c = A.cpu().numpy().conj(), B.cpu().numpy(), C.cpu().numpy()
+    spec = f"{Al},{Bl}->{Cl}"
+    want = 0.5 * c - 2.0 * np.einsum(spec, a, b, optimize=True)
+    mag = 0.5 * np.abs(c) + 2.0 * np.einsum(spec, np.abs(a), np.abs(b), optimize=True)
+    seen = launches(lambda: eg.einsum(0.5, Cl, C, -2.0, Al, A, Bl, B, conj_A=True))
+    assert seen.get("k_tc_split_gemm_f64") == 1 and seen.get("k_complex_blocks") == 1, seen
+    got = C.cpu().numpy()
+    # numpy's own sums of 2 K products may be as far off as theirs
+    bound = EPS * (8 + 2 * k + 8) * mag
+    assert np.all(np.abs(got.real - want.real) <= bound) and np.all(np.abs(got.imag - want.imag) <= bound)
