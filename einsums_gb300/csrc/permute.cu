@@ -64,15 +64,17 @@ __device__ __forceinline__ double combine(double a, const double *c, double ap, 
 
 // Fastest modes shared: rows of length L with strides sa/sc along the row, in elements
 // of T -- double, or double2 when rows are contiguous and every address is on a 16-byte
-// boundary.  A warp takes kRowChunk elements: a chunk of one row, or as many whole rows
+// boundary.  A warp takes `chunk` elements: a chunk of one row, or as many whole rows
 // as make it up, NR at a time.  The decomposition of the row index is paid once per run
 // along the fastest rest mode; eight loads of a thread are in flight (NR rows of 8 / NR
 // each), so rows shorter than 256 elements keep as many as long ones.  Bound: memory.
 // Rows of 126: 15e6 elements in 49 us (5.0 TB/s), scaled in place of a copy 47 us; a warp
 // per row took 54 us.
-constexpr int kRowChunk = 2048;
+// Fewer elements, down to 256, where there are not 32 warps of them for every SM: all
+// rank-4 permutations of 32^4 take 7 us on average so, with 2048 always 18.
+constexpr int kRowChunk = 2048, kRowChunkMin = 256;
 
-__host__ __device__ inline int rows_per_unit(int64_t L) { return L >= kRowChunk ? 1 : kRowChunk / (int)(L < 1 ? 1 : L); }
+__host__ __device__ inline int rows_per_unit(int64_t L, int chunk) { return L >= chunk ? 1 : chunk / (int)(L < 1 ? 1 : L); }
 
 template <int MODE>
 __device__ __forceinline__ double2 combine(double2 a, const double2 *c, double ap, double cp) {
@@ -80,18 +82,18 @@ __device__ __forceinline__ double2 combine(double2 a, const double2 *c, double a
 }
 
 template <int MODE, typename T, int NR>
-__global__ void __launch_bounds__(256) k_permute_rows(PermuteMap rest, int64_t L, int64_t sa, int64_t sc,
+__global__ void __launch_bounds__(256) k_permute_rows(PermuteMap rest, int64_t L, int64_t sa, int64_t sc, int chunk,
                                                       const T *__restrict__ A, T *C, double ap, double cp) {
     constexpr int Q = 8 / NR; // loads of a row at a time
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int per = rows_per_unit(L);
-    const int64_t chunks = (L + kRowChunk - 1) / kRowChunk;
+    const int per = rows_per_unit(L, chunk);
+    const int64_t chunks = (L + chunk - 1) / chunk;
     const int64_t groups = (rest.total + per - 1) / per, units = groups * chunks;
     const int last = rest.n - 1;
     const int64_t run = rest.n ? rest.ext[last] : 1, runA = rest.n ? rest.sA[last] : 0, runC = rest.n ? rest.sC[last] : 0;
     for (int64_t u = (int64_t)blockIdx.x * 8 + warp; u < units; u += (int64_t)gridDim.x * 8) {
-        const int64_t grp = u / chunks, x0 = (u - grp * chunks) * kRowChunk;
-        const int len = (int)min((int64_t)kRowChunk, L - x0); // this chunk's part of a row
+        const int64_t grp = u / chunks, x0 = (u - grp * chunks) * chunk;
+        const int len = (int)min((int64_t)chunk, L - x0); // this chunk's part of a row
         const int64_t row0 = grp * per;
         const int rows = (int)min((int64_t)per, rest.total - row0);
         int64_t oa, oc, left = run - row0 % run; // rows to the end of the run along the fastest rest mode
@@ -590,16 +592,18 @@ eg_status run_permute(const PermuteLaunch &pl, const double *A, double *C, cudaS
                 rest.sC[d] /= 2;
             }
         }
-        const int64_t per = rows_per_unit(L);
-        const int64_t work = ((rest.total + per - 1) / per * ((L + kRowChunk - 1) / kRowChunk) + 7) / 8;
+        int chunk = kRowChunk;
+        while (chunk > kRowChunkMin && rest.total * L < (int64_t)chunk * 32 * num_sms()) chunk /= 2;
+        const int64_t per = rows_per_unit(L, chunk);
+        const int64_t work = ((rest.total + per - 1) / per * ((L + chunk - 1) / chunk) + 7) / 8;
         const int grid = (int)std::min<int64_t>(work, (int64_t)num_sms() * 16);
         auto go = [&](auto mode, auto nr) {
             constexpr int MODE = decltype(mode)::value, NR = decltype(nr)::value;
             if (pairs)
-                k_permute_rows<MODE, double2, NR><<<grid, 256, 0, s>>>(rest, L, 1, 1, (const double2 *)A, (double2 *)C,
+                k_permute_rows<MODE, double2, NR><<<grid, 256, 0, s>>>(rest, L, 1, 1, chunk, (const double2 *)A, (double2 *)C,
                                                                        pl.ap, pl.cp);
             else
-                k_permute_rows<MODE, double, NR><<<grid, 256, 0, s>>>(rest, L, pl.sa, pl.sc, A, C, pl.ap, pl.cp);
+                k_permute_rows<MODE, double, NR><<<grid, 256, 0, s>>>(rest, L, pl.sa, pl.sc, chunk, A, C, pl.ap, pl.cp);
         };
         auto rows_at_once = [&](auto mode) {
             if (L <= 64)
