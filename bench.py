@@ -40,9 +40,9 @@ def flops(o, v):
 
 
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of the tensor kernel on the
-# o=32, v=160 workload, mean over the step's three launches (Wmnij 3.32 GB,
-# Wabef 18.17 GB, Wmbej 6.37 GB), from a separate capture of this workload.
-TC_TRAFFIC_O32_V160 = 9.44e9
+# o=32, v=160 workload, mean over the step's three launches (Wmnij 0.95 GB,
+# Wabef 21.31 GB, Wmbej 4.67 GB), from a separate capture of this workload.
+TC_TRAFFIC_O32_V160 = 8.98e9
 
 
 def tc_algorithmic_bytes(o, v, S):
@@ -399,13 +399,14 @@ def run_ours(args, rank, world):
     if headline == "split_bf16":
         dom = max((k for k in kernels if k.startswith("k_tc")), key=lambda k: kernels[k]["total_ms"], default=None)
     else:
-        dom = "k_contract_f64" if "k_contract_f64" in kernels else max(kernels, key=lambda k: kernels[k]["total_ms"])
+        dom = max(kernels, key=lambda k: kernels[k]["total_ms"])
     roof = None
     if dom:
         d = kernels[dom]
         avg_ms = d["total_ms"] / d["launches"]
-        if headline == "split_bf16":
-            pairs = (split_report or {}).get("slice_pairs", 0)
+        if headline == "split_bf16" or dom == "k_tc_split_gemm_f64":
+            # plain FP64 on the tensor cores: the 36 products of eight slices and two of its check
+            pairs = (split_report or {}).get("slice_pairs", 0) if headline == "split_bf16" else 38
             # bf16 flops issued by the tensor kernel per launch (slice pairs x 2MNK over the GEMM-shaped W's);
             # the kernel profile spans the warm-up and the timed steps
             launches_per_step = d["launches"] / (args.steps + args.warmup)
@@ -418,13 +419,13 @@ def run_ours(args, rank, world):
             roof = {"kernel": dom, "bound": "tensor", "achieved": ach, "peak": peak, "unit": "TFLOP/s",
                     "frac": ach / peak, "traffic": None,
                     "peak_source": f"bf16 {'sustained (power cap seen)' if capped else 'burst'}, {pk_kind}"}
-            if (o, v) == (32, 160) and (split_report or {}).get("slices") == 5:
+            if headline == "split_bf16" and (o, v) == (32, 160) and (split_report or {}).get("slices") == 5:
                 # DRAM bytes per tensor-kernel launch, mean over the step's three
                 # launches, from one ncu capture of this workload
                 # (dram__bytes_read.sum + dram__bytes_write.sum); algorithmic bytes
                 # per launch (digit planes read once, C read and written once) are
-                # 4.16 GB; the kernel moves 2.3x that (digit-plane panels re-read
-                # through L2 by the output tiles that share them).
+                # 4.16 GB; the kernel moves more (digit-plane panels re-read through
+                # L2 by the output tiles that share them).
                 roof["traffic"] = TC_TRAFFIC_O32_V160
                 roof["traffic_unit"] = ("bytes per launch, mean of the step's 3 launches, from an ncu capture of "
                                         "this workload (dram__bytes_read.sum + dram__bytes_write.sum), "
