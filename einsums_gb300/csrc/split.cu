@@ -307,7 +307,7 @@ constexpr int kFusedThreads = 256;
 template <int S, bool CHECK, int R>
 __global__ void __launch_bounds__(kFusedThreads) k_split_rows(const __grid_constant__ SplitJob ja,
                                                               const __grid_constant__ SplitJob jb, int kc, int ld,
-                                                              int C) {
+                                                              int C, int *clear) {
     extern __shared__ __align__(16) double tile[]; // [R][ld], then the tables
     int64_t *koff = (int64_t *)(tile + (size_t)R * ld);
     int64_t *roff = koff + kc;
@@ -315,6 +315,7 @@ __global__ void __launch_bounds__(kFusedThreads) k_split_rows(const __grid_const
     int *ex = (int *)(pmax + R);
     constexpr int W = kFusedThreads / 32, P = S + (CHECK ? 2 : 0);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (clear && blockIdx.x == 0 && tid == 0) *clear = 0; // a counter of the kernels that follow
     const int64_t id = blockIdx.x / C;
     const int rank = C > 1 ? (int)ptx::cluster_ctarank() : 0;
     const bool second = id >= ja.tiles;
@@ -578,7 +579,8 @@ eg_status split_operand(OperandMap om, const double *X, unsigned long long *rowm
 }
 
 template <int S, bool CHECK, int R>
-cudaError_t launch_split_rows(const SplitJob &a, const SplitJob &b, int kc, int ld, int C, size_t smem, cudaStream_t s) {
+cudaError_t launch_split_rows(const SplitJob &a, const SplitJob &b, int kc, int ld, int C, size_t smem, int *clear,
+                              cudaStream_t s) {
     static const cudaError_t attr = cudaFuncSetAttribute(k_split_rows<S, CHECK, R>,
                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (attr != cudaSuccess) return attr;
@@ -594,7 +596,7 @@ cudaError_t launch_split_rows(const SplitJob &a, const SplitJob &b, int kc, int 
     la.val.clusterDim.z = 1;
     cfg.attrs = &la;
     cfg.numAttrs = C > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_split_rows<S, CHECK, R>, a, b, kc, ld, C);
+    return cudaLaunchKernelEx(&cfg, k_split_rows<S, CHECK, R>, a, b, kc, ld, C, clear);
 }
 
 // Elements from row to row of the digit planes: K in whole blocks of 64, or for a short K
@@ -607,7 +609,8 @@ int64_t plane_pitch(int64_t K) {
     return K <= 512 && 8 * sectors <= 7 * blocks ? sectors : blocks;
 }
 
-// Splits the operands of a contraction (an operand without rows is left out).  The
+// Splits the operands of a contraction (an operand without rows is left out), and sets
+// *clear to zero (unless null).  The
 // fused launch when a range of K fits shared memory (K to about 25000); beyond, the
 // passes over each operand, with tables of offsets at tab (rows and K of each operand;
 // may be null).  Fused against passes, device time: both operands of 2304^3 in FP64
@@ -615,7 +618,8 @@ int64_t plane_pitch(int64_t K) {
 // 515 -> 211 us, the four of n = 75 quarter transformations 1.90 -> 0.72 ms (0.9 GB
 // each: 5.2 TB/s).
 eg_status split_both(OperandMap oa, const double *A, int *eA, __nv_bfloat16 *pA, OperandMap ob, const double *B, int *eB,
-                     __nv_bfloat16 *pB, unsigned long long *maxima, int64_t *tab, int S, bool f64, cudaStream_t s) {
+                     __nv_bfloat16 *pB, unsigned long long *maxima, int64_t *tab, int S, bool f64, int *clear,
+                     cudaStream_t s) {
     for (OperandMap *o : {&oa, &ob}) {
         o->sr = affine_stride(o->rg, o->comp);
         o->sk = affine_stride(o->kg, o->comp);
@@ -664,8 +668,8 @@ eg_status split_both(OperandMap oa, const double *A, int *eA, __nv_bfloat16 *pA,
             auto go = [&](auto slices, auto check) {
                 constexpr int SL = decltype(slices)::value;
                 constexpr bool CH = decltype(check)::value;
-                return R == 32 ? launch_split_rows<SL, CH, 32>(ja, jb, (int)kc, ld, C, smem, s)
-                               : launch_split_rows<SL, CH, 8>(ja, jb, (int)kc, ld, C, smem, s);
+                return R == 32 ? launch_split_rows<SL, CH, 32>(ja, jb, (int)kc, ld, C, smem, clear, s)
+                               : launch_split_rows<SL, CH, 8>(ja, jb, (int)kc, ld, C, smem, clear, s);
             };
             using std::integral_constant;
             if (f64)
@@ -683,6 +687,7 @@ eg_status split_both(OperandMap oa, const double *A, int *eA, __nv_bfloat16 *pA,
         EG_CHECK_LAUNCH("k_split_rows");
         return EG_SUCCESS;
     }
+    if (clear) EG_CUDA(cudaMemsetAsync(clear, 0, sizeof(int), s));
     unsigned long long *maxA = maxima, *maxB = maxima + (int64_t)oa.nbatch * oa.Rp;
     eg_status st;
     if (oa.rows && (st = split_operand(oa, A, maxA, eA, pA, S, s, tab, tab ? tab + oa.rows : nullptr, f64)) != EG_SUCCESS)
@@ -844,7 +849,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     OperandMap oa{c.batch, c.m, c.k, 0, M, Mp, K, Kp, (int)nb};
     OperandMap ob{c.batch, c.n, c.k, 1, N, Np, K, Kp, (int)nb};
     int64_t *tab = tables ? (int64_t *)(base + offTab) : nullptr;
-    if ((st = split_both(oa, c.A, eA, planesA, ob, c.B, eB, planesB, maxA, tab, S, false, s)) != EG_SUCCESS) return st;
+    if ((st = split_both(oa, c.A, eA, planesA, ob, c.B, eB, planesB, maxA, tab, S, false, nullptr, s)) != EG_SUCCESS) return st;
 
     CUtensorMap tmA, tmB, tmBh;
     if ((st = encode_planes(&tmA, planesA, Kp, Mp, nb * S)) != EG_SUCCESS) return st;
@@ -1049,7 +1054,7 @@ eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
     p.hid = kF64High;
     p.redo = (int4 *)(base + oRedo);
     p.redo_count = (int *)(base + oRedoN);
-    EG_CUDA(cudaMemsetAsync(p.redo_count, 0, sizeof(int), s));
+    bool first = true; // the first splitting launch clears redo_count
 
     for (int64_t b0 = 0; b0 < nb; b0 += bb) {
         const int64_t nbc = std::min(bb, nb - b0);
@@ -1069,8 +1074,9 @@ eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
                 if (n0 > 0) oa.rows = 0;
                 if (nbk >= Np_all && m0 > 0) ob.rows = 0;
                 if ((st = split_both(oa, c.A, eA, planesA, ob, c.B, eB, planesB, (unsigned long long *)(base + oMax), tab,
-                                     S, true, s)) != EG_SUCCESS)
+                                     S, true, first ? p.redo_count : nullptr, s)) != EG_SUCCESS)
                     return st;
+                first = false;
                 CUtensorMap tmA, tmB, tmBh;
                 if ((st = encode_planes(&tmA, planesA, Kp, Mp, nbc * P)) != EG_SUCCESS) return st;
                 if ((st = encode_planes(&tmB, planesB, Kp, Np, nbc * P)) != EG_SUCCESS) return st;
