@@ -6,7 +6,8 @@
 //   k_elementwise   no summed modes: DIRECT / GER / broadcasts
 //                   (replaces hipBLASVendor/src/direct_prod.hip:20-200, ger, and
 //                    GPUTensorAlgebra.hpp:87-140)
-//   k_dot_*         rank-0 C: deterministic two-pass reduction, no atomics
+//   k_dot_*         rank-0 C: deterministic reduction, no atomics, in one CTA for
+//                   short sums, else in two passes
 //                   (replaces GPULinearAlgebra.hpp:35-101 and GPUTensorAlgebra.hpp:146-198)
 //   k_gemv          one of the M/N groups empty: one CTA or warp per output
 //                   (replaces hipblasDgemv at GPULinearAlgebra.hpp:346-386)

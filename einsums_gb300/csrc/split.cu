@@ -1,5 +1,9 @@
-// Host orchestration of the split-BF16 form and its digit-splitting kernels.
+// Host orchestration of the split-BF16 form, of plain FP64 on the tensor cores
+// (launch_f64_tensor) and of their digit-splitting kernels.
 //
+//   k_split_rows     row maxima, exponents and digit planes of both operands in one
+//                    launch that reads every element once, for K up to about 25000;
+//                    beyond, passes over each operand:
 //   k_split_rowmax   max |x| of every operand row (atomicMax on the bit
 //                    pattern of |x|, which orders like the value; deterministic)
 //   k_split_exponent row exponent e with |x| < 2^e (INT_MIN for a row holding
@@ -16,12 +20,12 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
-#include <vector>
 #include <cstring>
 #include <map>
 #include <mutex>
 #include <tuple>
 #include <type_traits>
+#include <vector>
 
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
