@@ -848,7 +848,8 @@ __global__ void __launch_bounds__(32 * kFinishRows) k_tc_finish_slices(const __g
     long long lo[PER] = {}, hi[PER] = {};
     const long long *at =
         p.parts + (size_t)e0 * PLANES * kPlane + (size_t)(half * kCols + c0 + warp) * kBM + quad * 32 + lane;
-#pragma unroll 2
+    // (eight slices at a time: complex 300 x 170 x 257 in nine slices 16.3 -> 14.5 us)
+#pragma unroll 8
     for (int k = 0; k < p.ksplit; k++, at += CL * PLANES * kPlane) {
 #pragma unroll
         for (int i = 0; i < PER; i++) {
