@@ -739,6 +739,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 continue;
             }
             if (live == 0) continue;
+            __syncwarp(); // every lane has stored the tile before with the offsets replaced below
             pend_cols = live;
             pend_lo = sums;
             pend_hi = (int)(own_hi - sums);
