@@ -336,7 +336,7 @@ struct alignas(16) RowsUnit {
     int64_t rtab, ktab;
     int64_t pitch, pstride;
     int K, R, rows; // rows: of the R, those that exist
-    int flags;      // 1: contiguous along the rows, 2: the operand is B
+    int flags;      // 1: contiguous along the rows
 };
 constexpr int kUnitSlots = 4;
 static_assert(sizeof(RowsUnit) % 16 == 0 && sizeof(RowsUnit) / 16 <= 32, "fetched by one warp, 16 bytes a lane");
@@ -406,7 +406,6 @@ __global__ void __launch_bounds__(kGThreads, 3) k_grouped_rows(const RowsUnit *u
         // one after the other, so that rows of few k keep all lanes busy
         __nv_bfloat16 *const planes = g.planes;
         int *const rexp = g.rexp;
-        const float mark = g.flags & 2 ? split::kCheckB : split::kCheckA;
         for (int r = warp; r < nr; r += kGWarps) {
             const int e = split::row_exponent(split::row_max_bits(tile + r * ld, kw, lane));
             if (lane == 0) ex[r] = rexp[r] = e;
@@ -431,8 +430,8 @@ __global__ void __launch_bounds__(kGThreads, 3) k_grouped_rows(const RowsUnit *u
                 }
             }
             if constexpr (CHECK) {
-                p0[S + 1] = split::check_mark(v0.x, v0.y, mark);
-                p1[S + 1] = split::check_mark(v1.x, v1.y, mark);
+                p0[S + 1] = split::check_mark(v0.x, v0.y);
+                p1[S + 1] = split::check_mark(v1.x, v1.y);
             }
             __nv_bfloat16 *row = planes + r * pitch + 4 * k;
 #pragma unroll
@@ -905,7 +904,7 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
             x.K = (int)g.K;
             x.R = u.w;
             x.rows = (int)std::min<int64_t>(g.rows - r0, u.w);
-            x.flags = (g.row_fast ? 1 : 0) | (g.comp ? 2 : 0);
+            x.flags = g.row_fast ? 1 : 0;
             rows.push_back(x);
         }
         st = dev_copy(plan, rows.data(), rows.size() * sizeof(RowsUnit), &d_units);

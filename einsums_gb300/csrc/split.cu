@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(T *TR) k_split_digits(OperandMap m, const doub
                     digits_bf16x2<S>(x0, x1, e, pk);
                     if constexpr (CHECK) pk[S] = check_magnitude(pk[0]);
                 }
-                if constexpr (CHECK) pk[S + 1] = check_mark(x0, x1, m.comp ? kCheckB : kCheckA);
+                if constexpr (CHECK) pk[S + 1] = check_mark(x0, x1);
                 uint32_t *out = (uint32_t *)(planes + ((int64_t)b * P) * plane + r * m.Kp + k0) + tx;
 #pragma unroll
                 for (int s = 0; s < P; s++) out[(int64_t)s * (plane / 2)] = pk[s];
@@ -422,9 +422,8 @@ __global__ void __launch_bounds__(kFusedThreads) k_split_rows(const __grid_const
             }
         }
         if constexpr (CHECK) {
-            const float mark = m.comp ? kCheckB : kCheckA;
-            p0[S + 1] = check_mark(v0.x, v0.y, mark);
-            p1[S + 1] = check_mark(v1.x, v1.y, mark);
+            p0[S + 1] = check_mark(v0.x, v0.y);
+            p1[S + 1] = check_mark(v1.x, v1.y);
         }
         __nv_bfloat16 *row = first + r * m.Kp + 4 * k;
 #pragma unroll
@@ -962,14 +961,19 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
 //   |C - C_exact| <= 9.04 2^-64 N max|A_i| max|B_j|     N: the k where both are nonzero
 //
 // (7.03 from the slice pairs dropped, 2 from the digits, with max| | the power of
-// two above the row's largest element).  The check planes give, in one more slice
-// group and exactly, sum_k p_a p_b with p <= 128 |x| / max, and 20 N; where
-//   sum_k p_a p_b >= 20 N
+// two above the row's largest element).  The check planes give, in two more slice
+// products and exactly, M = sum_k p_a p_b with p <= 128 |x| / max, and N; where
+//   M >= 20 N   (M >= 20 N + 256 for N < 8)
 // the error is at most 4 2^-53 sum_k |A_ik| |B_jk| -- four roundings' worth, where
-// the bound of a chain of K FMAs is K of them.  A region of a tile in
-// which it fails anywhere (rows graded against each other, infinities, NaN) is
+// the bound of a chain of K FMAs is K of them; with two products, half a rounding.
+// A single product (N = 1), which an FMA rounds once and exactly, always fails; sums of
+// no products are zero and pass.  Random sums that just pass, against FMA chains in exact
+// arithmetic: rms error 0.82 of the chain's at N = 2, 0.65 at 4, 0.5 at 8, 0.25 at 32.
+// A region of a tile in
+// which the check fails anywhere (rows graded against each other, infinities, NaN) is
 // not written but listed, and k_contract_f64 computes it from C as it was.  The
-// sums of all 36 products are exact in two int64 words and rounded once.
+// sums of all 36 products are exact in two int64 words and rounded once.  Neither they
+// nor the check depend on how tiles are cut along K or shared by CTAs.
 //
 // The digit planes live in a scratch shared by the streams of the device and
 // bounded by kF64ScratchCap; larger operands are cut into panels of rows.  When
@@ -1018,7 +1022,7 @@ eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
     const size_t oFront = take(front);
     const size_t oPA = take((size_t)bb * P * mb * Kp * 2), oPB = take((size_t)bb * P * nbk * Kp * 2);
     const size_t oMax = take((size_t)bb * (mb + nbk) * 8);
-    const size_t oMargin = take((size_t)slices_max * kTileRegions * sizeof(int));
+    const size_t oCheck = take((size_t)slices_max * kBM * kBN * sizeof(int));
     const size_t oParts = take((size_t)slices_max * 2 * kBM * kBN * 8);
     const size_t oExp = take((size_t)bb * (mb + nbk) * 4);
     const size_t oTab = take(tables ? (size_t)(M + N + 2 * K) * 8 : 0);
@@ -1052,7 +1056,7 @@ eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
     p.timeout_ns = 2000ull * 1000 * 1000;
     p.rbuf = (long long *)(base + oR);
     p.parts = (long long *)(base + oParts);
-    p.parts_margin = (int *)(base + oMargin);
+    p.parts_check = (int *)(base + oCheck);
     p.d0 = 0;
     p.d1 = S;
     p.hid = kF64High;

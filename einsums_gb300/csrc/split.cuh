@@ -34,7 +34,18 @@ constexpr int kBM = 128, kBN = 128, kBK = 64;
 // The FP64 form: eight slices (63 bits below each row's power of two) and the
 // accuracy check of launch_f64_tensor.
 constexpr int kF64Slices = 8, kF64High = 4;
-constexpr float kCheckA = 4.0f, kCheckB = -5.0f;
+// The check of one output over its N products that are not zero, M the sum of their leading
+// magnitudes' products (p_a p_b): it passes when N = 0, or N >= 8 and M >= 20 N, or N >= 2 and
+// M >= 20 N + 256.  A product that stands alone is left to the FMA kernel, which rounds it once.
+constexpr int kCheckPer = 20, kCheckFew = 8, kCheckMore = 256;
+__host__ __device__ constexpr bool check_fails(int products, int excess) { // excess: M - 20 N
+    return products == 1 || (products > 1 && excess < (products < kCheckFew ? kCheckMore : 0));
+}
+// The check of one K slice of a tile, to be added up: the excess, below a bound that no sum
+// over the slices falls back from (the least is -20 65536), and N, where 8 stands for more.
+__host__ __device__ constexpr int pack_check(int products, int excess) {
+    return (excess < (1 << 22) ? excess : 1 << 22) * 16 + (products < kCheckFew ? products : kCheckFew);
+}
 constexpr int kTileRegions = 8; // parts of a tile, one per epilogue warp: 32 rows by 64 columns in turns of 16
 constexpr int kChunkKB = 16;    // 16 x 64 = 1024 products per exact FP32 chunk
 constexpr int kKStep = 2 * kBK;  // granularity of the longest exact pass (K itself is padded to kBK)
@@ -69,12 +80,12 @@ struct TcGemmParams {
     // (t - t0) % ksplit (kslice K blocks; the last slice takes the rest) of
     // tile t0 + (t - t0) / ksplit.  A slice's exact int64 sums go to parts ([t - t0]
     // [128 columns][128 rows], two planes in the FP64 form; with CTA pairs an entry is
-    // two tiles, one after the other) and the least sum of its check to parts_margin
-    // ([t - t0][8]); k_tc_finish_slices adds them up.  Unused when t0 is the number of tiles.
+    // two tiles, one after the other) and its outputs' checks (pack_check) to parts_check
+    // ([t - t0][128][128]); k_tc_finish_slices adds them up.  Unused when t0 is the number of tiles.
     int t0;
     int ksplit, kslice;
     long long *parts;
-    int *parts_margin;
+    int *parts_check;
     // Launch as CTA pairs (cta_group::2, 256x128 tiles): single contractions only.
     int pair;
     // Slice groups d0 <= d < d1 (anti-diagonals s + t = d of the digit pairs)
@@ -290,14 +301,14 @@ __device__ __forceinline__ void digits_bf16x2(double x0, double x1, int e, uint3
 
 // The two check planes of the FP64 form for the pair whose leading digits are
 // d0 (as floats in the halves of `lead`): max(|a_0| - 1, 0), at most 128 |x| 2^-e,
-// and `mark` where x is not zero (kCheckA or kCheckB by operand).
+// and 1 where x is not zero.
 __device__ __forceinline__ uint32_t check_magnitude(uint32_t lead) {
     const float f0 = fmaxf(fabsf(__uint_as_float(lead << 16)) - 1.0f, 0.0f);
     const float f1 = fmaxf(fabsf(__uint_as_float(lead & 0xFFFF0000u)) - 1.0f, 0.0f);
     return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
 }
-__device__ __forceinline__ uint32_t check_mark(double x0, double x1, float mark) {
-    return __byte_perm(abs_bits(x0) ? __float_as_uint(mark) : 0u, abs_bits(x1) ? __float_as_uint(mark) : 0u, 0x7632);
+__device__ __forceinline__ uint32_t check_mark(double x0, double x1) {
+    return (abs_bits(x0) ? 0x3F80u : 0u) | (abs_bits(x1) ? 0x3F800000u : 0u);
 }
 
 // Sets the kernels' shared-memory attribute once (call outside stream capture).

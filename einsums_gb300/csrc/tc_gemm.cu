@@ -51,10 +51,8 @@ static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 // that misses the few KB of L1 left beside the ring waits some 4000 clocks behind the
 // tiles in flight (25600 x 25600, K = 1024: 16.0 ms with 60 bytes of spills a thread,
 // 12.9 without).
-constexpr int regs_issue(int cl) { return cl == 2 ? 40 : 56; } // (single CTAs' issuer watches two slots)
-constexpr int regs_epilogue(int cl) { return cl == 2 ? 232 : 224; }
-static_assert(128 * regs_issue(1) + 32 * kEpiWarps * regs_epilogue(1) <= THREADS * 168, "registers of the launch");
-static_assert(128 * regs_issue(2) + 32 * kEpiWarps * regs_epilogue(2) <= THREADS * 168, "registers of the launch");
+constexpr int kRegsIssue = 56, kRegsEpilogue = 224;
+static_assert(128 * kRegsIssue + 32 * kEpiWarps * kRegsEpilogue <= THREADS * 168, "registers of the launch");
 constexpr int GROUP_M = 16; // tile rasterisation: groups of 16 row tiles share B tiles in L2
 constexpr unsigned long long DRAIN_NS = 200ull * 1000 * 1000;
 
@@ -172,12 +170,15 @@ __device__ __forceinline__ TileJob resolve(const TcGemmParams &p, const TcItem *
 // A_j and B_{hi-j} for j = 0 .. hi (hi the higher group), A_j meets B_{hi-j} in group
 // hi and B_{hi-1-j}, the next slot's, in group hi - 1, in one MMA of N = 256.  The
 // FP64 form starts with step -1, the two plane pairs of its accuracy check (planes S
-// and S + 1), each a product of its own slot's tiles.
+// and S + 1), each a product of its own slot's tiles in an accumulator of its own.
 struct Step {
     int hi;     // the higher group
     int slots;  // ring slots per K block
     bool two;   // groups hi - 1 and hi
-    int kbc;    // K blocks of a chunk: at most 16 tile products per accumulator, 1024 digit products
+    // K blocks of a chunk: at most 16 tile products per accumulator, 1024 digit products.
+    // The check's sums (of whole numbers, none negative) run over all of K: N stays below
+    // 2^24, and M is exact up to there, far above where it decides.
+    int kbc;
 };
 __device__ __forceinline__ int step_count(const TcGemmParams &p) { return (p.d1 - p.d0 + 1) / 2; }
 __device__ __forceinline__ Step step_of(const TcGemmParams &p, int q) {
@@ -186,13 +187,14 @@ __device__ __forceinline__ Step step_of(const TcGemmParams &p, int q) {
         s.hi = p.S;
         s.slots = 2;
         s.two = false;
+        s.kbc = INT_MAX;
     } else {
         const int odd = (p.d1 - p.d0) & 1;
         s.two = !(odd && q == 0);
         s.hi = p.d0 + 2 * q + 1 - odd;
         s.slots = s.hi + 1;
+        s.kbc = kChunkKB / s.slots;
     }
-    s.kbc = kChunkKB / s.slots;
     return s;
 }
 __device__ __forceinline__ int slot_a(const TcGemmParams &p, int q, int j) { return q < 0 ? p.S + j : j; }
@@ -299,7 +301,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         GROUPED ? p.ranges[blockIdx.x + 1] : p.t0 + (p.nbatch * ((p.mtiles + CL - 1) / CL) * p.ntiles - p.t0) * p.ksplit;
 
     if (warp < 4) {
-        ptx::regs_dec<regs_issue(CL)>();
+        ptx::regs_dec<kRegsIssue>();
         if (warp == 0 || warp == 2) {
             // -------------------------------------------- TMA producers: A tiles, B tiles
             // Two warps, each with uniform control flow and one elected lane issuing:
@@ -434,12 +436,13 @@ __global__ void __launch_bounds__(THREADS, 1)
                             if (leader) {
                                 const uint64_t a = desc0 + (uint64_t)stage * kTile;
                                 const uint64_t b = desc0 + (uint64_t)(kSlots + stage) * kTile;
-                                const uint32_t keep = (c > 0 || j > 0) ? 1u : 0u;
+                                const uint32_t keep = (c > 0 || (j > 0 && q >= 0)) ? 1u : 0u;
+                                const uint32_t Dj = q < 0 && j == 0 ? D + kBN : D; // the check's sums lie apart
                                 if (!dual || CL == 2 || next != 0) {
                                     const uint32_t idesc = dual ? idesc2 : idesc1;
 #pragma unroll
                                     for (int k = 0; k < 4; k++)
-                                        ptx::mma_bf16<CL>(D, a + k * kStep, b + k * kStep, idesc, k ? 1u : keep);
+                                        ptx::mma_bf16<CL>(Dj, a + k * kStep, b + k * kStep, idesc, k ? 1u : keep);
                                 } else { // the ring wraps between the two B tiles
                                     const uint64_t b2 = desc0 + (uint64_t)kSlots * kTile;
 #pragma unroll
@@ -478,7 +481,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     } else {
         // ------------------------------------------------ epilogue (warps 4..11)
         // Two warps per TMEM lane quadrant; each owns 64 of the tile's 128 columns.
-        ptx::regs_inc<regs_epilogue(CL)>();
+        ptx::regs_inc<kRegsEpilogue>();
         constexpr int FIN = F64 ? kFin / 2 : kFin; // the FP64 form holds two words per sum
         const int ew = warp - 4;              // 0..7
         const int quad = warp & 3;            // TMEM lane quadrant this warp may access
@@ -490,8 +493,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         int run_exp = kCols;
         double *finT = finTAll + ew * (kFin * FIN_T);
         double **rowAt = rowAtAll + ew * 33;
-        // FP64 form: the least sum of the check in the running tile, negative where it fails
-        volatile int *const margin = (volatile int *)(rowAt + 32);
+        volatile int *const failed = (volatile int *)(rowAt + 32); // FP64 form: the check, in the running tile
         int abuf = 0;
         uint32_t aphase = 0;
         bool ok = true;
@@ -562,7 +564,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 if ((int64_t)job.mt * kBM + quad * 32 < job.M)
                     live = cols / 32 * 16 + min(max(cols % 32 - half * 16, 0), 16);
                 const int64_t m = (int64_t)job.mt * kBM + row;
-                my_rowExp = m < job.M ? job.eA[m] : INT_MAX; // INT_MAX: past the output
+                my_rowExp = m < job.M ? job.eA[m] : 0;
 #pragma unroll
                 for (int i = 0; i < kCols / 32; i++) {
                     const int64_t n = (int64_t)job.nt * kBN + tile_col(half, lane + 32 * i);
@@ -591,7 +593,45 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                     ptx::tc_fence_after();
                     const uint32_t at = tl + (uint32_t)(abuf * 2 * kBN);
-                    if (st.two) {
+                    if (F64 && q < 0) { // the check; where it fails anywhere, the FMA kernel takes this warp's outputs
+                        // quickly: a sum of few products anywhere, or a lack of magnitude?
+                        float few = kCheckFew, least = 0.0f;
+#pragma unroll 1
+                        for (int cc = 0; cc < live; cc += 16) {
+                            uint32_t products[16], sums[16];
+                            ptx::tmem_ld16(at + 2 * cc, products);
+                            ptx::tmem_ld16(at + kBN + 2 * cc, sums);
+                            ptx::tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 16; i++) { // (past the output there are no products)
+                                const float n = __uint_as_float(products[i]);
+                                few = fminf(few, n > 0.0f ? n : (float)kCheckFew);
+                                least = fminf(least, fmaf(-(float)kCheckPer, n, __uint_as_float(sums[i])));
+                            }
+                        }
+                        const bool slice = !GROUPED && tile >= p.t0;
+                        bool bad = few < kCheckFew || least < 0.0f;
+                        if (slice || __any_sync(0xffffffffu, bad)) { // closely
+                            bad = false;
+#pragma unroll 1
+                            for (int cc = 0; cc < live; cc += 8) {
+                                const uint32_t from = at + 2 * cc - (cc & 8); // in turns of 16 columns
+                                uint32_t products[8], sums[8];
+                                ptx::tmem_ld8(from, products);
+                                ptx::tmem_ld8(from + kBN, sums);
+                                ptx::tmem_wait_ld();
+                                const uint32_t check = (uint32_t)(((tile - p.t0) * CL + rank) * kBN + half * kCols + cc) * kBM + row;
+#pragma unroll
+                                for (int i = 0; i < 8; i++) {
+                                    const int n = __float2int_rn(__uint_as_float(products[i]));
+                                    const int excess = __float2int_rn(__uint_as_float(sums[i])) - kCheckPer * n;
+                                    bad = bad || check_fails(n, excess);
+                                    if (slice) p.parts_check[check + i * kBM] = pack_check(n, excess);
+                                }
+                            }
+                        }
+                        *failed = __any_sync(0xffffffffu, bad) ? 1 : 0;
+                    } else if (st.two) {
 #pragma unroll
                         for (int cc = 0; cc < kCols; cc += 16) {
                             if (cc >= live) break;
@@ -629,15 +669,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if (kb >= nkb) { // the step is complete
                         kb = 0;
                         q++;
-                        if (F64 && q == 0) { // a negative margin anywhere: the FMA kernel takes this warp's outputs
-                            int worst = INT_MAX; // (the sums stay below 2^30)
-#pragma unroll
-                            for (int i = 0; i < kCols; i++) {
-                                if (i < live) worst = min(worst, (int)H[i]);
-                                H[i] = 0;
-                            }
-                            *margin = __reduce_min_sync(0xffffffffu, my_rowExp != INT_MAX ? worst : INT_MAX);
-                        } else if (F64 && st.hi + 1 == p.hid) { // the high sums are complete
+                        if (F64 && st.hi + 1 == p.hid) { // the high sums are complete
                             long long *const at_hi = !GROUPED && tile >= p.t0 ? part_of(tile) + kPlane : rbc + (1 + parity) * kPlane;
 #pragma unroll
                             for (int i = 0; i < kCols; i++) {
@@ -723,13 +755,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             long long *const sums = slice ? part_of(tile) : rbc;
 #pragma unroll
             for (int i = 0; i < kCols; i++) sums[i * kBM] = H[i];
-            if (slice) {
-                if (F64 && lane == 0) p.parts_margin[job.part * kTileRegions + ew] = *margin;
-                continue;
-            }
+            if (slice) continue;
             long long *const own_hi = rbc + (F64 ? 1 + parity : 0) * kPlane;
             parity ^= 1;
-            if (F64 && *margin < 0) {
+            if (F64 && *failed) {
                 if (lane == 0) {
                     const int at = atomicAdd(p.redo_count, 1);
                     const int m0 = job.mt * kBM + quad * 32, n0 = job.nt * kBN + half * 16;
@@ -795,7 +824,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 // (the whole contraction 190 -> 132 us, 2304 x 2304 715 -> 672 us).
 constexpr int kFinishRows = 8, kFinishCols = 32, kFinishParts = kCols / kFinishCols; // warps and columns of its CTAs
 template <int CL, bool F64>
-__global__ void __launch_bounds__(32 * kFinishRows) k_tc_finish_slices(const __grid_constant__ TcGemmParams p) {
+__global__ void __launch_bounds__(32 * kFinishRows, 3) k_tc_finish_slices(const __grid_constant__ TcGemmParams p) {
     __shared__ double tile[kFinishCols][33];
     constexpr int PLANES = F64 ? 2 : 1, PER = kFinishCols / kFinishRows;
     constexpr size_t kPlane = (size_t)kBM * kBN;
@@ -812,16 +841,25 @@ __global__ void __launch_bounds__(32 * kFinishRows) k_tc_finish_slices(const __g
     const int live = min(cols / 32 * 16 + min(max(cols % 32 - half * 16, 0), 16) - c0, kFinishCols);
     if (rows <= 0 || live <= 0) return;
     const int e0 = q * p.ksplit * CL + rank; // the tile's first slice; the next ones are CL further on
+    bool bad = false;
     if (F64) {
-        // the slices' least check sums add up to no more than the least of their sum
-        long long margin = 0;
-        for (int k = 0; k < p.ksplit; k++) margin += p.parts_margin[(e0 + k * CL) * kTileRegions + ew];
-        if (margin < 0) {
-            if (threadIdx.x == 0 && c0 == 0)
-                p.redo[atomicAdd(p.redo_count, 1)] =
-                    make_int4((int)p.b0 + b, (int)(p.m0 + m0), (int)(p.n0 + n0) + half * 16, 0);
-            return;
+        // the region's check, over the slices, as in a whole tile (both of its CTAs see all of it)
+        const int all = cols / 32 * 16 + min(max(cols % 32 - half * 16, 0), 16);
+        const int *at = p.parts_check + (size_t)e0 * kPlane + (size_t)(half * kCols) * kBM + quad * 32 + lane;
+        constexpr int COLS = kCols / kFinishRows; // of a warp: all of them and four slices at a time
+        int products[COLS] = {}, excess[COLS] = {};
+#pragma unroll 4
+        for (int k = 0; k < p.ksplit; k++, at += CL * kPlane) {
+#pragma unroll
+            for (int i = 0; i < COLS; i++) {
+                const int c = warp + i * kFinishRows, x = c < all ? __ldcg(at + c * kBM) : 0;
+                products[i] += x & 15;
+                excess[i] += x >> 4;
+            }
         }
+#pragma unroll
+        for (int i = 0; i < COLS; i++) bad = bad || check_fails(products[i], excess[i]);
+        bad = bad && lane < rows;
     }
     // where this thread will write, along C's rows or columns, and C's old values there
     const bool plain_store = p.zero && p.cp == 0.0;
@@ -867,7 +905,12 @@ __global__ void __launch_bounds__(32 * kFinishRows) k_tc_finish_slices(const __g
         const double v = finish_value<F64, false>(p, lo[i], hi[i], rowExp, colExp);
         tile[c][lane] = p.ab_pow2 ? v : p.ab * v;
     }
-    __syncthreads();
+    if (__syncthreads_or(bad)) { // the FMA kernel computes the region
+        if (threadIdx.x == 0 && c0 == 0)
+            p.redo[atomicAdd(p.redo_count, 1)] =
+                make_int4((int)p.b0 + b, (int)(p.m0 + m0), (int)(p.n0 + n0) + half * 16, 0);
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < PER; i++)
         if (out[i]) *out[i] = plain_store ? *from[i] : fma(p.cp, old[i], *from[i]);
