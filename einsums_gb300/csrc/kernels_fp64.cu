@@ -480,9 +480,11 @@ struct F64Args {
     int64_t ka, kb;        // single k strides of A and B (0: none)
     int64_t mtiles, ntiles, total; // total = batches * mtiles * ntiles
     int cs;                // CTAs of a cluster, each taking a range of the k chunks
-    // When set, the tiles are instead the halves of the blocks {batch, row, column}
-    // listed there (T = 32, one CTA each): 32 rows by the 16 columns from `column` and
-    // from 32, 64 and 96 further on.
+    // When set, the tiles are instead the parts of the blocks {batch, row, column}
+    // listed there: 32 rows by the 16 columns from `column` and from 32, 64 and 96 further
+    // on.  A part outside the output is skipped; with the parts of a block one after the
+    // other some CTAs had only such ones (120000 x 75, K = 75, all listed: 2097 us, all
+    // first parts first 1570).
     const int4 *list;
     const int *count;
 };
@@ -501,15 +503,20 @@ __global__ void __launch_bounds__(kThreads) k_contract_f64(const __grid_constant
     const int chunks = (int)((K + BK - 1) / BK);
     const int cbeg = (int)((int64_t)chunks * rank / p.cs), cend = (int)((int64_t)chunks * (rank + 1) / p.cs);
     const int64_t step = gridDim.x / p.cs;
-    const int64_t total = p.list ? 2 * (int64_t)__ldg(p.count) : p.total;
-    const int gap = p.list ? 16 : 0; // tile column j is column j + (j & gap) from the tile's first
+    constexpr int ROWS = 32 / T, PARTS = ROWS * (64 / T); // of a listed block
+    const uint32_t listed = p.list ? (uint32_t)__ldg(p.count) : 0;
+    const int64_t total = p.list ? (int64_t)PARTS * listed : p.total;
+    const int gap = T == 32 && p.list ? 16 : 0; // tile column j is column j + (j & gap) from the tile's first
     for (int64_t t = blockIdx.x / p.cs; t < total; t += step) {
         int64_t b, m0, n0;
         if (p.list) {
-            const int4 e = p.list[t >> 1];
+            const uint32_t part = (uint32_t)t / listed; // all first parts, then the second ones, ...
+            const int4 e = p.list[(uint32_t)t - part * listed];
+            const int col = part / ROWS * T;
             b = e.x;
-            m0 = e.y;
-            n0 = e.z + 2 * T * (t & 1);
+            m0 = e.y + part % ROWS * T;
+            n0 = e.z + (T == 32 ? 2 * col : 2 * col - col % 16);
+            if (m0 >= M || n0 >= N) continue;
         } else {
             const int64_t q = t / p.ntiles;
             b = q / p.mtiles;
@@ -664,7 +671,7 @@ double contract_plan(int64_t nb, int64_t M, int64_t N, int64_t K, int &T, int &c
 
 template <int T>
 cudaError_t launch_f64_tiles(const F64Args &p, cudaStream_t s) {
-    const int64_t clusters = std::min<int64_t>(p.total, int64_t(1) << 24);
+    const int64_t clusters = p.list ? num_sms() * (T == 32 ? 4 : 8) / p.cs : std::min<int64_t>(p.total, int64_t(1) << 24);
     if (p.cs == 1) {
         k_contract_f64<T><<<(unsigned)clusters, kThreads, 0, s>>>(p);
         return cudaGetLastError();
@@ -681,6 +688,10 @@ cudaError_t launch_f64_tiles(const F64Args &p, cudaStream_t s) {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_contract_f64<T>, p);
+}
+
+cudaError_t launch_f64_tiles(const F64Args &p, int T, cudaStream_t s) {
+    return T == 32 ? launch_f64_tiles<32>(p, s) : T == 16 ? launch_f64_tiles<16>(p, s) : launch_f64_tiles<8>(p, s);
 }
 
 ModeGroup concat(std::initializer_list<const ModeGroup *> groups) {
@@ -900,9 +911,7 @@ eg_status launch_contract_f64(const Contraction &c, cudaStream_t s) {
     if (p.total == 0) return EG_SUCCESS;
     {
         LaunchScope ls_("k_contract_f64", s);
-        const cudaError_t err = T == 32   ? launch_f64_tiles<32>(p, s)
-                                : T == 16 ? launch_f64_tiles<16>(p, s)
-                                          : launch_f64_tiles<8>(p, s);
+        const cudaError_t err = launch_f64_tiles(p, T, s);
         if (err != cudaSuccess) return cuda_fail(err, "k_contract_f64");
     }
     EG_CHECK_LAUNCH("k_contract_f64");
@@ -915,12 +924,20 @@ double contract_f64_seconds(const Contraction &c) {
 }
 
 eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, const int *count, cudaStream_t s) {
+    // Tiles and K cut as if the whole output were listed, but for outputs of six rounds of
+    // 32 x 32 tiles or more, where those are faster although the last round is not full
+    // (1024^3, all listed: 2.19 ms, 2.33 with 16 x 16).  Smaller ones: 300 x 300, K = 1000
+    // 591 -> 265 us in all, 128 x 128, K = 60000 17.0 -> 4.2 ms.
     F64Args p = f64_args(c);
+    int T = 32;
+    if (c.batch.total * ((c.m.total + 31) / 32) * ((c.n.total + 31) / 32) < 6 * num_sms())
+        contract_plan(c.batch.total, c.m.total, c.n.total, c.k.total, T, p.cs);
     p.list = list;
     p.count = count;
     {
         LaunchScope ls_("k_contract_f64_listed", s);
-        k_contract_f64<32><<<(unsigned)(num_sms() * 4), kThreads, 0, s>>>(p);
+        const cudaError_t err = launch_f64_tiles(p, T, s);
+        if (err != cudaSuccess) return cuda_fail(err, "k_contract_f64_listed");
     }
     EG_CHECK_LAUNCH("k_contract_f64_listed");
     return EG_SUCCESS;
