@@ -32,6 +32,7 @@
 
 #include <cuda_bf16.h>
 
+#include "f64_tile.cuh"
 #include "grouped.cuh"
 #include "ptx.cuh"
 #include "split.cuh"
@@ -57,13 +58,14 @@ struct F64Item {
     double *C;
     ModeGroup b, m, n, k;
     int a_kfast, b_kfast;
+    int64_t ka, kb; // single k strides of A and B (0: none)
 };
 
 constexpr int BK = 16, THREADS = 256, LD = 65;
 
 template <int T>
-__device__ __forceinline__ void f64_tile(const F64Item &it, int64_t bidx, int64_t m0, int64_t n0, int gap, double cp,
-                                         double ab, bool zero, double (*As)[LD], double (*Bs)[LD]) {
+__device__ __forceinline__ void f64_tile(const F64Item &it, int64_t bidx, int64_t m0, int64_t n0, double cp, double ab,
+                                         bool zero, double (*As)[LD], double (*Bs)[LD]) {
     constexpr int R = T / 16; // outputs per thread per dimension, and loads per thread per operand
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int64_t M = it.m.total, N = it.n.total, K = it.k.total;
@@ -83,9 +85,8 @@ __device__ __forceinline__ void f64_tile(const F64Item &it, int64_t bidx, int64_
         okA[i] = m0 + lm[i] < M;
         group_offsets32(it.m, (uint32_t)(okA[i] ? m0 + lm[i] : 0), oa, ob, oc);
         offA[i] = ba + oa;
-        const int64_t n = n0 + ln[i] + (ln[i] & gap);
-        okB[i] = n < N;
-        group_offsets32(it.n, (uint32_t)(okB[i] ? n : 0), oa, ob, oc);
+        okB[i] = n0 + ln[i] < N;
+        group_offsets32(it.n, (uint32_t)(okB[i] ? n0 + ln[i] : 0), oa, ob, oc);
         offB[i] = bb + ob;
     }
     double acc[R][R];
@@ -136,7 +137,7 @@ __device__ __forceinline__ void f64_tile(const F64Item &it, int64_t bidx, int64_
         group_offsets32(it.m, (uint32_t)m, ma, mb, mc);
 #pragma unroll
         for (int j = 0; j < R; j++) {
-            const int64_t n = n0 + tx + 16 * j + ((tx + 16 * j) & gap);
+            const int64_t n = n0 + tx + 16 * j;
             if (n >= N) continue;
             int64_t na, nb, nc;
             group_offsets32(it.n, (uint32_t)n, na, nb, nc);
@@ -156,23 +157,58 @@ __global__ void __launch_bounds__(THREADS) k_grouped_f64(const F64Item *items, c
         const int4 e = work[w];
         const F64Item &it = items[e.x];
         if (tiles[e.x] == 64)
-            f64_tile<64>(it, e.y, int64_t(64) * e.z, int64_t(64) * e.w, 0, cp, ab, zero != 0, As, Bs);
+            f64_tile<64>(it, e.y, int64_t(64) * e.z, int64_t(64) * e.w, cp, ab, zero != 0, As, Bs);
         else
-            f64_tile<32>(it, e.y, int64_t(32) * e.z, int64_t(32) * e.w, 0, cp, ab, zero != 0, As, Bs);
+            f64_tile<32>(it, e.y, int64_t(32) * e.z, int64_t(32) * e.w, cp, ab, zero != 0, As, Bs);
     }
 }
 
 // The blocks of outputs that the FP64 form on the tensor cores left out, *count of them:
 // {item, batch index, row, column}, 32 rows by the 16 columns from `column` and from 32,
-// 64 and 96 further on.  Tile column j is column j + (j & gap) from the tile's first.
-__global__ void __launch_bounds__(THREADS) k_grouped_f64_listed(const F64Item *items, const int4 *list, const int *count,
-                                                                 double cp, double ab, int zero) {
-    __shared__ double As[BK][LD];
-    __shared__ double Bs[BK][LD];
-    const int n = 2 * __ldg(count);
-    for (int w = blockIdx.x; w < n; w += gridDim.x) {
-        const int4 e = list[w >> 1];
-        f64_tile<32>(items[e.x], e.y, e.z, e.w + 64 * (w & 1), 16, cp, ab, zero != 0, As, Bs);
+// 64 and 96 further on.  A list that fails the check everywhere must not take longer than
+// as a plan for the FP64 pipe, so: tiles of 16 x 16, as items of lists are small, those
+// outside the output skipped, handed out one by one (count[1], cleared like the count), all
+// first tiles of the blocks first.  512 uneven items (4-32 x 4-32 summed, 20-120 x 20-120), all
+// graded: 876 us in all, in tiles of 32 x 32 dealt in turn 2691; as a plan for the FP64 pipe
+// 825 to 940.  2048 items: 2.97 ms, 8.11, 3.28.
+__global__ void __launch_bounds__(f64::kThreads) k_grouped_f64_listed(const F64Item *items, const int4 *list, int *count,
+                                                                      double cp, double ab, int zero) {
+    constexpr int T = 16;
+    __shared__ f64::Buffers<T> chunk;
+    __shared__ uint32_t next;
+    const int tx = threadIdx.x % T, ty = threadIdx.x / T;
+    const uint32_t listed = (uint32_t)__ldg(count), total = 8 * listed;
+    uint32_t fetched = blockIdx.x;
+    while (true) {
+        if (threadIdx.x == 0) {
+            next = fetched;
+            fetched = gridDim.x + atomicAdd((unsigned *)count + 1, 1u); // the one after, while this one runs
+        }
+        __syncthreads(); // and the chunks of the tile before are read
+        const uint32_t u = next;
+        if (u >= total) return;
+        const uint32_t part = u / listed;
+        const int4 e = list[u - part * listed];
+        const F64Item &it = items[e.x];
+        const int64_t m0 = e.z + part % 2 * T, n0 = e.w + part / 2 * 2 * T;
+        if (m0 >= it.m.total || n0 >= it.n.total) {
+            __syncthreads();
+            continue;
+        }
+        int64_t ba, bb, bc, oa, ob, oc;
+        group_offsets(it.b, e.y, ba, bb, bc);
+        double acc[1][1] = {};
+        constexpr int CK = f64::Tile<T>::BK;
+        f64::accumulate<T>(chunk, {it.m, it.n, it.k, it.A + ba, it.B + bb, it.a_kfast, it.b_kfast, it.ka, it.kb}, m0, n0, 0,
+                           0, (int)((it.k.total + CK - 1) / CK), acc);
+        if (m0 + ty < it.m.total && n0 + tx < it.n.total) {
+            group_offsets32(it.m, (uint32_t)(m0 + ty), oa, ob, oc);
+            bc += oc;
+            group_offsets32(it.n, (uint32_t)(n0 + tx), oa, ob, oc);
+            double *cptr = it.C + bc + oc;
+            const double v = ab * acc[0][0];
+            *cptr = (zero && cp == 0.0) ? v : cp * (*cptr) + v;
+        }
     }
 }
 
@@ -332,6 +368,7 @@ struct alignas(16) RowsUnit {
     const double *X;       // the operand at this batch index (and at the first row, when sr)
     __nv_bfloat16 *planes; // the first row's leading digits
     int *rexp;             // the rows' exponents
+    unsigned long long *magnitudes; // FP64 form: the operand's sum over all rows (TcGemmParams)
     int64_t sr, sk;        // strides of the rows and of k, 0: the tables at rtab (first row), ktab
     int64_t rtab, ktab;
     int64_t pitch, pstride;
@@ -406,6 +443,8 @@ __global__ void __launch_bounds__(kGThreads, 3) k_grouped_rows(const RowsUnit *u
         // one after the other, so that rows of few k keep all lanes busy
         __nv_bfloat16 *const planes = g.planes;
         int *const rexp = g.rexp;
+        unsigned long long *const magnitudes = g.magnitudes;
+        float leading = 0.0f; // whole numbers below 2^24
         for (int r = warp; r < nr; r += kGWarps) {
             const int e = split::row_exponent(split::row_max_bits(tile + r * ld, kw, lane));
             if (lane == 0) ex[r] = rexp[r] = e;
@@ -430,6 +469,7 @@ __global__ void __launch_bounds__(kGThreads, 3) k_grouped_rows(const RowsUnit *u
                 }
             }
             if constexpr (CHECK) {
+                leading += split::pair_sum(p0[S]) + split::pair_sum(p1[S]);
                 p0[S + 1] = split::check_mark(v0.x, v0.y);
                 p1[S + 1] = split::check_mark(v1.x, v1.y);
             }
@@ -442,6 +482,10 @@ __global__ void __launch_bounds__(kGThreads, 3) k_grouped_rows(const RowsUnit *u
                 k -= quads;
                 r++;
             }
+        }
+        if constexpr (CHECK) {
+            const unsigned sum = __reduce_add_sync(0xffffffffu, (unsigned)leading);
+            if (lane == 0) atomicAdd(magnitudes, (unsigned long long)sum);
         }
         __syncthreads(); // the tile is read before the loads of the unit after next replace it
         buf ^= 1;
@@ -570,6 +614,8 @@ F64Item f64_item(const Contraction &c) {
     it.k = c.k;
     it.a_kfast = c.k.n > 0 && c.k.s[0][c.k.n - 1] == 1 && !(c.m.n > 0 && c.m.s[0][c.m.n - 1] == 1);
     it.b_kfast = c.k.n > 0 && c.k.s[1][c.k.n - 1] == 1 && !(c.n.n > 0 && c.n.s[1][c.n.n - 1] == 1);
+    it.ka = mode_group_affine_stride(c.k, 0);
+    it.kb = mode_group_affine_stride(c.k, 1);
     return it;
 }
 
@@ -803,6 +849,7 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
         it.bg = c.batch;
         it.mg = c.m;
         it.ng = c.n;
+        it.tried = kTriedMean * (float)nb * (float)nb * (float)M * (float)N * (float)K * (float)K;
         items.push_back(it);
         for (int64_t bb = 0; bb < nb; bb++)
             for (int64_t x = 0; x < Mp / kBM; x++)
@@ -883,6 +930,12 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
     EG_CUDA(cudaMemsetAsync(eA, 0, (size_t)rowsA * 4, s));
     EG_CUDA(cudaMemsetAsync(eB, 0, (size_t)rowsB * 4, s));
     if ((st = dev_copy(plan, ops.data(), ops.size() * sizeof(GOp), &d_ops)) != EG_SUCCESS) return st;
+    // FP64 form, cleared by every replay: the counts of the blocks left out and of their tiles
+    // handed out, and from byte 16 on two sums an item
+    void *redo_count = nullptr;
+    const size_t counts = 16 + items.size() * 16;
+    if (f64 && (st = dev_alloc(plan, counts, &redo_count)) != EG_SUCCESS) return st;
+    unsigned long long *magnitudes = f64 ? (unsigned long long *)redo_count + 2 : nullptr;
     if (by_rows) {
         std::vector<RowsUnit> rows;
         rows.reserve(units.size());
@@ -895,6 +948,7 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
             x.X = g.X + pick(g.comp, oa, ob) + (g.sr ? r0 * g.sr : 0);
             x.planes = (__nv_bfloat16 *)(g.comp ? planesB : planesA) + g.plane0 + u.y * P * g.pstride + r0 * g.pitch;
             x.rexp = (int *)(g.comp ? eB : eA) + g.rowbase + u.y * g.Rp + r0;
+            if (f64) x.magnitudes = magnitudes + (size_t)u.x % items.size() * 2 + (g.comp ? 1 : 0);
             x.sr = g.sr;
             x.sk = g.sk;
             x.rtab = g.rtab + r0;
@@ -978,23 +1032,23 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
 
     if ((st = ensure_tc_attributes()) != EG_SUCCESS) return st;
     if (by_rows) EG_CUDA(allow_grouped_rows(S, f64));
-    void *d_fma = nullptr, *redo = nullptr, *redo_count = nullptr;
+    void *d_fma = nullptr, *redo = nullptr;
     if (f64) {
         std::vector<F64Item> fma;
         for (auto &c : cs) fma.push_back(f64_item(c));
         if ((st = dev_copy(plan, fma.data(), fma.size() * sizeof(F64Item), &d_fma)) != EG_SUCCESS) return st;
         if ((st = dev_alloc(plan, wl.size() * kTileRegions * sizeof(int4), &redo)) != EG_SUCCESS) return st;
-        if ((st = dev_alloc(plan, sizeof(int), &redo_count)) != EG_SUCCESS) return st;
         p.hid = kF64High;
         p.redo = (int4 *)redo;
         p.redo_count = (int *)redo_count;
+        p.magnitudes = magnitudes;
     }
     EG_CUDA(cudaEventCreateWithFlags(&plan.last, cudaEventDisableTiming));
     EG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     {
         CaptureGuard g;
         auto issue = [&]() -> eg_status {
-            if (f64) EG_CUDA(cudaMemsetAsync(redo_count, 0, sizeof(int), s));
+            if (f64) EG_CUDA(cudaMemsetAsync(redo_count, 0, counts, s));
             eg_status is =
                 by_rows ? launch_grouped_rows(S, f64, (const RowsUnit *)d_units, (int)units.size(),
                                               (const long long *)d_offs, rows_smem, s)
@@ -1004,8 +1058,8 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
             if (is != EG_SUCCESS) return is;
             is = launch_tc_gemm_grouped(maps[0], maps[1], p, (TcItem *)d_items, (int4 *)d_work, grid, s);
             if (is != EG_SUCCESS || !f64) return is;
-            k_grouped_f64_listed<<<num_sms() * 4, THREADS, 0, s>>>((const F64Item *)d_fma, (const int4 *)redo,
-                                                                   (const int *)redo_count, c0.cp, c0.ab, p.zero);
+            k_grouped_f64_listed<<<num_sms() * 8, f64::kThreads, 0, s>>>((const F64Item *)d_fma, (const int4 *)redo,
+                                                                   (int *)redo_count, c0.cp, c0.ab, p.zero);
             EG_CHECK_LAUNCH("k_grouped_f64_listed");
             return EG_SUCCESS;
         };

@@ -20,6 +20,7 @@
 #include <utility>
 
 #include "common.cuh"
+#include "f64_tile.cuh"
 #include "ptx.cuh"
 
 namespace eg {
@@ -445,30 +446,7 @@ __global__ void k_k_offsets(ModeGroup k, int64_t *out) {
 // (the call's host side), complex 300x170x257 (four launches) 1404 -> 156 us,
 // 144x2304x2304 2.93 -> 1.31 ms, 2304^3 21.7 -> 20.1 ms (1.22 TFLOP/s, 97 % of
 // the pipe).
-constexpr int kThreads = 256, kStages = 3;
-
-template <int T>
-struct F64Tile {
-    static constexpr int R = T == 32 ? 2 : 1;
-    static constexpr int KG = kThreads / ((T / R) * (T / R));
-    static constexpr int BK = T == 32 ? 16 : 32;
-    static constexpr int LD = T + 1;
-    static constexpr int PER = T * BK / kThreads; // elements a thread loads per operand and chunk
-};
-
-// How a k index becomes an element offset of one operand: a single stride when
-// the group's modes nest in it, else the decomposition over the modes.
-__device__ __forceinline__ int64_t k_offset(const ModeGroup &kg, int64_t stride, int comp, uint32_t k) {
-    if (stride) return (int64_t)k * stride;
-    int64_t oa, ob, oc;
-    group_offsets32(kg, k, oa, ob, oc);
-    return comp ? ob : oa;
-}
-
-__device__ __forceinline__ void copy_async8(double *dst, const double *src, bool valid) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
-}
+using f64::kThreads;
 
 struct F64Args {
     ModeGroup bg, mg, ng, kg;
@@ -490,11 +468,10 @@ struct F64Args {
 };
 
 template <int T>
-__global__ void __launch_bounds__(kThreads) k_contract_f64(const __grid_constant__ F64Args p) {
-    using Q = F64Tile<T>;
-    constexpr int R = Q::R, KG = Q::KG, BK = Q::BK, LD = Q::LD, PER = Q::PER, W = T / R;
-    __shared__ double As[kStages][BK][LD];
-    __shared__ double Bs[kStages][BK][LD];
+__global__ void __launch_bounds__(kThreads, T == 32 ? 4 : 3) k_contract_f64(const __grid_constant__ F64Args p) {
+    using Q = f64::Tile<T>;
+    constexpr int R = Q::R, KG = Q::KG, BK = Q::BK, W = T / R;
+    __shared__ f64::Buffers<T> chunk;
     __shared__ double part[T * T];
     const int tid = threadIdx.x;
     const int kgrp = tid / (W * W), tx = tid % W, ty = (tid / W) % W;
@@ -525,66 +502,15 @@ __global__ void __launch_bounds__(kThreads) k_contract_f64(const __grid_constant
         }
         int64_t ba, bb, bc;
         group_offsets(p.bg, b, ba, bb, bc);
-        int am[PER], ak[PER], bn[PER], bk[PER];
-        const double *pa[PER], *pb[PER];
-        bool oka[PER], okb[PER];
-#pragma unroll
-        for (int i = 0; i < PER; i++) {
-            const int e = tid + kThreads * i;
-            am[i] = p.a_kfast ? e / BK : e % T;
-            ak[i] = p.a_kfast ? e % BK : e / T;
-            bn[i] = p.b_kfast ? e / BK : e % T;
-            bk[i] = p.b_kfast ? e % BK : e / T;
-            int64_t oa, ob, oc;
-            oka[i] = m0 + am[i] < M;
-            group_offsets32(p.mg, (uint32_t)(oka[i] ? m0 + am[i] : 0), oa, ob, oc);
-            pa[i] = p.A + ba + oa;
-            const int64_t n = n0 + bn[i] + (bn[i] & gap);
-            okb[i] = n < N;
-            group_offsets32(p.ng, (uint32_t)(okb[i] ? n : 0), oa, ob, oc);
-            pb[i] = p.B + bb + ob;
-        }
-        auto load = [&](int c) {
-            if (c < cend) {
-                const int slot = (c - cbeg) % kStages;
-#pragma unroll
-                for (int i = 0; i < PER; i++) {
-                    const int64_t ka = (int64_t)c * BK + ak[i], kb = (int64_t)c * BK + bk[i];
-                    const bool va = oka[i] && ka < K, vb = okb[i] && kb < K;
-                    copy_async8(&As[slot][ak[i]][am[i]], va ? pa[i] + k_offset(p.kg, p.ka, 0, (uint32_t)ka) : p.A, va);
-                    copy_async8(&Bs[slot][bk[i]][bn[i]], vb ? pb[i] + k_offset(p.kg, p.kb, 1, (uint32_t)kb) : p.B, vb);
-                }
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
         double acc[R][R] = {};
-        load(cbeg);
-        load(cbeg + 1);
-        for (int c = cbeg; c < cend; c++) {
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-            __syncthreads(); // chunk c has landed for every thread, and chunk c - 1 is read
-            load(c + 2);
-            const int slot = (c - cbeg) % kStages;
-#pragma unroll 8
-            for (int kk = kgrp; kk < BK; kk += KG) {
-                double a[R], v[R];
-#pragma unroll
-                for (int i = 0; i < R; i++) a[i] = As[slot][kk][ty + W * i];
-#pragma unroll
-                for (int j = 0; j < R; j++) v[j] = Bs[slot][kk][tx + W * j];
-#pragma unroll
-                for (int i = 0; i < R; i++)
-#pragma unroll
-                    for (int j = 0; j < R; j++) acc[i][j] = fma(a[i], v[j], acc[i][j]);
-            }
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        f64::accumulate<T>(chunk, {p.mg, p.ng, p.kg, p.A + ba, p.B + bb, p.a_kfast, p.b_kfast, p.ka, p.kb}, m0, n0, gap,
+                           cbeg, cend, acc);
         // the k groups of the CTA, then the CTAs of the cluster, added in order
         const bool reduce = KG > 1 || p.cs > 1;
         if (KG > 1) {
             static_assert(KG == 1 || (R == 1 && KG * T * T == kThreads), "one output per thread and k group");
-            double *buf = &As[0][0][0]; // KG * T * T doubles fit one slot's space
-            static_assert(KG == 1 || KG * T * T <= kStages * BK * LD, "reduction buffer");
+            double *buf = &chunk.A[0][0][0];
+            static_assert(KG == 1 || sizeof(chunk.A) >= KG * T * T * sizeof(double), "reduction buffer");
             __syncthreads();
             buf[tid] = acc[0][0];
             __syncthreads();

@@ -37,6 +37,7 @@ constexpr int kF64Slices = 8, kF64High = 4;
 // The check of one output over its N products that are not zero, M the sum of their leading
 // magnitudes' products (p_a p_b): it passes when N = 0, or N >= 8 and M >= 20 N, or N >= 2 and
 // M >= 20 N + 256.  A product that stands alone is left to the FMA kernel, which rounds it once.
+constexpr float kTriedMean = 32.0f; // of p_a p_b over an item of a list, see left_out in tc_gemm.cu
 constexpr int kCheckPer = 20, kCheckFew = 8, kCheckMore = 256;
 __host__ __device__ constexpr bool check_fails(int products, int excess) { // excess: M - 20 N
     return products == 1 || (products > 1 && excess < (products < kCheckFew ? kCheckMore : 0));
@@ -108,6 +109,9 @@ struct TcGemmParams {
     // past M (N) and K blocks past K with zeros instead of reading the padding.
     const CUtensorMap *item_maps;
     const int *ranges; // each CTA's work entries
+    // Grouped launches, FP64 form: the sums of the leading magnitudes (p_a of the check) over all
+    // of A and all of B of every item, [item][2].
+    const unsigned long long *magnitudes;
 };
 
 // One item of a grouped launch: an independent contraction whose digit planes have
@@ -117,6 +121,7 @@ struct TcItem {
     double *C;
     int64_t M, N;
     int nkb;
+    float tried; // the product of its two magnitudes from which on the item is tried (left_out)
     int eAoff, eBoff;
     int Mp, Np;
     ModeGroup bg, mg, ng;
@@ -306,6 +311,9 @@ __device__ __forceinline__ uint32_t check_magnitude(uint32_t lead) {
     const float f0 = fmaxf(fabsf(__uint_as_float(lead << 16)) - 1.0f, 0.0f);
     const float f1 = fmaxf(fabsf(__uint_as_float(lead & 0xFFFF0000u)) - 1.0f, 0.0f);
     return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
+}
+__device__ __forceinline__ float pair_sum(uint32_t pair) { // of BF16 numbers
+    return __uint_as_float(pair << 16) + __uint_as_float(pair & 0xFFFF0000u);
 }
 __device__ __forceinline__ uint32_t check_mark(double x0, double x1) {
     return (abs_bits(x0) ? 0x3F80u : 0u) | (abs_bits(x1) ? 0x3F800000u : 0u);

@@ -211,6 +211,22 @@ __device__ __forceinline__ int entry_nkb(const TcGemmParams &p, const TcItem *it
     return min(p.kslice, p.nkb - kbeg);
 }
 
+// Lists, FP64 form: whether entry t's item is left to the FMA kernel without being tried.  The
+// splitting kernel adds up the check's magnitudes over each operand; where their means multiply
+// to less than 32, outputs with 20 N are few or none, and the FMA kernel would have to compute
+// (nearly) all of the item after the tensor cores did.  The kernel before wrote the sums, so
+// all roles decide alike.  (It saves such a list the 160 us that the tensor kernel takes for 512
+// uneven items, and costs an ordinary one 4.)
+template <bool GROUPED, bool F64>
+__device__ __forceinline__ bool left_out(const TcGemmParams &p, const TcItem *items, const int4 *work, int t) {
+    if constexpr (GROUPED && F64) {
+        const int i = work[t].x;
+        const ulonglong2 s = __ldg((const ulonglong2 *)p.magnitudes + i);
+        return (float)s.x * (float)s.y < items[i].tried;
+    }
+    return false;
+}
+
 // The FP64 value of one output's exact sums, scaled (but for an ab that is no power of
 // two), before C is added.  FAST: every
 // exponent of the tile lies where the result is a normal number (pend_fast).
@@ -320,6 +336,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             const uint32_t full0 = CL == 2 ? full_lead : ptx::smem_u32(full);
             for (int tile = cta0; tile < total_tiles && ok; tile += ctas) {
                 const TileJob job = resolve<GROUPED, CL>(p, items, work, tile, rank);
+                if (left_out<GROUPED, F64>(p, items, work, tile)) continue;
                 const int row0 = (isB ? job.nt : job.mt) * kBM, z0 = isB ? job.zB : job.zA;
                 const int kc0 = (p.kb0 + job.kbeg) * kBK, nkb = job.nkb;
                 const void *map = isB ? &tmB : &tmA;
@@ -415,6 +432,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             };
             for (int tile = cta0; tile < total_tiles && ok; tile += ctas) {
                 const int nkb = entry_nkb<GROUPED>(p, items, work, tile);
+                if (left_out<GROUPED, F64>(p, items, work, tile)) continue;
                 for (int q = qbeg; q < qend && ok; q++) {
                     const Step st = step_of(p, q);
                     int c = 0; // K blocks in the open chunk
@@ -576,7 +594,8 @@ __global__ void __launch_bounds__(THREADS, 1)
             long long H[kCols];
 #pragma unroll
             for (int i = 0; i < kCols; i++) H[i] = 0;
-            int q = drain ? qend : qbeg, kb = 0;
+            const bool untried = !drain && left_out<GROUPED, F64>(p, items, work, tile);
+            int q = drain || untried ? qend : qbeg, kb = 0;
             Step st = step_of(p, q);
             while (true) {
                 const bool last = q == qend;
@@ -751,6 +770,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             pend_done = pend_cols = 0;
             const TileJob job = resolve<GROUPED, CL>(p, items, work, tile, rank);
             if (!GROUPED && job.part == -2) continue; // the odd half of a pair's last row of tiles
+            if (untried) {
+                if (live > 0 && lane == 0) p.redo[atomicAdd(p.redo_count, 1)] = make_int4(job.item, job.b, job.mt * kBM + quad * 32, job.nt * kBN + half * 16);
+                continue;
+            }
             const bool slice = !GROUPED && job.part >= 0; // k_tc_finish_slices adds it up
             long long *const sums = slice ? part_of(tile) : rbc;
 #pragma unroll

@@ -79,3 +79,59 @@ def test_narrow_outputs(eg, m, n, k):
     assert set(plain) == {"k_contract_f64"}
     # the listed blocks are all of the output, in tiles of as many outputs: a fifth more for their order
     assert times["k_contract_f64_listed"] <= 1.2 * plain["k_contract_f64"]
+
+
+def replay_us(plan):
+    times = []
+    for _ in range(9):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        plan.execute()
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b) * 1e3)
+    return sorted(times)[4]
+
+
+def test_lists(eg):
+    """An uneven list: all graded, every second item, and magnitudes that are worth a try but fail."""
+    from einsums_gb300 import _lib, workloads
+    lib = _lib.load()
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    normal = lambda *s: torch.randn(s, generator=gen, dtype=torch.float64, device="cuda")
+    shapes = workloads.batched_shapes(512, seed=5)
+    used = ctypes.c_size_t()
+    for kind in ("graded", "half", "apart"):
+        As, Bs = [], []
+        for q, (i, j, a, b) in enumerate(shapes):
+            A, B = normal(i, j, a), normal(i, j, b)
+            if kind == "apart":  # two fifths of the summed indices each, elements of the other 1e-5
+                at = torch.arange(i * j, device="cuda").view(i, j, 1) * 5 // (i * j)
+                A, B = torch.where(at < 2, A, A * 1e-5), torch.where(at > 2, B, B * 1e-5)
+            elif kind == "graded" or q % 2:
+                d = 10.0 ** torch.linspace(-9, 9, i * j, dtype=torch.float64, device="cuda").view(i, j, 1)
+                A, B = A * d, B / d
+            As.append(A.contiguous()), Bs.append(B.contiguous())
+        Cs = [torch.full((a, b), float("nan"), dtype=torch.float64, device="cuda") for i, j, a, b in shapes]
+        plan = eg.GroupedPlan(0.0, "ab", Cs, 1.0, "ija", As, "ijb", Bs)
+        plan.execute()
+        torch.cuda.synchronize()
+        for q in range(0, 512, 3):
+            i, j, a, b = shapes[q]
+            x, y = As[q].reshape(i * j, a).cpu().numpy(), Bs[q].reshape(i * j, b).cpu().numpy()
+            want = (x.T.astype(np.longdouble) @ y.astype(np.longdouble)).astype(float)
+            assert np.all(np.abs(Cs[q].cpu().numpy() - want) <= (i * j + 4) * U * (np.abs(x.T) @ np.abs(y))), (kind, q)
+        ours = replay_us(plan)
+        plan.close()
+        _lib.check(lib.eg_memory_in_use(ctypes.byref(used)))
+        try:
+            _lib.check(lib.eg_set_memory_budget(used.value + (16 << 20)))
+            plan = eg.GroupedPlan(0.0, "ab", Cs, 1.0, "ija", As, "ijb", Bs)
+            plain = replay_us(plan)
+            plan.close()
+        finally:
+            _lib.check(lib.eg_set_memory_budget(0))
+        if kind != "apart":
+            assert ours <= 1.1 * plain, (kind, ours, plain)
+        print(kind, ours, plain)
