@@ -129,6 +129,13 @@ eg_status run_plan(Plan &plan, cudaStream_t stream) {
     if (ordered) {
         lk = std::unique_lock<std::mutex>(plan.mu);
         EG_CUDA(cudaStreamWaitEvent(stream, plan.last, 0));
+        int *status = nullptr;
+        if (eg::status_word(stream, &status) != EG_SUCCESS)
+            eg::set_error(""); // the word before stays
+        else if (status != plan.status_on) {
+            EG_CUDA(cudaMemcpyAsync(plan.status_at, &status, sizeof status, cudaMemcpyHostToDevice, stream));
+            plan.status_on = status;
+        }
     }
     cudaError_t err = cudaGraphLaunch(plan.exec, stream);
     if (err != cudaSuccess) return eg::cuda_fail(err, "cudaGraphLaunch");

@@ -151,6 +151,9 @@ class ScratchLease {
 // reads and clears it.
 eg_status status_word(cudaStream_t stream, int **ptr);
 
+// Self-test: sets *lost as eg_selftest_lose_next asked this thread's next call to.
+eg_status inject_lost(int *lost, cudaStream_t s);
+
 // Device memory accounting used by eg_device_alloc and the workspace.
 eg_status tracked_malloc(size_t bytes, void **ptr);
 eg_status tracked_free(void *ptr);
@@ -184,9 +187,12 @@ eg_status launch_scale(const ModeGroup &g, double *C, double cp, cudaStream_t s)
 eg_status launch_dot(const Contraction &c, cudaStream_t s);
 eg_status launch_gemv(const Contraction &c, cudaStream_t s);
 eg_status launch_contract_f64(const Contraction &c, cudaStream_t s);
-// The blocks of outputs listed at `list` ({batch, row, column}), *count of them: 32 rows by
-// the 16 columns from `column` and from 32, 64 and 96 further on.
-eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, const int *count, cudaStream_t s);
+// The blocks of outputs listed at `list` ({batch, row, column}), count[0] of them: 32 rows by
+// the 16 columns from `column` and from 32, 64 and 96 further on; count[2], zero before,
+// numbers the tiles handed out.  Where count[1] is set, the tensor kernel before gave up: all
+// of C becomes NaN, and count[1] goes to *status.
+constexpr int kListWords = 3;
+eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, int *count, int *status, cudaStream_t s);
 double contract_f64_seconds(const Contraction &c); // its estimated time
 bool f64_tensor_pays(const Contraction &c);
 // `front` bytes of the scratch are the caller's: fill(c, them) issues what writes them and

@@ -163,6 +163,25 @@ __global__ void __launch_bounds__(THREADS) k_grouped_f64(const F64Item *items, c
     }
 }
 
+// All outputs of all items (work: {item, batch index, mt, nt} of every 128 x 128 tile): what the
+// tensor kernel did not finish must not pass for results.
+__device__ __noinline__ void fill_nan(const F64Item *items, const int4 *work, int nwork, int *const *status_at, int lost) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) split::report_lost(status_at, nullptr, lost);
+    for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
+        const int4 e = work[w];
+        const F64Item &it = items[e.x];
+        const int64_t m0 = (int64_t)e.z * split::kBM, n0 = (int64_t)e.w * split::kBN;
+        const int64_t rows = min((int64_t)split::kBM, it.m.total - m0), cols = min((int64_t)split::kBN, it.n.total - n0);
+        int64_t oa, ob, oc, om, on;
+        group_offsets(it.b, e.y, oa, ob, oc);
+        for (int64_t i = threadIdx.x; i < rows * cols; i += blockDim.x) {
+            group_offsets(it.m, m0 + i / cols, oa, ob, om);
+            group_offsets(it.n, n0 + i % cols, oa, ob, on);
+            it.C[oc + om + on] = __longlong_as_double(0x7ff8000000000000ll);
+        }
+    }
+}
+
 // The blocks of outputs that the FP64 form on the tensor cores left out, *count of them:
 // {item, batch index, row, column}, 32 rows by the 16 columns from `column` and from 32,
 // 64 and 96 further on.  A list that fails the check everywhere must not take longer than
@@ -172,12 +191,15 @@ __global__ void __launch_bounds__(THREADS) k_grouped_f64(const F64Item *items, c
 // graded: 876 us in all, in tiles of 32 x 32 dealt in turn 2691; as a plan for the FP64 pipe
 // 825 to 940.  2048 items: 2.97 ms, 8.11, 3.28.
 __global__ void __launch_bounds__(f64::kThreads) k_grouped_f64_listed(const F64Item *items, const int4 *list, int *count,
-                                                                      double cp, double ab, int zero) {
+                                                                      double cp, double ab, int zero,
+                                                                      int *const *status_at, const int4 *work, int nwork) {
     constexpr int T = 16;
     __shared__ f64::Buffers<T> chunk;
     __shared__ uint32_t next;
     const int tx = threadIdx.x % T, ty = threadIdx.x / T;
     const uint32_t listed = (uint32_t)__ldg(count), total = 8 * listed;
+    const int lost = __ldg(count + 2);
+    if (lost) return fill_nan(items, work, nwork, status_at, lost);
     uint32_t fetched = blockIdx.x;
     while (true) {
         if (threadIdx.x == 0) {
@@ -930,11 +952,11 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
     EG_CUDA(cudaMemsetAsync(eA, 0, (size_t)rowsA * 4, s));
     EG_CUDA(cudaMemsetAsync(eB, 0, (size_t)rowsB * 4, s));
     if ((st = dev_copy(plan, ops.data(), ops.size() * sizeof(GOp), &d_ops)) != EG_SUCCESS) return st;
-    // FP64 form, cleared by every replay: the counts of the blocks left out and of their tiles
-    // handed out, and from byte 16 on two sums an item
+    // cleared by every replay: the counts of the blocks left out and of their tiles handed out,
+    // the record of a wait that gave up, and in the FP64 form from byte 16 on two sums an item
     void *redo_count = nullptr;
-    const size_t counts = 16 + items.size() * 16;
-    if (f64 && (st = dev_alloc(plan, counts, &redo_count)) != EG_SUCCESS) return st;
+    const size_t counts = 16 + (f64 ? items.size() * 16 : 0);
+    if ((st = dev_alloc(plan, counts, &redo_count)) != EG_SUCCESS) return st;
     unsigned long long *magnitudes = f64 ? (unsigned long long *)redo_count + 2 : nullptr;
     if (by_rows) {
         std::vector<RowsUnit> rows;
@@ -988,8 +1010,10 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
     }
     void *d_maps = nullptr;
     if ((st = dev_copy(plan, maps.data(), maps.size() * sizeof(CUtensorMap), &d_maps)) != EG_SUCCESS) return st;
-    int *status = nullptr;
-    if ((st = status_word(s, &status)) != EG_SUCCESS) return st;
+    if ((st = status_word(s, &plan.status_on)) != EG_SUCCESS) return st;
+    void *status_at = nullptr;
+    if ((st = dev_copy(plan, &plan.status_on, sizeof(int *), &status_at)) != EG_SUCCESS) return st;
+    plan.status_at = (int **)status_at;
 
     const Contraction &c0 = cs[0];
     TcGemmParams p{};
@@ -1009,7 +1033,8 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
         p.ab_neg = (p.ab_pow2 && c0.ab < 0) ? 1 : 0;
         if (p.ab_pow2) p.shift_const += k - 1;
     }
-    p.status = status;
+    p.status_at = plan.status_at;
+    p.lost = (int *)redo_count + 2;
     p.timeout_ns = 2000ull * 1000 * 1000;
     p.d0 = 0; // every slice group in one launch (K fits one exact pass)
     p.d1 = S;
@@ -1048,8 +1073,10 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
     {
         CaptureGuard g;
         auto issue = [&]() -> eg_status {
-            if (f64) EG_CUDA(cudaMemsetAsync(redo_count, 0, counts, s));
-            eg_status is =
+            EG_CUDA(cudaMemsetAsync(redo_count, 0, counts, s));
+            eg_status is = inject_lost(p.lost, s);
+            if (is != EG_SUCCESS) return is;
+            is =
                 by_rows ? launch_grouped_rows(S, f64, (const RowsUnit *)d_units, (int)units.size(),
                                               (const long long *)d_offs, rows_smem, s)
                         : launch_grouped_split(S, (const GOp *)d_ops, (const int4 *)d_units, (int)units.size(),
@@ -1059,7 +1086,8 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
             is = launch_tc_gemm_grouped(maps[0], maps[1], p, (TcItem *)d_items, (int4 *)d_work, grid, s);
             if (is != EG_SUCCESS || !f64) return is;
             k_grouped_f64_listed<<<num_sms() * 8, f64::kThreads, 0, s>>>((const F64Item *)d_fma, (const int4 *)redo,
-                                                                   (int *)redo_count, c0.cp, c0.ab, p.zero);
+                                                                   (int *)redo_count, c0.cp, c0.ab, p.zero, p.status_at,
+                                                                   (const int4 *)d_work, (int)wl.size());
             EG_CHECK_LAUNCH("k_grouped_f64_listed");
             return EG_SUCCESS;
         };

@@ -38,6 +38,9 @@ struct Plan {
     // plans with scratch of their own: a replay waits for the one before, on whatever stream
     std::mutex mu;
     cudaEvent_t last = nullptr;
+    // device copy of the address of the executing stream's status word, and that address
+    int **status_at = nullptr;
+    int *status_on = nullptr;
     ~Plan();
 };
 eg_status build_f64_plan(Plan &plan, const std::vector<Contraction> &cs, cudaStream_t s);

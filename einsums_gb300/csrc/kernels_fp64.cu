@@ -464,11 +464,27 @@ struct F64Args {
     // other some CTAs had only such ones (120000 x 75, K = 75, all listed: 2097 us, all
     // first parts first 1570).
     const int4 *list;
-    const int *count;
+    int *count; // entries, the record of a wait that gave up, tiles handed out
+    int *status;
 };
 
-template <int T>
-__global__ void __launch_bounds__(kThreads, T == 32 ? 4 : 3) k_contract_f64(const __grid_constant__ F64Args p) {
+// All of C, by all threads of the grid: outputs that the tensor kernel did not finish must not
+// pass for results.
+__device__ __forceinline__ void fill_nan(const F64Args &p) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(p.status, 0, p.count[1]);
+    const int64_t M = p.mg.total, N = p.ng.total, all = p.bg.total * M * N;
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < all; i += (int64_t)gridDim.x * kThreads) {
+        const int64_t q = i / N, b = q / M;
+        int64_t oa, ob, oc, om, on;
+        group_offsets(p.bg, b, oa, ob, oc);
+        group_offsets(p.mg, q - b * M, oa, ob, om);
+        group_offsets(p.ng, i - q * N, oa, ob, on);
+        p.C[oc + om + on] = __longlong_as_double(0x7ff8000000000000ll);
+    }
+}
+
+template <int T, bool LISTED>
+__global__ void __launch_bounds__(kThreads, T == 32 && !LISTED ? 4 : 3) k_contract_f64(const __grid_constant__ F64Args p) {
     using Q = f64::Tile<T>;
     constexpr int R = Q::R, KG = Q::KG, BK = Q::BK, W = T / R;
     __shared__ f64::Buffers<T> chunk;
@@ -481,19 +497,36 @@ __global__ void __launch_bounds__(kThreads, T == 32 ? 4 : 3) k_contract_f64(cons
     const int cbeg = (int)((int64_t)chunks * rank / p.cs), cend = (int)((int64_t)chunks * (rank + 1) / p.cs);
     const int64_t step = gridDim.x / p.cs;
     constexpr int ROWS = 32 / T, PARTS = ROWS * (64 / T); // of a listed block
-    const uint32_t listed = p.list ? (uint32_t)__ldg(p.count) : 0;
-    const int64_t total = p.list ? (int64_t)PARTS * listed : p.total;
-    const int gap = T == 32 && p.list ? 16 : 0; // tile column j is column j + (j & gap) from the tile's first
-    for (int64_t t = blockIdx.x / p.cs; t < total; t += step) {
+    const uint32_t listed = LISTED ? (uint32_t)__ldg(p.count) : 0;
+    if (LISTED && __ldg(p.count + 1)) return fill_nan(p);
+    const int64_t total = LISTED ? (int64_t)PARTS * listed : p.total;
+    constexpr int gap = LISTED && T == 32 ? 16 : 0; // tile column j is column j + (j & gap) from the tile's first
+    // listed tiles are handed out one by one (to clusters, in turn)
+    __shared__ uint32_t next;
+    const bool handed = LISTED && p.cs == 1;
+    uint32_t fetched = blockIdx.x;
+    for (int64_t t = blockIdx.x / p.cs;; t += step) {
+        if (handed) {
+            if (tid == 0) {
+                next = fetched;
+                fetched = gridDim.x + atomicAdd((unsigned *)p.count + 2, 1u); // the one after, while this one runs
+            }
+            __syncthreads(); // and the chunks of the tile before are read
+            t = next;
+        }
+        if (t >= total) break;
         int64_t b, m0, n0;
-        if (p.list) {
+        if (LISTED) {
             const uint32_t part = (uint32_t)t / listed; // all first parts, then the second ones, ...
             const int4 e = p.list[(uint32_t)t - part * listed];
             const int col = part / ROWS * T;
             b = e.x;
             m0 = e.y + part % ROWS * T;
             n0 = e.z + (T == 32 ? 2 * col : 2 * col - col % 16);
-            if (m0 >= M || n0 >= N) continue;
+            if (m0 >= M || n0 >= N) {
+                if (handed) __syncthreads();
+                continue;
+            }
         } else {
             const int64_t q = t / p.ntiles;
             b = q / p.mtiles;
@@ -561,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, T == 32 ? 4 : 3) k_contract_f64(cons
         }
         if (p.cs > 1)
             ptx::cluster_sync(); // the peers' sums are read; the next tile may overwrite them
-        else if (reduce || t + step < total)
+        else if (!handed && (reduce || t + step < total))
             __syncthreads();
     }
 }
@@ -595,11 +628,11 @@ double contract_plan(int64_t nb, int64_t M, int64_t N, int64_t K, int &T, int &c
     return best;
 }
 
-template <int T>
+template <int T, bool LISTED>
 cudaError_t launch_f64_tiles(const F64Args &p, cudaStream_t s) {
-    const int64_t clusters = p.list ? num_sms() * (T == 32 ? 4 : 8) / p.cs : std::min<int64_t>(p.total, int64_t(1) << 24);
+    const int64_t clusters = LISTED ? (p.cs == 1 ? 3 : 8) * num_sms() / p.cs : std::min<int64_t>(p.total, int64_t(1) << 24);
     if (p.cs == 1) {
-        k_contract_f64<T><<<(unsigned)clusters, kThreads, 0, s>>>(p);
+        k_contract_f64<T, LISTED><<<(unsigned)clusters, kThreads, 0, s>>>(p);
         return cudaGetLastError();
     }
     cudaLaunchConfig_t cfg = {};
@@ -613,11 +646,14 @@ cudaError_t launch_f64_tiles(const F64Args &p, cudaStream_t s) {
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_contract_f64<T>, p);
+    return cudaLaunchKernelEx(&cfg, k_contract_f64<T, LISTED>, p);
 }
 
+template <bool LISTED>
 cudaError_t launch_f64_tiles(const F64Args &p, int T, cudaStream_t s) {
-    return T == 32 ? launch_f64_tiles<32>(p, s) : T == 16 ? launch_f64_tiles<16>(p, s) : launch_f64_tiles<8>(p, s);
+    return T == 32   ? launch_f64_tiles<32, LISTED>(p, s)
+           : T == 16 ? launch_f64_tiles<16, LISTED>(p, s)
+                     : launch_f64_tiles<8, LISTED>(p, s);
 }
 
 ModeGroup concat(std::initializer_list<const ModeGroup *> groups) {
@@ -837,7 +873,7 @@ eg_status launch_contract_f64(const Contraction &c, cudaStream_t s) {
     if (p.total == 0) return EG_SUCCESS;
     {
         LaunchScope ls_("k_contract_f64", s);
-        const cudaError_t err = launch_f64_tiles(p, T, s);
+        const cudaError_t err = launch_f64_tiles<false>(p, T, s);
         if (err != cudaSuccess) return cuda_fail(err, "k_contract_f64");
     }
     EG_CHECK_LAUNCH("k_contract_f64");
@@ -849,20 +885,23 @@ double contract_f64_seconds(const Contraction &c) {
     return contract_plan(c.batch.total, c.m.total, c.n.total, c.k.total, T, cs) / 2.0e9;
 }
 
-eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, const int *count, cudaStream_t s) {
+eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, int *count, int *status,
+                                     cudaStream_t s) {
     // Tiles and K cut as if the whole output were listed, but for outputs of six rounds of
     // 32 x 32 tiles or more, where those are faster although the last round is not full
-    // (1024^3, all listed: 2.19 ms, 2.33 with 16 x 16).  Smaller ones: 300 x 300, K = 1000
-    // 591 -> 265 us in all, 128 x 128, K = 60000 17.0 -> 4.2 ms.
+    // (1024^3, all listed, dealt in turn: 2.19 ms, 2.33 with 16 x 16; handed out one by one
+    // 1.97).  Smaller ones: 300 x 300, K = 1000 591 -> 270 us in all, 128 x 128, K = 60000
+    // 17.0 -> 4.2 ms.
     F64Args p = f64_args(c);
     int T = 32;
     if (c.batch.total * ((c.m.total + 31) / 32) * ((c.n.total + 31) / 32) < 6 * num_sms())
         contract_plan(c.batch.total, c.m.total, c.n.total, c.k.total, T, p.cs);
     p.list = list;
     p.count = count;
+    p.status = status;
     {
         LaunchScope ls_("k_contract_f64_listed", s);
-        const cudaError_t err = launch_f64_tiles(p, T, s);
+        const cudaError_t err = launch_f64_tiles<true>(p, T, s);
         if (err != cudaSuccess) return cuda_fail(err, "k_contract_f64_listed");
     }
     EG_CHECK_LAUNCH("k_contract_f64_listed");

@@ -16,6 +16,7 @@ namespace eg {
 namespace {
 
 constexpr int kSelftestCode = 6;
+thread_local int g_lose_next = 0;
 
 __global__ void __launch_bounds__(64, 1) k_selftest_wait(int *status, unsigned long long limit_ns) {
     __shared__ __align__(8) uint64_t bar;
@@ -51,7 +52,21 @@ __global__ void __launch_bounds__(64, 1) k_selftest_wait(int *status, unsigned l
 }
 
 } // namespace
+
+eg_status inject_lost(int *lost, cudaStream_t s) {
+    if (g_lose_next == 0) return EG_SUCCESS;
+    EG_CUDA(cudaMemsetAsync(lost, g_lose_next, 1, s)); // (the other bytes are zero)
+    g_lose_next = 0;
+    return EG_SUCCESS;
+}
 } // namespace eg
+
+extern "C" eg_status eg_selftest_lose_next(int32_t code) {
+    eg::set_error("");
+    if (code < 0 || code > 127) return eg::fail(EG_ERROR_INVALID_ARGUMENT, "eg_selftest_lose_next: code must be in 0..127");
+    eg::g_lose_next = code;
+    return EG_SUCCESS;
+}
 
 extern "C" eg_status eg_selftest_wait_timeout(uint64_t limit_ns, void *stream) {
     eg::set_error("");

@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(kFusedThreads) k_split_rows(const __grid_const
     int *ex = (int *)(pmax + R);
     constexpr int W = kFusedThreads / 32, P = S + (CHECK ? 2 : 0);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (clear && blockIdx.x == 0 && tid == 0) *clear = 0; // a counter of the kernels that follow
+    if (clear && blockIdx.x == 0 && tid < kListWords) clear[tid] = 0; // words of the kernels that follow
     const int64_t id = blockIdx.x / C;
     const int rank = C > 1 ? (int)ptx::cluster_ctarank() : 0;
     const bool second = id >= ja.tiles;
@@ -613,7 +613,7 @@ int64_t plane_pitch(int64_t K) {
 }
 
 // Splits the operands of a contraction (an operand without rows is left out), and sets
-// *clear to zero (unless null).  The
+// the kListWords words at clear to zero (unless null).  The
 // fused launch when a range of K fits shared memory (K to about 25000); beyond, the
 // passes over each operand, with tables of offsets at tab (rows and K of each operand;
 // may be null).  Fused against passes, device time: both operands of 2304^3 in FP64
@@ -690,7 +690,7 @@ eg_status split_both(OperandMap oa, const double *A, int *eA, __nv_bfloat16 *pA,
         EG_CHECK_LAUNCH("k_split_rows");
         return EG_SUCCESS;
     }
-    if (clear) EG_CUDA(cudaMemsetAsync(clear, 0, sizeof(int), s));
+    if (clear) EG_CUDA(cudaMemsetAsync(clear, 0, kListWords * sizeof(int), s));
     unsigned long long *maxA = maxima, *maxB = maxima + (int64_t)oa.nbatch * oa.Rp;
     eg_status st;
     if (oa.rows && (st = split_operand(oa, A, maxA, eA, pA, S, s, tab, tab ? tab + oa.rows : nullptr, f64)) != EG_SUCCESS)
@@ -827,7 +827,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     const size_t offR = offEB + round_up(nb * Np * 4, 256);
     // offset tables (rows and k of each operand) unless they would be large
     const bool tables = M + K <= (int64_t(1) << 25) && N + K <= (int64_t(1) << 25);
-    const size_t offTab = offR + rbuf_bytes();
+    const size_t offLost = offR + rbuf_bytes(), offTab = offLost + 256;
     const size_t tabBytes = tables ? (size_t)(M + N + 2 * K) * 8 : 0;
     const int64_t tiles = nb * (Mp / kBM) * (Np / kBN);
     const size_t offRacc = round_up((int64_t)(offTab + tabBytes), 256);
@@ -846,13 +846,14 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     __nv_bfloat16 *planesA = (__nv_bfloat16 *)base, *planesB = (__nv_bfloat16 *)(base + offB);
     unsigned long long *maxA = (unsigned long long *)(base + offMaxA);
     int *eA = (int *)(base + offEA), *eB = (int *)(base + offEB);
-    int *status = nullptr;
+    int *status = nullptr, *lost = (int *)(base + offLost); // kListWords, the second this call's record
     if ((st = status_word(s, &status)) != EG_SUCCESS) return st;
 
     OperandMap oa{c.batch, c.m, c.k, 0, M, Mp, K, Kp, (int)nb};
     OperandMap ob{c.batch, c.n, c.k, 1, N, Np, K, Kp, (int)nb};
     int64_t *tab = tables ? (int64_t *)(base + offTab) : nullptr;
-    if ((st = split_both(oa, c.A, eA, planesA, ob, c.B, eB, planesB, maxA, tab, S, false, nullptr, s)) != EG_SUCCESS) return st;
+    if ((st = split_both(oa, c.A, eA, planesA, ob, c.B, eB, planesB, maxA, tab, S, false, lost, s)) != EG_SUCCESS) return st;
+    if ((st = inject_lost(lost + 1, s)) != EG_SUCCESS) return st;
 
     CUtensorMap tmA, tmB, tmBh;
     if ((st = encode_planes(&tmA, planesA, Kp, Mp, nb * S)) != EG_SUCCESS) return st;
@@ -878,6 +879,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
     p.shift_const = -2 * kTopBits - kBits * (S - 1);
     set_ab(p, c.ab);
     p.status = status;
+    p.lost = lost + 1;
     p.timeout_ns = 2000ull * 1000 * 1000;
     p.rbuf = (long long *)(base + offR);
     p.parts = (long long *)(base + offRacc);
@@ -1027,7 +1029,7 @@ eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
     const size_t oExp = take((size_t)bb * (mb + nbk) * 4);
     const size_t oTab = take(tables ? (size_t)(M + N + 2 * K) * 8 : 0);
     const size_t oR = take(rbuf_bytes(3));
-    const size_t oRedoN = take(sizeof(int)), oRedo = take((size_t)all_tiles * kTileRegions * sizeof(int4));
+    const size_t oRedoN = take(kListWords * sizeof(int)), oRedo = take((size_t)all_tiles * kTileRegions * sizeof(int4));
     ScratchLease lease(s, at);
     if (!lease.ptr()) return EG_ERROR_NOT_SUPPORTED;
     int *status = nullptr;
@@ -1062,7 +1064,8 @@ eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
     p.hid = kF64High;
     p.redo = (int4 *)(base + oRedo);
     p.redo_count = (int *)(base + oRedoN);
-    bool first = true; // the first splitting launch clears redo_count
+    p.lost = p.redo_count + 1;
+    bool first = true; // the first splitting launch clears redo_count and the record
 
     for (int64_t b0 = 0; b0 < nb; b0 += bb) {
         const int64_t nbc = std::min(bb, nb - b0);
@@ -1084,6 +1087,7 @@ eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
                 if ((st = split_both(oa, c.A, eA, planesA, ob, c.B, eB, planesB, (unsigned long long *)(base + oMax), tab,
                                      S, true, first ? p.redo_count : nullptr, s)) != EG_SUCCESS)
                     return st;
+                if (first && (st = inject_lost(p.lost, s)) != EG_SUCCESS) return st;
                 first = false;
                 CUtensorMap tmA, tmB, tmBh;
                 if ((st = encode_planes(&tmA, planesA, Kp, Mp, nbc * P)) != EG_SUCCESS) return st;
@@ -1103,7 +1107,7 @@ eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
             }
         }
     }
-    return launch_contract_f64_listed(c, p.redo, p.redo_count, s);
+    return launch_contract_f64_listed(c, p.redo, p.redo_count, status, s);
 }
 
 // Whether an FP64 contraction is worth its detour over the tensor cores, from

@@ -68,7 +68,12 @@ struct TcGemmParams {
     const int *eA; // [nbatch][Mp] row exponents; INT_MIN marks a non-finite row
     const int *eB; // [nbatch][Np]
     int shift_const; // -14 - 8 (S-1), plus k when ab = +-2^k
+    // Where a wait that gives up is recorded: the executing stream's word -- *status_at when set
+    // (lists, which do not know the stream before they run) -- and this call's own, which the
+    // launches that follow look at.
     int *status;
+    int *const *status_at;
+    int *lost;
     unsigned long long timeout_ns;
     // Optional per-CTA cycle counters (null in normal runs): see kProf* in tc_gemm.cu.
     unsigned long long *prof;
@@ -113,6 +118,11 @@ struct TcGemmParams {
     // of A and all of B of every item, [item][2].
     const unsigned long long *magnitudes;
 };
+
+// Records a wait that gave up in the executing stream's word.
+__device__ __forceinline__ void report_lost(int *const *status_at, int *status, int code) {
+    atomicCAS(status_at ? *status_at : status, 0, code);
+}
 
 // One item of a grouped launch: an independent contraction whose digit planes have
 // tensor maps of their own (TcGemmParams::item_maps) and whose exponents start at

@@ -18,8 +18,9 @@
 // Bound: the tensor pipe (64 clocks per 128 x 128 x 16 product and SM).  What kept
 // it idle before was the issue loop, not operand delivery (see the issuer).
 // Every mbarrier wait is bounded (split.cuh, ptx.cuh): on a timeout the CTA
-// records an error code in *status, raises its abort flag, waits for its own
-// TMA loads and MMAs to land, frees TMEM and returns.
+// records an error code (report_lost), raises its abort flag, waits for its own
+// TMA loads and MMAs to land, frees TMEM and returns.  The launches after it then
+// add up no slices, and in the FP64 form write NaN to all of C.
 #include <climits>
 #include <cstdlib>
 #include <mutex>
@@ -55,6 +56,7 @@ constexpr int kRegsIssue = 56, kRegsEpilogue = 224;
 static_assert(128 * kRegsIssue + 32 * kEpiWarps * kRegsEpilogue <= THREADS * 168, "registers of the launch");
 constexpr int GROUP_M = 16; // tile rasterisation: groups of 16 row tiles share B tiles in L2
 constexpr unsigned long long DRAIN_NS = 200ull * 1000 * 1000;
+constexpr unsigned long long ODD_DRAIN_NS = 10ull * 1000 * 1000; // longer than any load takes
 
 // Optional cycle counters per CTA (TcGemmParams::prof, 8 slots per CTA).
 enum { kProfProducerWaitEmpty, kProfMmaWaitFull, kProfMmaWaitAcc, kProfEpiWaitAcc, kProfEpiFlush, kProfEpiFinal,
@@ -242,7 +244,8 @@ __device__ __forceinline__ double finish_value(const TcGemmParams &p, long long 
 // (peer_flag: shared::cluster address of its abort flag, 0 without a peer).
 __device__ __forceinline__ void raise_abort(const TcGemmParams &p, volatile int *abort_flag, int code,
                                             uint32_t peer_flag = 0) {
-    atomicCAS(p.status, 0, code);
+    report_lost(p.status_at, p.status, code);
+    atomicCAS(p.lost, 0, code);
     *abort_flag = 1;
     if (peer_flag) ptx::st_cluster_u32(peer_flag, 1u);
 }
@@ -399,6 +402,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                 for (int i = 0; i < issued; i++)
                     if (!ptx::mbar_wait(&full[i], i < stage ? phase : phase ^ 1, DRAIN_NS, nullptr))
                         raise_abort(p, abort_flag, 4, peer_flag);
+            // An odd CTA that gives up may be slots ahead of the even one's count.
+            if (CL == 2 && rank != 0 && !ok && leader)
+                for (const uint64_t t0 = ptx::globaltimer_ns(); ptx::globaltimer_ns() - t0 < ODD_DRAIN_NS;) {}
             __syncwarp();
         } else if (warp == 1 && rank == 0) {
             // -------------------------------------------- MMA issuer (the even CTA of a pair)
@@ -864,6 +870,7 @@ __global__ void __launch_bounds__(32 * kFinishRows, 3) k_tc_finish_slices(const 
     const int live = min(cols / 32 * 16 + min(max(cols % 32 - half * 16, 0), 16) - c0, kFinishCols);
     if (rows <= 0 || live <= 0) return;
     const int e0 = q * p.ksplit * CL + rank; // the tile's first slice; the next ones are CL further on
+    const int lost = __ldcg(p.lost); // with a slice missing there is nothing to add up
     bool bad = false;
     if (F64) {
         // the region's check, over the slices, as in a whole tile (both of its CTAs see all of it)
@@ -928,8 +935,9 @@ __global__ void __launch_bounds__(32 * kFinishRows, 3) k_tc_finish_slices(const 
         const double v = finish_value<F64, false>(p, lo[i], hi[i], rowExp, colExp);
         tile[c][lane] = p.ab_pow2 ? v : p.ab * v;
     }
-    if (__syncthreads_or(bad)) { // the FMA kernel computes the region
-        if (threadIdx.x == 0 && c0 == 0)
+    if (__syncthreads_or(bad) || lost) { // the FMA kernel computes the region
+        if (lost && blockIdx.x == 0 && threadIdx.x == 0) report_lost(p.status_at, p.status, lost);
+        if (!lost && threadIdx.x == 0 && c0 == 0)
             p.redo[atomicAdd(p.redo_count, 1)] =
                 make_int4((int)p.b0 + b, (int)(p.m0 + m0), (int)(p.n0 + n0) + half * 16, 0);
         return;

@@ -260,11 +260,14 @@ eg_status eg_device_free(void *ptr);
 eg_status eg_set_memory_budget(size_t bytes);
 eg_status eg_memory_in_use(size_t *bytes);
 
-/* Error record of kernels with bounded device-side waits (the split form's tensor-core
- * pipeline) for work issued on `stream`: synchronises the stream, returns EG_ERROR_TIMEOUT
+/* Error record of kernels with bounded device-side waits (the tensor-core pipeline of
+ * the split form and of FP64) for work issued on `stream`: synchronises the stream, returns EG_ERROR_TIMEOUT
  * with the kernel's code in *device_code (may be NULL) when a wait gave up, and clears
  * the record.  Such a kernel returns early instead of hanging, leaving its outputs
- * incomplete; the context stays usable.  No reference counterpart (the reference's
+ * incomplete; the context stays usable.  An FP64 contraction that ran on the tensor
+ * cores (eg_einsum, eg_einsum_complex, lists) then holds NaN in all of C, so that it
+ * cannot be taken for a result by callers that do not ask.  For a list the record is
+ * that of the stream it was executed on.  No reference counterpart (the reference's
  * kernels have no bounded waits). */
 eg_status eg_stream_status(void *stream, int32_t *device_code);
 
@@ -274,6 +277,12 @@ eg_status eg_stream_status(void *stream, int32_t *device_code);
  * and returns -- the steps the tensor-core pipeline takes when one of its waits gives up.
  * No reference counterpart. */
 eg_status eg_selftest_wait_timeout(uint64_t limit_ns, void *stream);
+
+/* Self-test of what follows such a wait: the next contraction of this host thread that runs on
+ * the tensor cores, or every replay of the next list plan that it creates, goes on as if a wait
+ * of its tensor kernel had given up with `code` (1..127; 0 takes the request back).  The kernels
+ * themselves run undisturbed.  No reference counterpart. */
+eg_status eg_selftest_lose_next(int32_t code);
 
 /* Host<->device copies on `stream` (DeviceTensor::read / operator= in DeviceTensor.hpp). */
 eg_status eg_copy_to_device(void *dst, const void *src, size_t bytes, void *stream);
