@@ -54,15 +54,7 @@ eg_status cuda_fail(cudaError_t err, const char *what) {
     return err == cudaErrorMemoryAllocation ? EG_ERROR_OUT_OF_MEMORY : EG_ERROR_CUDA;
 }
 
-// Calls that may not run while a stream of any thread is being captured (in the
-// global capture mode) are made in the relaxed mode: they touch no captured stream.
 namespace {
-struct RelaxedCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
-
 eg_status malloc_once(size_t bytes, void **ptr) {
     std::lock_guard<std::mutex> lk(g_mem_mutex);
     if (g_budget && g_in_use + bytes > g_budget)
@@ -239,10 +231,22 @@ eg_status status_word(cudaStream_t stream, int **ptr) {
     }
     for (const WsKey &key : {shared_key, WsKey{dev, stream}}) {
         int *&w = g_status[key];
-        if (!w) {
-            EG_CUDA(cudaMalloc(&w, 256));
-            EG_CUDA(cudaMemset(w, 0, 256));
+        if (w) continue;
+        // (a stream of its own: the legacy one must not be used beside some captures)
+        RelaxedCapture relaxed;
+        cudaStream_t own = nullptr;
+        int *fresh = nullptr;
+        cudaError_t err = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
+        if (err == cudaSuccess) err = cudaMalloc(&fresh, 256);
+        if (err == cudaSuccess) err = cudaMemsetAsync(fresh, 0, 256, own);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(own);
+        if (own) cudaStreamDestroy(own);
+        if (err != cudaSuccess) {
+            if (fresh) cudaFree(fresh);
+            cudaGetLastError(); // leave no trace for later checks
+            return cuda_fail(err, "status word");
         }
+        w = fresh;
     }
     *ptr = g_status[WsKey{dev, stream}];
     return EG_SUCCESS;

@@ -146,6 +146,17 @@ class ScratchLease {
     void *ptr_ = nullptr;
 };
 
+// While it lives, calls of this thread that may not run while a stream of any thread is being
+// captured (in the global capture mode), such as allocations, may: for code that touches no
+// captured stream.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture &) = delete;
+    RelaxedCapture &operator=(const RelaxedCapture &) = delete;
+};
+
 // Device-side error word of kernels with bounded waits, one per (device,
 // stream); kernels set it with atomicCAS(ptr, 0, code) and eg_stream_status
 // reads and clears it.

@@ -979,7 +979,7 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
 //
 // The digit planes live in a scratch shared by the streams of the device and
 // bounded by kF64ScratchCap; larger operands are cut into panels of rows.  When
-// the scratch cannot be had (a memory budget, a full device) or the stream is
+// the scratch or the stream's status word cannot be had (a memory budget, a full device) or the stream is
 // being captured (a graph must not hold the scratch), EG_ERROR_NOT_SUPPORTED
 // comes back with nothing launched and the FMA kernel runs instead.
 constexpr size_t kF64ScratchCap = size_t(2) << 30;
@@ -993,6 +993,7 @@ eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     EG_CUDA(cudaStreamIsCapturing(s, &cap));
     if (cap != cudaStreamCaptureStatusNone) return EG_ERROR_NOT_SUPPORTED;
+    RelaxedCapture relaxed; // another thread's capture neither stops nor suffers from the scratch
     // panels: all rows of both operands when they fit, else whole 128-row blocks of
     // each (and, with batches, as many batch indices as fit)
     const int64_t row_bytes = P * Kp * 2 + 32, Mp_all = round_up(M, kBM), Np_all = round_up(N, kBN);
@@ -1034,7 +1035,10 @@ eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
     if (!lease.ptr()) return EG_ERROR_NOT_SUPPORTED;
     int *status = nullptr;
     eg_status st = status_word(s, &status);
-    if (st != EG_SUCCESS) return st;
+    if (st != EG_SUCCESS) {
+        set_error("");
+        return EG_ERROR_NOT_SUPPORTED;
+    }
     char *base = (char *)lease.ptr();
     if (fill && (st = fill(c, base + oFront)) != EG_SUCCESS) return st;
     __nv_bfloat16 *planesA = (__nv_bfloat16 *)(base + oPA), *planesB = (__nv_bfloat16 *)(base + oPB);
