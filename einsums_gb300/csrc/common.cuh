@@ -11,6 +11,7 @@
 #include <string>
 
 #include "../../include/einsums_gb300.h"
+#include "per_device.cuh"
 
 namespace eg {
 
@@ -168,6 +169,11 @@ eg_status inject_lost(int *lost, cudaStream_t s);
 // Device memory accounting used by eg_device_alloc and the workspace.
 eg_status tracked_malloc(size_t bytes, void **ptr);
 eg_status tracked_free(void *ptr);
+
+inline int current_device() {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess ? dev : 0;
+}
 
 inline int num_sms() {
     static int sms = [] {

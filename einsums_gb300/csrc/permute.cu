@@ -16,7 +16,6 @@
 // ap*A without reading C (a plain copy when ap == 1, so the copy is bit-exact),
 // otherwise ap*A + cp*C without fused multiply-adds.
 #include <algorithm>
-#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -500,9 +499,9 @@ eg_status launch_tma(const PermuteLaunch &pl, int grid, const CUtensorMap &mA, c
 }
 
 eg_status ensure_tma_attributes() {
-    static std::once_flag once;
-    static cudaError_t err = cudaSuccess;
-    std::call_once(once, [] {
+    static PerDevice<cudaError_t> attributes;
+    const cudaError_t err = attributes.get(current_device(), [] {
+        cudaError_t err = cudaSuccess;
         auto set = [&](const void *f) {
             if (err == cudaSuccess) err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kTmaSmem);
         };
@@ -514,6 +513,7 @@ eg_status ensure_tma_attributes() {
         set((const void *)k_permute_tma<3, 1>);
         set((const void *)k_permute_tma<4, 1>);
         set((const void *)k_permute_tma<5, 1>);
+        return err;
     });
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(k_permute_tma)");
     return EG_SUCCESS;
@@ -521,18 +521,15 @@ eg_status ensure_tma_attributes() {
 
 // Resident CTAs of the TMA permute per SM (its ring takes 65 KB of shared memory).
 int tma_blocks_per_sm() {
-    static std::once_flag once;
-    static int per_sm = 1;
-    std::call_once(once, [] {
+    static PerDevice<int> per_sm;
+    return per_sm.get(current_device(), [] {
         int n = 0;
-        if (ensure_tma_attributes() == EG_SUCCESS &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_permute_tma<4, 0>, kTmaThreads, kTmaSmem) ==
-                cudaSuccess &&
-            n > 0)
-            per_sm = n;
+        const bool known = ensure_tma_attributes() == EG_SUCCESS &&
+                           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_permute_tma<4, 0>, kTmaThreads, kTmaSmem) ==
+                               cudaSuccess;
         cudaGetLastError();
+        return known && n > 0 ? n : 1;
     });
-    return per_sm;
 }
 
 // Encodes the two maps for these pointers and launches; EG_ERROR_NOT_SUPPORTED

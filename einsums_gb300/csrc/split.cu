@@ -543,7 +543,8 @@ eg_status split_operand(OperandMap om, const double *X, unsigned long long *rowm
     EG_CUDA(cudaMemsetAsync(rowmax, 0, (size_t)om.nbatch * om.Rp * sizeof(unsigned long long), s));
     const int cap = num_sms() * 8;
     {
-        static const int resident = resident_grid(k_split_rowmax);
+        static PerDevice<int> grids;
+        const int resident = grids.get(current_device(), [] { return resident_grid(k_split_rowmax); });
         const int64_t unit_rows = r_fast ? kRowFastRows : T;
         const int64_t rows_units = (int64_t)om.nbatch * ((om.rows + unit_rows - 1) / unit_rows);
         const int kchunk = balanced_chunk(rows_units, om.K, resident, r_fast ? kRowFastBatch : T);
@@ -561,9 +562,9 @@ eg_status split_operand(OperandMap om, const double *X, unsigned long long *rowm
     EG_CHECK_LAUNCH("k_split_exponent");
     {
         const int64_t work = (int64_t)om.nbatch * (om.Rp / T) * ((om.Kp / TK + kDigitStrip - 1) / kDigitStrip);
-        static const int resident = resident_grid(k_split_digits<5, false>); // the S variants share a register budget
-        static const int resident_f64 = resident_grid(k_split_digits<kF64Slices, true>);
-        const int cta = f64 ? resident_f64 : resident;
+        static PerDevice<int> grids, grids_f64; // (the S variants share a register budget)
+        const int cta = f64 ? grids_f64.get(current_device(), [] { return resident_grid(k_split_digits<kF64Slices, true>); })
+                            : grids.get(current_device(), [] { return resident_grid(k_split_digits<5, false>); });
         const int grid = (int)(work < cta ? work : cta);
         LaunchScope ls_("k_split_digits", s);
         const int rf = r_fast ? 1 : 0;
@@ -584,8 +585,10 @@ eg_status split_operand(OperandMap om, const double *X, unsigned long long *rowm
 template <int S, bool CHECK, int R>
 cudaError_t launch_split_rows(const SplitJob &a, const SplitJob &b, int kc, int ld, int C, size_t smem, int *clear,
                               cudaStream_t s) {
-    static const cudaError_t attr = cudaFuncSetAttribute(k_split_rows<S, CHECK, R>,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    static PerDevice<cudaError_t> attributes;
+    const cudaError_t attr = attributes.get(current_device(), [] {
+        return cudaFuncSetAttribute(k_split_rows<S, CHECK, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    });
     if (attr != cudaSuccess) return attr;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((a.tiles + b.tiles) * C));

@@ -329,7 +329,7 @@ __device__ __forceinline__ uint32_t check_mark(double x0, double x1) {
     return (abs_bits(x0) ? 0x3F80u : 0u) | (abs_bits(x1) ? 0x3F800000u : 0u);
 }
 
-// Sets the kernels' shared-memory attribute once (call outside stream capture).
+// Sets the kernels' shared-memory attribute, once for a device (call outside stream capture).
 eg_status ensure_tc_attributes();
 // Clusters of two k_tc_split_gemm CTAs that fit on the GPU at once (0 when CTA pairs
 // are switched off with EINSUMS_GB300_TC_PAIRS=0), and whether they are asked for

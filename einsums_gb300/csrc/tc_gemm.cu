@@ -23,7 +23,6 @@
 // add up no slices, and in the FP64 form write NaN to all of C.
 #include <climits>
 #include <cstdlib>
-#include <mutex>
 
 #include "ptx.cuh"
 #include "split.cuh"
@@ -950,13 +949,14 @@ __global__ void __launch_bounds__(32 * kFinishRows, 3) k_tc_finish_slices(const 
 } // namespace
 
 eg_status ensure_tc_attributes() {
-    static std::once_flag once;
-    static cudaError_t err = cudaSuccess;
-    std::call_once(once, [] {
+    static PerDevice<cudaError_t> attributes;
+    const cudaError_t err = attributes.get(current_device(), [] {
+        cudaError_t err = cudaSuccess;
         for (const void *f : {(const void *)k_tc_split_gemm<false, 1, false>, (const void *)k_tc_split_gemm<true, 1, false>,
                               (const void *)k_tc_split_gemm<false, 2, false>, (const void *)k_tc_split_gemm<false, 1, true>,
                               (const void *)k_tc_split_gemm<false, 2, true>, (const void *)k_tc_split_gemm<true, 1, true>})
             if (err == cudaSuccess) err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        return err;
     });
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute(k_tc_split_gemm)");
     return EG_SUCCESS;
@@ -990,17 +990,16 @@ int pairs_wish() {
 } // namespace
 
 int tc_pair_clusters() {
-    static std::once_flag once;
-    static int n = 0;
-    std::call_once(once, [] {
-        if (pairs_wish() == 0 || ensure_tc_attributes() != EG_SUCCESS) return;
+    static PerDevice<int> clusters;
+    return clusters.get(current_device(), [] {
+        if (pairs_wish() == 0 || ensure_tc_attributes() != EG_SUCCESS) return 0;
         cudaLaunchAttribute attr;
         cudaLaunchConfig_t cfg = pair_config(num_sms(), nullptr, &attr);
         int c = 0;
-        if (cudaOccupancyMaxActiveClusters(&c, (void *)k_tc_split_gemm<false, 2, false>, &cfg) == cudaSuccess) n = c;
+        if (cudaOccupancyMaxActiveClusters(&c, (void *)k_tc_split_gemm<false, 2, false>, &cfg) != cudaSuccess) c = 0;
         cudaGetLastError();
+        return c;
     });
-    return n;
 }
 
 bool tc_pairs_forced() { return pairs_wish() == 1 && tc_pair_clusters() > 0; }
