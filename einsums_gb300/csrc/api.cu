@@ -3,6 +3,7 @@
 // and dispatch to the kernels.  No exception crosses this file's entry points.
 #include <algorithm>
 #include <cmath>
+#include <condition_variable>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -73,41 +74,124 @@ eg_status malloc_once(size_t bytes, void **ptr) {
 }
 } // namespace
 
-struct SharedScratch {
-    std::mutex mu; // held from a lease's start to its end
+// The scratch buffers of a device (ScratchLease).  Several, so that work waiting on one stream
+// does not hold up another: a call takes the buffer that its stream used last, else one whose
+// work is done, else a new one while all of them stay below kScratchTotal; only then does it
+// wait on the GPU for another stream's work.
+struct Scratch {
     void *ptr = nullptr;
     size_t bytes = 0;
     cudaEvent_t last = nullptr; // after the last lease's work
+    cudaStream_t stream = nullptr;
+    bool taken = false; // by a lease that has not ended
+    uint64_t turn = 0;
+};
+
+constexpr int kScratchBuffers = 8;
+constexpr size_t kScratchTotal = size_t(5) << 30, kScratchUnit = size_t(64) << 20;
+struct ScratchPool {
+    std::mutex mu;
+    std::condition_variable ended; // a lease
+    Scratch buffers[kScratchBuffers];
+    uint64_t turns = 0;
 };
 
 namespace {
 std::mutex &g_scratch_mutex = *new std::mutex;
-std::map<int, SharedScratch> &g_scratch = *new std::map<int, SharedScratch>;
+std::map<int, ScratchPool> &g_scratch = *new std::map<int, ScratchPool>;
 
-// Waits for the buffer's last user and frees it (its lock is held).
-void drop_scratch(SharedScratch &x) {
+bool done(const Scratch &x) { // the work of its last lease
+    if (!x.last) return true;
+    const cudaError_t err = cudaEventQuery(x.last);
+    if (err == cudaErrorNotReady) cudaGetLastError();
+    return err == cudaSuccess;
+}
+
+// Waits for the buffer's last user and frees it (not taken, its pool locked).
+void drop_scratch(Scratch &x) {
     if (!x.ptr) return;
     RelaxedCapture relaxed;
-    cudaEventSynchronize(x.last);
+    if (x.last) cudaEventSynchronize(x.last);
     tracked_free(x.ptr);
     x.ptr = nullptr;
     x.bytes = 0;
 }
 
-// Gives back every device's shared scratch; false when there was none.
+// Gives back every device's scratch; false when there was none.
 bool trim_scratch() {
-    std::vector<SharedScratch *> all;
+    std::vector<ScratchPool *> all;
     {
         std::lock_guard<std::mutex> lk(g_scratch_mutex);
         for (auto &kv : g_scratch) all.push_back(&kv.second);
     }
     bool any = false;
-    for (SharedScratch *x : all) {
-        std::lock_guard<std::mutex> lk(x->mu);
-        any |= x->ptr != nullptr;
-        drop_scratch(*x);
+    for (ScratchPool *p : all) {
+        std::unique_lock<std::mutex> lk(p->mu);
+        for (Scratch &x : p->buffers) {
+            p->ended.wait(lk, [&] { return !x.taken; });
+            any |= x.ptr != nullptr;
+            drop_scratch(x);
+        }
     }
     return any;
+}
+
+// Whether `want` bytes can be allocated once `back` bytes have been freed: under the memory
+// budget, and with a thirty-second of the device's memory left free.
+bool scratch_fits(size_t want, size_t back) {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b + back < want + total_b / 32) return false;
+    std::lock_guard<std::mutex> lk(g_mem_mutex);
+    return !g_budget || g_in_use + want <= g_budget + back;
+}
+
+// A buffer of at least `bytes` that is not taken (its pool locked), or null; `wait`: all that would
+// do are taken, and one may come back.
+Scratch *choose_scratch(ScratchPool &p, cudaStream_t s, size_t bytes, bool &wait) {
+    Scratch *own = nullptr, *idle = nullptr, *busy = nullptr, *empty = nullptr, *small = nullptr;
+    size_t held = 0;
+    wait = false;
+    for (Scratch &x : p.buffers) {
+        held += x.bytes;
+        if (x.taken) {
+            wait |= x.bytes >= bytes;
+        } else if (!x.ptr) {
+            empty = &x;
+        } else if (x.bytes < bytes) {
+            if (!small || (x.stream == s) > (small->stream == s) ||
+                ((x.stream == s) == (small->stream == s) && x.turn < small->turn))
+                small = &x;
+        } else if (x.stream == s) {
+            if (!own || x.bytes < own->bytes) own = &x;
+        } else if (done(x)) {
+            if (!idle || x.bytes < idle->bytes) idle = &x;
+        } else if (!busy || x.turn < busy->turn) {
+            busy = &x;
+        }
+    }
+    if (own) return own;
+    if (idle) return idle;
+    const size_t want = (bytes + kScratchUnit - 1) / kScratchUnit * kScratchUnit;
+    auto allocate = [&](Scratch &x) -> Scratch * {
+        if (malloc_once(want, &x.ptr) != EG_SUCCESS) {
+            set_error("");
+            return nullptr;
+        }
+        x.bytes = want;
+        return &x;
+    };
+    // in place of one that is too small and done, or else beside it; of the others only what
+    // makes the new one fit is given back
+    if (small && done(*small) && scratch_fits(want, small->bytes)) {
+        drop_scratch(*small);
+        if (Scratch *x = allocate(*small)) return x;
+    } else if (empty && (held + want <= kScratchTotal || held == 0) && scratch_fits(want, 0)) {
+        if (Scratch *x = allocate(*empty)) return x;
+    } else if (!busy && !wait && small && scratch_fits(want, small->bytes)) {
+        drop_scratch(*small);
+        if (Scratch *x = allocate(*small)) return x;
+    }
+    return busy;
 }
 } // namespace
 
@@ -121,42 +205,43 @@ eg_status tracked_malloc(size_t bytes, void **ptr) {
 ScratchLease::ScratchLease(cudaStream_t s, size_t bytes) : s_(s) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return;
-    SharedScratch *x = nullptr;
+    ScratchPool *p = nullptr;
     {
         std::lock_guard<std::mutex> lk(g_scratch_mutex);
-        x = &g_scratch[dev];
+        p = &g_scratch[dev];
     }
-    x->mu.lock();
-    bool ok = x->last || cudaEventCreateWithFlags(&x->last, cudaEventDisableTiming) == cudaSuccess;
-    if (ok && x->bytes < bytes) {
-        RelaxedCapture relaxed;
-        drop_scratch(*x);
-        const size_t want = (bytes + 0x3FFFFFF) & ~size_t(0x3FFFFFF); // whole 64 MB
-        size_t free_b = 0, total_b = 0;
-        ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b >= want + total_b / 32 &&
-             malloc_once(want, &x->ptr) == EG_SUCCESS;
-        if (ok)
-            x->bytes = want;
-        else
-            set_error("");
-    } else if (ok) {
-        ok = cudaStreamWaitEvent(s, x->last, 0) == cudaSuccess;
+    RelaxedCapture relaxed;
+    std::unique_lock<std::mutex> lk(p->mu);
+    Scratch *x = nullptr;
+    for (bool wait = true; wait;) {
+        x = choose_scratch(*p, s, bytes, wait);
+        if (x) break;
+        if (wait) p->ended.wait(lk);
     }
-    if (!ok) {
-        x->mu.unlock();
+    if (!x || (!x->last && cudaEventCreateWithFlags(&x->last, cudaEventDisableTiming) != cudaSuccess) ||
+        cudaStreamWaitEvent(s, x->last, 0) != cudaSuccess) {
+        cudaGetLastError();
         return;
     }
-    owner_ = x;
+    x->taken = true;
+    x->stream = s;
+    x->turn = ++p->turns;
+    pool_ = p;
+    buffer_ = x;
     ptr_ = x->ptr;
 }
 
 ScratchLease::~ScratchLease() {
-    if (!owner_) return;
-    if (cudaEventRecord(owner_->last, s_) != cudaSuccess) { // never leave the buffer unguarded
+    if (!pool_) return;
+    if (cudaEventRecord(buffer_->last, s_) != cudaSuccess) { // never leave the buffer unguarded
         cudaStreamSynchronize(s_);
         cudaGetLastError();
     }
-    owner_->mu.unlock();
+    {
+        std::lock_guard<std::mutex> lk(pool_->mu);
+        buffer_->taken = false;
+    }
+    pool_->ended.notify_all();
 }
 
 eg_status tracked_free(void *ptr) {

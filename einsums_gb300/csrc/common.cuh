@@ -126,13 +126,11 @@ struct Contraction {
 // library is loaded.  Calls that share a stream are ordered, so reuse is safe.
 eg_status workspace(cudaStream_t stream, size_t bytes, void **ptr);
 
-// A device's shared scratch for calls that need much of it for a short time: one
-// buffer per device, handed from call to call in the order of the calls (each
-// waits on the GPU for the one before, whatever its stream), locked to the
-// calling thread while its launches are issued, and given back when another
-// allocation of the library does not fit.  ptr() is null when the buffer cannot
-// be had: under the memory budget, or without leaving a thirty-second of the
-// device's memory free.
+// Scratch for calls that need much of it for a short time, out of a device's few buffers: one
+// goes from call to call in the order of their work (the next one's waits on the GPU for it),
+// is the calling thread's while it issues its launches, and is given back when another
+// allocation of the library does not fit.  ptr() is null when no buffer can be had: under the
+// memory budget, or without leaving a thirty-second of the device's memory free.
 class ScratchLease {
   public:
     ScratchLease(cudaStream_t s, size_t bytes);
@@ -143,7 +141,8 @@ class ScratchLease {
 
   private:
     cudaStream_t s_;
-    struct SharedScratch *owner_ = nullptr;
+    struct ScratchPool *pool_ = nullptr;
+    struct Scratch *buffer_ = nullptr;
     void *ptr_ = nullptr;
 };
 

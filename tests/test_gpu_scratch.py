@@ -1,0 +1,83 @@
+"""The scratch of FP64 contractions on the tensor cores: a stream that is held up does not hold up
+another one's contraction, and a size that cannot be had leaves the buffer of smaller ones alone."""
+import ctypes
+import time
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def eg():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import einsums_gb300
+    from einsums_gb300 import build
+    build.build()
+    return einsums_gb300
+
+
+def operands(dtype, m, n, k):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(m + n)
+    A, B = (torch.randn(s, generator=gen, dtype=dtype, device="cuda") for s in ((m, k), (k, n)))
+    return A, B, A @ B
+
+
+@pytest.mark.parametrize("dtype,m,n,k", [(torch.float64, 700, 500, 600), (torch.complex128, 300, 170, 257),
+                                         (torch.complex128, 40, 30, 50)])
+def test_streams_apart(eg, dtype, m, n, k):
+    A, B, want = operands(dtype, m, n, k)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    Cs = [torch.zeros_like(want) for _ in streams]
+    for C, s in zip(Cs, streams):  # every stream has run a call before
+        eg.einsum(0.0, "ij", C, 1.0, "ik", A, "kj", B, stream=s)
+        torch.cuda.synchronize()
+        C.zero_()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(streams[0]):
+        torch.cuda._sleep(3_000_000_000)  # about 1.5 s at the highest clock
+    start = time.perf_counter()
+    for C, s in zip(Cs, streams):
+        eg.einsum(0.0, "ij", C, 1.0, "ik", A, "kj", B, stream=s)
+    streams[1].synchronize()
+    streams[2].synchronize()
+    apart = time.perf_counter() - start
+    held = not streams[0].query()
+    for C in Cs[1:]:
+        assert torch.allclose(C, want, rtol=0, atol=1e-10)
+    torch.cuda.synchronize()
+    assert torch.allclose(Cs[0], want, rtol=0, atol=1e-10)
+    assert held and apart < 1.0
+
+
+def test_too_large_a_size_takes_nothing_away(eg):
+    from einsums_gb300 import _lib
+    lib = _lib.load()
+    small, large = operands(torch.float64, 600, 500, 400), operands(torch.float64, 6000, 5000, 900)
+    used, p = ctypes.c_size_t(), ctypes.c_void_p()
+
+    def run(x):
+        A, B, want = x
+        C = torch.zeros_like(want)
+        eg.einsum(0.0, "ij", C, 1.0, "ik", A, "kj", B)
+        torch.cuda.synchronize()
+        assert torch.allclose(C, want, rtol=0, atol=1e-10)
+        _lib.check(lib.eg_memory_in_use(ctypes.byref(used)))
+        return used.value
+
+    _lib.check(lib.eg_set_memory_budget(1))
+    assert lib.eg_device_alloc(1 << 20, ctypes.byref(p)) != 0  # what was held is given back
+    _lib.check(lib.eg_set_memory_budget(0))
+    before = run(small)
+    try:
+        _lib.check(lib.eg_set_memory_budget(before + (32 << 20)))
+        assert run(large) == before  # on the FMA kernel
+        assert run(small) == before
+    finally:
+        _lib.check(lib.eg_set_memory_budget(0))
+    after = run(large)
+    assert after > before
+    assert run(small) == after
