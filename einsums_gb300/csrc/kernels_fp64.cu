@@ -500,13 +500,12 @@ __global__ void __launch_bounds__(kThreads, T == 32 && !LISTED ? 4 : 3) k_contra
     const uint32_t listed = LISTED ? (uint32_t)__ldg(p.count) : 0;
     if (LISTED && __ldg(p.count + 1)) return fill_nan(p);
     const int64_t total = LISTED ? (int64_t)PARTS * listed : p.total;
+    if (LISTED && blockIdx.x >= total) return;
     constexpr int gap = LISTED && T == 32 ? 16 : 0; // tile column j is column j + (j & gap) from the tile's first
-    // listed tiles are handed out one by one (to clusters, in turn)
-    __shared__ uint32_t next;
-    const bool handed = LISTED && p.cs == 1;
+    __shared__ uint32_t next; // listed tiles are handed out one by one
     uint32_t fetched = blockIdx.x;
     for (int64_t t = blockIdx.x / p.cs;; t += step) {
-        if (handed) {
+        if (LISTED) {
             if (tid == 0) {
                 next = fetched;
                 fetched = gridDim.x + atomicAdd((unsigned *)p.count + 2, 1u); // the one after, while this one runs
@@ -524,7 +523,7 @@ __global__ void __launch_bounds__(kThreads, T == 32 && !LISTED ? 4 : 3) k_contra
             m0 = e.y + part % ROWS * T;
             n0 = e.z + (T == 32 ? 2 * col : 2 * col - col % 16);
             if (m0 >= M || n0 >= N) {
-                if (handed) __syncthreads();
+                __syncthreads();
                 continue;
             }
         } else {
@@ -594,7 +593,7 @@ __global__ void __launch_bounds__(kThreads, T == 32 && !LISTED ? 4 : 3) k_contra
         }
         if (p.cs > 1)
             ptx::cluster_sync(); // the peers' sums are read; the next tile may overwrite them
-        else if (!handed && (reduce || t + step < total))
+        else if (!LISTED && (reduce || t + step < total))
             __syncthreads();
     }
 }
@@ -604,14 +603,14 @@ __global__ void __launch_bounds__(kThreads, T == 32 && !LISTED ? 4 : 3) k_contra
 // 2000 clocks per resident round (prologue, first loads, stores) and 1500 for a
 // cluster's exchange.  A smaller tile wins only where larger ones leave SMs
 // idle: it issues more loads and index arithmetic per FMA (the factors).
-double contract_plan(int64_t nb, int64_t M, int64_t N, int64_t K, int &T, int &cs) { // returns the clocks
+double contract_plan(int64_t nb, int64_t M, int64_t N, int64_t K, int &T, int &cs, int most = 8) { // returns the clocks
     double best = -1.0;
     T = 32;
     cs = 1;
     for (int e : {32, 16, 8}) {
         const int bk = e == 32 ? 16 : 32;
         const double factor = e == 32 ? 1.0 : e == 16 ? 1.05 : 1.15;
-        for (int c = 1; c <= 8; c *= 2) {
+        for (int c = 1; c <= most; c *= 2) {
             const int64_t chunks = (K + bk - 1) / bk;
             if (c > 1 && chunks < 2 * c) break;
             const double blocks = (double)nb * (double)((M + e - 1) / e) * (double)((N + e - 1) / e) * c;
@@ -630,7 +629,7 @@ double contract_plan(int64_t nb, int64_t M, int64_t N, int64_t K, int &T, int &c
 
 template <int T, bool LISTED>
 cudaError_t launch_f64_tiles(const F64Args &p, cudaStream_t s) {
-    const int64_t clusters = LISTED ? (p.cs == 1 ? 3 : 8) * num_sms() / p.cs : std::min<int64_t>(p.total, int64_t(1) << 24);
+    const int64_t clusters = LISTED ? 3 * num_sms() : std::min<int64_t>(p.total, int64_t(1) << 24);
     if (p.cs == 1) {
         k_contract_f64<T, LISTED><<<(unsigned)clusters, kThreads, 0, s>>>(p);
         return cudaGetLastError();
@@ -887,15 +886,14 @@ double contract_f64_seconds(const Contraction &c) {
 
 eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, int *count, int *status,
                                      cudaStream_t s) {
-    // Tiles and K cut as if the whole output were listed, but for outputs of six rounds of
-    // 32 x 32 tiles or more, where those are faster although the last round is not full
-    // (1024^3, all listed, dealt in turn: 2.19 ms, 2.33 with 16 x 16; handed out one by one
-    // 1.97).  Smaller ones: 300 x 300, K = 1000 591 -> 270 us in all, 128 x 128, K = 60000
-    // 17.0 -> 4.2 ms.
+    // Tiles as if the whole output were listed (K in one piece: launching clusters takes 2 us
+    // more, mostly for nothing), but for outputs of six rounds of 32 x 32 tiles or more, where
+    // those are faster although the last round is not full (1024^3, all listed, dealt in turn:
+    // 2.19 ms, 2.33 with 16 x 16; handed out one by one 1.97).
     F64Args p = f64_args(c);
     int T = 32;
     if (c.batch.total * ((c.m.total + 31) / 32) * ((c.n.total + 31) / 32) < 6 * num_sms())
-        contract_plan(c.batch.total, c.m.total, c.n.total, c.k.total, T, p.cs);
+        contract_plan(c.batch.total, c.m.total, c.n.total, c.k.total, T, p.cs, 1);
     p.list = list;
     p.count = count;
     p.status = status;

@@ -620,8 +620,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if (F64 && q < 0) { // the check; where it fails anywhere, the FMA kernel takes this warp's outputs
                         // quickly: a sum of few products anywhere, or a lack of magnitude?
                         float few = kCheckFew, least = 0.0f;
+                        const bool slice = !GROUPED && tile >= p.t0; // (keeps each output's check)
 #pragma unroll 1
-                        for (int cc = 0; cc < live; cc += 16) {
+                        for (int cc = 0; cc < live && !slice; cc += 16) {
                             uint32_t products[16], sums[16];
                             ptx::tmem_ld16(at + 2 * cc, products);
                             ptx::tmem_ld16(at + kBN + 2 * cc, sums);
@@ -633,20 +634,18 @@ __global__ void __launch_bounds__(THREADS, 1)
                                 least = fminf(least, fmaf(-(float)kCheckPer, n, __uint_as_float(sums[i])));
                             }
                         }
-                        const bool slice = !GROUPED && tile >= p.t0;
                         bool bad = few < kCheckFew || least < 0.0f;
                         if (slice || __any_sync(0xffffffffu, bad)) { // closely
                             bad = false;
 #pragma unroll 1
-                            for (int cc = 0; cc < live; cc += 8) {
-                                const uint32_t from = at + 2 * cc - (cc & 8); // in turns of 16 columns
-                                uint32_t products[8], sums[8];
-                                ptx::tmem_ld8(from, products);
-                                ptx::tmem_ld8(from + kBN, sums);
+                            for (int cc = 0; cc < live; cc += 16) {
+                                uint32_t products[16], sums[16];
+                                ptx::tmem_ld16(at + 2 * cc, products);
+                                ptx::tmem_ld16(at + kBN + 2 * cc, sums);
                                 ptx::tmem_wait_ld();
                                 const uint32_t check = (uint32_t)(((tile - p.t0) * CL + rank) * kBN + half * kCols + cc) * kBM + row;
 #pragma unroll
-                                for (int i = 0; i < 8; i++) {
+                                for (int i = 0; i < 16; i++) {
                                     const int n = __float2int_rn(__uint_as_float(products[i]));
                                     const int excess = __float2int_rn(__uint_as_float(sums[i])) - kCheckPer * n;
                                     bad = bad || check_fails(n, excess);
