@@ -10,7 +10,7 @@ from .blocks import BlockTensor, TiledTensor
 from .core import (ALGORITHMS, EinsumDirectProductPlan, EinsumDotPlan, EinsumGemmPlan, EinsumGemvPlan,
                    EinsumGenericPlan, EinsumGerPlan, GroupedPlan, PermutePlan, compile_permute, compile_plan, einsum,
                    fock_jk_symmetric, last_split_report,
-                   permute)
+                   permute, trim_memory)
 
-__all__ = ["compile_plan", "einsum", "permute", "compile_permute", "PermutePlan", "fock_jk_symmetric", "BlockTensor", "TiledTensor", "GroupedPlan", "Einsum", "einsum_ag", "last_split_report", "ALGORITHMS", "EinsumGenericPlan",
+__all__ = ["compile_plan", "einsum", "permute", "compile_permute", "PermutePlan", "fock_jk_symmetric", "BlockTensor", "TiledTensor", "GroupedPlan", "Einsum", "einsum_ag", "last_split_report", "trim_memory", "ALGORITHMS", "EinsumGenericPlan",
            "EinsumDotPlan", "EinsumDirectProductPlan", "EinsumGerPlan", "EinsumGemvPlan", "EinsumGemmPlan"]

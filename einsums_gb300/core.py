@@ -408,3 +408,10 @@ def last_split_report() -> dict:
     _lib.check(_lib.load().eg_last_split_report(ctypes.byref(r)))
     return {"slices": r.slices, "slice_pairs": r.slice_pairs, "bits_per_slice": r.bits_per_slice,
             "error_bound": r.error_bound}
+
+
+def trim_memory() -> None:
+    """Free the device memory the library keeps between calls and can make anew: the scratch of FP64
+    contractions on the tensor cores (up to 5 GiB a device) and the plans kept for list einsums.
+    For programs that need it for another allocator; waits for the work that uses it."""
+    _lib.check(_lib.load().eg_trim_memory())

@@ -195,9 +195,13 @@ Scratch *choose_scratch(ScratchPool &p, cudaStream_t s, size_t bytes, bool &wait
 }
 } // namespace
 
+bool drop_cached_plans(); // batched.cu
+
 eg_status tracked_malloc(size_t bytes, void **ptr) {
     const eg_status st = malloc_once(bytes, ptr);
-    if (st != EG_ERROR_OUT_OF_MEMORY || !trim_scratch()) return st;
+    if (st != EG_ERROR_OUT_OF_MEMORY) return st;
+    const bool scratch = trim_scratch(), plans = drop_cached_plans();
+    if (!scratch && !plans) return st;
     set_error("");
     return malloc_once(bytes, ptr);
 }
@@ -746,6 +750,18 @@ eg_status eg_memory_in_use(size_t *bytes) {
     std::lock_guard<std::mutex> lk(eg::g_mem_mutex);
     *bytes = eg::g_in_use;
     return EG_SUCCESS;
+}
+
+eg_status eg_trim_memory(void) {
+    eg::set_error("");
+    try {
+        eg::RelaxedCapture relaxed;
+        eg::trim_scratch();
+        eg::drop_cached_plans();
+        return EG_SUCCESS;
+    } catch (const std::exception &e) {
+        return eg::fail(EG_ERROR_OUT_OF_MEMORY, e.what());
+    }
 }
 
 eg_status eg_copy_to_device(void *dst, const void *src, size_t bytes, void *stream) {

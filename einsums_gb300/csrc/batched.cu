@@ -147,8 +147,22 @@ eg_status run_plan(Plan &plan, cudaStream_t stream) {
 
 } // namespace
 
+namespace eg {
+// Gives up the plans kept for eg_einsum_batched (one that is being executed lives until then);
+// false when there were none.
+bool drop_cached_plans() {
+    std::list<std::pair<uint64_t, std::shared_ptr<Plan>>> plans;
+    {
+        std::lock_guard<std::mutex> lk(g_cache_mu);
+        plans.swap(g_cache);
+    }
+    return !plans.empty();
+}
+} // namespace eg
+
 namespace eg::grouped {
 Plan::~Plan() {
+    if (last) cudaEventSynchronize(last);
     if (prof) {
         // tracing aid (EINSUMS_GB300_TC_PROFILE): the tensor kernel's per-role cycles over all replays
         std::vector<unsigned long long> h((size_t)num_sms() * 8);

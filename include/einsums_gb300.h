@@ -259,6 +259,12 @@ eg_status eg_device_alloc(size_t bytes, void **ptr);
 eg_status eg_device_free(void *ptr);
 eg_status eg_set_memory_budget(size_t bytes);
 eg_status eg_memory_in_use(size_t *bytes);
+/* Frees what the library keeps between calls and can make anew: the scratch of FP64
+ * contractions on the tensor cores (up to 5 GiB a device) and the plans that eg_einsum_batched
+ * keeps (up to eight).  Waits for the work that uses them.  Done by itself when an allocation of
+ * the library fails; for programs whose memory is handed out elsewhere.  No reference
+ * counterpart. */
+eg_status eg_trim_memory(void);
 
 /* Error record of kernels with bounded device-side waits (the tensor-core pipeline of
  * the split form and of FP64) for work issued on `stream`: synchronises the stream, returns EG_ERROR_TIMEOUT

@@ -81,3 +81,60 @@ def test_too_large_a_size_takes_nothing_away(eg):
     after = run(large)
     assert after > before
     assert run(small) == after
+
+
+def test_trim_gives_back_scratch_and_kept_plans(eg):
+    from einsums_gb300 import _lib
+    lib = _lib.load()
+    A, B, want = operands(torch.float64, 900, 800, 700)
+    C = torch.zeros_like(want)
+    As = [A[:, 10 * q:10 * q + 60 + q % 9].contiguous() for q in range(60)] * 6
+    Bs = [A[:, 5 * q:5 * q + 50 + q % 7].contiguous() for q in range(60)] * 6
+    Cs = [torch.zeros((a.shape[1], b.shape[1]), dtype=torch.float64, device="cuda") for a, b in zip(As, Bs)]
+    used = ctypes.c_size_t()
+
+    def in_use():
+        _lib.check(lib.eg_memory_in_use(ctypes.byref(used)))
+        return used.value
+
+    eg.einsum(0.0, "ij", C, 1.0, "ik", A, "kj", B)  # (the workspace of this stream, which stays, is there)
+    eg.trim_memory()
+    before = in_use()
+    for _ in range(2):
+        C.zero_()
+        eg.einsum(0.0, "ij", C, 1.0, "ik", A, "kj", B)
+        scratch = in_use()
+        assert scratch >= before + (64 << 20)
+        plan = eg.compile_plan("ab", "ka", "kb")
+        plan.execute(0.0, Cs, 1.0, As, Bs)
+        assert in_use() > scratch + (16 << 20)
+        eg.trim_memory()  # with both still under way
+        assert in_use() == before
+        assert torch.allclose(C, want, rtol=0, atol=1e-10)
+        for a, b, c in zip(As, Bs, Cs):
+            assert torch.allclose(c, a.T @ b, rtol=0, atol=1e-10)
+            c.zero_()
+
+
+def test_kept_plans_make_room(eg):
+    """An allocation that fails while list plans are kept gets their memory."""
+    from einsums_gb300 import _lib
+    lib = _lib.load()
+    A, _, _ = operands(torch.float64, 900, 800, 700)
+    As = [A[:, 10 * q:10 * q + 60].contiguous() for q in range(60)] * 6
+    Cs = [torch.zeros((60, 60), dtype=torch.float64, device="cuda") for _ in As]
+    eg.trim_memory()
+    used, p = ctypes.c_size_t(), ctypes.c_void_p()
+    _lib.check(lib.eg_memory_in_use(ctypes.byref(used)))
+    before = used.value
+    eg.compile_plan("ab", "ka", "kb").execute(0.0, Cs, 1.0, As, As)
+    try:
+        _lib.check(lib.eg_memory_in_use(ctypes.byref(used)))
+        assert used.value > before + (16 << 20)
+        _lib.check(lib.eg_set_memory_budget(used.value + 4096))
+        _lib.check(lib.eg_device_alloc(16 << 20, ctypes.byref(p)))
+        _lib.check(lib.eg_device_free(p))
+    finally:
+        _lib.check(lib.eg_set_memory_budget(0))
+    for a, c in zip(As, Cs):
+        assert torch.allclose(c, a.T @ a, rtol=0, atol=1e-10)
