@@ -121,7 +121,7 @@ eg_status create_plan(double cp, const int32_t *Cl, const eg_tensor *Cs, double 
     return EG_SUCCESS;
 }
 
-eg_status run_plan(Plan &plan, cudaStream_t stream) {
+eg_status run_plan(Plan &plan, cudaStream_t stream) try {
     std::unique_lock<std::mutex> lk;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     const bool ordered = plan.last && cudaStreamIsCapturing(stream, &capturing) == cudaSuccess &&
@@ -143,6 +143,8 @@ eg_status run_plan(Plan &plan, cudaStream_t stream) {
     eg::count_launches(plan.kernels);
     if (plan.precision == EG_PRECISION_SPLIT_BF16) eg::set_split_report(plan.report);
     return EG_SUCCESS;
+} catch (const std::exception &e) {
+    return eg::fail(EG_ERROR_OUT_OF_MEMORY, e.what());
 }
 
 } // namespace

@@ -173,12 +173,13 @@ eg_status launch_complex_blocks(Contraction c, double sa, double sb, cudaStream_
 
 } // namespace eg
 
-extern "C" eg_status eg_einsum_complex(const double *C_prefactor, const int32_t *C_labels, const eg_tensor *C,
-                                       const double *AB_prefactor, const int32_t *A_labels, const eg_tensor *A,
-                                       const int32_t *B_labels, const eg_tensor *B, int32_t conj_A, int32_t conj_B,
-                                       const eg_options *opt, void *stream, int32_t *algorithm_choice) {
+namespace {
+
+eg_status einsum_complex(const double *C_prefactor, const int32_t *C_labels, const eg_tensor *C,
+                         const double *AB_prefactor, const int32_t *A_labels, const eg_tensor *A,
+                         const int32_t *B_labels, const eg_tensor *B, int32_t conj_A, int32_t conj_B,
+                         const eg_options *opt, void *stream, int32_t *algorithm_choice) {
     using namespace eg;
-    set_error("");
     if (!C_prefactor || !AB_prefactor) return fail(EG_ERROR_INVALID_ARGUMENT, "eg_einsum_complex: NULL prefactor");
     if (!C || !A || !B) return fail(EG_ERROR_INVALID_ARGUMENT, "eg_einsum_complex: NULL tensor");
     if (C->rank < 0 || C->rank > EG_MAX_RANK) return fail(EG_ERROR_RANK, "eg_einsum_complex: C rank out of range");
@@ -250,4 +251,19 @@ extern "C" eg_status eg_einsum_complex(const double *C_prefactor, const int32_t 
         first[part] = false;
     }
     return EG_SUCCESS;
+}
+
+} // namespace
+
+extern "C" eg_status eg_einsum_complex(const double *C_prefactor, const int32_t *C_labels, const eg_tensor *C,
+                                       const double *AB_prefactor, const int32_t *A_labels, const eg_tensor *A,
+                                       const int32_t *B_labels, const eg_tensor *B, int32_t conj_A, int32_t conj_B,
+                                       const eg_options *opt, void *stream, int32_t *algorithm_choice) {
+    eg::set_error("");
+    try {
+        return einsum_complex(C_prefactor, C_labels, C, AB_prefactor, A_labels, A, B_labels, B, conj_A, conj_B, opt,
+                              stream, algorithm_choice);
+    } catch (const std::exception &e) {
+        return eg::fail(EG_ERROR_OUT_OF_MEMORY, e.what());
+    }
 }
