@@ -384,8 +384,9 @@ struct Mode {
 };
 
 // Sort by the given operand's stride (descending) and merge neighbours that
-// are contiguous in all three operands.
-ModeGroup fold(std::vector<Mode> modes, int primary) {
+// are contiguous in all three operands.  False when more modes are left than a group holds
+// (summed indices of A alone and of B alone may be sixteen).
+bool fold(std::vector<Mode> modes, int primary, ModeGroup &g) {
     std::stable_sort(modes.begin(), modes.end(), [&](const Mode &a, const Mode &b) {
         if (a.s[primary] != b.s[primary]) return a.s[primary] > b.s[primary];
         for (int t = 0; t < 3; t++)
@@ -408,15 +409,15 @@ ModeGroup fold(std::vector<Mode> modes, int primary) {
         }
         out.push_back(m);
     }
-    ModeGroup g;
+    if (out.size() > kMaxModes) return false;
+    g = ModeGroup{};
     g.n = (int)out.size();
-    g.total = 1;
     for (int d = 0; d < g.n; d++) {
         g.ext[d] = out[d].ext;
         for (int t = 0; t < 3; t++) g.s[t][d] = out[d].s[t];
         g.total *= out[d].ext;
     }
-    return g;
+    return true;
 }
 
 struct Lowered {
@@ -475,10 +476,8 @@ eg_status lower(const int32_t *Cl, const eg_tensor *C, const int32_t *Al, const 
     // Repeated C labels address the diagonal only; the number of C positions
     // written is the product over unique labels, as in the reference loops.
     out.c = Contraction{};
-    out.c.batch = fold(batch, 2);
-    out.c.m = fold(m, 0);
-    out.c.n = fold(n, 1);
-    out.c.k = fold(k, 0);
+    if (!fold(batch, 2, out.c.batch) || !fold(m, 0, out.c.m) || !fold(n, 1, out.c.n) || !fold(k, 0, out.c.k))
+        return fail(EG_ERROR_NOT_SUPPORTED, "more than " + std::to_string(kMaxModes) + " separate indices in one role");
     out.c.A = A->data;
     out.c.B = B->data;
     out.c.C = C->data;
