@@ -6,6 +6,7 @@
 #include <condition_variable>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <utility>
@@ -383,39 +384,40 @@ struct Mode {
     int64_t s[3];
 };
 
+struct Modes {
+    int n = 0;
+    Mode m[2 * EG_MAX_RANK]; // summed indices of A alone and of B alone
+};
+
 // Sort by the given operand's stride (descending) and merge neighbours that
 // are contiguous in all three operands.  False when more modes are left than a group holds
 // (summed indices of A alone and of B alone may be sixteen).
-bool fold(std::vector<Mode> modes, int primary, ModeGroup &g) {
-    std::stable_sort(modes.begin(), modes.end(), [&](const Mode &a, const Mode &b) {
+bool fold(Modes &modes, int primary, ModeGroup &g) {
+    auto before = [&](const Mode &a, const Mode &b) {
         if (a.s[primary] != b.s[primary]) return a.s[primary] > b.s[primary];
         for (int t = 0; t < 3; t++)
             if (a.s[t] != b.s[t]) return a.s[t] > b.s[t];
         return false;
-    });
-    std::vector<Mode> out;
-    for (const Mode &m : modes) {
-        if (m.ext == 1) continue; // extent-1 modes contribute nothing
-        if (!out.empty()) {
-            Mode &p = out.back();
-            bool merge = true;
-            for (int t = 0; t < 3; t++)
-                if (p.s[t] != m.s[t] * m.ext) merge = false;
-            if (merge) {
-                p.ext *= m.ext;
-                for (int t = 0; t < 3; t++) p.s[t] = m.s[t];
-                continue;
-            }
-        }
-        out.push_back(m);
+    };
+    for (int i = 1; i < modes.n; i++) { // (few: insertion, which keeps the order of equals)
+        const Mode x = modes.m[i];
+        int j = i;
+        for (; j > 0 && before(x, modes.m[j - 1]); j--) modes.m[j] = modes.m[j - 1];
+        modes.m[j] = x;
     }
-    if (out.size() > kMaxModes) return false;
     g = ModeGroup{};
-    g.n = (int)out.size();
-    for (int d = 0; d < g.n; d++) {
-        g.ext[d] = out[d].ext;
-        for (int t = 0; t < 3; t++) g.s[t][d] = out[d].s[t];
-        g.total *= out[d].ext;
+    for (int i = 0; i < modes.n; i++) {
+        const Mode &m = modes.m[i];
+        if (m.ext == 1) continue; // extent-1 modes contribute nothing
+        bool merge = g.n > 0;
+        for (int t = 0; t < 3 && merge; t++) merge = g.s[t][g.n - 1] == m.s[t] * m.ext;
+        if (!merge) {
+            if (g.n == kMaxModes) return false;
+            g.ext[g.n++] = 1;
+        }
+        g.ext[g.n - 1] *= m.ext;
+        for (int t = 0; t < 3; t++) g.s[t][g.n - 1] = m.s[t];
+        g.total *= m.ext;
     }
     return true;
 }
@@ -428,19 +430,18 @@ struct Lowered {
 eg_status lower(const int32_t *Cl, const eg_tensor *C, const int32_t *Al, const eg_tensor *A, const int32_t *Bl,
                 const eg_tensor *B, int semantics, Lowered &out) {
     struct U {
-        int32_t label;
+        int32_t label = 0;
         int64_t ext = -1;
         int64_t s[3] = {0, 0, 0};
         bool in[3] = {false, false, false};
     };
-    std::vector<U> us;
+    U us[3 * EG_MAX_RANK];
+    int count = 0;
     auto add = [&](const int32_t *labels, const eg_tensor *t, int which, const char *name) -> eg_status {
         for (int i = 0; i < t->rank; i++) {
-            auto it = std::find_if(us.begin(), us.end(), [&](const U &u) { return u.label == labels[i]; });
-            if (it == us.end()) {
-                us.push_back(U{labels[i]});
-                it = us.end() - 1;
-            }
+            U *it = us;
+            while (it != us + count && it->label != labels[i]) it++;
+            if (it == us + count) us[count++].label = labels[i];
             if (it->ext >= 0 && it->ext != t->extent[i])
                 return fail(EG_ERROR_DIMENSION, std::string("index ") + std::to_string(labels[i]) + " of " + name +
                                                     " has extent " + std::to_string(t->extent[i]) + " but " +
@@ -456,21 +457,22 @@ eg_status lower(const int32_t *Cl, const eg_tensor *C, const int32_t *Al, const 
     if ((st = add(Al, A, 0, "A")) != EG_SUCCESS) return st;
     if ((st = add(Bl, B, 1, "B")) != EG_SUCCESS) return st;
 
-    std::vector<Mode> batch, m, n, k;
+    Modes batch, m, n, k;
+    auto put = [](Modes &to, const U &u) { to.m[to.n++] = Mode{u.ext, {u.s[0], u.s[1], u.s[2]}}; };
     int64_t c_elems = 1;
-    for (const U &u : us) {
-        Mode md{u.ext, {u.s[0], u.s[1], u.s[2]}};
+    for (int i = 0; i < count; i++) {
+        const U &u = us[i];
         if (u.in[2]) c_elems *= u.ext;
         if (u.in[2] && u.in[0] && u.in[1])
-            batch.push_back(md);
+            put(batch, u);
         else if (u.in[2] && u.in[1] && !u.in[0])
-            n.push_back(md);
+            put(n, u);
         else if (u.in[2])
-            m.push_back(md); // in A only, or C-only broadcast (A stride 0)
+            put(m, u); // in A only, or C-only broadcast (A stride 0)
         else if (u.in[0] && u.in[1])
-            k.push_back(md);
+            put(k, u);
         else if (semantics == EG_SEMANTICS_PYTHON)
-            k.push_back(md); // operand-only index: summed over the unique-index space
+            put(k, u); // operand-only index: summed over the unique-index space
         // else: C++ semantics hold an operand-only index at 0
     }
     // Repeated C labels address the diagonal only; the number of C positions
@@ -486,11 +488,16 @@ eg_status lower(const int32_t *Cl, const eg_tensor *C, const int32_t *Al, const 
     return EG_SUCCESS;
 }
 
-eg_status classify_labels(const int32_t *Cl, int cr, const int32_t *Al, int ar, const int32_t *Bl, int br, int semantics,
-                          Algorithm &alg) {
-    Labels C = labels_of(Cl, cr), A = labels_of(Al, ar), B = labels_of(Bl, br);
-    alg = semantics == EG_SEMANTICS_PYTHON ? detail::classify_py(C, A, B) : detail::classify_cpp(C, A, B);
-    return EG_SUCCESS;
+Algorithm classify_labels(const detail::Analysis &an, int semantics) {
+    return semantics == EG_SEMANTICS_PYTHON ? detail::classify_py(an) : detail::classify_cpp(an);
+}
+
+// The algorithm of a call: that of its pattern, or the generic one where the views or the
+// options say so.
+Algorithm choose(const detail::Analysis &an, Algorithm of_pattern, const eg_options &opt, const eg_tensor *C,
+                 const eg_tensor *A, const eg_tensor *B) {
+    const Algorithm alg = opt.only_generic ? Algorithm::GENERIC : of_pattern;
+    return opt.semantics == EG_SEMANTICS_CPP ? detail::apply_vetoes(alg, an, view_of(C), view_of(A), view_of(B)) : alg;
 }
 
 } // namespace
@@ -506,12 +513,8 @@ eg_status classify_call(const int32_t *Cl, const eg_tensor *C, const int32_t *Al
     if ((st = check_tensor(C, Cl, "C")) != EG_SUCCESS) return st;
     if ((st = check_tensor(A, Al, "A")) != EG_SUCCESS) return st;
     if ((st = check_tensor(B, Bl, "B")) != EG_SUCCESS) return st;
-    Algorithm alg;
-    classify_labels(Cl, C->rank, Al, A->rank, Bl, B->rank, opt.semantics, alg);
-    if (opt.only_generic) alg = Algorithm::GENERIC;
-    if (opt.semantics == EG_SEMANTICS_CPP)
-        alg = detail::apply_vetoes(alg, labels_of(Cl, C->rank), view_of(C), labels_of(Al, A->rank), view_of(A),
-                                   labels_of(Bl, B->rank), view_of(B));
+    const detail::Analysis an(labels_of(Cl, C->rank), labels_of(Al, A->rank), labels_of(Bl, B->rank));
+    const Algorithm alg = choose(an, classify_labels(an, opt.semantics), opt, C, A, B);
     *alg_out = (int32_t)alg;
     return EG_SUCCESS;
 }
@@ -531,12 +534,8 @@ eg_status einsum_impl(double cp, const int32_t *Cl, const eg_tensor *C, double a
     if ((st = check_tensor(A, Al, "A")) != EG_SUCCESS) return st;
     if ((st = check_tensor(B, Bl, "B")) != EG_SUCCESS) return st;
 
-    Algorithm alg;
-    classify_labels(Cl, C->rank, Al, A->rank, Bl, B->rank, opt.semantics, alg);
-    if (opt.only_generic) alg = Algorithm::GENERIC;
-    if (opt.semantics == EG_SEMANTICS_CPP)
-        alg = detail::apply_vetoes(alg, labels_of(Cl, C->rank), view_of(C), labels_of(Al, A->rank), view_of(A),
-                                   labels_of(Bl, B->rank), view_of(B));
+    const detail::Analysis an(labels_of(Cl, C->rank), labels_of(Al, A->rank), labels_of(Bl, B->rank));
+    const Algorithm alg = choose(an, classify_labels(an, opt.semantics), opt, C, A, B);
     if (alg_out) *alg_out = (int32_t)alg;
 
     Lowered low;
@@ -593,20 +592,24 @@ eg_status einsum_impl(double cp, const int32_t *Cl, const eg_tensor *C, double a
 
 // Validates, classifies and lowers one item of a batch; gemm_shaped tells
 // whether it can join a grouped launch (summed modes, an output with more
-// than one position, no repeated output index).
+// than one position, no repeated output index).  What `pattern` knows of the labels is found
+// for the first item and used for the others, which have the same ones.
 eg_status lower_for_group(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al,
                           const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options &opt,
-                          Contraction &out, int32_t *alg_out, bool &gemm_shaped) {
+                          Contraction &out, int32_t *alg_out, bool &gemm_shaped, ListPattern &pattern) {
     eg_status st;
     if ((st = check_tensor(C, Cl, "C")) != EG_SUCCESS) return st;
     if ((st = check_tensor(A, Al, "A")) != EG_SUCCESS) return st;
     if ((st = check_tensor(B, Bl, "B")) != EG_SUCCESS) return st;
-    Algorithm alg;
-    classify_labels(Cl, C->rank, Al, A->rank, Bl, B->rank, opt.semantics, alg);
-    if (opt.only_generic) alg = Algorithm::GENERIC;
-    if (opt.semantics == EG_SEMANTICS_CPP)
-        alg = detail::apply_vetoes(alg, labels_of(Cl, C->rank), view_of(C), labels_of(Al, A->rank), view_of(A),
-                                   labels_of(Bl, B->rank), view_of(B));
+    if (pattern.ranks[0] != C->rank || pattern.ranks[1] != A->rank || pattern.ranks[2] != B->rank) {
+        pattern.analysis = std::make_shared<detail::Analysis>(labels_of(Cl, C->rank), labels_of(Al, A->rank),
+                                                              labels_of(Bl, B->rank));
+        pattern.algorithm = (int32_t)classify_labels(*pattern.analysis, opt.semantics);
+        pattern.ranks[0] = C->rank;
+        pattern.ranks[1] = A->rank;
+        pattern.ranks[2] = B->rank;
+    }
+    const Algorithm alg = choose(*pattern.analysis, (Algorithm)pattern.algorithm, opt, C, A, B);
     if (alg_out) *alg_out = (int32_t)alg;
     Lowered low;
     if ((st = lower(Cl, C, Al, A, Bl, B, opt.semantics, low)) != EG_SUCCESS) return st;
@@ -700,9 +703,9 @@ eg_status eg_classify(int32_t C_rank, const int32_t *C_labels, int32_t A_rank, c
         if (r < 0 || r > EG_MAX_RANK) return eg::fail(EG_ERROR_RANK, "rank out of range");
     if ((C_rank && !C_labels) || (A_rank && !A_labels) || (B_rank && !B_labels))
         return eg::fail(EG_ERROR_INVALID_ARGUMENT, "labels are NULL");
-    eg::detail::Algorithm alg;
-    eg::classify_labels(C_labels, C_rank, A_labels, A_rank, B_labels, B_rank, semantics, alg);
-    *algorithm_choice = (int32_t)alg;
+    const eg::detail::Analysis an(eg::labels_of(C_labels, C_rank), eg::labels_of(A_labels, A_rank),
+                                  eg::labels_of(B_labels, B_rank));
+    *algorithm_choice = (int32_t)eg::classify_labels(an, semantics);
     return EG_SUCCESS;
 }
 

@@ -17,9 +17,6 @@ namespace eg {
 eg_status einsum_impl(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al, const eg_tensor *A,
                       const int32_t *Bl, const eg_tensor *B, const eg_options *opt_in, cudaStream_t stream,
                       int32_t *alg_out);
-eg_status lower_for_group(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al,
-                          const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options &opt,
-                          Contraction &out, int32_t *alg_out, bool &gemm_shaped);
 void set_split_report(const eg_split_report &r);
 void set_error(const std::string &msg);
 void count_launches(uint64_t n);
@@ -74,11 +71,12 @@ eg_status create_plan(double cp, const int32_t *Cl, const eg_tensor *Cs, double 
     cs.reserve((size_t)count);
     groupable = true;
     int32_t alg0 = 0;
+    eg::ListPattern pattern;
     for (int64_t i = 0; i < count; i++) {
         eg::Contraction c;
         int32_t alg = 0;
         bool g = false;
-        eg_status st = eg::lower_for_group(cp, Cl, &Cs[i], ab, Al, &As[i], Bl, &Bs[i], opt, c, &alg, g);
+        eg_status st = eg::lower_for_group(cp, Cl, &Cs[i], ab, Al, &As[i], Bl, &Bs[i], opt, c, &alg, g, pattern);
         if (st != EG_SUCCESS) return st;
         if (i == 0) alg0 = alg;
         groupable &= g;

@@ -8,10 +8,15 @@
 #include <cstdint>
 #include <cstdio>
 #include <functional>
+#include <memory>
 #include <string>
 
 #include "../../include/einsums_gb300.h"
 #include "per_device.cuh"
+
+namespace einsums_gb300::detail {
+struct Analysis;
+}
 
 namespace eg {
 
@@ -216,6 +221,16 @@ bool f64_tensor_pays(const Contraction &c);
 eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front = 0,
                             const std::function<eg_status(Contraction &, void *)> &fill = nullptr);
 eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s, eg_split_report *rep);
+
+// The labels of a list's items, analysed (api.cu) for these ranks.
+struct ListPattern {
+    int ranks[3] = {-1, -1, -1};
+    int32_t algorithm = 0;
+    std::shared_ptr<const ::einsums_gb300::detail::Analysis> analysis;
+};
+eg_status lower_for_group(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al,
+                          const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options &opt,
+                          Contraction &out, int32_t *alg_out, bool &gemm_shaped, ListPattern &pattern);
 
 struct PermuteDesc {
     int rank = 0;

@@ -31,9 +31,6 @@ namespace eg {
 eg_status einsum_impl(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al,
                       const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options *opt_in,
                       cudaStream_t stream, int32_t *alg_out);
-eg_status lower_for_group(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al,
-                          const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options &opt,
-                          Contraction &out, int32_t *alg_out, bool &gemm_shaped);
 void set_split_report(const eg_split_report &r);
 eg_status classify_call(const int32_t *Cl, const eg_tensor *C, const int32_t *Al, const eg_tensor *A,
                         const int32_t *Bl, const eg_tensor *B, const eg_options *opt_in, int32_t *alg_out);
@@ -226,7 +223,9 @@ eg_status einsum_complex(const double *C_prefactor, const int32_t *C_labels, con
         Contraction c;
         int32_t alg = 0;
         bool gemm_shaped = false;
-        eg_status st = lower_for_group(cp0, C_labels, &Cr, abr, A_labels, &Ar, B_labels, &Br, o, c, &alg, gemm_shaped);
+        ListPattern pattern;
+        eg_status st = lower_for_group(cp0, C_labels, &Cr, abr, A_labels, &Ar, B_labels, &Br, o, c, &alg, gemm_shaped,
+                                       pattern);
         if (st != EG_SUCCESS) return st;
         if (gemm_shaped && (st = launch_complex_blocks(c, sa, sb, s)) != EG_ERROR_NOT_SUPPORTED) return st;
     }

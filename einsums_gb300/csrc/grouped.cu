@@ -38,9 +38,6 @@
 #include "split.cuh"
 
 namespace eg {
-eg_status lower_for_group(double cp, const int32_t *Cl, const eg_tensor *C, double ab, const int32_t *Al,
-                          const eg_tensor *A, const int32_t *Bl, const eg_tensor *B, const eg_options &opt,
-                          Contraction &out, int32_t *alg_out, bool &gemm_shaped);
 int64_t mode_group_affine_stride(const ModeGroup &g, int comp);
 eg_status encode_planes_extent(CUtensorMap *map, void *base, int64_t K, int64_t rows, int64_t planes, int64_t Kp,
                                int64_t Rp);

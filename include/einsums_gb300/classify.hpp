@@ -43,8 +43,8 @@ struct Labels {
 
 // (label, position) pairs as produced by find_type_with_position.
 struct Positions {
-    int32_t label[3 * kMaxRank * kMaxRank] = {};
-    int32_t pos[3 * kMaxRank * kMaxRank] = {};
+    int32_t label[kMaxRank * kMaxRank] = {}; // (of two tensors' indices, all the same at most)
+    int32_t pos[kMaxRank * kMaxRank] = {};
     int n = 0;
 };
 
@@ -152,8 +152,8 @@ struct Analysis {
 
 // Compile-time choice of the C++ einsum (Dispatch.hpp:893-951) for real,
 // same-typed basic tensors, before any runtime stride veto.
-constexpr Algorithm classify_cpp(const Labels &C, const Labels &A, const Labels &B) {
-    Analysis an(C, A, B);
+constexpr Algorithm classify_cpp(const Analysis &an) {
+    const Labels &C = an.C, &A = an.A, &B = an.B;
     if (an.hadamard) return Algorithm::GENERIC;
     if (an.is_dot()) return Algorithm::DOT;
     if (an.is_direct()) return Algorithm::DIRECT;
@@ -163,9 +163,11 @@ constexpr Algorithm classify_cpp(const Labels &C, const Labels &A, const Labels 
     return Algorithm::GENERIC;
 }
 
+constexpr Algorithm classify_cpp(const Labels &C, const Labels &A, const Labels &B) { return classify_cpp(Analysis(C, A, B)); }
+
 // Plan type of compile_plan (PyTensorAlgebra.cpp:168-554).
-constexpr Algorithm classify_py(const Labels &C, const Labels &A, const Labels &B) {
-    Analysis an(C, A, B);
+constexpr Algorithm classify_py(const Analysis &an) {
+    const Labels &C = an.C, &A = an.A, &B = an.B;
     if (an.hadamard) return Algorithm::GENERIC;
     if (C.n == 0 && equal(A, B)) return Algorithm::DOT;
     if (equal(C, A) && equal(C, B)) return Algorithm::DIRECT;
@@ -174,6 +176,8 @@ constexpr Algorithm classify_py(const Labels &C, const Labels &A, const Labels &
     if (an.is_gemm()) return Algorithm::GEMM;
     return Algorithm::GENERIC;
 }
+
+constexpr Algorithm classify_py(const Labels &C, const Labels &A, const Labels &B) { return classify_py(Analysis(C, A, B)); }
 
 // ---- runtime stride vetoes (Dispatch.hpp) ----------------------------------
 // A tensor view: extents and element strides, row-major position order.
@@ -215,9 +219,7 @@ inline int64_t last_stride(const Positions &p, const View &x) { return p.n ? x.s
 // Applies the runtime vetoes of einsum_do_outer_product (:267-401),
 // einsum_do_matrix_vector (:444-560) and einsum_do_matrix_product (:614-837):
 // a choice whose views are not BLAS-compatible falls back to GENERIC (:953-955).
-inline Algorithm apply_vetoes(Algorithm alg, const Labels &Cl, const View &C, const Labels &Al, const View &A,
-                              const Labels &Bl, const View &B) {
-    Analysis an(Cl, Al, Bl);
+inline Algorithm apply_vetoes(Algorithm alg, const Analysis &an, const View &C, const View &A, const View &B) {
     switch (alg) {
     case Algorithm::GER:
         if (!totally_vectorable(A) || !totally_vectorable(B) ||
