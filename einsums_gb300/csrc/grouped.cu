@@ -10,7 +10,7 @@
 //     kernel over the blocks that failed it;
 //   * FP64 otherwise: one persistent launch of k_grouped_f64 over the work list; each
 //     entry computes a 32x32 or 64x64 tile with the DFMA core, the tile size
-//     chosen per shape bucket by the autotuner (autotune.cpp);
+//     chosen per shape bucket by the autotuner (autotune.cu);
 //   * split-BF16: one digit-splitting launch over every operand of every item, then
 //     one persistent launch of the tcgen05 GEMM over the work list
 //     (k_tc_split_gemm<true>).

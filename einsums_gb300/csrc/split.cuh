@@ -12,7 +12,7 @@
 // which keeps every partial sum an integer of at most 2^24 and therefore
 // exact; the epilogue converts each chunk to an integer and accumulates
 //     R = sum_d 2^(8 (S-1-d)) G_d
-// exactly in int64 in tensor memory.  The only roundings of the whole
+// exactly in int64 in registers.  The only roundings of the whole
 // product are the digit truncation and the final int64 -> FP64 conversion.
 // This is the scheme of Ozaki, Ogita, Oishi and Rump (Numer. Algorithms 59,
 // 2012) as mapped to integer-exact tensor-core products by Ootomo, Ozaki and
