@@ -606,7 +606,8 @@ def run_e2e(eg, T, precision, args, o, v, step_flops, chunks=8, return_outputs=F
 def link_rates(h_in, h_out, bufs, rows, s_in, s_out, reps=2):
     """Host-link copy rates (GB/s) measured just before the timed e2e steps with the same
     pinned buffers and streams: Wabef's initial value up in row slabs, its result down,
-    and both at once -- the e2e step's floor is its bytes over the concurrent rate."""
+    and both at once -- the e2e step's bytes over the concurrent rate are its floor at that
+    moment's rate; the link is shared, and passes have been seen to beat it."""
     import torch
     nv = h_in.shape[0]
     bounds = [(a0, min(a0 + rows, nv)) for a0 in range(0, nv, rows)]

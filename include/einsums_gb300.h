@@ -106,9 +106,12 @@ eg_status eg_einsum(double C_prefactor, const int32_t *C_labels, const eg_tensor
  * (real, imaginary) doubles; their extents and strides count complex elements.  C_prefactor and
  * AB_prefactor are (real, imaginary) pairs.  Replaces einsum<ConjA, ConjB>(...) on
  * std::complex<double> tensors (Backends/Dispatch.hpp:48,136, conjugation in the generic loops
- * of Backends/BaseAlgebra.hpp:33-38).  Runs as the real contractions of the parts' strided views
- * through eg_einsum (four when AB_prefactor is real, eight otherwise), with opt's precision; a
- * complex C_prefactor is applied to C first.  *algorithm_choice: the choice for the pattern.
+ * of Backends/BaseAlgebra.hpp:33-38).  A GEMM-shaped FP64 product with a real
+ * AB_prefactor runs as one real contraction on the 2 x 2 blocks of its smaller operand's elements
+ * (not on a capturing stream, nor without scratch); everything else as the real contractions of
+ * the parts' strided views through eg_einsum (four when AB_prefactor is real, eight otherwise),
+ * with opt's precision.  A complex C_prefactor is applied to C first.  *algorithm_choice: the
+ * choice for the pattern.
  */
 eg_status eg_einsum_complex(const double *C_prefactor, const int32_t *C_labels, const eg_tensor *C,
                             const double *AB_prefactor, const int32_t *A_labels, const eg_tensor *A,
@@ -308,8 +311,8 @@ eg_status eg_measure_fp64_peak_clock(double *dfma_tflops, double *dmma_tflops, d
  * cta_group::2 MMAs) that the tensor kernel fits on the GPU when the process asked
  * for them wherever the output has two row tiles (EINSUMS_GB300_TC_PAIRS=1), else 0:
  * each call then takes pairs or single CTAs by its estimated time, or always single
- * CTAs with EINSUMS_GB300_TC_PAIRS=0.  Results are the same bit for bit.  No
- * reference counterpart. */
+ * CTAs with EINSUMS_GB300_TC_PAIRS=0.  Results are the same bit for bit, in the split
+ * form and in FP64.  No reference counterpart. */
 eg_status eg_tc_pair_clusters(int32_t *clusters);
 
 /* Kernel accounting.  eg_kernel_launches: kernels this library has launched in the
