@@ -97,7 +97,7 @@ bool append_part(ModeGroup &g, int64_t s0, int64_t s1, int64_t s2) {
 
 // The contraction c of the real parts as one real contraction of the whole complex
 // operands (file comment).  NOT_SUPPORTED: the caller's four contractions, when the shape,
-// a capture or the scratch say so.  300 x 170 x 257: 52 us on the tensor cores; FMAs take
+// a capture or the scratch say so.  300 x 170 x 257: 55 us on the tensor cores; FMAs take
 // 125 us in one launch (83 us of the FP64 pipe) and in four 156 us, each with a last wave
 // of its own and operands at stride 2.
 constexpr int64_t kBlocksMax = int64_t(1) << 23; // elements of the smaller operand: 256 MB of blocks

@@ -967,24 +967,24 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
 //
 // (7.03 from the slice pairs dropped, 2 from the digits, with max| | the power of
 // two above the row's largest element).  The check planes give, in two more slice
-// products and exactly, M = sum_k p_a p_b with p <= 128 |x| / max, and N; where
+// products and exactly where it decides, M = sum_k p_a p_b with p <= 128 |x| / max, and N; where
 //   M >= 20 N   (M >= 20 N + 256 for N < 8)
 // the error is at most 4 2^-53 sum_k |A_ik| |B_jk| -- four roundings' worth, where
 // the bound of a chain of K FMAs is K of them; with two products, half a rounding.
 // A single product (N = 1), which an FMA rounds once and exactly, always fails; sums of
 // no products are zero and pass.  Random sums that just pass, against FMA chains in exact
 // arithmetic: rms error 0.82 of the chain's at N = 2, 0.65 at 4, 0.5 at 8, 0.25 at 32.
-// A region of a tile in
-// which the check fails anywhere (rows graded against each other, infinities, NaN) is
-// not written but listed, and k_contract_f64 computes it from C as it was.  The
+// A region of a tile in which the check fails anywhere (rows graded against each other,
+// infinities, NaN) is not written but listed, and k_contract_f64 computes it from C as it
+// was; inputs that fail everywhere so take the FP64 pipe's time and a little more.  The
 // sums of all 36 products are exact in two int64 words and rounded once.  Neither they
 // nor the check depend on how tiles are cut along K or shared by CTAs.
 //
-// The digit planes live in a scratch shared by the streams of the device and
-// bounded by kF64ScratchCap; larger operands are cut into panels of rows.  When
-// the scratch or the stream's status word cannot be had (a memory budget, a full device) or the stream is
-// being captured (a graph must not hold the scratch), EG_ERROR_NOT_SUPPORTED
-// comes back with nothing launched and the FMA kernel runs instead.
+// The digit planes live in scratch of the device's pool (ScratchLease), bounded by
+// kF64ScratchCap; larger operands are cut into panels of rows.  When the scratch or the
+// stream's status word cannot be had (a memory budget, a full device) or the stream is
+// being captured (a graph must not hold the scratch), EG_ERROR_NOT_SUPPORTED comes back
+// with nothing launched and the FMA kernel runs instead.
 constexpr size_t kF64ScratchCap = size_t(2) << 30;
 
 eg_status launch_f64_tensor(Contraction c, cudaStream_t s, size_t front,
