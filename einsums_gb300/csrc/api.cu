@@ -198,9 +198,9 @@ Scratch *choose_scratch(ScratchPool &p, cudaStream_t s, size_t bytes, bool &wait
 
 bool drop_cached_plans(); // batched.cu
 
-eg_status tracked_malloc(size_t bytes, void **ptr) {
+eg_status tracked_malloc(size_t bytes, void **ptr, bool make_room) {
     const eg_status st = malloc_once(bytes, ptr);
-    if (st != EG_ERROR_OUT_OF_MEMORY) return st;
+    if (st != EG_ERROR_OUT_OF_MEMORY || !make_room) return st;
     const bool scratch = trim_scratch(), plans = drop_cached_plans();
     if (!scratch && !plans) return st;
     set_error("");

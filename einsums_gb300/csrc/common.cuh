@@ -171,7 +171,8 @@ eg_status status_word(cudaStream_t stream, int **ptr);
 eg_status inject_lost(int *lost, cudaStream_t s);
 
 // Device memory accounting used by eg_device_alloc and the workspace.
-eg_status tracked_malloc(size_t bytes, void **ptr);
+// (make_room: what the library keeps between calls is given back when it does not fit.)
+eg_status tracked_malloc(size_t bytes, void **ptr, bool make_room = true);
 eg_status tracked_free(void *ptr);
 
 inline int current_device() {

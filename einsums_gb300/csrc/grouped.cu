@@ -569,7 +569,7 @@ namespace {
 
 eg_status dev_copy(Plan &plan, const void *host, size_t bytes, void **dev) {
     void *p = nullptr;
-    eg_status st = tracked_malloc(bytes ? bytes : 16, &p);
+    eg_status st = tracked_malloc(bytes ? bytes : 16, &p, !plan.optional);
     if (st != EG_SUCCESS) return st;
     plan.owned.push_back(p);
     if (bytes) EG_CUDA(cudaMemcpy(p, host, bytes, cudaMemcpyHostToDevice));
@@ -579,7 +579,7 @@ eg_status dev_copy(Plan &plan, const void *host, size_t bytes, void **dev) {
 
 eg_status dev_alloc(Plan &plan, size_t bytes, void **dev) {
     void *p = nullptr;
-    eg_status st = tracked_malloc(bytes ? bytes : 16, &p);
+    eg_status st = tracked_malloc(bytes ? bytes : 16, &p, !plan.optional);
     if (st != EG_SUCCESS) return st;
     plan.owned.push_back(p);
     *dev = p;
@@ -807,6 +807,7 @@ eg_status build_split_plan(Plan &plan, const std::vector<Contraction> &given, in
     for (auto &c : given) cs.push_back(better_side_first(c));
     const int S = f64 ? kF64Slices : slices ? slices : 5, P = f64 ? S + 2 : S;
     if (!f64 && (S < 2 || S > kMaxSlices)) return fail(EG_ERROR_INVALID_ARGUMENT, "split form: slices must be in 2..6");
+    plan.optional = f64; // (the FMA plan)
     const int64_t kmax = f64 ? kRowsMaxK : max_k_per_pass(S);
     int64_t elemsA = 0, elemsB = 0, rowsA = 0, rowsB = 0;
     for (auto &c : cs) {

@@ -29,6 +29,7 @@ struct Plan {
     int64_t count = 0;
     int32_t algorithm = 0;
     std::vector<void *> owned; // device buffers owned by the plan
+    bool optional = false;     // another plan serves where this one's buffers do not fit
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint64_t kernels = 0; // kernels in one replay

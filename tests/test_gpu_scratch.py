@@ -138,3 +138,34 @@ def test_kept_plans_make_room(eg):
         _lib.check(lib.eg_set_memory_budget(0))
     for a, c in zip(As, Cs):
         assert torch.allclose(c, a.T @ a, rtol=0, atol=1e-10)
+
+
+def test_plans_do_not_push_scratch_out(eg):
+    """An FP64 list plan that does not fit beside the scratch takes the FMA kernel, whatever is held."""
+    from einsums_gb300 import _lib
+    lib = _lib.load()
+    A, B, want = operands(torch.float64, 3000, 2500, 900)
+    C = torch.zeros_like(want)
+    As = [A[:, 10 * q:10 * q + 60].contiguous() for q in range(60)] * 6
+    Cs = [torch.zeros((60, 60), dtype=torch.float64, device="cuda") for _ in As]
+    used, n = ctypes.c_size_t(), ctypes.c_uint64()
+    eg.einsum(0.0, "ij", C, 1.0, "ik", A, "kj", B)  # some scratch
+    torch.cuda.synchronize()
+    _lib.check(lib.eg_memory_in_use(ctypes.byref(used)))
+    before = used.value
+    try:
+        _lib.check(lib.eg_set_memory_budget(before + (16 << 20)))
+        plan = eg.GroupedPlan(0.0, "ab", Cs, 1.0, "ka", As, "kb", As)
+        _lib.check(lib.eg_memory_in_use(ctypes.byref(used)))
+        assert before < used.value < before + (16 << 20)
+        _lib.check(lib.eg_kernel_launches(ctypes.byref(n)))
+        start = n.value
+        plan.execute()
+        _lib.check(lib.eg_kernel_launches(ctypes.byref(n)))
+        assert n.value - start == 1
+    finally:
+        _lib.check(lib.eg_set_memory_budget(0))
+    torch.cuda.synchronize()
+    for a, c in zip(As, Cs):
+        assert torch.allclose(c, a.T @ a, rtol=0, atol=1e-9)
+    plan.close()
