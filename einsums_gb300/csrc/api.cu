@@ -181,16 +181,14 @@ Scratch *choose_scratch(ScratchPool &p, cudaStream_t s, size_t bytes, bool &wait
         x.bytes = want;
         return &x;
     };
-    // in place of one that is too small and done, or else beside it; of the others only what
-    // makes the new one fit is given back
-    if (small && done(*small) && scratch_fits(want, small->bytes)) {
-        drop_scratch(*small);
-        if (Scratch *x = allocate(*small)) return x;
-    } else if (empty && (held + want <= kScratchTotal || held == 0) && scratch_fits(want, 0)) {
+    // beside those that are too small: freeing one waits for all work on the device, which may be
+    // held up, so that is left for when there is no other way
+    if (empty && (held + want <= kScratchTotal || held == 0) && scratch_fits(want, 0)) {
         if (Scratch *x = allocate(*empty)) return x;
-    } else if (!busy && !wait && small && scratch_fits(want, small->bytes)) {
+    }
+    if (!busy && !wait && small && scratch_fits(want, small->bytes)) {
         drop_scratch(*small);
-        if (Scratch *x = allocate(*small)) return x;
+        return allocate(*small);
     }
     return busy;
 }

@@ -16,6 +16,7 @@ def eg():
     import einsums_gb300
     from einsums_gb300 import build
     build.build()
+    einsums_gb300.trim_memory()  # buffers of other tests
     return einsums_gb300
 
 
@@ -50,6 +51,26 @@ def test_streams_apart(eg, dtype, m, n, k):
         assert torch.allclose(C, want, rtol=0, atol=1e-10)
     torch.cuda.synchronize()
     assert torch.allclose(Cs[0], want, rtol=0, atol=1e-10)
+    assert held and apart < 1.0
+
+
+def test_small_buffers_stay(eg):
+    """A stream's larger contraction while another stream is held up, with smaller buffers held: none of
+    them is freed, which would wait for the device."""
+    small, large = operands(torch.float64, 600, 500, 400), operands(torch.float64, 2500, 2000, 600)
+    s, t = torch.cuda.Stream(), torch.cuda.Stream()
+    eg.trim_memory()
+    C, D = torch.zeros_like(small[2]), torch.zeros_like(large[2])
+    eg.einsum(0.0, "ij", C, 1.0, "ik", small[0], "kj", small[1], stream=s)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(3_000_000_000)
+    start = time.perf_counter()
+    eg.einsum(0.0, "ij", D, 1.0, "ik", large[0], "kj", large[1], stream=t)
+    t.synchronize()
+    apart, held = time.perf_counter() - start, not s.query()
+    torch.cuda.synchronize()
+    assert torch.allclose(D, large[2], rtol=0, atol=1e-10)
     assert held and apart < 1.0
 
 
