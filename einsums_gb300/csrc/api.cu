@@ -85,6 +85,7 @@ struct Scratch {
     cudaEvent_t last = nullptr; // after the last lease's work
     cudaStream_t stream = nullptr;
     bool taken = false; // by a lease that has not ended
+    bool fresh = false; // allocated, its header not yet cleared
     uint64_t turn = 0;
 };
 
@@ -179,6 +180,7 @@ Scratch *choose_scratch(ScratchPool &p, cudaStream_t s, size_t bytes, bool &wait
             return nullptr;
         }
         x.bytes = want;
+        x.fresh = true;
         return &x;
     };
     // beside those that are too small: freeing one waits for all work on the device, which may be
@@ -217,21 +219,23 @@ ScratchLease::ScratchLease(cudaStream_t s, size_t bytes) : s_(s) {
     std::unique_lock<std::mutex> lk(p->mu);
     Scratch *x = nullptr;
     for (bool wait = true; wait;) {
-        x = choose_scratch(*p, s, bytes, wait);
+        x = choose_scratch(*p, s, bytes + kHeader, wait);
         if (x) break;
         if (wait) p->ended.wait(lk);
     }
     if (!x || (!x->last && cudaEventCreateWithFlags(&x->last, cudaEventDisableTiming) != cudaSuccess) ||
-        cudaStreamWaitEvent(s, x->last, 0) != cudaSuccess) {
+        cudaStreamWaitEvent(s, x->last, 0) != cudaSuccess ||
+        (x->fresh && cudaMemsetAsync(x->ptr, 0, kHeader, s) != cudaSuccess)) {
         cudaGetLastError();
         return;
     }
     x->taken = true;
+    x->fresh = false;
     x->stream = s;
     x->turn = ++p->turns;
     pool_ = p;
     buffer_ = x;
-    ptr_ = x->ptr;
+    ptr_ = (char *)x->ptr + kHeader;
 }
 
 ScratchLease::~ScratchLease() {

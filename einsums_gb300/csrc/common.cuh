@@ -143,6 +143,10 @@ class ScratchLease {
     ScratchLease(const ScratchLease &) = delete;
     ScratchLease &operator=(const ScratchLease &) = delete;
     void *ptr() const { return ptr_; }
+    // kHeader bytes before it that no lease's bytes cover: zero when the buffer is new, and from
+    // then on as its users leave them.
+    void *header() const { return (char *)ptr_ - kHeader; }
+    static constexpr size_t kHeader = 1024; // (the layouts behind it count on its multiples)
 
   private:
     cudaStream_t s_;
@@ -212,9 +216,11 @@ eg_status launch_contract_f64(const Contraction &c, cudaStream_t s);
 // The blocks of outputs listed at `list` ({batch, row, column}), count[0] of them: 32 rows by
 // the 16 columns from `column` and from 32, 64 and 96 further on; count[2], zero before,
 // numbers the tiles handed out.  Where count[1] is set, the tensor kernel before gave up: all
-// of C becomes NaN, and count[1] goes to *status.
-constexpr int kListWords = 3;
-eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, int *count, int *status, cudaStream_t s);
+// of C becomes NaN, and count[1] goes to *status.  The kMagnitudeWords words at `magnitudes`
+// are left zero (unless null).
+constexpr int kListWords = 3, kMagnitudeWords = 4;
+eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, int *count, int *status,
+                                     unsigned long long *magnitudes, cudaStream_t s);
 double contract_f64_seconds(const Contraction &c); // its estimated time
 bool f64_tensor_pays(const Contraction &c);
 // `front` bytes of the scratch are the caller's: fill(c, them) issues what writes them and

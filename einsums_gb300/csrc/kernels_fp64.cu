@@ -466,6 +466,7 @@ struct F64Args {
     const int4 *list;
     int *count; // entries, the record of a wait that gave up, tiles handed out
     int *status;
+    unsigned long long *magnitudes; // left zero for the next call
 };
 
 // All of C, by all threads of the grid: outputs that the tensor kernel did not finish must not
@@ -498,6 +499,7 @@ __global__ void __launch_bounds__(kThreads, T == 32 && !LISTED ? 4 : 3) k_contra
     const int64_t step = gridDim.x / p.cs;
     constexpr int ROWS = 32 / T, PARTS = ROWS * (64 / T); // of a listed block
     const uint32_t listed = LISTED ? (uint32_t)__ldg(p.count) : 0;
+    if (LISTED && p.magnitudes && blockIdx.x == 0 && tid < kMagnitudeWords) p.magnitudes[tid] = 0;
     if (LISTED && __ldg(p.count + 1)) return fill_nan(p);
     const int64_t total = LISTED ? (int64_t)PARTS * listed : p.total;
     if (LISTED && blockIdx.x >= total) return;
@@ -885,7 +887,7 @@ double contract_f64_seconds(const Contraction &c) {
 }
 
 eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, int *count, int *status,
-                                     cudaStream_t s) {
+                                     unsigned long long *magnitudes, cudaStream_t s) {
     // Tiles as if the whole output were listed (K in one piece: launching clusters takes 2 us
     // more, mostly for nothing), but for outputs of six rounds of 32 x 32 tiles or more, where
     // those are faster although the last round is not full (1024^3, all listed, dealt in turn:
@@ -897,6 +899,7 @@ eg_status launch_contract_f64_listed(const Contraction &c, const int4 *list, int
     p.list = list;
     p.count = count;
     p.status = status;
+    p.magnitudes = magnitudes;
     {
         LaunchScope ls_("k_contract_f64_listed", s);
         const cudaError_t err = launch_f64_tiles<true>(p, T, s);

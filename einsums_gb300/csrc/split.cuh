@@ -37,7 +37,7 @@ constexpr int kF64Slices = 8, kF64High = 4;
 // The check of one output over its N products that are not zero, M the sum of their leading
 // magnitudes' products (p_a p_b): it passes when N = 0, or N >= 8 and M >= 20 N, or N >= 2 and
 // M >= 20 N + 256.  A product that stands alone is left to the FMA kernel, which rounds it once.
-constexpr float kTriedMean = 32.0f; // of p_a p_b over an item of a list, see left_out in tc_gemm.cu
+constexpr float kTriedMean = 32.0f; // of p_a p_b, see left_out in tc_gemm.cu
 constexpr int kCheckPer = 20, kCheckFew = 8, kCheckMore = 256;
 __host__ __device__ constexpr bool check_fails(int products, int excess) { // excess: M - 20 N
     return products == 1 || (products > 1 && excess < (products < kCheckFew ? kCheckMore : 0));
@@ -114,8 +114,9 @@ struct TcGemmParams {
     // past M (N) and K blocks past K with zeros instead of reading the padding.
     const CUtensorMap *item_maps;
     const int *ranges; // each CTA's work entries
-    // Grouped launches, FP64 form: the sums of the leading magnitudes (p_a of the check) over all
-    // of A and all of B of every item, [item][2].
+    // FP64 form: the sums of the leading magnitudes (p_a of the check) over all of A and all of B.
+    // Grouped launches: [item][2].  Else, may be null, of a sample of rows: A's sum, the number of
+    // its elements that are not zero, and the same of B.
     const unsigned long long *magnitudes;
 };
 

@@ -212,10 +212,11 @@ __device__ __forceinline__ int entry_nkb(const TcGemmParams &p, const TcItem *it
     return min(p.kslice, p.nkb - kbeg);
 }
 
-// Lists, FP64 form: whether entry t's item is left to the FMA kernel without being tried.  The
-// splitting kernel adds up the check's magnitudes over each operand; where their means multiply
-// to less than 32, outputs with 20 N are few or none, and the FMA kernel would have to compute
-// (nearly) all of the item after the tensor cores did.  The kernel before wrote the sums, so
+// FP64 form: whether entry t's item of a list, or the whole of a single contraction, is left to
+// the FMA kernel without being tried.  The splitting kernel adds up the check's magnitudes over
+// each operand; where their means (over the elements that are not zero, in lists over all)
+// multiply to less than 32, outputs with 20 N are few or none, and the FMA kernel would have to
+// compute (nearly) all of it after the tensor cores did.  The kernel before wrote the sums, so
 // all roles decide alike.  (It saves such a list the 160 us that the tensor kernel takes for 512
 // uneven items, and costs an ordinary one 4.)
 template <bool GROUPED, bool F64>
@@ -226,6 +227,12 @@ __device__ __forceinline__ bool left_out(const TcGemmParams &p, const TcItem *it
         return (float)s.x * (float)s.y < items[i].tried;
     }
     return false;
+}
+template <bool F64>
+__device__ __forceinline__ bool all_left_out(const TcGemmParams &p) {
+    if (!F64 || !p.magnitudes) return false;
+    const ulonglong2 a = __ldg((const ulonglong2 *)p.magnitudes), b = __ldg((const ulonglong2 *)p.magnitudes + 1);
+    return (float)a.x * (float)b.x < kTriedMean * (float)a.y * (float)b.y;
 }
 
 // The FP64 value of one output's exact sums, scaled (but for an ab that is no power of
@@ -276,6 +283,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     uint64_t *done = acce + 2;
     uint32_t *tmem_slot = (uint32_t *)(done + 1);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+    volatile int *none_tried = abort_flag + 1; // single contractions: all_left_out
     // per-epilogue-warp copies of the tile's column offsets and exponents, so
     // the epilogue warps never wait on one another
     int64_t *colOffAll = (int64_t *)(smem + 2 * kSlots * TILE_BYTES + AUX_BYTES);
@@ -302,6 +310,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         ptx::mbar_init(done, 1);
         *abort_flag = 0;
         ptx::fence_mbar_init();
+    }
+    if (!GROUPED && F64 && warp == 3) {
+        const bool out = all_left_out<F64>(p);
+        if (lane == 0) *none_tried = out;
     }
     if (warp == 1) {
         ptx::tmem_alloc<CL>(tmem_slot, TMEM_COLS);
@@ -336,7 +348,8 @@ __global__ void __launch_bounds__(THREADS, 1)
             bool ok = true;
             const uint32_t ring0 = ptx::smem_u32(isB ? smB : smA);
             const uint32_t full0 = CL == 2 ? full_lead : ptx::smem_u32(full);
-            for (int tile = cta0; tile < total_tiles && ok; tile += ctas) {
+            const int end = !GROUPED && F64 && *none_tried ? 0 : total_tiles;
+            for (int tile = cta0; tile < end && ok; tile += ctas) {
                 const TileJob job = resolve<GROUPED, CL>(p, items, work, tile, rank);
                 if (left_out<GROUPED, F64>(p, items, work, tile)) continue;
                 const int row0 = (isB ? job.nt : job.mt) * kBM, z0 = isB ? job.zB : job.zA;
@@ -435,7 +448,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                 else
                     ptx::mma_commit_both(bar);
             };
-            for (int tile = cta0; tile < total_tiles && ok; tile += ctas) {
+            const int end = !GROUPED && F64 && *none_tried ? 0 : total_tiles;
+            for (int tile = cta0; tile < end && ok; tile += ctas) {
                 const int nkb = entry_nkb<GROUPED>(p, items, work, tile);
                 if (left_out<GROUPED, F64>(p, items, work, tile)) continue;
                 for (int q = qbeg; q < qend && ok; q++) {
@@ -572,7 +586,21 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
             if (!F64) load_sums(c0);
         };
-        for (int tile = cta0;; tile += ctas) {
+        auto list_region = [&](const TileJob &job) { // this warp's, for the FMA kernel
+            const int m0 = job.mt * kBM + quad * 32, n0 = job.nt * kBN + half * 16;
+            p.redo[atomicAdd(p.redo_count, 1)] = GROUPED ? make_int4(job.item, job.b, m0, n0)
+                                                         : make_int4(job.b, (int)p.m0 + m0, (int)p.n0 + n0, 0);
+        };
+        int first = cta0;
+        if (!GROUPED && F64 && *none_tried) { // (k_tc_finish_slices lists what is cut along K)
+            for (; first < p.t0 && first < total_tiles; first += ctas) {
+                const TileJob job = resolve<GROUPED, CL>(p, items, work, first, rank);
+                if (lane == 0 && (int64_t)job.mt * kBM + quad * 32 < job.M && (int64_t)job.nt * kBN + half * 16 < job.N)
+                    list_region(job);
+            }
+            first = total_tiles;
+        }
+        for (int tile = first;; tile += ctas) {
             // after the last tile one more pass, without chunks, finishes what is pending
             const bool drain = tile >= total_tiles;
             if (drain && pend_done >= pend_cols) break;
@@ -775,7 +803,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             const TileJob job = resolve<GROUPED, CL>(p, items, work, tile, rank);
             if (!GROUPED && job.part == -2) continue; // the odd half of a pair's last row of tiles
             if (untried) {
-                if (live > 0 && lane == 0) p.redo[atomicAdd(p.redo_count, 1)] = make_int4(job.item, job.b, job.mt * kBM + quad * 32, job.nt * kBN + half * 16);
+                if (live > 0 && lane == 0) list_region(job);
                 continue;
             }
             const bool slice = !GROUPED && job.part >= 0; // k_tc_finish_slices adds it up
@@ -786,12 +814,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             long long *const own_hi = rbc + (F64 ? 1 + parity : 0) * kPlane;
             parity ^= 1;
             if (F64 && *failed) {
-                if (lane == 0) {
-                    const int at = atomicAdd(p.redo_count, 1);
-                    const int m0 = job.mt * kBM + quad * 32, n0 = job.nt * kBN + half * 16;
-                    p.redo[at] = GROUPED ? make_int4(job.item, job.b, m0, n0)
-                                         : make_int4(job.b, (int)p.m0 + m0, (int)p.n0 + n0, 0);
-                }
+                if (lane == 0) list_region(job);
                 continue;
             }
             if (live == 0) continue;
@@ -867,10 +890,13 @@ __global__ void __launch_bounds__(32 * kFinishRows, 3) k_tc_finish_slices(const 
     const int rows = (int)min((int64_t)32, p.M - m0), cols = (int)min((int64_t)kBN, p.N - n0);
     const int live = min(cols / 32 * 16 + min(max(cols % 32 - half * 16, 0), 16) - c0, kFinishCols);
     if (rows <= 0 || live <= 0) return;
+    auto list_region = [&] {
+        p.redo[atomicAdd(p.redo_count, 1)] = make_int4((int)p.b0 + b, (int)(p.m0 + m0), (int)(p.n0 + n0) + half * 16, 0);
+    };
     const int e0 = q * p.ksplit * CL + rank; // the tile's first slice; the next ones are CL further on
     const int lost = __ldcg(p.lost); // with a slice missing there is nothing to add up
-    bool bad = false;
-    if (F64) {
+    bool bad = all_left_out<F64>(p);
+    if (F64 && !bad) {
         // the region's check, over the slices, as in a whole tile (both of its CTAs see all of it)
         const int all = cols / 32 * 16 + min(max(cols % 32 - half * 16, 0), 16);
         const int *at = p.parts_check + (size_t)e0 * kPlane + (size_t)(half * kCols) * kBM + quad * 32 + lane;
@@ -935,9 +961,7 @@ __global__ void __launch_bounds__(32 * kFinishRows, 3) k_tc_finish_slices(const 
     }
     if (__syncthreads_or(bad) || lost) { // the FMA kernel computes the region
         if (lost && blockIdx.x == 0 && threadIdx.x == 0) report_lost(p.status_at, p.status, lost);
-        if (!lost && threadIdx.x == 0 && c0 == 0)
-            p.redo[atomicAdd(p.redo_count, 1)] =
-                make_int4((int)p.b0 + b, (int)(p.m0 + m0), (int)(p.n0 + n0) + half * 16, 0);
+        if (!lost && threadIdx.x == 0 && c0 == 0) list_region();
         return;
     }
 #pragma unroll

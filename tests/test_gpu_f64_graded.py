@@ -135,3 +135,31 @@ def test_lists(eg):
         if kind != "apart":
             assert ours <= 1.1 * plain, (kind, ours, plain)
         print(kind, ours, plain)
+
+
+@pytest.mark.parametrize("m,n,k", [(4000, 2100, 300), (300, 260, 4100), (100000, 24, 33)])
+def test_not_tried_in_vain(eg, m, n, k):
+    """Operands whose magnitudes say that nothing can pass are left to the FMA kernel at once, whole
+    tiles and tiles cut along K; then ordinary and sparse ones with the same scratch are not."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(k)
+    A, B = graded(gen, m, n, k)
+    C = torch.full((m, n), float("nan"), dtype=torch.float64, device="cuda")
+    call = lambda: eg.einsum(0.0, "ij", C, 1.0, "ik", A, "kj", B)
+    tensor = {}
+    for kind in ("graded", "ordinary", "sparse", "graded again"):
+        if kind == "ordinary":
+            gA, gB = A, B
+            A, B = (torch.randn(x.shape, generator=gen, dtype=torch.float64, device="cuda") for x in (A, B))
+        elif kind == "sparse":  # a tenth of A's elements
+            A = A * (torch.rand(A.shape, generator=gen, device="cuda") < 0.1)
+        elif kind == "graded again":
+            A, B = gA, gB
+        tensor[kind] = profiled(call)["k_tc_split_gemm_f64"]
+        rows = np.arange(0, m, max(1, m // 40))
+        a, b = A[rows].cpu().numpy(), B.cpu().numpy()
+        want = (a.astype(np.longdouble) @ b.astype(np.longdouble)).astype(float)
+        assert np.all(np.abs(C[rows].cpu().numpy() - want) <= (k + 4) * U * (np.abs(a) @ np.abs(b))), kind
+    # without loads and products: the kernel's start, 8 us, and the listing
+    assert max(tensor["graded"], tensor["graded again"]) <= 15
+    assert min(tensor["ordinary"], tensor["sparse"]) >= 18
