@@ -1000,7 +1000,8 @@ eg_status launch_split_contract(const Contraction &c, int slices, cudaStream_t s
 // arithmetic: rms error 0.82 of the chain's at N = 2, 0.65 at 4, 0.5 at 8, 0.25 at 32.
 // A region of a tile in which the check fails anywhere (rows graded against each other,
 // infinities, NaN) is not written but listed, and k_contract_f64 computes it from C as it
-// was; inputs that fail everywhere so take the FP64 pipe's time and a little more.  The
+// was.  Inputs that fail everywhere so take the FP64 pipe's time and a little more; where the
+// operands' magnitudes say so, nothing is tried (all_left_out in tc_gemm.cu).  The
 // sums of all 36 products are exact in two int64 words and rounded once.  Neither they
 // nor the check depend on how tiles are cut along K or shared by CTAs.
 //
