@@ -160,6 +160,6 @@ def test_not_tried_in_vain(eg, m, n, k):
         a, b = A[rows].cpu().numpy(), B.cpu().numpy()
         want = (a.astype(np.longdouble) @ b.astype(np.longdouble)).astype(float)
         assert np.all(np.abs(C[rows].cpu().numpy() - want) <= (k + 4) * U * (np.abs(a) @ np.abs(b))), kind
-    # without loads and products: the kernel's start, 8 us, and the listing
-    assert max(tensor["graded"], tensor["graded again"]) <= 15
-    assert min(tensor["ordinary"], tensor["sparse"]) >= 18
+    # without loads and products (an eighth and less of the time): the kernel's start and the listing
+    assert max(tensor["graded"], tensor["graded again"]) <= 0.25 * tensor["ordinary"]
+    assert tensor["sparse"] >= 0.5 * tensor["ordinary"]
